@@ -118,3 +118,14 @@ def test_tensor_core_full_size_equals_fp32(efg):
         out[screening] = (ids.cpu().numpy(), dist.cpu().numpy())
     assert np.array_equal(out["auto"][0], out["fp32"][0])
     assert np.array_equal(out["auto"][1], out["fp32"][1])
+
+
+@pytest.mark.parametrize("n,nq,k", [(129, 1, 104), (20_000, 3, 100), (33_001, 130, 104), (70_000, 300, 60)])
+def test_few_queries_over_many_chunks(efg, n, nq, k):
+    """A few queries with long lists: the base is cut into more chunks than 4096 keys per query would
+    allow (one tile of rows at the least); byte data, so ids and distances equal the FP32 screening's."""
+    x = datasets.mixture_u8(n, 40, seed=3)
+    q = datasets.mixture_u8(nq, 40, seed=3, queries=True)
+    tc = _knn(efg, x, q, k, "auto")
+    f32 = _knn(efg, x, q, k, "fp32")
+    assert np.array_equal(tc[0], f32[0]) and np.array_equal(tc[1], f32[1])
