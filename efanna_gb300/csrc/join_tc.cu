@@ -12,17 +12,16 @@
 //     with more rows goes to a list that tiles of TR = 256 rows (two CTAs per SM) pack next; a node
 //     with more than 128 new entries or 256 rows goes to a second list, scored tile by tile: a
 //     block of new entries (the tile's first rows) with a chunk of the candidates after the block,
-//     the block's first chunk also covering the pairs within the block.  Each row's pairs in a
-//     tile are consecutive slots of its node's pair array.
+//     the block's first chunk also covering the pairs within the block.
 //   * CTAs are persistent.  Warps 0 and 2-9 gather a tile's rows with 16-byte cp.async copies
 //     (eight threads per 128-byte row segment) into a ring of stages in the 128-byte-swizzle
 //     K-major layout; each thread waits for its copies, fences them for the tensor cores
 //     (fence.proxy.async) and arrives on the stage's barrier.  The same stage is both MMA operands.
 //     One thread of warp 1 issues the MMAs into TMEM.  Warps 2-9 copy the Gram rows of 32 new
 //     entries at a time out of TMEM (the two warps of each TMEM lane quarter taking alternate
-//     32-column groups) into shared memory, then walk those entries' pairs in pair-array order, one
-//     pair per thread: distance ||x||^2 + ||y||^2 - 2 x.y, then the join's record step -- the same
-//     per-pair array, per-target counts and `found` flags as the FP32 join kernel.
+//     32-column groups) into shared memory, then walk those entries' pairs, one pair
+//     per thread: distance ||x||^2 + ||y||^2 - 2 x.y, then the join's record step -- the same records
+//     and `found` flags as the FP32 join kernel.
 //   * When BF16 holds every value of the base, one product per value; with integer values and
 //     squared norms below 2^23 (byte data up to 128 dimensions) every sum is exact, so the distances
 //     equal the FP32 join's and the graph is identical.  Other data take the hi + lo split
@@ -61,24 +60,19 @@ enum : uint32_t {
 struct JoinArgs {
   const __nv_bfloat16 *hi, *lo;  // BF16 rows of W values (lo only read when terms = 3)
   const uint32_t *new_ids, *new_cnt, *old_ids, *old_cnt;
-  const uint64_t* pair_off;
   const float* bound;
   const float* xnorm;  // FP32 squared norms of the base rows
-  float* pairdist;
-  uint32_t* cnt;
+  RecordSink sink;
   uint8_t* found;
   uint32_t* next_node;  // node counter of the launch
   uint32_t* mid;        // nodes of 129 to 256 rows: mid[0] their count, then their ids
   uint32_t* big;        // nodes larger than a tile: big[0] their count, then their ids
   int* err;
   uint64_t n;
+  unsigned long long* nlarge;  // counts the nodes larger than a tile
   uint32_t W, cap, P, check_k, kblocks, terms, nstages, mode;
+  uint32_t count, step, skip;  // MODE_ORDER: the nodes k * step (skip 0), or the others (skip 1)
 };
-
-// Offset of new entry p's first pair within the node's pairs (nn new, no old entries).
-__device__ __forceinline__ uint64_t pair_row(uint32_t nn, uint32_t no, uint32_t p) {
-  return p == 0 ? 0 : (uint64_t)p * (nn - 1) - (uint64_t)p * (p - 1) / 2 + (uint64_t)p * no;
-}
 
 __device__ __forceinline__ void rec_sync() { asm volatile("bar.sync 1, %0;" ::"r"(JRT) : "memory"); }
 
@@ -105,8 +99,6 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
   constexpr uint32_t PART = TL::PART, DLD = TL::DLD;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[2], bar_empty[2], bar_mma, bar_drain;
-  __shared__ uint64_t po_ch[JCH];                  // pair-array offset of each node of the chunk
-  __shared__ uint64_t rstart[JM];                  // slot of each tile new entry's first pair
   __shared__ uint32_t id_ch[JCH], nn_ch[JCH], no_ch[JCH];  // the chunk's nodes (nn 0: no pairs here)
   __shared__ uint32_t tslot[JCH], tnb[JCH], tob[JCH];  // tile nodes: chunk slot, first new row, first old row
   __shared__ uint32_t cum[JM + 1];                 // pairs of the tile's new entries before each one
@@ -116,10 +108,9 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
   __shared__ uint32_t tmem_base_sh, chn_sh, chpos_sh, tn_sh, nsum_sh, tsum_sh;
   __shared__ uint32_t next_k0_sh, next_cn_sh;  // the chunk being fetched (published after a barrier)
   __shared__ int abort_sh, rec_fail_sh, bad_sh;
-  // MODE_BIG: the node (id, list lengths, pair offset), the next tile's block of new entries and
-  // candidate chunk start, whether it is the block's first (the one with the triangle), the tile
+  // MODE_BIG: the node (id, list lengths), the next tile's block of new entries and candidate chunk
+  // start, whether it is the block's first (the one with the triangle), the tile
   __shared__ uint32_t bm_node, bm_nn, bm_no, bm_a0, bm_c0, bm_first, bm_tri, bm_tc0, bm_ch;
-  __shared__ uint64_t bm_po;
   const uint32_t raw = smem_addr(smem_raw);
   const uint32_t pad = ((raw + 1023u) & ~1023u) - raw;
   const uint32_t sbase = raw + pad;
@@ -171,7 +162,6 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
             bm_node = i;
             bm_nn = a.new_cnt[i];
             bm_no = a.old_cnt[i];
-            bm_po = a.pair_off[i];
             bm_a0 = 0;
             bm_c0 = min(TL::BLOCK, bm_nn);
             bm_first = 1;
@@ -200,7 +190,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
       }
       __syncthreads();
       if (tn_sh == 0) break;
-      const uint32_t A = nsum_sh, nn = bm_nn, no = bm_no, a0 = bm_a0, c0 = bm_tc0, tri = bm_tri;
+      const uint32_t A = nsum_sh, nn = bm_nn, a0 = bm_a0, c0 = bm_tc0;
       const uint64_t i = bm_node;
       for (uint32_t b = threadIdx.x; b < tsum_sh; b += JTHREADS) {
         const uint32_t c = b < A ? a0 + b : c0 + (b - A);  // entry of the node's lists (new, then old)
@@ -211,11 +201,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
         }
         rows_sh[b] = r;
         norm_sh[b] = a.xnorm[r];
-        if (b < A) {
-          const uint32_t pe = a0 + b;
-          rnode[b] = 0;
-          rstart[b] = bm_po + pair_row(nn, no, pe) + (tri ? 0 : c0 - pe - 1);
-        }
+        if (b < A) rnode[b] = 0;
       }
     } else {
       // ---------------------------------------------------------- packed tiles
@@ -225,7 +211,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
       __syncthreads();
       if (fetch) {  // the chunk is packed: the next JCH nodes
         if (threadIdx.x == 0) {
-          const uint32_t total = a.mode == MODE_LIST ? a.mid[0] : (uint32_t)a.n;
+          const uint32_t total = a.mode == MODE_LIST ? a.mid[0] : a.count;
           const uint32_t k0 = *abort_flag ? total : atomicAdd(a.next_node, JCH);
           next_cn_sh = k0 < total ? min(JCH, total - k0) : 0;
           next_k0_sh = k0;
@@ -235,21 +221,24 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
         if (cn == 0) break;
         if (threadIdx.x < cn) {
           const uint32_t k = next_k0_sh + threadIdx.x;
-          const uint32_t i = a.mode == MODE_LIST ? a.mid[1 + k] : k;
+          const uint32_t i = a.mode == MODE_LIST ? a.mid[1 + k] : a.skip ? k + k / (a.step - 1) + 1 : k * a.step;
           uint32_t nn = a.new_cnt[i];
           const uint32_t no = a.old_cnt[i];
           if (nn > a.cap || no > a.cap) {  // not a list: reported, the node left out
             atomicOr(a.err, 4);
             nn = 0;
           } else if (nn > 0 && a.mode == MODE_ORDER && (nn > JM || nn + no > TR)) {
-            if (nn <= JM && nn + no <= 256) a.mid[1 + atomicAdd(a.mid, 1u)] = i;  // for TR = 256
-            else a.big[1 + atomicAdd(a.big, 1u)] = i;                                // tile by tile
+            if (nn <= JM && nn + no <= 256) {  // for TR = 256
+              a.mid[1 + atomicAdd(a.mid, 1u)] = i;
+            } else {  // tile by tile
+              a.big[1 + atomicAdd(a.big, 1u)] = i;
+              atomicAdd(a.nlarge, 1ull);
+            }
             nn = 0;
           }
           id_ch[threadIdx.x] = i;
           nn_ch[threadIdx.x] = nn;
           no_ch[threadIdx.x] = no;
-          po_ch[threadIdx.x] = a.pair_off[i];
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -300,10 +289,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
           const uint32_t b = e < nn ? tnb[j] + e : tob[j] + e - nn;
           rows_sh[b] = r;
           norm_sh[b] = a.xnorm[r];
-          if (e < nn) {
-            rnode[b] = (uint8_t)j;
-            rstart[b] = po_ch[sl] + pair_row(nn, no, e);
-          }
+          if (e < nn) rnode[b] = (uint8_t)j;
         }
       }
     }
@@ -429,7 +415,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
             }
           }
           rec_sync();
-          // pairs of new entries q0 .. q1 - 1 (in order of entry, then candidate), one per thread
+          // pairs of new entries q0 .. q1 - 1, one per thread
           const uint32_t q1 = min(Ns, q0 + 32), u1 = cum[q1];
           uint32_t r = q0;
           for (uint32_t u = cum[q0] + t; u < u1; u += JRT) {
@@ -457,8 +443,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
             }
             const float dot = gram[(r - q0) * DLD + bc];
             const float d = fmaxf(fmaf(-2.f, dot, norm_sh[r] + norm_sh[bc]), 0.f);
-            if (join_lane_record<0>(node, rows_sh[r], rows_sh[bc], cand_new, d, rstart[r] + off, a.P, a.check_k,
-                                    a.bound, a.pairdist, a.cnt, nullptr, nullptr, nullptr, nullptr))
+            if (join_pair_records(a.sink, node, rows_sh[r], rows_sh[bc], cand_new, d, a.P, a.check_k, a.bound))
               a.found[node] = 1;
           }
           rec_sync();  // the Gram rows are overwritten by the next 32 entries
@@ -518,30 +503,45 @@ int launch_join(const JoinArgs& a, int sms, int smem_max, cudaStream_t s) {
 
 }  // namespace
 
-// The BF16 rows (hi, and lo = x - hi), FP32 squared norms and the inexact flag (some lo not zero)
-// of the base, for the tensor-core join: rows of W = round_up(dim, 64) values.
+// flags[2] is set when some value is not an integer or some squared norm not below 2^22: otherwise
+// every product, partial sum and distance (at most 4 x 2^22) is an integer of 24 bits, exact in any order.
+__global__ void not_exact_kernel(const float* __restrict__ base, uint64_t n, uint32_t ld4,
+                                 const float* __restrict__ norms, int* __restrict__ flags) {
+  bool bad = false;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * ld4; i += (uint64_t)gridDim.x * blockDim.x) {
+    const float4 x = __ldg(reinterpret_cast<const float4*>(base) + i);
+    bad |= rintf(x.x) != x.x || rintf(x.y) != x.y || rintf(x.z) != x.z || rintf(x.w) != x.w;
+    if (i < n) bad |= !(norms[i] < 4194304.f);
+  }
+  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flags + 2, 1);
+}
+
+// The BF16 rows (hi, and lo = x - hi) and FP32 squared norms of the base, for the tensor-core join:
+// rows of W = round_up(dim, 64) values.  flags[0]: some lo is not zero; flags[2]: see above.
 int tc_join_prepare(const float* base, uint64_t n, uint32_t dim, uint32_t ld, __nv_bfloat16* hi, __nv_bfloat16* lo,
-                    float* norms, int* inexact, cudaStream_t s) {
+                    float* norms, int* flags, cudaStream_t s) {
   const uint32_t W = (dim + 63) / 64 * 64;
   int dev = 0, sms = 148;
   EFG_CUDA(cudaGetDevice(&dev));
   EFG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  EFG_CUDA(cudaMemsetAsync(inexact, 0, sizeof(int), s));
+  EFG_CUDA(cudaMemsetAsync(flags, 0, 3 * sizeof(int), s));
   const uint64_t warps = std::max<uint64_t>(1, std::min<uint64_t>(n, (uint64_t)sms * 64));
-  to_bf16_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(base, n, dim, ld, W, hi, lo, norms, n, inexact);
+  to_bf16_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(base, n, dim, ld, W, hi, lo, norms, n, flags);
+  EFG_CUDA(cudaGetLastError());
+  not_exact_kernel<<<(unsigned)sms * 8, 256, 0, s>>>(base, n, ld / 4, norms, flags);
   EFG_CUDA(cudaGetLastError());
   return EFG_OK;
 }
 
-// Join pass 0 on the tensor cores: three launches (tiles of 128 rows over every node, tiles of 256
+// The join on the tensor cores: three launches (tiles of 128 rows over every node, tiles of 256
 // rows over the nodes listed in mid, and the nodes listed in big tile by tile).  counters: three
 // node counters, zero on entry; mid and big: n + 1 words each, their counts (word 0) zero on entry;
-// *err zero on entry.  terms: 1 (BF16 holds the base) or 3 (hi + lo products).
+// *err zero on entry; *nlarge counts the nodes larger than a tile.  step, skip: the nodes k * step (skip 0) or the others (skip 1).  terms: 1 (BF16 holds the base) or 3 (hi + lo products).
 int tc_join(const __nv_bfloat16* hi, const __nv_bfloat16* lo, const float* norms, uint64_t n, uint32_t dim,
             uint32_t terms, uint32_t cap, uint32_t P, uint32_t check_k, const uint32_t* new_ids,
-            const uint32_t* new_cnt, const uint32_t* old_ids, const uint32_t* old_cnt, const uint64_t* pair_off,
-            const float* bound, float* pairdist, uint32_t* cnt, uint8_t* found, uint32_t* counters, uint32_t* mid,
-            uint32_t* big, int* err, cudaStream_t s) {
+            const uint32_t* new_cnt, const uint32_t* old_ids, const uint32_t* old_cnt, const float* bound,
+            const RecordSink& sink, uint8_t* found, uint32_t* counters, uint32_t* mid, uint32_t* big,
+            unsigned long long* nlarge, int* err, uint32_t step, uint32_t skip, cudaStream_t s) {
   if (terms != 1 && terms != 3) return fail(EFG_ERR_ARG, "tensor-core join: terms must be 1 or 3");
   if (n >= 0xffffffffull) return fail(EFG_ERR_ARG, "tensor-core join: more than 2^32 - 2 rows");
   const uint32_t W = (dim + 63) / 64 * 64;
@@ -556,11 +556,9 @@ int tc_join(const __nv_bfloat16* hi, const __nv_bfloat16* lo, const float* norms
   a.new_cnt = new_cnt;
   a.old_ids = old_ids;
   a.old_cnt = old_cnt;
-  a.pair_off = pair_off;
   a.bound = bound;
   a.xnorm = norms;
-  a.pairdist = pairdist;
-  a.cnt = cnt;
+  a.sink = sink;
   a.found = found;
   a.mid = mid;
   a.big = big;
@@ -573,6 +571,11 @@ int tc_join(const __nv_bfloat16* hi, const __nv_bfloat16* lo, const float* norms
   a.kblocks = W / JKB;
   a.terms = terms;
   a.nstages = terms == 1 ? 2 : 1;
+  a.nlarge = nlarge;
+  a.step = step;
+  a.skip = skip;
+  const uint64_t first = (n + step - 1) / step;
+  a.count = (uint32_t)(skip ? n - first : first);
   a.mode = MODE_ORDER;
   a.next_node = counters;
   EFG_TRY(launch_join<128>(a, sms, smem_max, s));

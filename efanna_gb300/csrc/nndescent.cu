@@ -43,22 +43,30 @@ struct NNDev {
   DevBuf<uint32_t> pid, Lc, Range, new_ids, new_cnt, old_ids, old_cnt;
   DevBuf<uint8_t> found;
   // scratch
-  DevBuf<uint64_t> pair_off, rec_off64, scan64;
-  DevBuf<float> pairdist;
-  DevBuf<uint32_t> cnt, cursor, rec_aux, rcnt, rcur, roff, rbuf, scan32, ucnt;
-  DevBuf<uint64_t> rec_key;
+  DevBuf<uint64_t> task_len, off64, scan64;
+  DevBuf<uint64_t> rec_key;  // leaf merge: records per target
+  DevBuf<uint32_t> cnt, cursor, rcnt, rcur, roff, rbuf, scan32;
+  DevBuf<float> bound;
+  DevBuf<unsigned long long> totals;  // pairs, records, overflow records, nodes larger than a tile
+  DevBuf<uint32_t> jctr;              // node counters: the merge's, the join's (up to three launches in each of two parts)
+  DevBuf<uint4> bucket, ovf, ovfrec;  // join records: per-target buckets, overflow list, hub targets' records
+  DevBuf<uint32_t> ovf_slot;
   // tensor-core join: BF16 rows (hi, lo), FP32 norms, flags {inexact, error}, nodes left to FP32
   DevBuf<__nv_bfloat16> jhi, jlo;
   DevBuf<float> jnorm;
-  DevBuf<int> jflag;
+  DevBuf<int> jflag;  // inexact, error, not integers
   DevBuf<uint32_t> jmid, jbig;  // nodes of 129-256 rows, and larger ones (count in word 0)
   uint32_t jterms = 0;  // 0: not prepared; 1 or 3 products per value
+  bool jexact = false;  // the tensor cores' distances are exact (integers, squared norms below 2^22)
+  uint32_t W = 0;          // records per bucket
+  uint64_t bucket_cap = 0, ovf_cap = 0;
   void release_all() {
     pd.release(); radius.release(); radiusM.release(); pid.release(); Lc.release(); Range.release();
     new_ids.release(); new_cnt.release(); old_ids.release(); old_cnt.release(); found.release();
-    pair_off.release(); rec_off64.release(); scan64.release(); pairdist.release(); cnt.release(); cursor.release();
-    rec_aux.release(); rcnt.release(); rcur.release(); roff.release(); rbuf.release(); scan32.release();
-    ucnt.release(); rec_key.release(); jhi.release(); jlo.release(); jnorm.release(); jflag.release();
+    task_len.release(); off64.release(); scan64.release(); cnt.release(); cursor.release(); bound.release();
+    rcnt.release(); rcur.release(); roff.release(); rbuf.release(); scan32.release(); totals.release();
+    jctr.release(); bucket.release(); ovf.release(); ovfrec.release(); ovf_slot.release();
+    rec_key.release(); jhi.release(); jlo.release(); jnorm.release(); jflag.release();
     jmid.release();
     jbig.release();
     jterms = 0;
@@ -400,168 +408,309 @@ __global__ void init_select_kernel(const float* __restrict__ base, uint32_t ld4,
 // Join.
 // =============================================================================================
 
-// Pairs of node i's join: new x new with p < q (skipped when the ids are equal) and new x old.
-__global__ void pair_count_kernel(uint64_t n, const uint32_t* __restrict__ new_cnt,
-                                  const uint32_t* __restrict__ old_cnt, uint64_t* __restrict__ pairs) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint64_t a = new_cnt[i], b = old_cnt[i];
-  pairs[i] = a * (a - (a > 0 ? 1 : 0)) / 2 + a * b;
-}
-
-// The largest distance any insert aimed at node t can still be accepted at during this join:
-// max(radius, pool[L-1].dist).  Inserts beyond it are rejected by Neighbor::insert whatever the
-// order (the radius never rises above it), so their records need not be materialised.
-__global__ void bound_kernel(uint64_t n, uint32_t P, const float* __restrict__ pd, const uint32_t* __restrict__ Lc,
-                             const float* __restrict__ radius, float* __restrict__ bound) {
+// bound[t]: the largest distance any insert aimed at node t can still be accepted at during this join:
+// max(radius, pool[L-1].dist).  Inserts beyond it are rejected by Neighbor::insert whatever the order
+// (the radius never rises above it), so their records need not be materialised.  total: the pairs of
+// the nodes' joins, new x new with p < q and new x old.
+__global__ void __launch_bounds__(256) bound_kernel(uint64_t n, uint32_t P, const float* __restrict__ pd,
+                                                    const uint32_t* __restrict__ Lc, const float* __restrict__ radius,
+                                                    const uint32_t* __restrict__ new_cnt,
+                                                    const uint32_t* __restrict__ old_cnt, float* __restrict__ bound,
+                                                    unsigned long long* __restrict__ total) {
+  __shared__ unsigned long long wsum[8];
   uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long pairs = 0;
+  if (t < n) {
+    float r = radius[t];
+    float w = pd[t * P + Lc[t] - 1];
+    bound[t] = r > w ? r : w;
+    uint64_t a = new_cnt[t], b = old_cnt[t];
+    pairs = a * (a - (a > 0 ? 1 : 0)) / 2 + a * b;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = pairs;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) pairs += wsum[w];
+    if (pairs) atomicAdd(total, pairs);
+  }
+}
+
+// Targets with more records than a bucket holds: their record counts (0 for the others), whose scan
+// places their records in one exactly sized array.
+__global__ void hub_len_kernel(uint64_t n, uint32_t W, const uint32_t* __restrict__ cnt, uint64_t* __restrict__ len) {
+  uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) len[t] = cnt[t] > W ? cnt[t] : 0;
+}
+
+// The bucket's share of those targets' records (a warp per target) ...
+__global__ void hub_copy_kernel(uint64_t n, uint32_t W, const uint32_t* __restrict__ cnt,
+                                const uint64_t* __restrict__ off, const uint4* __restrict__ bucket,
+                                uint4* __restrict__ out) {
+  const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (t >= n || cnt[t] <= W) return;
+  for (uint32_t b = threadIdx.x & 31; b < W; b += 32) out[off[t] + b] = bucket[t * W + b];
+}
+
+// ... and the overflow list's.
+__global__ void hub_scatter_kernel(uint64_t m, const uint4* __restrict__ ovf, const uint32_t* __restrict__ slot,
+                                   const uint64_t* __restrict__ off, uint4* __restrict__ out) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  const uint4 r = ovf[i];
+  out[off[r.w] + slot[i]] = r;
+}
+
+__device__ __forceinline__ K96 rec_k96(const uint4& r) { return K96{rec_key(r), r.z}; }
+
+// A target's P-th smallest distance over distinct ids of its pool and the records found so far lowers
+// its bound: P entries at or below it fill the pool and its overflow slot, after which the radius is at
+// most that distance, so a record beyond it is rejected whatever else arrives.  A pair's distance is the
+// same wherever it is computed (the caller sees to that), so equal ids have equal keys.  The 64 smallest
+// keys, whatever order the records arrived in, are kept over chunks of 32; targets of more records than
+// a bucket holds keep their bound.  A warp per target.
+constexpr uint32_t TIGHTEN_MAX_P = 48;
+__global__ void __launch_bounds__(256) tighten_kernel(uint64_t n, uint32_t P, uint32_t W,
+                                                      const uint32_t* __restrict__ cnt,
+                                                      const uint4* __restrict__ bucket, const float* __restrict__ pd,
+                                                      const uint32_t* __restrict__ pid,
+                                                      const uint32_t* __restrict__ Lc, float* __restrict__ bound) {
+  const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t lane = threadIdx.x & 31;
   if (t >= n) return;
-  float r = radius[t];
-  float w = pd[t * P + Lc[t] - 1];
-  bound[t] = r > w ? r : w;
-}
-
-// Join pass 0: the distances of node i's pairs, stored, and record counts per target.  One warp
-// per node, nodes taken from a shared counter as warps come free (pair counts differ by an order
-// of magnitude, so a fixed assignment leaves most warps of a block idle behind its longest node).
-// New entries are taken two at a time: x0 = new[p] pairs with Y = new[p+1..] + old, x1 = new[p+1]
-// with Y[1..], so every candidate row loaded serves both; four rows per pass, the 2 x 4 sums
-// reduced together.
-__global__ void __launch_bounds__(256, 4) join_dist_kernel(
-    const float* __restrict__ base, uint32_t ld4, uint64_t n, uint32_t cap, uint32_t P, uint32_t check_k,
-    const uint32_t* __restrict__ new_ids, const uint32_t* __restrict__ new_cnt, const uint32_t* __restrict__ old_ids,
-    const uint32_t* __restrict__ old_cnt, const uint64_t* __restrict__ pair_off, const float* __restrict__ bound,
-    float* __restrict__ pairdist, uint32_t* __restrict__ cnt, uint8_t* __restrict__ found,
-    uint32_t* __restrict__ next_node) {
-  const uint32_t lane = threadIdx.x & 31;
-  for (;;) {
-    uint32_t ii = 0;
-    if (lane == 0) ii = atomicAdd(next_node, 1u);
-    const uint64_t i = __shfl_sync(0xffffffffu, ii, 0);
-    if (i >= n) return;
-    const uint32_t nn = new_cnt[i], no = old_cnt[i];
-    if (nn == 0) continue;
-    const uint32_t* nw = new_ids + i * cap;
-    const uint32_t* od = old_ids + i * cap;
-    const uint64_t po = pair_off[i];
-    bool found_drop = false;
-    for (uint32_t p = 0; p < nn; p += 2) {
-      const bool two = p + 1 < nn;
-      const uint32_t x0 = nw[p], x1 = two ? nw[p + 1] : x0;
-      const uint32_t nl = nn - 1 - p;  // new-list candidates of x0
-      const uint32_t m = nl + no;      // Y positions (x1 takes positions 1..m-1)
-      const float4* r0 = reinterpret_cast<const float4*>(base) + (uint64_t)x0 * ld4;
-      const float4* r1 = reinterpret_cast<const float4*>(base) + (uint64_t)x1 * ld4;
-      for (uint32_t cb = 0; cb < m; cb += 32) {
-        const uint32_t cm = min(32u, m - cb);
-        // lane l's candidate (position cb + l; the last one repeated past cm), loaded once per
-        // chunk and handed to the passes by shuffles
-        const uint32_t cl = cb + min(lane, cm - 1);
-        const uint32_t cand = cl < nl ? nw[p + 1 + cl] : od[cl - nl];
-        float mine0 = 0.f, mine1 = 0.f;
-        for (uint32_t u0 = 0; u0 < cm; u0 += 4) {
-          float acc[8];  // [0..4): x0 against rows u0..u0+3, [4..8): x1 against them
-          const float4* ry[4];
+  const uint32_t L = Lc[t], B = cnt[t];
+  if (L + B < P || B > W) return;
+  uint64_t v[2] = {~0ull, ~0ull};  // the 64 smallest, ascending over v[0] then v[1]
+  for (uint32_t b = 0; b < L + B; b += 32) {
+    const uint32_t e = b + lane;
+    uint64_t x = ~0ull;
+    if (e < L) x = pack_key(pd[t * P + e], pid[t * P + e] & IDM);
+    else if (e < L + B) x = rec_key(bucket[t * W + e - L]);
+    const uint64_t worst = __shfl_sync(0xffffffffu, v[1], 31);
+    if (__all_sync(0xffffffffu, x >= worst)) continue;
+    x = warp_sort32(x);
+    // v[1] and x, both ascending: the 32 smallest into v[1], then with v[0] likewise
+    v[1] = warp_merge_min32(v[1], x);
+    const uint64_t hi = shfl_idx(v[1], 31 - lane);  // bitonic split of v[0] (ascending) and v[1] reversed
+    uint64_t lo0 = lt(hi, v[0]) ? hi : v[0], hi0 = lt(hi, v[0]) ? v[0] : hi;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint32_t yu = __shfl_sync(0xffffffffu, cand, min(u0 + u, cm - 1));
-            ry[u] = reinterpret_cast<const float4*>(base) + (uint64_t)yu * ld4;
-            acc[u] = 0.f;
-            acc[u + 4] = 0.f;
-          }
-          for (uint32_t c4 = lane; c4 < ld4; c4 += 32) {
-            const float4 a = __ldg(r0 + c4), b = __ldg(r1 + c4);
-            float4 yv[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) yv[u] = __ldg(ry[u] + c4);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              float d0 = a.x - yv[u].x, d1 = a.y - yv[u].y, d2 = a.z - yv[u].z, d3 = a.w - yv[u].w;
-              acc[u] += d0 * d0;
-              acc[u] += d1 * d1;
-              acc[u] += d2 * d2;
-              acc[u] += d3 * d3;
-              float e0 = b.x - yv[u].x, e1 = b.y - yv[u].y, e2 = b.z - yv[u].z, e3 = b.w - yv[u].w;
-              acc[u + 4] += e0 * e0;
-              acc[u + 4] += e1 * e1;
-              acc[u + 4] += e2 * e2;
-              acc[u + 4] += e3 * e3;
-            }
-          }
-          // lanes 4r .. 4r+3 end with sum r: r < 4 x0's row u0+r, r >= 4 x1's row u0+r-4; row
-          // u's sums move to lane u0 + u
-          const float tot = reduce8_rows(acc, lane);
-          const uint32_t u = (lane - u0) & 3;
-          const float d0 = __shfl_sync(0xffffffffu, tot, u * 4), d1 = __shfl_sync(0xffffffffu, tot, (u + 4) * 4);
-          if (lane - u0 < 4u) {
-            mine0 = d0;
-            mine1 = d1;
-          }
-        }
-        const uint32_t c = cb + lane;
-        if (lane < cm) {
-          const bool my_new = c < nl;
-          found_drop |= join_lane_record<0>(i, x0, cand, my_new, mine0, join_slot(po, nn, no, p, c), P, check_k,
-                                            bound, pairdist, cnt, nullptr, nullptr, nullptr, nullptr);
-          if (two && c >= 1)  // x1's candidate c - 1 (new exactly when x0's candidate c is)
-            found_drop |= join_lane_record<0>(i, x1, cand, my_new, mine1, join_slot(po, nn, no, p + 1, c - 1), P,
-                                              check_k, bound, pairdist, cnt, nullptr, nullptr, nullptr, nullptr);
-        }
-      }
+    for (int j = 16; j > 0; j >>= 1) {
+      const bool lower = (lane & j) == 0;
+      uint64_t y = shfl_xor(lo0, j);
+      lo0 = (lower == lt(y, lo0)) ? y : lo0;
+      y = shfl_xor(hi0, j);
+      hi0 = (lower == lt(y, hi0)) ? y : hi0;
     }
-    if (__any_sync(0xffffffffu, found_drop) && lane == 0) found[i] = 1;
+    v[0] = lo0;
+    v[1] = hi0;
+  }
+  uint32_t seen = 0;  // distinct keys before this register
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    uint64_t prev = __shfl_up_sync(0xffffffffu, v[r], 1);
+    const uint64_t last = __shfl_sync(0xffffffffu, v[0], 31);
+    if (lane == 0) prev = r == 0 ? ~v[0] : last;
+    const uint32_t m = __ballot_sync(0xffffffffu, v[r] != ~0ull && v[r] != prev);
+    const uint32_t mine = seen + __popc(m & ((2u << lane) - 1));
+    if ((m >> lane & 1u) && mine == P) bound[t] = fminf(bound[t], key_dist(v[r]));
+    seen += __popc(m);
   }
 }
 
-// Join pass 1: node i's records written from the stored distances (warps take nodes from a
-// shared counter, as in pass 0).
-__global__ void __launch_bounds__(256, 4) join_records_kernel(
-    uint64_t n, uint32_t cap, uint32_t P, uint32_t check_k, const uint32_t* __restrict__ new_ids,
-    const uint32_t* __restrict__ new_cnt, const uint32_t* __restrict__ old_ids, const uint32_t* __restrict__ old_cnt,
-    const uint64_t* __restrict__ pair_off, const float* __restrict__ bound, float* __restrict__ pairdist,
-    const uint64_t* __restrict__ rec_off, uint32_t* __restrict__ cursor, uint64_t* __restrict__ rec_key,
-    uint32_t* __restrict__ rec_aux, uint32_t* __restrict__ next_node) {
-  const uint32_t lane = threadIdx.x & 31;
-  for (;;) {
-    uint32_t ii = 0;
-    if (lane == 0) ii = atomicAdd(next_node, 1u);
-    const uint64_t i = __shfl_sync(0xffffffffu, ii, 0);
-    if (i >= n) return;
-    const uint32_t nn = new_cnt[i], no = old_cnt[i];
-    if (nn == 0) continue;
-    const uint32_t* nw = new_ids + i * cap;
-    const uint32_t* od = old_ids + i * cap;
-    const uint64_t po = pair_off[i];
-    for (uint32_t p = 0; p < nn; ++p) {
-      const uint32_t x = nw[p], nl = nn - 1 - p, m = nl + no;
-      for (uint32_t c = lane; c < m; c += 32) {
-        const bool my_new = c < nl;
-        const uint32_t y = my_new ? nw[p + 1 + c] : od[c - nl];
-        join_lane_record<1>(i, x, y, my_new, 0.f, join_slot(po, nn, no, p, c), P, check_k, bound, pairdist, nullptr,
-                            rec_off, cursor, rec_key, rec_aux);
-      }
-    }
-  }
-}
+constexpr uint32_t MERGE_WARPS = 4;  // warps per merge block
 
-// Pool of one node held by a warp: entry e on lane e % 32, slot e / 32.
+// Records sorted at a time (a window): 64 for pools of up to 64 entries, which reject soon after as
+// many, 256 for larger ones.
 template <int NS>
-struct WarpPool {
-  float d[NS];
-  uint32_t id[NS];  // with FLAG
+struct Merge {
+  static constexpr uint32_t WIN = NS <= 2 ? 64 : 256;
+  static constexpr uint32_t WARP_BYTES = WIN * 12 + NS * 32 * 8;
 };
 
-// Next 32 records of a bucket in ascending (key, aux) order from `last` on (copies of `last`
-// included: the caller skips the ones it has applied).
-__device__ __forceinline__ K96 next_batch(const uint64_t* __restrict__ rk, const uint32_t* __restrict__ ra,
-                                          uint32_t B, K96 last, bool first) {
-  uint32_t lane = threadIdx.x & 31;
+// The pool of one node in a warp's shared memory, entries [0, L) ascending, slot P - 1 the overflow
+// slot, with Neighbor::insert / InsertIntoKnn applied to it (base_index.hpp:37-61).
+template <int NS>
+struct Pool {
+  float* pd;
+  uint32_t* pid;
+  uint8_t* found;
+  uint32_t P, check_k, L;
+  float rad;
+  bool any_dist, rejected;
+  K96 rej;
+
+  // One record as the reference applies it; true when it is rejected (every later one is too).
+  __device__ __forceinline__ bool apply(const K96 r) {
+    const uint32_t lane = threadIdx.x & 31;
+    const float d = key_dist(r.k);
+    const uint32_t cand = key_id(r.k);
+    if (d > rad) {
+      rejected = true;
+      rej = r;
+      return true;
+    }
+    float v[NS], up[NS];
+    uint32_t id[NS], upid[NS], i = 0, dup = 0;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const uint32_t e = s * 32 + lane;
+      v[s] = pd[e];
+      id[s] = pid[e];
+      up[s] = e ? pd[e - 1] : 0.f;
+      upid[s] = e ? pid[e - 1] : 0u;
+      i += __popc(__ballot_sync(0xffffffffu, e < L && v[s] <= d));  // entries of [0, L) with dist <= d
+    }
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const uint32_t e = s * 32 + lane;
+      dup |= __ballot_sync(0xffffffffu, (any_dist ? e < L : (e < i && v[s] == d)) && (id[s] & IDM) == cand);
+    }
+    uint32_t rank = L + 1;
+    if (!dup) {  // [i, L) moves up by one; entry L (<= P - 1) receives entry L - 1
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const uint32_t e = s * 32 + lane;
+        if (e > i && e <= L) {
+          pd[e] = up[s];
+          pid[e] = upid[s];
+        } else if (e == i) {
+          pd[e] = d;
+          pid[e] = cand | FLAG;
+        }
+      }
+      __syncwarp();
+      rank = i;
+      if (L + 1 < P) ++L;
+      else rad = pd[L - 1];
+    }
+    if ((r.a & 1u) == 0 && rank < check_k && lane == 0) found[r.a >> 1] = 1;
+    __syncwarp();
+    return false;
+  }
+
+  // Up to 32 ascending records, one per lane (lanes >= m hold none); true when one is rejected.
+  //
+  // The records that land strictly inside the pool are placed at once: with `j` of the records before
+  // it inserted and `pa` entries at or below its distance, a record's rank is pa + j (earlier records
+  // are no larger, so all of them precede it), and an entry moves up by the records placed before it.
+  // Duplicates are recognised among the entries and, as equal neighbours (with any_dist: equal ids),
+  // among the records.  From the first record on for which this does not hold -- one that is rejected,
+  // lands in the overflow slot, or whose duplicate may have left the pool -- they are applied one by one.
+  __device__ __forceinline__ bool apply_batch(const K96 r, uint32_t m) {
+    const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1;
+    const float d = key_dist(r.k);
+    const uint32_t cand = key_id(r.k);
+    uint32_t pa = 0;  // entries with dist <= d
+    {
+      uint32_t hi = L;
+      while (__any_sync(0xffffffffu, pa < hi)) {
+        if (pa < hi) {
+          const uint32_t mid = (pa + hi) >> 1;
+          if (pd[mid] <= d) pa = mid + 1;
+          else hi = mid;
+        }
+      }
+    }
+    bool dup = false;
+    uint32_t at = 0;  // (any_dist) the duplicate entry
+    if (any_dist) {
+      for (uint32_t e = 0; e < L; e += 4) {
+        const uint4 q = *reinterpret_cast<const uint4*>(pid + e);
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if ((w[c] & IDM) == cand && e + c < L) {
+            dup = true;
+            at = e + c;
+          }
+      }
+      const uint32_t same = __match_any_sync(0xffffffffu, lane < m ? cand : ~lane);  // (ids are < 2^30)
+      dup |= (same & below) != 0;
+    } else {
+      for (uint32_t e = pa; e > 0 && pd[e - 1] == d; --e)
+        if ((pid[e - 1] & IDM) == cand) {
+          dup = true;
+          break;
+        }
+      __syncwarp();
+      const uint64_t prev = __shfl_up_sync(0xffffffffu, r.k, 1);
+      dup |= lane > 0 && prev == r.k;
+    }
+    const uint32_t valid = m >= 32 ? 0xffffffffu : (1u << m) - 1;
+    const uint32_t j = __popc(__ballot_sync(0xffffffffu, !dup) & valid & below);
+    const bool accept = d <= rad || j >= P - L;  // (the radius is an inner entry's after an insert at capacity)
+    const bool ok = accept && pa + j < P - 1 && at + j < P - 1;
+    const uint32_t bad = ~__ballot_sync(0xffffffffu, ok) & valid;
+    const uint32_t f = bad ? __ffs(bad) - 1 : m;
+    const bool mine = lane < f;
+    if (mine && (r.a & 1u) == 0 && (dup ? min(L + j, P - 1) + 1 : pa + j) < check_k) found[r.a >> 1] = 1;
+    const uint32_t J = __popc(__ballot_sync(0xffffffffu, mine && !dup));
+    if (J) {
+      const uint32_t pos = pa + j, end = min(L + J, P);
+      uint32_t before = 0;
+      float nv[NS];
+      uint32_t ni[NS];
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {  // slot x takes entry x - (records placed below x)
+        const uint32_t word = __reduce_or_sync(0xffffffffu, mine && !dup && pos / 32 == (uint32_t)s ? 1u << (pos & 31) : 0u);
+        const uint32_t x = s * 32 + lane;
+        const uint32_t src = x < end ? x - min(x, before + __popc(word & below)) : x;
+        nv[s] = pd[src];
+        ni[s] = pid[src];
+        before += __popc(word);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        pd[s * 32 + lane] = nv[s];
+        pid[s * 32 + lane] = ni[s];
+      }
+      __syncwarp();
+      if (mine && !dup) {
+        pd[pos] = d;
+        pid[pos] = cand | FLAG;
+      }
+      __syncwarp();
+      if (J >= P - L) rad = pd[P - 2];
+      L = min(L + J, P - 1);
+    }
+    for (uint32_t u = f; u < m; ++u)
+      if (apply(shfl_idx(r, u))) return true;
+    return false;
+  }
+};
+
+// Sorts m <= 32 NR records of the warp's window (keys wk, aux wa) in registers.
+template <int NR>
+__device__ __forceinline__ void sort_window(uint64_t* wk, uint32_t* wa, uint32_t m) {
+  const uint32_t lane = threadIdx.x & 31;
+  K96 v[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const uint32_t e = r * 32 + lane;
+    v[r] = e < m ? K96{wk[e], wa[e]} : k96_max();
+  }
+  warp_sort_regs<NR>(v);
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    wk[r * 32 + lane] = v[r].k;
+    wa[r * 32 + lane] = v[r].a;
+  }
+  __syncwarp();
+}
+
+// Next 32 records of distance bits g in ascending (key, aux) order after `last`.
+__device__ __forceinline__ K96 next_batch(const uint4* __restrict__ rec, uint32_t B, uint32_t g, K96 last, bool first) {
+  const uint32_t lane = threadIdx.x & 31;
   K96 run = k96_max();
   for (uint32_t b = 0; b < B; b += 32) {
     K96 x = k96_max();
     if (b + lane < B) {
-      K96 y{rk[b + lane], ra[b + lane]};
-      if (first || !lt(y, last)) x = y;
+      const uint4 q = rec[b + lane];
+      const K96 y = rec_k96(q);
+      if (q.y == g && (first || lt(last, y))) x = y;
     }
     if (__all_sync(0xffffffffu, is_max(x))) continue;
     x = warp_sort32(x);
@@ -570,275 +719,174 @@ __device__ __forceinline__ K96 next_batch(const uint64_t* __restrict__ rk, const
   return run;
 }
 
-// Ascending bitonic sort of Bp records (keys sk, aux sa; Bp a power of two >= 32) in shared
-// memory by one warp.
-__device__ __forceinline__ void warp_sort_smem(uint64_t* sk, uint32_t* sa, uint32_t Bp) {
-  const uint32_t lane = threadIdx.x & 31;
-  for (uint32_t k = 2; k <= Bp; k <<= 1) {
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      for (uint32_t t = lane; t < Bp / 2; t += 32) {
-        const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), l = i + j;
-        const K96 x{sk[i], sa[i]}, y{sk[l], sa[l]};
-        if ((i & k) == 0 ? lt(y, x) : lt(x, y)) {
-          sk[i] = y.k;
-          sa[i] = y.a;
-          sk[l] = x.k;
-          sa[l] = x.a;
-        }
-      }
-      __syncwarp();
-    }
-  }
-}
-
-constexpr uint32_t MERGE_WARPS = 4;  // warps per merge block
-
-// Lane of the smallest of the warp's 32 records (the lower lane on a tie), on every lane.
-__device__ __forceinline__ uint32_t warp_argmin(K96 x) {
-  uint32_t who = threadIdx.x & 31;
-#pragma unroll
-  for (int m = 16; m > 0; m >>= 1) {
-    const K96 y = shfl_xor(x, m);
-    const uint32_t wy = __shfl_xor_sync(0xffffffffu, who, m);
-    if (lt(y, x) || (!lt(x, y) && wy < who)) {
-      x = y;
-      who = wy;
-    }
-  }
-  return who;
-}
-
-// One warp per target node: applies its records in ascending (dist, id, source, side) order,
-// every one of them (repeats of a record included), with Neighbor::insert / InsertIntoKnn
-// semantics (base_index.hpp:37-61).  The order comes from one of three sources:
-//   * 129 to msort records: sorted once in the warp's shared memory;
-//   * up to 32 x msort: runs of msort sorted in shared memory and written back in place, then
-//     merged 32 ways (lane l holds run l's head; msort / 32 records of each run staged in shared
-//     memory);
-//   * up to 128, or more than 32 x msort: pulled 32 at a time by scanning all of them.
+// One warp per target node: applies its records in ascending (dist, id, source, side) order until one
+// is rejected.  The records are taken a window at a time: those below a distance chosen (by
+// interpolation and bisection on the distance bits) so that at most WIN and, as a rule, at least half
+// as many fall below it, sorted in registers and applied 32 at once (Pool::apply_batch); a pool of 30
+// is done after one window of the 78 records per node and iteration that 1M x 128 has.  More than WIN
+// records at one distance are pulled 32 at a time.  A record equal to an earlier one in all four fields
+// changes nothing, so the windows need not keep its copies apart.
 // The reference rejects a candidate whose id sits among the entries of equal distance; a pair's
 // distance is the same wherever the reference computes it, so that finds every repeat.  With
 // any_dist a repeat is found at any distance: the tensor-core join's distances can differ in the
 // last bits from the FP32 ones a pool entry was inserted with, and an equal-distance test would
 // let the id in twice.
+// Bound: instruction issue and the latency of the record reads.  Sorting every record in shared memory
+// and inserting them one by one took 40 ms of the 1M x 128 build's 8 iterations and 65 ms of 6
+// iterations at 100k x 960 (P = 201).
 template <int NS>
-__global__ void merge_kernel(uint64_t n, uint32_t P, uint32_t check_k, bool any_dist, uint32_t msort,
-                 const uint32_t* __restrict__ cnt, const uint64_t* __restrict__ rec_off, uint64_t* __restrict__ rec_key,
-                 uint32_t* __restrict__ rec_aux, float* __restrict__ pd, uint32_t* __restrict__ pid,
-                 uint32_t* __restrict__ Lc, float* __restrict__ radius, uint8_t* __restrict__ found,
-                 uint32_t* __restrict__ next_node) {
-  extern __shared__ uint64_t merge_smem[];  // per warp: msort keys, then msort aux
-  const uint32_t lane = threadIdx.x & 31;
-  uint64_t* sk = merge_smem + (size_t)(threadIdx.x >> 5) * (msort + msort / 2);
-  uint32_t* sa = reinterpret_cast<uint32_t*>(sk + msort);
+__global__ void __launch_bounds__(MERGE_WARPS * 32) merge_kernel(
+    uint64_t n, uint32_t P, uint32_t check_k, bool any_dist, const uint32_t* __restrict__ cnt, uint32_t W,
+    const uint4* __restrict__ bucket, const uint64_t* __restrict__ hub_off, const uint4* __restrict__ hub,
+    float* __restrict__ pd, uint32_t* __restrict__ pid, uint32_t* __restrict__ Lc, float* __restrict__ radius,
+    uint8_t* __restrict__ found, uint32_t* __restrict__ next_node, unsigned long long* __restrict__ nrec) {
+  constexpr uint32_t WIN = Merge<NS>::WIN;
+  extern __shared__ __align__(16) unsigned char merge_smem[];
+  const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1;
+  unsigned char* mine = merge_smem + (size_t)(threadIdx.x >> 5) * Merge<NS>::WARP_BYTES;
+  uint64_t* wk = reinterpret_cast<uint64_t*>(mine);
+  Pool<NS> pool;
+  pool.pd = reinterpret_cast<float*>(mine + WIN * 8);
+  pool.pid = reinterpret_cast<uint32_t*>(pool.pd + NS * 32);
+  uint32_t* wa = pool.pid + NS * 32;
+  pool.found = found;
+  pool.P = P;
+  pool.check_k = check_k;
+  pool.any_dist = any_dist;
+  unsigned long long records = 0;
   for (;;) {  // nodes taken from a shared counter as warps come free (their record counts differ)
-  uint32_t tt = 0;
-  if (lane == 0) tt = atomicAdd(next_node, 1u);
-  const uint64_t t = __shfl_sync(0xffffffffu, tt, 0);
-  if (t >= n) return;
-  const uint32_t B = cnt[t];
-  if (B == 0) continue;
-  uint64_t* rk = rec_key + rec_off[t];
-  uint32_t* ra = rec_aux + rec_off[t];
-  WarpPool<NS> pool;
-  const uint64_t prow = t * P;
-#pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    uint32_t e = s * 32 + lane;
-    pool.d[s] = e < P ? pd[prow + e] : 0.f;
-    pool.id[s] = e < P ? pid[prow + e] : 0u;
-  }
-  uint32_t L = Lc[t];
-  float rad = radius[t];
-  bool rejected = false;
-  K96 rej{0, 0};
-
-  // Applies record r; true when r is rejected (every later record is too).
-  auto apply = [&](const K96 r) -> bool {
-    const float d = key_dist(r.k);
-    const uint32_t cand = key_id(r.k);
-    uint32_t rank;
-    if (d > rad) {
-      rejected = true;
-      rej = r;
-      return true;
+    uint32_t tt = 0;
+    if (lane == 0) tt = atomicAdd(next_node, 1u);
+    const uint64_t t = __shfl_sync(0xffffffffu, tt, 0);
+    if (t >= n) {
+      if (lane == 0 && records) atomicAdd(nrec, records);
+      return;
     }
-    // i = entries of [0, L) with dist <= d
-    uint32_t i = 0, dup = 0;
+    const uint32_t B = cnt[t];
+    if (B == 0) continue;
+    records += B;
+    const uint4* rec = B <= W ? bucket + t * W : hub + hub_off[t];  // (the hub array holds targets of B > W)
+    const uint64_t prow = t * P;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      uint32_t e = s * 32 + lane;
-      i += __popc(__ballot_sync(0xffffffffu, e < L && pool.d[s] <= d));
+      const uint32_t e = s * 32 + lane;
+      pool.pd[e] = e < P ? pd[prow + e] : 0.f;
+      pool.pid[e] = e < P ? pid[prow + e] : 0u;
     }
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      uint32_t e = s * 32 + lane;
-      dup |= __ballot_sync(0xffffffffu,
-                           (any_dist ? e < L : (e < i && pool.d[s] == d)) && (pool.id[s] & IDM) == cand);
-    }
-    if (dup) {
-      rank = L + 1;
-    } else {
-      // shift [i, L) up by one; entry L (<= P-1) receives entry L-1
-#pragma unroll
-      for (int s = NS - 1; s >= 0; --s) {
-        float ud = __shfl_up_sync(0xffffffffu, pool.d[s], 1);
-        uint32_t ui = __shfl_up_sync(0xffffffffu, pool.id[s], 1);
-        if (s > 0) {
-          float cd = __shfl_sync(0xffffffffu, pool.d[s > 0 ? s - 1 : 0], 31);
-          uint32_t ci = __shfl_sync(0xffffffffu, pool.id[s > 0 ? s - 1 : 0], 31);
-          if (lane == 0) {
-            ud = cd;
-            ui = ci;
-          }
-        }
-        uint32_t e = s * 32 + lane;
-        if (e > i && e <= L) {
-          pool.d[s] = ud;
-          pool.id[s] = ui;
-        } else if (e == i) {
-          pool.d[s] = d;
-          pool.id[s] = cand | FLAG;
-        }
-      }
-      rank = i;
-      if (L + 1 < P) {
-        ++L;
-      } else {
-        uint32_t e = L - 1;
-        float v = 0.f;
-#pragma unroll
-        for (int s = 0; s < NS; ++s) {
-          float w = __shfl_sync(0xffffffffu, pool.d[s], e & 31);
-          if ((uint32_t)s == e / 32) v = w;
-        }
-        rad = v;
-      }
-    }
-    if ((r.a & 1u) == 0 && rank < check_k && lane == 0) found[r.a >> 1] = 1;
-    return false;
-  };
+    pool.L = Lc[t];
+    pool.rad = radius[t];
+    pool.rejected = false;
+    __syncwarp();
 
-  const uint32_t runs = (B + msort - 1) / msort;
-  if (B > 128 && runs <= 32) {  // (a few batches of a small node: scanning, which stops at a rejection)
-    // sort each run of msort records in shared memory (a single run stays there)
-    for (uint32_t q = 0; q < runs; ++q) {
-      const uint32_t b0 = q * msort, len = min(msort, B - b0);
-      uint32_t Bp = 32;
-      while (Bp < len) Bp <<= 1;
-      for (uint32_t b = lane; b < Bp; b += 32) {
-        sk[b] = b < len ? rk[b0 + b] : ~0ULL;
-        sa[b] = b < len ? ra[b0 + b] : 0xffffffffu;
-      }
-      __syncwarp();
-      warp_sort_smem(sk, sa, Bp);
-      if (runs > 1) {
-        for (uint32_t b = lane; b < len; b += 32) {
-          rk[b0 + b] = sk[b];
-          ra[b0 + b] = sa[b];
-        }
-        __syncwarp();
-      }
-    }
-    if (runs == 1) {
-      bool stop = false;
-      for (uint32_t base = 0; base < B && !stop; base += 32) {
-        const K96 batch = base + lane < B ? K96{sk[base + lane], sa[base + lane]} : k96_max();
-        const uint32_t m = min(32u, B - base);
-        for (uint32_t u = 0; u < m; ++u)
-          if (apply(shfl_idx(batch, u))) {
-            stop = true;
-            break;
-          }
-      }
-    } else {
-      // 32-way merge: lane q holds run q's head; run q's records [ws, ws + SD) staged at
-      // sk/sa[SD q ..]
-      const uint32_t SD = msort / 32;
-      const uint32_t my_len = lane < runs ? min(msort, B - lane * msort) : 0;
-      uint32_t at = 0, ws = 0;  // lane q: next record of run q, first staged record of run q
-      for (uint32_t q = 0; q < runs; ++q) {
-        const uint32_t len = min(msort, B - q * msort);
-        if (lane < SD && lane < len) {
-          sk[SD * q + lane] = rk[q * msort + lane];
-          sa[SD * q + lane] = ra[q * msort + lane];
-        }
-      }
-      __syncwarp();
-      for (;;) {
-        const K96 head = at < my_len ? K96{sk[SD * lane + at - ws], sa[SD * lane + at - ws]} : k96_max();
-        const uint32_t w = warp_argmin(head);
-        const K96 r = shfl_idx(head, w);
-        if (is_max(r)) break;
-        if (apply(r)) break;
-        if (lane == w) ++at;
-        const uint32_t wat = __shfl_sync(0xffffffffu, at, w), wws = __shfl_sync(0xffffffffu, ws, w);
-        const uint32_t wlen = __shfl_sync(0xffffffffu, my_len, w);
-        if (wat == wws + SD && wat < wlen) {  // run w's staged records are spent: stage the next SD
-          __syncwarp();
-          if (lane < SD && wat + lane < wlen) {
-            sk[SD * w + lane] = rk[w * msort + wat + lane];
-            sa[SD * w + lane] = ra[w * msort + wat + lane];
-          }
-          __syncwarp();
-          if (lane == w) ws = wat;
-        }
-      }
-    }
-  } else {
-    // scanning: the next 32 records from the last applied one on, copies of it included
-    K96 last{0, 0};
-    uint32_t last_n = 0;  // copies of `last` applied so far
-    bool first = true, stop = false;
+    uint32_t tlo = 0;  // every record below these distance bits is done
+    bool stop = false;
     while (!stop) {
-      const K96 batch = next_batch(rk, ra, B, last, first);
-      first = false;
-      uint32_t skip = last_n;  // the batch starts with every copy of `last`
-      bool applied = false;
-      for (int u = 0; u < 32; ++u) {
-        const K96 r = shfl_idx(batch, u);
-        if (is_max(r)) {
-          stop = true;
-          break;
+      uint32_t thi = 0xffffffffu, total = B;
+      if (B > WIN || tlo) {
+        uint32_t mn = 0xffffffffu, mx = 0;
+        total = 0;
+        for (uint32_t b = lane; b < B; b += 32) {
+          const uint32_t q = rec[b].y;
+          if (q >= tlo) {
+            mn = min(mn, q);
+            mx = max(mx, q);
+            ++total;
+          }
         }
-        if (skip) {
-          --skip;
-          continue;
-        }
-        applied = true;
-        if (last_n && r.k == last.k && r.a == last.a) {
-          ++last_n;
-        } else {
-          last = r;
-          last_n = 1;
-        }
-        if (apply(r)) {
-          stop = true;
-          break;
+        mn = __reduce_min_sync(0xffffffffu, mn);
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        total = __reduce_add_sync(0xffffffffu, total);
+        if (total == 0) break;
+        if (total > WIN) {
+          uint32_t lo = mn, hi = mx + 1, clo = 0, chi = total;  // records in [tlo, lo) and [tlo, hi)
+          for (uint32_t it = 0; hi - lo > 1 && (clo == 0 || (clo < WIN / 2 && it < 8)); ++it) {
+            uint32_t mid = lo + (hi - lo) / 2;
+            if (!(it & 1)) mid = lo + (uint32_t)((float)(hi - lo) * ((float)(WIN * 3 / 4 - clo) / (float)(chi - clo)));
+            mid = min(max(mid, lo + 1), hi - 1);
+            uint32_t c = 0;
+            for (uint32_t b = lane; b < B; b += 32) {
+              const uint32_t q = rec[b].y;
+              c += q >= tlo && q < mid;
+            }
+            c = __reduce_add_sync(0xffffffffu, c);
+            if (c <= WIN) {
+              lo = mid;
+              clo = c;
+            } else {
+              hi = mid;
+              chi = c;
+            }
+          }
+          if (clo == 0) {  // more than WIN records at distance bits lo
+            K96 last{0, 0};
+            for (bool first = true; !stop; first = false) {
+              const K96 batch = next_batch(rec, B, lo, last, first);
+              const uint32_t m = __popc(__ballot_sync(0xffffffffu, !is_max(batch)));
+              if (m == 0) break;
+              stop = pool.apply_batch(batch, m);
+              last = shfl_idx(batch, m - 1);
+            }
+            tlo = lo + 1;
+            continue;
+          }
+          thi = lo;
+          total = clo;
         }
       }
-      if (!applied) break;  // a batch of nothing but applied copies (more than 32 repeats)
+      // the records of [tlo, thi), sorted
+      if (tlo == 0 && thi == 0xffffffffu) {
+        for (uint32_t b = lane; b < B; b += 32) {
+          const K96 y = rec_k96(rec[b]);
+          wk[b] = y.k;
+          wa[b] = y.a;
+        }
+      } else {
+        uint32_t at = 0;
+        for (uint32_t b = 0; b < B; b += 32) {
+          const uint4 q = b + lane < B ? rec[b + lane] : make_uint4(0, 0xffffffffu, 0, 0);
+          const bool take = b + lane < B && q.y >= tlo && q.y < thi;
+          const uint32_t bal = __ballot_sync(0xffffffffu, take);
+          if (take) {
+            const uint32_t o = at + __popc(bal & below);
+            wk[o] = rec_key(q);
+            wa[o] = q.z;
+          }
+          at += __popc(bal);
+        }
+      }
+      __syncwarp();
+      if (total <= 32) sort_window<1>(wk, wa, total);
+      else if (total <= 64) sort_window<2>(wk, wa, total);
+      else if (WIN > 64 && total <= 128) sort_window<(WIN > 64 ? 4 : 1)>(wk, wa, total);
+      else if (WIN > 64) sort_window<(WIN > 64 ? 8 : 1)>(wk, wa, total);
+      for (uint32_t b = 0; b < total && !stop; b += 32) {
+        const K96 batch = b + lane < total ? K96{wk[b + lane], wa[b + lane]} : k96_max();
+        stop = pool.apply_batch(batch, min(32u, total - b));
+      }
+      if (thi == 0xffffffffu) break;
+      tlo = thi;
     }
-  }
-  if (rejected && P < check_k) {
-    // every record from `rej` on was rejected with rank P < check_k
-    for (uint32_t b = lane; b < B; b += 32) {
-      K96 y{rk[b], ra[b]};
-      if (!lt(y, rej) && (y.a & 1u) == 0) found[y.a >> 1] = 1;
+    if (pool.rejected && P < check_k) {
+      // every record from `rej` on was rejected with rank P < check_k
+      for (uint32_t b = lane; b < B; b += 32) {
+        const K96 y = rec_k96(rec[b]);
+        if (!lt(y, pool.rej) && (y.a & 1u) == 0) found[y.a >> 1] = 1;
+      }
     }
-  }
+    __syncwarp();
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    uint32_t e = s * 32 + lane;
-    if (e < P) {
-      pd[prow + e] = pool.d[s];
-      pid[prow + e] = pool.id[s];
+    for (int s = 0; s < NS; ++s) {
+      const uint32_t e = s * 32 + lane;
+      if (e < P) {
+        pd[prow + e] = pool.pd[e];
+        pid[prow + e] = pool.pid[e];
+      }
     }
-  }
-  if (lane == 0) {
-    Lc[t] = L;
-    radius[t] = rad;
-  }
+    if (lane == 0) {
+      Lc[t] = pool.L;
+      radius[t] = pool.rad;
+    }
+    __syncwarp();
   }
 }
 
@@ -1020,15 +1068,15 @@ static int nnd_init_device(efg_index* idx, NNDev& S) {
   EFG_TRY(nn_alloc(S, n, bp.L, cap));
   TreeView tv{F.nodes.p, F.n_left.p, F.n_right.p, F.n_level.p, F.n_tree.p, F.n_start.p, F.n_end.p, F.leaves.p, F.n};
   // task offsets over nodes
-  EFG_TRY(S.pair_off.reserve(F.nnodes + 1));
-  EFG_TRY(S.rec_off64.reserve(F.nnodes + 1));
+  EFG_TRY(S.task_len.reserve(F.nnodes + 1));
+  EFG_TRY(S.off64.reserve(std::max<uint64_t>(F.nnodes, n) + 1));
   EFG_TRY(S.scan64.reserve(scan_tmp_elems<uint64_t>(std::max<uint64_t>(F.nnodes, n)) + 1));
   merge_task_len_kernel<<<blocks_for(F.nnodes, 256), 256, 0, s>>>(tv, F.nnodes, bp.trees_build,
-                                                                   (int32_t)bp.merge_level, S.pair_off.p);
+                                                                   (int32_t)bp.merge_level, S.task_len.p);
   EFG_CUDA(cudaGetLastError());
-  EFG_TRY(device_scan<uint64_t>(S.pair_off.p, F.nnodes, S.rec_off64.p, S.scan64.p, s));
+  EFG_TRY(device_scan<uint64_t>(S.task_len.p, F.nnodes, S.off64.p, S.scan64.p, s));
   uint64_t ntasks = 0;
-  EFG_CUDA(cudaMemcpyAsync(&ntasks, S.rec_off64.p + F.nnodes, 8, cudaMemcpyDeviceToHost, s));
+  EFG_CUDA(cudaMemcpyAsync(&ntasks, S.off64.p + F.nnodes, 8, cudaMemcpyDeviceToHost, s));
   EFG_CUDA(cudaStreamSynchronize(s));
   // per-target record counts -> offsets
   EFG_TRY(S.cnt.reserve(n));
@@ -1063,7 +1111,7 @@ static int nnd_init_device(efg_index* idx, NNDev& S) {
     EFG_TRY(task_d.reserve(ntasks * maxl));
   }
   if (ntasks) {
-    merge_route_kernel<0><<<rgrid, 256, 0, s>>>(idx->d_base, ld4, tv, S.rec_off64.p, F.nnodes, ntasks, S.cnt.p,
+    merge_route_kernel<0><<<rgrid, 256, 0, s>>>(idx->d_base, ld4, tv, S.off64.p, F.nnodes, ntasks, S.cnt.p,
                                                  nullptr, nullptr, nullptr, nd.p, task_p.p, task_leaf.p, task_d.p,
                                                  maxl);
     EFG_CUDA(cudaGetLastError());
@@ -1083,7 +1131,7 @@ static int nnd_init_device(efg_index* idx, NNDev& S) {
         tv, ntasks, task_p.p, task_leaf.p, task_d.p, maxl, off64.p, S.cursor.p, S.rec_key.p);
     EFG_CUDA(cudaGetLastError());
   } else if (ntasks) {
-    merge_route_kernel<1><<<rgrid, 256, 0, s>>>(idx->d_base, ld4, tv, S.rec_off64.p, F.nnodes, ntasks, nullptr,
+    merge_route_kernel<1><<<rgrid, 256, 0, s>>>(idx->d_base, ld4, tv, S.off64.p, F.nnodes, ntasks, nullptr,
                                                 off64.p, S.cursor.p, S.rec_key.p, nullptr, nullptr, nullptr, nullptr,
                                                 0);
     EFG_CUDA(cudaGetLastError());
@@ -1105,101 +1153,130 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   uint64_t n = S.n;
   uint32_t ld4 = idx->ld / 4;
   // ---- join
-  EFG_TRY(S.pair_off.reserve(n + 1));
-  EFG_TRY(S.rec_off64.reserve(n + 1));
+  EFG_TRY(S.off64.reserve(n + 1));
   EFG_TRY(S.scan64.reserve(scan_tmp_elems<uint64_t>(2 * n) + 1));
-  LocalBuf<uint64_t> tmp64;
-  EFG_TRY(tmp64.reserve(2 * n + 1));
-  pair_count_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, S.new_cnt.p, S.old_cnt.p, tmp64.p);
-  EFG_CUDA(cudaGetLastError());
-  EFG_TRY(device_scan<uint64_t>(tmp64.p, n, S.pair_off.p, S.scan64.p, s));
-  uint64_t npairs = 0;
-  EFG_CUDA(cudaMemcpyAsync(&npairs, S.pair_off.p + n, 8, cudaMemcpyDeviceToHost, s));
-  EFG_CUDA(cudaStreamSynchronize(s));
-  EFG_TRY(S.pairdist.reserve(npairs + 1));
+  EFG_TRY(S.task_len.reserve(n + 1));
   EFG_TRY(S.cnt.reserve(2 * n));
-  EFG_TRY(S.cursor.reserve(2 * n));
-  LocalBuf<float> bound;
-  EFG_TRY(bound.reserve(n));
-  bound_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, S.P, S.pd.p, S.Lc.p, S.radius.p, bound.p);
-  EFG_CUDA(cudaMemsetAsync(S.cnt.p, 0, n * 4, s));
-  EFG_CUDA(cudaMemsetAsync(S.cursor.p, 0, n * 4, s));
-  EFG_CUDA(cudaMemsetAsync(S.found.p, 0, n, s));
-  LocalBuf<uint32_t> jctr;  // node counters of the two join passes, the merge, the tensor-core join's three
-  EFG_TRY(jctr.reserve(6));
-  EFG_CUDA(cudaMemsetAsync(jctr.p, 0, 24, s));
-  int sms = 152, per0 = 1, per1 = 1, dev = 0;
+  EFG_TRY(S.bound.reserve(n));
+  EFG_TRY(S.totals.reserve(4));
+  EFG_TRY(S.jctr.reserve(8));
+  // The first join keeps every pair of the seeded lists, mean = 2 S (2S - 1) records per node (380 for
+  // S = 10), of which a pool of P - 1 takes a few dozen.  So in FP32 it runs on 1 of `part` nodes first,
+  // where that leaves about P entries per target, the targets' bounds are tightened, and the other
+  // nodes follow: 1M x 128 keeps 221 records per node instead of 380.  (On the tensor cores only
+  // where their distances are exact: else an id may be found at two distances, and would count twice.)
+  const uint64_t mean = 2ull * bp.S * (2 * bp.S - 1);
+  const bool tc = idx->build_precision == EFG_PRECISION_BF16;
+  if (tc && !S.jterms) {
+    const uint64_t W = (idx->dim + 63) / 64 * 64;
+    EFG_TRY(S.jhi.reserve(n * W));
+    EFG_TRY(S.jlo.reserve(n * W));
+    EFG_TRY(S.jnorm.reserve(n));
+    EFG_TRY(S.jflag.reserve(3));
+    EFG_TRY(S.jmid.reserve(n + 1));
+    EFG_TRY(S.jbig.reserve(n + 1));
+    EFG_TRY(tc_join_prepare(idx->d_base, n, idx->dim, idx->ld, S.jhi.p, S.jlo.p, S.jnorm.p, S.jflag.p, s));
+    int inexact[3] = {0, 0, 0};
+    EFG_CUDA(cudaMemcpyAsync(inexact, S.jflag.p, 12, cudaMemcpyDeviceToHost, s));
+    EFG_CUDA(cudaStreamSynchronize(s));
+    S.jterms = inexact[0] ? 3 : 1;
+    S.jexact = !inexact[0] && !inexact[2];
+  }
+  const uint32_t part = iter == 0 && (!tc || S.jexact) && S.P <= TIGHTEN_MAX_P && mean / 8 + bp.S >= S.P + S.P / 4 ? 8 : 1;
+  // Bucket width: about the records a node receives in the first join, then three times the last
+  // iteration's mean (past the buffer's size only up to 4 GiB or when the mean itself nears its width:
+  // allocating costs about 1 ms per GB, more than a few overflowing hubs do), within a quarter of the
+  // memory free at the start; the rest goes to the overflow list.
+  if (!S.W) {
+    size_t free_b = 0, total_b = 0;
+    EFG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    S.bucket_cap = std::max<uint64_t>(1, (uint64_t)free_b / 4 / sizeof(uint4) / n);
+    const uint64_t expect = part > 1 ? mean / part + 8 * S.P : mean + mean / 4;
+    S.W = (uint32_t)std::min<uint64_t>(S.bucket_cap, expect + 32);
+    S.ovf_cap = std::max<uint64_t>(n * (expect / 4 + 8), 1 << 16);
+    EFG_TRY(S.ovf.reserve(S.ovf_cap));
+    EFG_TRY(S.ovf_slot.reserve(S.ovf_cap));
+  }
+  EFG_TRY(S.bucket.reserve(n * S.W));
+  int sms = 152, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per0, join_dist_kernel, 256, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, join_records_kernel, 256, 0);
-  const unsigned jgrid0 = (unsigned)std::min<uint64_t>(blocks_for(n * 32, 256), (uint64_t)sms * std::max(per0, 1));
-  const unsigned jgrid1 = (unsigned)std::min<uint64_t>(blocks_for(n * 32, 256), (uint64_t)sms * std::max(per1, 1));
-  const bool tc = idx->build_precision == EFG_PRECISION_BF16;
-  if (tc) {
-    // pass 0 on the tensor cores: nodes that fit one tile packed together, then the larger ones
-    if (!S.jterms) {
-      const uint64_t W = (idx->dim + 63) / 64 * 64;
-      EFG_TRY(S.jhi.reserve(n * W));
-      EFG_TRY(S.jlo.reserve(n * W));
-      EFG_TRY(S.jnorm.reserve(n));
-      EFG_TRY(S.jflag.reserve(2));
-      EFG_TRY(S.jmid.reserve(n + 1));
-      EFG_TRY(S.jbig.reserve(n + 1));
-      EFG_TRY(tc_join_prepare(idx->d_base, n, idx->dim, idx->ld, S.jhi.p, S.jlo.p, S.jnorm.p, S.jflag.p, s));
-      int inexact = 0;
-      EFG_CUDA(cudaMemcpyAsync(&inexact, S.jflag.p, 4, cudaMemcpyDeviceToHost, s));
-      EFG_CUDA(cudaStreamSynchronize(s));
-      S.jterms = inexact ? 3 : 1;
+  EFG_CUDA(cudaMemsetAsync(S.found.p, 0, n, s));
+  uint64_t npairs = 0, novf = 0;
+  for (;;) {  // again only when the overflow list was too short for its records
+    EFG_CUDA(cudaMemsetAsync(S.totals.p, 0, 32, s));
+    EFG_CUDA(cudaMemsetAsync(S.cnt.p, 0, n * 4, s));
+    EFG_CUDA(cudaMemsetAsync(S.jctr.p, 0, 32, s));
+    bound_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, S.P, S.pd.p, S.Lc.p, S.radius.p, S.new_cnt.p, S.old_cnt.p,
+                                                    S.bound.p, S.totals.p);
+    EFG_CUDA(cudaGetLastError());
+    const RecordSink sink{S.cnt.p, S.bucket.p, S.ovf.p, S.ovf_slot.p, S.totals.p + 2, S.ovf_cap, S.W};
+    if (tc) EFG_CUDA(cudaMemsetAsync(S.jflag.p + 1, 0, 4, s));
+    auto join = [&](uint32_t counter, uint32_t step, uint32_t skip) -> int {
+      if (!tc)
+        return join_fp32(idx->d_base, n, idx->ld, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p, S.old_ids.p,
+                         S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, step, skip, s);
+      EFG_CUDA(cudaMemsetAsync(S.jmid.p, 0, 4, s));
+      EFG_CUDA(cudaMemsetAsync(S.jbig.p, 0, 4, s));
+      return tc_join(S.jhi.p, S.jlo.p, S.jnorm.p, n, idx->dim, S.jterms, S.cap, S.P, bp.check_k, S.new_ids.p,
+                     S.new_cnt.p, S.old_ids.p, S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, S.jmid.p,
+                     S.jbig.p, S.totals.p + 3, S.jflag.p + 1, step, skip, s);
+    };
+    if (part > 1) {
+      EFG_TRY(join(1, part, 0));
+      tighten_kernel<<<blocks_for(n * 32, 256), 256, 0, s>>>(n, S.P, S.W, S.cnt.p, S.bucket.p, S.pd.p, S.pid.p,
+                                                             S.Lc.p, S.bound.p);
+      EFG_CUDA(cudaGetLastError());
+      EFG_TRY(join(4, part, 1));
+    } else {
+      EFG_TRY(join(1, 1, 0));
     }
-    EFG_CUDA(cudaMemsetAsync(S.jflag.p + 1, 0, 4, s));
-    EFG_CUDA(cudaMemsetAsync(S.jmid.p, 0, 4, s));
-    EFG_CUDA(cudaMemsetAsync(S.jbig.p, 0, 4, s));
-    EFG_TRY(tc_join(S.jhi.p, S.jlo.p, S.jnorm.p, n, idx->dim, S.jterms, S.cap, S.P, bp.check_k, S.new_ids.p,
-                    S.new_cnt.p, S.old_ids.p, S.old_cnt.p, S.pair_off.p, bound.p, S.pairdist.p, S.cnt.p, S.found.p,
-                    jctr.p + 3, S.jmid.p, S.jbig.p, S.jflag.p + 1, s));
-  } else {
-    join_dist_kernel<<<jgrid0, 256, 0, s>>>(idx->d_base, ld4, n, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p,
-                                            S.old_ids.p, S.old_cnt.p, S.pair_off.p, bound.p, S.pairdist.p, S.cnt.p,
-                                            S.found.p, jctr.p);
+    unsigned long long tot[4] = {0, 0, 0, 0};
+    EFG_CUDA(cudaMemcpyAsync(tot, S.totals.p, 32, cudaMemcpyDeviceToHost, s));
+    int jerr = 0;  // the tensor-core join's error word
+    if (tc) EFG_CUDA(cudaMemcpyAsync(&jerr, S.jflag.p + 1, 4, cudaMemcpyDeviceToHost, s));
+    EFG_CUDA(cudaStreamSynchronize(s));
+    if (jerr & 4) return fail(EFG_ERR_ARG, "tensor-core join: a join list holds an id >= n");
+    if (jerr) return fail(EFG_ERR_DEVICE_LIMIT, "tensor-core join: a wait ran out on the device");
+    npairs = tot[0];
+    novf = tot[2];
+    if (novf <= S.ovf_cap) {
+      idx->bstats.join_large_nodes += tot[3];
+      break;
+    }
+    S.ovf_cap = novf + novf / 4;
+    EFG_TRY(S.ovf.reserve(S.ovf_cap));
+    EFG_TRY(S.ovf_slot.reserve(S.ovf_cap));
+  }
+  if (novf) {  // the hub targets' records gathered in one array
+    hub_len_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, S.W, S.cnt.p, S.task_len.p);
+    EFG_CUDA(cudaGetLastError());
+    EFG_TRY(device_scan<uint64_t>(S.task_len.p, n, S.off64.p, S.scan64.p, s));
+    uint64_t hub_total = 0;
+    EFG_CUDA(cudaMemcpyAsync(&hub_total, S.off64.p + n, 8, cudaMemcpyDeviceToHost, s));
+    EFG_CUDA(cudaStreamSynchronize(s));
+    EFG_TRY(S.ovfrec.reserve(hub_total));
+    hub_copy_kernel<<<blocks_for(n * 32, 256), 256, 0, s>>>(n, S.W, S.cnt.p, S.off64.p, S.bucket.p, S.ovfrec.p);
+    EFG_CUDA(cudaGetLastError());
+    hub_scatter_kernel<<<blocks_for(novf, 256), 256, 0, s>>>(novf, S.ovf.p, S.ovf_slot.p, S.off64.p, S.ovfrec.p);
     EFG_CUDA(cudaGetLastError());
   }
-  widen_kernel<<<blocks_for(n, 256), 256, 0, s>>>(S.cnt.p, tmp64.p, n);
-  EFG_TRY(device_scan<uint64_t>(tmp64.p, n, S.rec_off64.p, S.scan64.p, s));
-  uint64_t nrec = 0;
-  EFG_CUDA(cudaMemcpyAsync(&nrec, S.rec_off64.p + n, 8, cudaMemcpyDeviceToHost, s));
-  int jstat[2] = {0, 0};  // tensor-core join: error word, nodes larger than one tile
-  if (tc) {
-    EFG_CUDA(cudaMemcpyAsync(&jstat[0], S.jflag.p + 1, 4, cudaMemcpyDeviceToHost, s));
-    EFG_CUDA(cudaMemcpyAsync(&jstat[1], S.jbig.p, 4, cudaMemcpyDeviceToHost, s));
-  }
-  EFG_CUDA(cudaStreamSynchronize(s));
-  if (jstat[0] & 4) return fail(EFG_ERR_ARG, "tensor-core join: a join list holds an id >= n");
-  if (jstat[0]) return fail(EFG_ERR_DEVICE_LIMIT, "tensor-core join: a wait ran out on the device");
-  idx->bstats.join_large_nodes += (uint32_t)jstat[1];
-  EFG_TRY(S.rec_key.reserve(nrec + 1));
-  EFG_TRY(S.rec_aux.reserve(nrec + 1));
-  join_records_kernel<<<jgrid1, 256, 0, s>>>(n, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p, S.old_ids.p,
-                                             S.old_cnt.p, S.pair_off.p, bound.p, S.pairdist.p, S.rec_off64.p,
-                                             S.cursor.p, S.rec_key.p, S.rec_aux.p, jctr.p + 1);
-  EFG_CUDA(cudaGetLastError());
-  // merge: a warp per target node; records of up to msort per node sorted in shared memory
-  const uint32_t msort = S.P > 64 ? 1024 : 256;
-  const size_t msmem = (size_t)MERGE_WARPS * msort * 12;
-  auto launch_merge = [&](auto kern) -> int {
+  auto launch_merge = [&](auto kern, uint32_t warp_bytes) -> int {
+    const size_t msmem = (size_t)MERGE_WARPS * warp_bytes;
     EFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem));
     int per = 1;
     EFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, MERGE_WARPS * 32, msmem));
     const unsigned grid = (unsigned)std::min<uint64_t>(blocks_for(n * 32, MERGE_WARPS * 32),
                                                        (uint64_t)sms * std::max(per, 1));
-    kern<<<grid, MERGE_WARPS * 32, msmem, s>>>(n, S.P, bp.check_k, tc, msort, S.cnt.p, S.rec_off64.p, S.rec_key.p,
-                                               S.rec_aux.p, S.pd.p, S.pid.p, S.Lc.p, S.radius.p, S.found.p, jctr.p + 2);
+    kern<<<grid, MERGE_WARPS * 32, msmem, s>>>(n, S.P, bp.check_k, tc, S.cnt.p, S.W, S.bucket.p, S.off64.p,
+                                               S.ovfrec.p, S.pd.p, S.pid.p, S.Lc.p, S.radius.p, S.found.p,
+                                               S.jctr.p, S.totals.p + 1);
     return EFG_OK;
   };
-  if (S.P <= 32) EFG_TRY(launch_merge(merge_kernel<1>));
-  else if (S.P <= 64) EFG_TRY(launch_merge(merge_kernel<2>));
-  else if (S.P <= 128) EFG_TRY(launch_merge(merge_kernel<4>));
-  else EFG_TRY(launch_merge(merge_kernel<8>));
+  if (S.P <= 32) EFG_TRY(launch_merge(merge_kernel<1>, Merge<1>::WARP_BYTES));
+  else if (S.P <= 64) EFG_TRY(launch_merge(merge_kernel<2>, Merge<2>::WARP_BYTES));
+  else if (S.P <= 128) EFG_TRY(launch_merge(merge_kernel<4>, Merge<4>::WARP_BYTES));
+  else EFG_TRY(launch_merge(merge_kernel<8>, Merge<8>::WARP_BYTES));
   EFG_CUDA(cudaGetLastError());
   // ---- update
   update_range_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, S.P, bp.S, S.pd.p, S.pid.p, S.Lc.p, S.Range.p,
@@ -1228,9 +1305,12 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
                                                                     S.roff.p, S.rbuf.p, S.new_ids.p, S.new_cnt.p,
                                                                     S.old_ids.p, S.old_cnt.p);
   EFG_CUDA(cudaGetLastError());
+  unsigned long long nrec = 0;
+  EFG_CUDA(cudaMemcpyAsync(&nrec, S.totals.p + 1, 8, cudaMemcpyDeviceToHost, s));
   EFG_CUDA(cudaStreamSynchronize(s));
-  bound.release();
-  tmp64.release();
+  const uint64_t avg = nrec / n, have = std::max<uint64_t>(S.bucket.cap / n, (4ull << 30) / sizeof(uint4) / n);
+  S.W = (uint32_t)std::max<uint64_t>(
+      1, std::min<uint64_t>({S.bucket_cap, 3 * avg + 64, std::max<uint64_t>(have, avg + avg / 4 + 32)}));
   if (pairs_out) *pairs_out = npairs;
   if (recs_out) *recs_out = nrec;
   return EFG_OK;

@@ -49,6 +49,41 @@ __device__ __forceinline__ T warp_sort32(T x) {
   return x;
 }
 
+// Ascending bitonic sort of NR x 32 elements, element r * 32 + i in v[r] of lane i: partners 32 or more
+// apart are two registers of one lane.
+template <int NR, typename T>
+__device__ __forceinline__ void warp_sort_regs(T (&v)[NR]) {
+  const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 2; k <= 32 * NR; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j >= 32) {
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+          const int q = r ^ (j / 32);
+          if (q > r) {
+            const bool asc = ((r * 32) & k) == 0;
+            if (lt(v[q], v[r]) == asc) {
+              const T x = v[r];
+              v[r] = v[q];
+              v[q] = x;
+            }
+          }
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+          const T y = shfl_xor(v[r], j);
+          const bool asc = ((r * 32 + lane) & k) == 0, lower = (lane & j) == 0;
+          const bool ylt = lt(y, v[r]);
+          v[r] = ((lower == asc) == ylt) ? y : v[r];
+        }
+      }
+    }
+  }
+}
+
 // t and x ascending across lanes -> the 32 smallest of both, ascending.
 template <typename T>
 __device__ __forceinline__ T warp_merge_min32(T t, T x) {
