@@ -289,6 +289,7 @@ int efg_index_create(const float* data, uint64_t n, uint32_t dim, uint64_t row_s
   efg_index* idx = *out;
   cudaError_t e = cudaMemcpy2D(idx->d_base, idx->ld * sizeof(float), data, row_stride * sizeof(float),
                                dim * sizeof(float), n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // (the last piece may still be on its way)
   if (e != cudaSuccess) {
     efg_index_destroy(idx);
     *out = nullptr;
@@ -305,6 +306,9 @@ int efg_index_create_device(const float* d_data, uint64_t n, uint32_t dim, uint6
   efg_index* idx = *out;
   cudaError_t e = cudaMemcpy2D(idx->d_base, idx->ld * sizeof(float), d_data, row_stride * sizeof(float),
                                dim * sizeof(float), n, cudaMemcpyDeviceToDevice);
+  // (a device-to-device copy returns before it is done, and the index's stream does not wait for the
+  // default stream)
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   if (e != cudaSuccess) {
     efg_index_destroy(idx);
     *out = nullptr;
@@ -326,6 +330,8 @@ void efg_index_destroy(efg_index* idx) {
   idx->base16.release();
   idx->base8.release();
   idx->scale8.release();
+  idx->bytes.release();
+  idx->bnorm.release();
   idx->kg_keys.release();
   idx->qp_buf.release();
   idx->kg_bits.release();

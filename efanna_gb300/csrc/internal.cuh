@@ -144,6 +144,12 @@ struct efg_index {
   efg::DevBuf<uint8_t> base8;   // FP8 e4m3 screening copy (ld8 bytes per row) and per-row scales
   efg::DevBuf<float> scale8;
   uint32_t ld8 = 0;
+  // byte rows (ldb bytes each) and squared norms of a base of integers in [0, 255] with at most 258
+  // dimensions; bytes_state 0: not looked yet, 1: present, 2: other data
+  efg::DevBuf<uint8_t> bytes;
+  efg::DevBuf<uint32_t> bnorm;
+  uint32_t ldb = 0;
+  int bytes_state = 0;
   // kgraph search scratch: pool keys per query, visited bitsets per warp
   efg::DevBuf<uint64_t> kg_keys;
   efg::DevBuf<uint32_t> kg_bits;
@@ -191,6 +197,14 @@ int join_fp32(const float* base, uint64_t n, uint32_t ld, uint32_t cap, uint32_t
               const uint32_t* new_ids, const uint32_t* new_cnt, const uint32_t* old_ids, const uint32_t* old_cnt,
               const float* bound, const RecordSink& sink, uint8_t* found, uint32_t* counter, uint32_t step,
               uint32_t skip, cudaStream_t s);
+// bytes.cu: the byte rows of an index's base, where it has them (idx->bytes_state == 1 afterwards), and
+// the join over byte rows, with the FP32 join's records.
+int make_bytes(efg_index* idx);
+int join_bytes(const uint8_t* rows, const uint32_t* norm, uint64_t n, uint32_t ldb, uint32_t cap, uint32_t P,
+               uint32_t check_k, const uint32_t* new_ids, const uint32_t* new_cnt, const uint32_t* old_ids,
+               const uint32_t* old_cnt, const float* bound, const RecordSink& sink, uint8_t* found, uint32_t* counter,
+               uint32_t step, uint32_t skip, cudaStream_t s);
+__host__ __device__ __forceinline__ bool is_byte(float x) { return x >= 0.f && x <= 255.f && (float)(uint32_t)x == x; }
 // mlp_tc.cu: the learned form's dense layers on the tensor cores, C = act(A W^T + bias) (A: M x K,
 // W: N x K, BF16 row-major; C FP32 and / or Cb BF16, M x N); EFG_ERR_ARG when the shape does not fit.
 int tc_gemm_bf16(uint32_t M, uint32_t N, uint32_t K, const __nv_bfloat16* A, const __nv_bfloat16* W,

@@ -1201,6 +1201,7 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   int sms = 152, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (!tc) EFG_TRY(make_bytes(idx));
   EFG_CUDA(cudaMemsetAsync(S.found.p, 0, n, s));
   uint64_t npairs = 0, novf = 0;
   for (;;) {  // again only when the overflow list was too short for its records
@@ -1213,6 +1214,9 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
     const RecordSink sink{S.cnt.p, S.bucket.p, S.ovf.p, S.ovf_slot.p, S.totals.p + 2, S.ovf_cap, S.W};
     if (tc) EFG_CUDA(cudaMemsetAsync(S.jflag.p + 1, 0, 4, s));
     auto join = [&](uint32_t counter, uint32_t step, uint32_t skip) -> int {
+      if (!tc && idx->bytes_state == 1)
+        return join_bytes(idx->bytes.p, idx->bnorm.p, n, idx->ldb, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p,
+                          S.old_ids.p, S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, step, skip, s);
       if (!tc)
         return join_fp32(idx->d_base, n, idx->ld, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p, S.old_ids.p,
                          S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, step, skip, s);
