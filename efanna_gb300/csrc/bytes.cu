@@ -88,6 +88,7 @@ __global__ void __launch_bounds__(BW * 32, 5) join_bytes_kernel(const JoinBytesA
   uint32_t* norm_sh = norm_all[warp];
   float* bound_sh = bound_all[warp];
   const uint32_t rows0 = (uint32_t)__cvta_generic_to_shared(smem) + warp * BROWS * a.stride;
+  uint32_t* dot_sh = reinterpret_cast<uint32_t*>(smem + BW * BROWS * a.stride) + warp * 512;
   uint32_t nk = 0;
   if (lane == 0) nk = atomicAdd(a.next_node, 1u);
   for (;;) {
@@ -158,41 +159,58 @@ __global__ void __launch_bounds__(BW * 32, 5) join_bytes_kernel(const JoinBytesA
               acc[i * 4 + j] = s;
             }
         }
+        // the lane's 16 products through shared memory, so that the record code below exists once per
+        // column and not 16 times: unrolled over the rows too it outgrew the instruction cache
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4*>(dot_sh + (i * 32 + lane) * 4) =
+              make_uint4(acc[i * 4], acc[i * 4 + 1], acc[i * 4 + 2], acc[i * 4 + 3]);
+#pragma unroll 1
+        for (uint32_t i = 0; i < 4; ++i) {
           const uint32_t rx = gx * 4 + i;
           if (rx >= A) break;
           const uint32_t x = id_sh[rx], nx = norm_sh[rx];
           const float bx = bound_sh[rx];
+          const uint4 dv = *reinterpret_cast<const uint4*>(dot_sh + (i * 32 + lane) * 4);
+          const uint32_t dot[4] = {dv.x, dv.y, dv.z, dv.w};
           // four pairs' slots first, then their records: the atomics' latencies overlap
-          uint32_t slot[8], ta[8], ca[8];
+          uint32_t slot[8], ta[8];
           float dd[4];
-          bool put[8];
+          uint32_t put = 0;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const uint32_t ry = gy * 4 + j;
             const bool pair = ry < R && (tri ? ry > rx : ry >= A);
-            const uint32_t y = pair ? id_sh[ry] : 0;
-            const float by = pair ? bound_sh[ry] : 0.f;
+            const uint32_t y = id_sh[ry];
+            const float by = bound_sh[ry];
             const bool my_new = (ry < A ? a0 + ry : c0 + (ry - A)) < nn;
-            const float d = (float)(nx + (pair ? norm_sh[ry] : 0) - 2 * acc[i * 4 + j]);
+            dd[j] = (float)(nx + norm_sh[ry] - 2 * dot[j]);
             const bool ok = pair && !(my_new && y == x);
             const bool swap = my_new && y < x;  // side 0: the larger id into the smaller id's node
-            const float b0 = swap ? by : bx, b1 = swap ? bx : by;
-            dd[j] = d;
-            put[2 * j] = ok && d <= b0;
-            put[2 * j + 1] = ok && d <= b1;
-            drop |= ok && !(d <= b0);
+            const bool in0 = dd[j] <= (swap ? by : bx), in1 = dd[j] <= (swap ? bx : by);
+            put |= (ok && in0 ? 1u : 0u) << (2 * j) | (ok && in1 ? 2u : 0u) << (2 * j);
+            drop |= ok && !in0;
             ta[2 * j] = swap ? y : x;
             ta[2 * j + 1] = swap ? x : y;
-            ca[2 * j] = ta[2 * j + 1];
-            ca[2 * j + 1] = ta[2 * j];
           }
 #pragma unroll
-          for (int q = 0; q < 8; ++q) slot[q] = put[q] ? atomicAdd(&a.sink.cnt[ta[q]], 1u) : 0u;
+          for (int q = 0; q < 8; ++q)
+            if (put >> q & 1u) slot[q] = atomicAdd(&a.sink.cnt[ta[q]], 1u);
+          uint32_t over = 0;
 #pragma unroll
           for (int q = 0; q < 8; ++q)
-            if (put[q]) place_record(a.sink, ta[q], slot[q], dd[q >> 1], ca[q], (uint32_t)(node << 1) | (q & 1));
+            if (put >> q & 1u) {
+              if (slot[q] < a.sink.W)
+                a.sink.bucket[(uint64_t)ta[q] * a.sink.W + slot[q]] =
+                    make_uint4(ta[q ^ 1], __float_as_uint(dd[q >> 1]), (uint32_t)(node << 1) | (q & 1), ta[q]);
+              else over |= 1u << q;
+            }
+          if (over) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              if (over >> q & 1u)
+                place_overflow(a.sink, ta[q], slot[q], dd[q >> 1], ta[q ^ 1], (uint32_t)(node << 1) | (q & 1));
+          }
         }
       }
       __syncwarp();  // the tile's rows are no longer read
@@ -277,7 +295,7 @@ int join_bytes(const uint8_t* rows, const uint32_t* norm, uint64_t n, uint32_t l
   int dev = 0, sms = 152, per = 1;
   EFG_CUDA(cudaGetDevice(&dev));
   EFG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const size_t smem = (size_t)BW * BROWS * a.stride;
+  const size_t smem = (size_t)BW * (BROWS * a.stride + 2048);
   EFG_CUDA(cudaFuncSetAttribute(join_bytes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   EFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, join_bytes_kernel, BW * 32, smem));
   const unsigned grid = (unsigned)std::min<uint64_t>((a.count + BW - 1) / BW, (uint64_t)sms * std::max(per, 1));

@@ -27,19 +27,22 @@ struct RecordSink {
   uint32_t W;
 };
 
+// A record whose slot lies past its target's bucket.  (Not inlined: rare, and its code would be
+// repeated at every place that makes records.)
+static __device__ __noinline__ void place_overflow(const RecordSink& s, uint32_t t, uint32_t slot, float d,
+                                                   uint32_t cand, uint32_t aux) {
+  const unsigned long long o = atomicAdd(s.ovf_n, 1ull);
+  if (o < s.ovf_cap) {
+    s.ovf[o] = make_uint4(cand, __float_as_uint(d), aux, t);
+    s.ovf_slot[o] = slot;
+  }
+}
+
 // Writes a record to slot `slot` (taken from cnt[t]) of target t.
 __device__ __forceinline__ void place_record(const RecordSink& s, uint32_t t, uint32_t slot, float d, uint32_t cand,
                                              uint32_t aux) {
-  const uint4 r = make_uint4(cand, __float_as_uint(d), aux, t);
-  if (slot < s.W) {
-    s.bucket[(uint64_t)t * s.W + slot] = r;
-  } else {
-    const unsigned long long o = atomicAdd(s.ovf_n, 1ull);
-    if (o < s.ovf_cap) {
-      s.ovf[o] = r;
-      s.ovf_slot[o] = slot;
-    }
-  }
+  if (slot < s.W) s.bucket[(uint64_t)t * s.W + slot] = make_uint4(cand, __float_as_uint(d), aux, t);
+  else place_overflow(s, t, slot, d, cand, aux);
 }
 
 __device__ __forceinline__ void emit_record(const RecordSink& s, uint32_t t, float d, uint32_t cand, uint32_t aux) {
