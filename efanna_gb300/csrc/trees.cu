@@ -57,118 +57,176 @@ __global__ void roots_init_kernel(NodeArrays na, uint32_t ntrees, uint64_t n) {
   na.split_at[t] = 0;
 }
 
-// (value desc, index asc): the rank order of selectDivision.
-__device__ __forceinline__ bool var_better(float va, int32_t ia, float vb, int32_t ib) {
-  return va > vb || (va == vb && ia < ib);
+// Four consecutive values of a row, from FP32 rows or from byte rows (ldw floats or bytes per row).
+__device__ __forceinline__ float4 row_quad(const float* __restrict__ rows, uint32_t ldw, uint32_t id, uint32_t q) {
+  return __ldg(reinterpret_cast<const float4*>(rows + (uint64_t)id * ldw) + q);
+}
+__device__ __forceinline__ float4 row_quad(const uint8_t* __restrict__ rows, uint32_t ldw, uint32_t id, uint32_t q) {
+  const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(rows + (uint64_t)id * ldw) + q);
+  // byte b as the low mantissa bits of 2^23: exact, and off the conversion unit
+  float4 v;
+  v.x = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440)) - 8388608.f;
+  v.y = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7441)) - 8388608.f;
+  v.z = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7442)) - 8388608.f;
+  v.w = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7443)) - 8388608.f;
+  return v;
 }
 
-// One warp per active node: statistics, split dimension and cut value.
-__global__ void split_stats_kernel(const float* __restrict__ base, uint32_t dim, uint32_t ld, uint64_t n,
-                                   const uint32_t* __restrict__ ids, NodeArrays na, const int32_t* __restrict__ active,
-                                   uint32_t nactive, int32_t level, int phaseB, uint32_t tns, uint64_t seed,
-                                   uint32_t* __restrict__ split_flag) {
-  extern __shared__ float smean[];  // (blockDim.x / 32) * dim
-  uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  uint32_t a = blockIdx.x * (blockDim.x >> 5) + wib;
-  if (a >= nactive) return;
-  float* mean = smean + (size_t)wib * dim;
-  int32_t v = active[a];
-  uint32_t s = na.start[v], e = na.end[v], count = e - s;
-  int32_t t = na.tree[v];
-  if (phaseB && count <= tns) {  // DFSbuild leaf (kdtreeub_index.hpp:1142-1149)
+// Takes the T_RAND_DIM best of the warp's candidates (c per lane; taken[i]: not one) in selectDivision's
+// rank order, value descending, then index ascending; lane r returns the r-th (value -1, index
+// 0x7fffffff when there are fewer).  Variances are not negative, so their bits order like them.
+template <int C>
+__device__ __forceinline__ void warp_top(const float (&val)[C], const int32_t (&idx)[C], bool (&taken)[C],
+                                         float& out_v, int32_t& out_i) {
+  const uint32_t lane = threadIdx.x & 31;
+  out_v = -1.0f;
+  out_i = 0x7fffffff;
+#pragma unroll
+  for (int r = 0; r < T_RAND_DIM; ++r) {
+    uint32_t key = 0;  // best value's bits + 1 (0: no candidate left)
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      if (!taken[c]) key = max(key, __float_as_uint(val[c]) + 1u);
+    const uint32_t best = __reduce_max_sync(0xffffffffu, key);
+    if (best == 0) break;
+    uint32_t who = 0x7fffffffu;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      if (!taken[c] && __float_as_uint(val[c]) + 1u == best) who = min(who, (uint32_t)idx[c]);
+    const uint32_t win = __reduce_min_sync(0xffffffffu, who);
+#pragma unroll
+    for (int c = 0; c < C; ++c) taken[c] |= (uint32_t)idx[c] == win;
+    if (lane == (uint32_t)r) {
+      out_v = __uint_as_float(best - 1u);
+      out_i = (int32_t)win;
+    }
+  }
+}
+
+// Statistics, split dimension and cut value of the active nodes: `wpn` warps of a block of eight per
+// node, each over its blocks of 128 dimensions, a lane four of them (one 16-byte load per row, or one
+// 4-byte load from byte rows); the sums of a dimension run in id order in one lane, eight rows in
+// flight.  Bound: the latency of the dependent sums at the top levels (few nodes), the row reads below.
+// With one warp per node and one dimension per lane this took 15.3 ms of the 1M x 128 build's trees
+// (8 trees, 27 levels) and 27.3 ms at 100k x 960.
+template <typename Row>
+__global__ void __launch_bounds__(256) split_stats_kernel(
+    const Row* __restrict__ rows, uint32_t ldw, uint32_t dim, uint64_t n, const uint32_t* __restrict__ ids,
+    NodeArrays na, const int32_t* __restrict__ active, uint32_t nactive, uint32_t wpn, int32_t level, int phaseB,
+    uint32_t tns, uint64_t seed, uint32_t* __restrict__ split_flag) {
+  extern __shared__ float smean[];  // (8 / wpn) * dim
+  __shared__ float cand_v[8][T_RAND_DIM];
+  __shared__ int32_t cand_i[8][T_RAND_DIM];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t slot = warp / wpn, part = warp - slot * wpn;
+  const uint32_t a = blockIdx.x * (8 / wpn) + slot;
+  const bool here = a < nactive;
+  float* mean = smean + (size_t)slot * dim;
+  const int32_t v = here ? active[a] : 0;
+  const uint32_t s = here ? na.start[v] : 0, count = here ? na.end[v] - s : 0;
+  const int32_t t = here ? na.tree[v] : 0;
+  const bool split = here && !(phaseB && count <= tns);  // else a DFSbuild leaf (kdtreeub_index.hpp:1142-1149)
+  if (split) {
+    const uint32_t* seg = ids + (uint64_t)t * n + s;
+    const uint32_t cnt = min((uint32_t)T_SAMPLE, count);
+    const float inv = __fdiv_rn(1.0f, (float)cnt);
+    uint32_t sid[4];  // lane l: sample ids l, l + 32, l + 64, l + 96
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sid[j] = j * 32 + lane < cnt ? __ldg(seg + j * 32 + lane) : 0u;
+    float bv = -1.0f;  // lane r: the best r-th of this warp's dimensions so far
+    int32_t bi = 0x7fffffff;
+    for (uint32_t kb = part * 128; kb < dim; kb += wpn * 128) {
+      const uint32_t k = kb + lane * 4;
+      const bool in = k < dim;
+      const uint32_t q = in ? k / 4 : 0;
+      float4 m = make_float4(0.f, 0.f, 0.f, 0.f), var = m;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t jc = cnt > j * 32u ? min(32u, cnt - j * 32u) : 0u;
+        for (uint32_t u0 = 0; u0 < jc; u0 += 8) {
+          float4 x[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) x[u] = row_quad(rows, ldw, __shfl_sync(0xffffffffu, sid[j], min(u0 + u, jc - 1)), q);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (u0 + u < jc) {
+              m.x = __fadd_rn(m.x, x[u].x);
+              m.y = __fadd_rn(m.y, x[u].y);
+              m.z = __fadd_rn(m.z, x[u].z);
+              m.w = __fadd_rn(m.w, x[u].w);
+            }
+        }
+      }
+      m.x = __fmul_rn(m.x, inv);
+      m.y = __fmul_rn(m.y, inv);
+      m.z = __fmul_rn(m.z, inv);
+      m.w = __fmul_rn(m.w, inv);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t jc = cnt > j * 32u ? min(32u, cnt - j * 32u) : 0u;
+        for (uint32_t u0 = 0; u0 < jc; u0 += 8) {
+          float4 x[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) x[u] = row_quad(rows, ldw, __shfl_sync(0xffffffffu, sid[j], min(u0 + u, jc - 1)), q);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (u0 + u < jc) {
+              const float d0 = __fsub_rn(x[u].x, m.x), d1 = __fsub_rn(x[u].y, m.y);
+              const float d2 = __fsub_rn(x[u].z, m.z), d3 = __fsub_rn(x[u].w, m.w);
+              var.x = __fadd_rn(var.x, __fmul_rn(d0, d0));
+              var.y = __fadd_rn(var.y, __fmul_rn(d1, d1));
+              var.z = __fadd_rn(var.z, __fmul_rn(d2, d2));
+              var.w = __fadd_rn(var.w, __fmul_rn(d3, d3));
+            }
+        }
+      }
+      const float mk[4] = {m.x, m.y, m.z, m.w};
+      float cv[5] = {var.x, var.y, var.z, var.w, bv};
+      int32_t ci[5];
+      bool taken[5];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const bool is = in && k + c < dim;
+        if (is) mean[k + c] = mk[c];
+        ci[c] = (int32_t)(k + c);
+        taken[c] = !is;
+      }
+      ci[4] = bi;
+      taken[4] = bi == 0x7fffffff;
+      warp_top<5>(cv, ci, taken, bv, bi);
+    }
+    if (lane < T_RAND_DIM) {
+      cand_v[warp][lane] = bv;
+      cand_i[warp][lane] = bi;
+    }
+  }
+  __syncthreads();
+  if (!here || part != 0) return;
+  if (!split) {
     if (lane == 0) {
       na.dim[v] = -1;
       split_flag[a] = 0;
     }
     return;
   }
-  const uint32_t* seg = ids + (uint64_t)t * n + s;
-  uint32_t cnt = min((uint32_t)T_SAMPLE, count);
-  float inv = __fdiv_rn(1.0f, (float)cnt);
-  // running top-5, identical on all lanes
-  float tv[T_RAND_DIM];
-  int32_t ti[T_RAND_DIM];
+  // the node's best over its warps' (at most 40 candidates)
+  float cv[2];
+  int32_t ci[2];
+  bool taken[2];
 #pragma unroll
-  for (int r = 0; r < T_RAND_DIM; ++r) {
-    tv[r] = -1.0f;
-    ti[r] = 0x7fffffff;
+  for (int c = 0; c < 2; ++c) {
+    const uint32_t e = c * 32 + lane, w = e / T_RAND_DIM;
+    const bool is = w < wpn;
+    cv[c] = is ? cand_v[warp + w][e - w * T_RAND_DIM] : -1.0f;
+    ci[c] = is ? cand_i[warp + w][e - w * T_RAND_DIM] : 0x7fffffff;
+    taken[c] = ci[c] == 0x7fffffff;
   }
-  for (uint32_t kb = 0; kb < dim; kb += 32) {
-    uint32_t k = kb + lane;
-    float m = 0.f, var = 0.f;
-    if (k < dim) {
-      for (uint32_t j = 0; j < cnt; ++j) m = __fadd_rn(m, __ldg(base + (uint64_t)seg[j] * ld + k));
-      m = __fmul_rn(m, inv);
-      for (uint32_t j = 0; j < cnt; ++j) {
-        float dd = __fsub_rn(__ldg(base + (uint64_t)seg[j] * ld + k), m);
-        var = __fadd_rn(var, __fmul_rn(dd, dd));
-      }
-      mean[k] = m;
-    }
-    // merge this block's 32 candidates into the running top-5
-    float cv = k < dim ? var : -1.0f;
-    int32_t ci = k < dim ? (int32_t)k : 0x7fffffff;
-    bool taken_c = k >= dim;
-    bool taken_r[T_RAND_DIM];
-#pragma unroll
-    for (int r = 0; r < T_RAND_DIM; ++r) taken_r[r] = ti[r] == 0x7fffffff;
-    float nv[T_RAND_DIM];
-    int32_t ni[T_RAND_DIM];
-#pragma unroll
-    for (int r = 0; r < T_RAND_DIM; ++r) {
-      // best remaining running entry (uniform) vs best remaining lane candidate (warp argmax)
-      float bv = -1.0f;
-      int32_t bi = 0x7fffffff;
-      int br = -1;
-#pragma unroll
-      for (int q = 0; q < T_RAND_DIM; ++q)
-        if (!taken_r[q] && (br < 0 || var_better(tv[q], ti[q], bv, bi))) {
-          bv = tv[q];
-          bi = ti[q];
-          br = q;
-        }
-      float lv = taken_c ? -1.0f : cv;
-      int32_t li = taken_c ? 0x7fffffff : ci;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, lv, o);
-        int32_t oi = __shfl_xor_sync(0xffffffffu, li, o);
-        if (var_better(ov, oi, lv, li)) {
-          lv = ov;
-          li = oi;
-        }
-      }
-      bool lane_wins = li != 0x7fffffff && (br < 0 || var_better(lv, li, bv, bi));
-      if (lane_wins) {
-        nv[r] = lv;
-        ni[r] = li;
-        if (!taken_c && ci == li) taken_c = true;
-      } else if (br >= 0) {
-        nv[r] = bv;
-        ni[r] = bi;
-#pragma unroll
-        for (int q = 0; q < T_RAND_DIM; ++q)
-          if (q == br) taken_r[q] = true;
-      } else {
-        nv[r] = -1.0f;
-        ni[r] = 0x7fffffff;
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < T_RAND_DIM; ++r) {
-      tv[r] = nv[r];
-      ti[r] = ni[r];
-    }
-  }
-  __syncwarp();
-  int num = 0;
-#pragma unroll
-  for (int r = 0; r < T_RAND_DIM; ++r) num += ti[r] != 0x7fffffff;
-  uint32_t rnd = (uint32_t)(hash4(seed, TAG_DIM, (uint64_t)t, (uint64_t)level, (uint64_t)s) % (uint64_t)num);
-  int32_t cutdim = ti[0];
-#pragma unroll
-  for (int r = 0; r < T_RAND_DIM; ++r)
-    if ((uint32_t)r == rnd) cutdim = ti[r];
+  float tv;
+  int32_t ti;
+  warp_top<2>(cv, ci, taken, tv, ti);
+  const int num = __popc(__ballot_sync(0xffffffffu, lane < T_RAND_DIM && ti != 0x7fffffff));
+  const uint32_t rnd = (uint32_t)(hash4(seed, TAG_DIM, (uint64_t)t, (uint64_t)level, (uint64_t)s) % (uint64_t)num);
+  const int32_t cutdim = __shfl_sync(0xffffffffu, ti, rnd);
   if (lane == 0) {
     na.dim[v] = cutdim;
     na.val[v] = mean[cutdim];
@@ -374,16 +432,23 @@ int build_forest(efg_index* idx, uint32_t ntrees) {
   int32_t level = 0;
   uint32_t* cur = F.leaves.p;
   uint32_t* other = ids_b.p;
-  const int wpb = 8;
-  size_t smem = (size_t)wpb * idx->dim * sizeof(float);
+  EFG_TRY(make_bytes(idx));
+  const bool bytes = idx->bytes_state == 1;
+  const uint32_t blocks128 = (idx->dim + 127) / 128;
+  const uint32_t wpn = blocks128 > 4 ? 8 : blocks128 > 2 ? 4 : blocks128;  // warps per node
+  const size_t smem = (size_t)(8 / wpn) * idx->dim * sizeof(float);
   if (smem > 48 * 1024)
-    EFG_CUDA(cudaFuncSetAttribute(split_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EFG_CUDA(cudaFuncSetAttribute(split_stats_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   while (nactive > 0) {
     if (phaseA && nactive >= 1100) phaseA = false;
     int phaseB = phaseA ? 0 : 1;
-    split_stats_kernel<<<(nactive + wpb - 1) / wpb, wpb * 32, smem, s>>>(idx->d_base, idx->dim, idx->ld, n, cur, na,
-                                                                         act.p, nactive, level, phaseB, tns, seed,
-                                                                         split_flag.p);
+    const unsigned sgrid = (nactive * wpn + 7) / 8;
+    if (bytes)
+      split_stats_kernel<<<sgrid, 256, smem, s>>>(idx->bytes.p, idx->ldb, idx->dim, n, cur, na, act.p, nactive, wpn,
+                                                  level, phaseB, tns, seed, split_flag.p);
+    else
+      split_stats_kernel<<<sgrid, 256, smem, s>>>(idx->d_base, idx->ld, idx->dim, n, cur, na, act.p, nactive, wpn,
+                                                  level, phaseB, tns, seed, split_flag.p);
     EFG_CUDA(cudaGetLastError());
     EFG_TRY(device_scan<uint32_t>(split_flag.p, nactive, child_off.p, tmp32.p, s));
     classify_kernel<<<grid_for(total, 256), 256, 0, s>>>(idx->d_base, idx->ld, n, ntrees, cur, owner.p, na, level,
