@@ -141,21 +141,29 @@ __global__ void min_leaf_level_kernel(TreeView tv, uint64_t nnodes, uint32_t tre
   if (tv.left[v] < 0 && (uint32_t)tv.tree[v] < trees_build) atomicMin(out, tv.level[v]);
 }
 
-// One warp per routed point: descend the larger child to a leaf (SearchToLeaf,
-// kdtreeub_index.hpp:1012-1021) and compare with each leaf point.  pass 0 counts records per
-// target, pass 1 writes them: key = (dist bits << 32) | candidate.  With task_d set, pass 0 also
-// keeps each task's point, leaf and distances (maxl per task), and merge_emit_kernel writes the
-// records from them instead of a second routing pass.
-template <int PASS>
-__global__ void __launch_bounds__(256, 3) merge_route_kernel(const float* __restrict__ base, uint32_t ld4, TreeView tv,
+// Byte rows for the leaf merge's distances (rows null: FP32 rows).
+struct ByteRows {
+  const uint8_t* rows;
+  const uint32_t* norm;
+  uint32_t chunks, gshift;  // 16-byte chunks per row; 2^gshift >= chunks lanes take one row
+};
+
+// Routed points: descend the larger child to a leaf (SearchToLeaf, kdtreeub_index.hpp:1012-1021) and
+// compare with each leaf point.  pass 0 counts records per target, pass 1 writes them: key = (dist
+// bits << 32) | candidate.  With task_d set, pass 0 also keeps each task's point, leaf and distances
+// (maxl per task), and merge_emit_kernel writes the records from them instead of a second routing pass.
+// A warp routes 32 consecutive tasks at once, one per lane (search and descent are chains of dependent
+// loads: the lanes run theirs side by side), then the whole warp computes each task's leaf distances in
+// turn.  Bound: the latency of the leaf rows' reads, one task's at a time per warp; byte rows bring
+// a leaf of ten points in one pass of four 16-byte loads per lane (8 lanes per row at 128 dimensions).
+template <int PASS, bool BYTES>
+__global__ void __launch_bounds__(256, 3) merge_route_kernel(const float* __restrict__ base, uint32_t ld4,
+                                   const ByteRows br, TreeView tv,
                                    const uint64_t* __restrict__ task_off, uint64_t nnodes, uint64_t ntasks,
                                    uint32_t* __restrict__ cnt, const uint64_t* __restrict__ off,
                                    uint32_t* __restrict__ cursor, uint64_t* __restrict__ keys,
                                    unsigned long long* __restrict__ ndist, uint32_t* __restrict__ task_p,
                                    int32_t* __restrict__ task_leaf, float* __restrict__ task_d, uint32_t maxl) {
-  // a warp routes 32 consecutive tasks at once, one per lane (search and descent are chains of
-  // dependent loads: the lanes run theirs side by side), then the whole warp computes each task's
-  // leaf distances in turn
   const uint64_t gwarp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
@@ -165,9 +173,26 @@ __global__ void __launch_bounds__(256, 3) merge_route_kernel(const float* __rest
     const uint64_t myw = wb + lane;
     uint32_t myp = 0, mls = 0, mle = 0;
     uint64_t mt = 0;
+    // node owning task wb, the last v with task_off[v] <= wb: 32 probes at a time
+    uint64_t lo = 0, hi = nnodes;
+    while (hi - lo > 1) {
+      const uint64_t step = (hi - lo + 32) / 33;
+      const uint64_t probe = lo + (lane + 1) * step;
+      const uint32_t le = __popc(__ballot_sync(0xffffffffu, probe < hi && task_off[probe] <= wb));
+      const uint64_t nlo = lo + le * step;
+      hi = nlo + step < hi ? nlo + step : hi;
+      lo = nlo;
+    }
     if (myw < ntasks) {
-      // node owning task myw: last v with task_off[v] <= myw
-      uint64_t lo = 0, hi = nnodes;
+      // the lane's own task: a few nodes further
+      uint64_t step = 1;
+      hi = lo + 1;
+      while (hi < nnodes && task_off[hi] <= myw) {
+        lo = hi;
+        hi += step;
+        step *= 2;
+      }
+      if (hi > nnodes) hi = nnodes;
       while (hi - lo > 1) {
         uint64_t mid = (lo + hi) >> 1;
         if (task_off[mid] <= myw) lo = mid;
@@ -200,6 +225,57 @@ __global__ void __launch_bounds__(256, 3) merge_route_kernel(const float* __rest
       const uint32_t ls = __shfl_sync(0xffffffffu, mls, j), le = __shfl_sync(0xffffffffu, mle, j);
       const uint64_t t = __shfl_sync(0xffffffffu, mt, j);
       const uint32_t* ll = tv.leaves + t * tv.n;
+      if (BYTES) {
+        const uint32_t G = 1u << br.gshift, rpi = 32u >> br.gshift, sub = lane >> br.gshift, cl = lane & (G - 1);
+        const bool on = cl < br.chunks;
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        const uint4* row4 = reinterpret_cast<const uint4*>(br.rows);
+        const uint4 y = on ? __ldg(row4 + (uint64_t)p * br.chunks + cl) : zero;
+        const uint32_t np = __ldg(br.norm + p);
+        const uint32_t span = min(4 * rpi, 32u);
+        for (uint32_t i0 = ls; i0 < le; i0 += span) {
+          const uint32_t m = min(span, le - i0);  // leaf points of this pass, point i with lane i
+          const uint32_t q = lane < m ? ll[i0 + lane] : 0u;
+          const uint32_t nq = lane < m ? __ldg(br.norm + q) : 0u;
+          uint4 x[4];
+          uint32_t dot[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t r = u * rpi + sub, id = __shfl_sync(0xffffffffu, q, r < m ? r : 0u);
+            x[u] = on && r < m ? __ldg(row4 + (uint64_t)id * br.chunks + cl) : zero;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            dot[u] = __dp4a(x[u].x, y.x, __dp4a(x[u].y, y.y, __dp4a(x[u].z, y.z, __dp4a(x[u].w, y.w, 0u))));
+          for (uint32_t o = G >> 1; o > 0; o >>= 1) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) dot[u] += __shfl_xor_sync(0xffffffffu, dot[u], o);
+          }
+          uint32_t mine = 0;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t v = __shfl_sync(0xffffffffu, dot[u], (lane & (rpi - 1)) << br.gshift);
+            if (lane / rpi == (uint32_t)u) mine = v;
+          }
+          const float d = (float)(np + nq - 2 * mine);
+          local += m;
+          if (PASS == 0) {
+            if (lane < m) {
+              if (task_d) task_d[w * maxl + (i0 - ls) + lane] = d;
+              atomicAdd(&cnt[q], 1u);
+            }
+            if (lane == 0) atomicAdd(&cnt[p], m);
+          } else {
+            uint32_t b = lane == 0 ? atomicAdd(&cursor[p], m) : 0u;
+            b = __shfl_sync(0xffffffffu, b, 0);
+            if (lane < m) {
+              keys[off[q] + atomicAdd(&cursor[q], 1u)] = pack_key(d, p);
+              keys[off[p] + b + lane] = pack_key(d, q);
+            }
+          }
+        }
+        continue;
+      }
       const float4* rp = reinterpret_cast<const float4*>(base) + (uint64_t)p * ld4;
       for (uint32_t i0 = ls; i0 < le; i0 += 8) {  // eight leaf points at a time, their loads in flight together
         const uint32_t cnt8 = min(8u, le - i0);
@@ -231,16 +307,19 @@ __global__ void __launch_bounds__(256, 3) merge_route_kernel(const float* __rest
         for (int u = 1; u < 8; ++u)
           if (r == (uint32_t)u) q = qq[u];
         local += cnt8;
-        if ((lane & 3) == 0 && r < cnt8) {
-          if (PASS == 0) {
+        const bool put = (lane & 3) == 0 && r < cnt8;
+        if (PASS == 0) {
+          if (put) {
             if (task_d) task_d[w * maxl + (i0 - ls) + r] = d;
             atomicAdd(&cnt[q], 1u);
-            atomicAdd(&cnt[p], 1u);
-          } else {
-            uint32_t a = atomicAdd(&cursor[q], 1u);
-            keys[off[q] + a] = pack_key(d, p);
-            uint32_t b = atomicAdd(&cursor[p], 1u);
-            keys[off[p] + b] = pack_key(d, q);
+          }
+          if (lane == 0) atomicAdd(&cnt[p], cnt8);
+        } else {
+          uint32_t b = lane == 0 ? atomicAdd(&cursor[p], cnt8) : 0u;
+          b = __shfl_sync(0xffffffffu, b, 0);
+          if (put) {
+            keys[off[q] + atomicAdd(&cursor[q], 1u)] = pack_key(d, p);
+            keys[off[p] + b + r] = pack_key(d, q);
           }
         }
       }
@@ -249,7 +328,8 @@ __global__ void __launch_bounds__(256, 3) merge_route_kernel(const float* __rest
   if (PASS == 0 && lane == 0 && local) atomicAdd(ndist, local);
 }
 
-// Records of the leaf merge from what pass 0 kept: one thread per task.
+// Records of the leaf merge from what pass 0 kept: one thread per task, whose own records (the point
+// with every leaf point) take their slots by one atomic.
 __global__ void merge_emit_kernel(TreeView tv, uint64_t ntasks, const uint32_t* __restrict__ task_p,
                                   const int32_t* __restrict__ task_leaf, const float* __restrict__ task_d,
                                   uint32_t maxl, const uint64_t* __restrict__ off, uint32_t* __restrict__ cursor,
@@ -261,13 +341,25 @@ __global__ void merge_emit_kernel(TreeView tv, uint64_t ntasks, const uint32_t* 
     const DNode nd = tv.nodes[leaf];
     const uint32_t* ll = tv.leaves + (uint64_t)tv.tree[leaf] * tv.n;
     const uint32_t ls = (uint32_t)(-(nd.left + 1)), le = (uint32_t)nd.right;
-    for (uint32_t i = ls; i < le; ++i) {
-      const uint32_t q = ll[i];
-      const float d = task_d[w * maxl + (i - ls)];
-      uint32_t a = atomicAdd(&cursor[q], 1u);
-      keys[off[q] + a] = pack_key(d, p);
-      uint32_t b = atomicAdd(&cursor[p], 1u);
-      keys[off[p] + b] = pack_key(d, q);
+    const uint64_t mine = off[p] + atomicAdd(&cursor[p], le - ls);
+    for (uint32_t i0 = ls; i0 < le; i0 += 4) {  // four atomics in flight
+      uint32_t q[4], slot[4];
+      float d[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i0 + u < le) {
+          q[u] = ll[i0 + u];
+          d[u] = task_d[w * maxl + (i0 + u - ls)];
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i0 + u < le) slot[u] = atomicAdd(&cursor[q[u]], 1u);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i0 + u < le) {
+          keys[off[q[u]] + slot[u]] = pack_key(d[u], p);
+          keys[mine + (i0 + u - ls)] = pack_key(d[u], q[u]);
+        }
     }
   }
 }
@@ -304,8 +396,42 @@ __device__ __forceinline__ uint64_t fold_distinct(uint64_t run, uint64_t x) {
   return warp_merge_min32(run, x);
 }
 
+// Keys waiting to be folded into a warp's running list: those below the list's `rank`-th key, which
+// few are once the list has settled (of 494 records per node about 70 in all), so a fold -- a match, a
+// sort and a merge of 32 -- runs for every 32 of them and not for every 32 records (15.5 ms of the
+// 1M x 128 build without the queue).
+struct FoldQueue {
+  uint64_t* q;  // 64 keys in shared memory
+  uint32_t n, rank;
+  uint64_t run, limit;
+  __device__ __forceinline__ FoldQueue(uint64_t* mem, uint32_t rank_) : q(mem), n(0), rank(rank_), run(~0ULL), limit(~0ULL) {}
+  __device__ __forceinline__ void fold(uint32_t m) {  // the first m <= 32
+    const uint32_t lane = threadIdx.x & 31;
+    __syncwarp();
+    const uint64_t x = lane < m ? q[lane] : ~0ULL;
+    const uint64_t rest = lane + 32 < n ? q[lane + 32] : ~0ULL;
+    run = fold_distinct(run, x);
+    limit = __shfl_sync(0xffffffffu, run, rank - 1);
+    __syncwarp();
+    if (lane + 32 < n) q[lane] = rest;
+    n -= m;
+    __syncwarp();
+  }
+  __device__ __forceinline__ void push(uint64_t x) {  // one key per lane, ~0 = none
+    const uint32_t lane = threadIdx.x & 31;
+    const bool take = x < limit;
+    const uint32_t bal = __ballot_sync(0xffffffffu, take);
+    if (take) q[n + __popc(bal & ((1u << lane) - 1))] = x;
+    n += __popc(bal);
+    if (n >= 32) fold(32);
+  }
+  __device__ __forceinline__ void finish() {
+    if (n) fold(n);
+  }
+};
+
 // One warp per node: S best distinct (dist, id) keys, S extra join candidates, pool seeding.
-__global__ void init_select_kernel(const float* __restrict__ base, uint32_t ld4, uint64_t n, uint32_t S, uint32_t P,
+__global__ void __launch_bounds__(256) init_select_kernel(const float* __restrict__ base, uint32_t ld4, uint64_t n, uint32_t S, uint32_t P,
                                    uint32_t cap, uint64_t seed, const uint32_t* __restrict__ cnt,
                                    const uint64_t* __restrict__ off, const uint64_t* __restrict__ keys,
                                    float* __restrict__ pd, uint32_t* __restrict__ pid, uint32_t* __restrict__ Lc,
@@ -318,12 +444,12 @@ __global__ void init_select_kernel(const float* __restrict__ base, uint32_t ld4,
   if (t >= n) return;
   const uint64_t* R = keys + off[t];
   uint32_t B = cnt[t];
-  // 1. the smallest distinct keys (up to 32)
-  uint64_t run = ~0ULL;
-  for (uint32_t b = 0; b < B; b += 32) {
-    uint64_t x = b + lane < B ? R[b + lane] : ~0ULL;
-    run = fold_distinct(run, x);
-  }
+  __shared__ uint64_t queue[8][64];
+  // 1. the S smallest distinct keys
+  FoldQueue best(queue[threadIdx.x >> 5], S);
+  for (uint32_t b = 0; b < B; b += 32) best.push(b + lane < B ? R[b + lane] : ~0ULL);
+  best.finish();
+  uint64_t run = best.run;
   uint32_t nvalid = __popc(__ballot_sync(0xffffffffu, run != ~0ULL));
   // 2. top up to S distinct with counter-hash random ids (kdtreeub_index.hpp:1399-1405)
   if (nvalid < S) {
@@ -340,20 +466,23 @@ __global__ void init_select_kernel(const float* __restrict__ base, uint32_t ld4,
   }
   uint64_t kth = __shfl_sync(0xffffffffu, run, S - 1);
   // 3. extras: S of the distinct keys beyond the S best, by smallest (hash, id); needs >= 2S
-  uint64_t hrun = ~0ULL;
+  FoldQueue more(queue[threadIdx.x >> 5], 2 * S);
   if (kth != ~0ULL) {
+    const uint64_t hkey = mix64(mix64(seed ^ (TAG_EXTRA * 0x9E3779B97F4A7C15ULL)) ^ t);  // hash4's first two steps
     for (uint32_t b = 0; b < B; b += 32) {
       uint64_t x = ~0ULL;
       if (b + lane < B) {
         uint64_t k = R[b + lane];
         if (k > kth) {
           uint32_t c = (uint32_t)k;
-          x = ((hash4(seed, TAG_EXTRA, t, c, 0) >> 32) << 32) | c;
+          x = ((mix64(mix64(hkey ^ c)) >> 32) << 32) | c;
         }
       }
-      hrun = fold_distinct(hrun, x);
+      more.push(x);
     }
+    more.finish();
   }
+  const uint64_t hrun = more.run;
   uint32_t nh = __popc(__ballot_sync(0xffffffffu, hrun != ~0ULL));
   uint32_t extra = 0;  // lane l < S holds extra id l
   if (nh >= 2 * S) {
@@ -919,46 +1048,42 @@ __global__ void update_range_kernel(uint64_t n, uint32_t P, uint32_t S, const fl
   radiusM[t] = pd[row + R - 1];
 }
 
-// Forward lists of node t (pool order) and reverse-edge counts per target.
+// Forward lists of node t (pool order) and reverse-edge counts per target; a warp per node, an entry per
+// lane, so that the pool's rows are read in lines and the targets' radii and counts side by side.
 // PASS 0: counts; PASS 1: writes reverse edges and clears the new flags.
 template <int PASS>
-__global__ void update_lists_kernel(uint64_t n, uint32_t P, uint32_t cap, const float* __restrict__ pd,
-                                    uint32_t* __restrict__ pid, const uint32_t* __restrict__ Range,
-                                    const float* __restrict__ radiusM, uint32_t* __restrict__ new_ids,
-                                    uint32_t* __restrict__ new_cnt, uint32_t* __restrict__ old_ids,
-                                    uint32_t* __restrict__ old_cnt, uint32_t* __restrict__ rcnt,
-                                    const uint32_t* __restrict__ roff, uint32_t* __restrict__ rcur,
-                                    uint32_t* __restrict__ rbuf) {
-  uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) update_lists_kernel(
+    uint64_t n, uint32_t P, uint32_t cap, const float* __restrict__ pd, uint32_t* __restrict__ pid,
+    const uint32_t* __restrict__ Range, const float* __restrict__ radiusM, uint32_t* __restrict__ new_ids,
+    uint32_t* __restrict__ new_cnt, uint32_t* __restrict__ old_ids, uint32_t* __restrict__ old_cnt,
+    uint32_t* __restrict__ rcnt, const uint32_t* __restrict__ roff, uint32_t* __restrict__ rcur,
+    uint32_t* __restrict__ rbuf) {
+  const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1;
   if (t >= n) return;
-  uint64_t row = t * P;
-  uint32_t R = Range[t];
+  const uint64_t row = t * P;
+  const uint32_t R = Range[t];
   uint32_t cn = 0, co = 0;
-  for (uint32_t l = 0; l < R; ++l) {
-    uint32_t v = pid[row + l];
-    uint32_t id = v & IDM;
-    float d = pd[row + l];
-    bool rev = d > radiusM[id];
-    if (v & FLAG) {
-      if (PASS == 0) {
-        new_ids[t * cap + cn] = id;
-        if (rev) atomicAdd(&rcnt[id], 1u);
-      } else {
-        if (rev) rbuf[roff[id] + atomicAdd(&rcur[id], 1u)] = (uint32_t)t;
-        pid[row + l] = id;  // flag cleared
-      }
-      ++cn;
+  for (uint32_t l0 = 0; l0 < R; l0 += 32) {
+    const uint32_t l = l0 + lane;
+    const bool in = l < R;
+    const uint32_t v = in ? pid[row + l] : 0u, id = v & IDM;
+    const bool isnew = in && (v & FLAG), isold = in && !(v & FLAG);
+    const bool rev = in && pd[row + l] > radiusM[id];
+    const uint64_t slot = isnew ? id : n + id;  // the target's new or old reverse list
+    if (PASS == 0) {
+      const uint32_t bn = __ballot_sync(0xffffffffu, isnew), bo = __ballot_sync(0xffffffffu, isold);
+      if (isnew) new_ids[t * cap + cn + __popc(bn & below)] = id;
+      if (isold) old_ids[t * cap + co + __popc(bo & below)] = id;
+      cn += __popc(bn);
+      co += __popc(bo);
+      if (rev) atomicAdd(&rcnt[slot], 1u);
     } else {
-      if (PASS == 0) {
-        old_ids[t * cap + co] = id;
-        if (rev) atomicAdd(&rcnt[n + id], 1u);
-      } else {
-        if (rev) rbuf[roff[n + id] + atomicAdd(&rcur[n + id], 1u)] = (uint32_t)t;
-      }
-      ++co;
+      if (rev) rbuf[roff[slot] + atomicAdd(&rcur[slot], 1u)] = (uint32_t)t;
+      if (isnew) pid[row + l] = id;  // flag cleared
     }
   }
-  if (PASS == 0) {
+  if (PASS == 0 && lane == 0) {
     new_cnt[t] = cn;
     old_cnt[t] = co;
   }
@@ -1110,10 +1235,16 @@ static int nnd_init_device(efg_index* idx, NNDev& S) {
     EFG_TRY(task_leaf.reserve(ntasks));
     EFG_TRY(task_d.reserve(ntasks * maxl));
   }
+  EFG_TRY(make_bytes(idx));
+  ByteRows br{nullptr, nullptr, 0, 0};
+  if (idx->bytes_state == 1) {
+    br = ByteRows{idx->bytes.p, idx->bnorm.p, idx->ldb / 16, 0};
+    while ((1u << br.gshift) < br.chunks) ++br.gshift;
+  }
   if (ntasks) {
-    merge_route_kernel<0><<<rgrid, 256, 0, s>>>(idx->d_base, ld4, tv, S.off64.p, F.nnodes, ntasks, S.cnt.p,
-                                                 nullptr, nullptr, nullptr, nd.p, task_p.p, task_leaf.p, task_d.p,
-                                                 maxl);
+    auto route = br.rows ? merge_route_kernel<0, true> : merge_route_kernel<0, false>;
+    route<<<rgrid, 256, 0, s>>>(idx->d_base, ld4, br, tv, S.off64.p, F.nnodes, ntasks, S.cnt.p, nullptr, nullptr,
+                                nullptr, nd.p, task_p.p, task_leaf.p, task_d.p, maxl);
     EFG_CUDA(cudaGetLastError());
   }
   widen_kernel<<<blocks_for(n, 256), 256, 0, s>>>(S.cnt.p, cnt64.p, n);
@@ -1131,9 +1262,9 @@ static int nnd_init_device(efg_index* idx, NNDev& S) {
         tv, ntasks, task_p.p, task_leaf.p, task_d.p, maxl, off64.p, S.cursor.p, S.rec_key.p);
     EFG_CUDA(cudaGetLastError());
   } else if (ntasks) {
-    merge_route_kernel<1><<<rgrid, 256, 0, s>>>(idx->d_base, ld4, tv, S.off64.p, F.nnodes, ntasks, nullptr,
-                                                off64.p, S.cursor.p, S.rec_key.p, nullptr, nullptr, nullptr, nullptr,
-                                                0);
+    auto route = br.rows ? merge_route_kernel<1, true> : merge_route_kernel<1, false>;
+    route<<<rgrid, 256, 0, s>>>(idx->d_base, ld4, br, tv, S.off64.p, F.nnodes, ntasks, nullptr, off64.p, S.cursor.p,
+                                S.rec_key.p, nullptr, nullptr, nullptr, nullptr, 0);
     EFG_CUDA(cudaGetLastError());
   }
   init_select_kernel<<<blocks_for(n * 32, 256), 256, 0, s>>>(
@@ -1292,7 +1423,7 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   EFG_TRY(S.scan32.reserve(scan_tmp_elems<uint32_t>(2 * n) + 1));
   EFG_CUDA(cudaMemsetAsync(S.rcnt.p, 0, 2 * n * 4, s));
   EFG_CUDA(cudaMemsetAsync(S.rcur.p, 0, 2 * n * 4, s));
-  update_lists_kernel<0><<<blocks_for(n, 128), 128, 0, s>>>(n, S.P, S.cap, S.pd.p, S.pid.p, S.Range.p, S.radiusM.p,
+  update_lists_kernel<0><<<blocks_for(n * 32, 256), 256, 0, s>>>(n, S.P, S.cap, S.pd.p, S.pid.p, S.Range.p, S.radiusM.p,
                                                             S.new_ids.p, S.new_cnt.p, S.old_ids.p, S.old_cnt.p,
                                                             S.rcnt.p, nullptr, nullptr, nullptr);
   EFG_CUDA(cudaGetLastError());
@@ -1301,7 +1432,7 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   EFG_CUDA(cudaMemcpyAsync(&nrev, S.roff.p + 2 * n, 4, cudaMemcpyDeviceToHost, s));
   EFG_CUDA(cudaStreamSynchronize(s));
   EFG_TRY(S.rbuf.reserve((uint64_t)nrev + 1));
-  update_lists_kernel<1><<<blocks_for(n, 128), 128, 0, s>>>(n, S.P, S.cap, S.pd.p, S.pid.p, S.Range.p, S.radiusM.p,
+  update_lists_kernel<1><<<blocks_for(n * 32, 256), 256, 0, s>>>(n, S.P, S.cap, S.pd.p, S.pid.p, S.Range.p, S.radiusM.p,
                                                             S.new_ids.p, S.new_cnt.p, S.old_ids.p, S.old_cnt.p,
                                                             S.rcnt.p, S.roff.p, S.rcur.p, S.rbuf.p);
   EFG_CUDA(cudaGetLastError());
