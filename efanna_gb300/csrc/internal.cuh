@@ -192,11 +192,11 @@ int tc_join(const __nv_bfloat16* hi, const __nv_bfloat16* lo, const float* norms
             const RecordSink& sink, uint8_t* found, uint32_t* counters, uint32_t* mid, uint32_t* big,
             unsigned long long* nlarge, int* err, uint32_t step, uint32_t skip, cudaStream_t s);
 // join_fp32.cu: the NN-descent join in FP32 over the nodes k * step (skip 0) or the others (skip 1);
-// counter: a node counter, zero on entry.
+// counters: two node counters, zero on entry; big: n + 1 words, word 0 zero on entry.
 int join_fp32(const float* base, uint64_t n, uint32_t ld, uint32_t cap, uint32_t P, uint32_t check_k,
               const uint32_t* new_ids, const uint32_t* new_cnt, const uint32_t* old_ids, const uint32_t* old_cnt,
-              const float* bound, const RecordSink& sink, uint8_t* found, uint32_t* counter, uint32_t step,
-              uint32_t skip, cudaStream_t s);
+              const float* bound, const RecordSink& sink, uint8_t* found, uint32_t* counters, uint32_t* big,
+              uint32_t step, uint32_t skip, cudaStream_t s);
 // bytes.cu: the byte rows of an index's base, where it has them (idx->bytes_state == 1 afterwards), and
 // the join over byte rows, with the FP32 join's records.
 int make_bytes(efg_index* idx);

@@ -55,7 +55,7 @@ struct NNDev {
   DevBuf<__nv_bfloat16> jhi, jlo;
   DevBuf<float> jnorm;
   DevBuf<int> jflag;  // inexact, error, not integers
-  DevBuf<uint32_t> jmid, jbig;  // nodes of 129-256 rows, and larger ones (count in word 0)
+  DevBuf<uint32_t> jmid, jbig;  // nodes of 129-256 rows, and larger ones (FP32: of many pairs); count in word 0
   uint32_t jterms = 0;  // 0: not prepared; 1 or 3 products per value
   bool jexact = false;  // the tensor cores' distances are exact (integers, squared norms below 2^22)
   uint32_t W = 0;          // records per bucket
@@ -1305,7 +1305,6 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
     EFG_TRY(S.jnorm.reserve(n));
     EFG_TRY(S.jflag.reserve(3));
     EFG_TRY(S.jmid.reserve(n + 1));
-    EFG_TRY(S.jbig.reserve(n + 1));
     EFG_TRY(tc_join_prepare(idx->d_base, n, idx->dim, idx->ld, S.jhi.p, S.jlo.p, S.jnorm.p, S.jflag.p, s));
     int inexact[3] = {0, 0, 0};
     EFG_CUDA(cudaMemcpyAsync(inexact, S.jflag.p, 12, cudaMemcpyDeviceToHost, s));
@@ -1348,11 +1347,12 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
       if (!tc && idx->bytes_state == 1)
         return join_bytes(idx->bytes.p, idx->bnorm.p, n, idx->ldb, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p,
                           S.old_ids.p, S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, step, skip, s);
+      EFG_TRY(S.jbig.reserve(n + 1));
+      EFG_CUDA(cudaMemsetAsync(S.jbig.p, 0, 4, s));
       if (!tc)
         return join_fp32(idx->d_base, n, idx->ld, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p, S.old_ids.p,
-                         S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, step, skip, s);
+                         S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, S.jbig.p, step, skip, s);
       EFG_CUDA(cudaMemsetAsync(S.jmid.p, 0, 4, s));
-      EFG_CUDA(cudaMemsetAsync(S.jbig.p, 0, 4, s));
       return tc_join(S.jhi.p, S.jlo.p, S.jnorm.p, n, idx->dim, S.jterms, S.cap, S.P, bp.check_k, S.new_ids.p,
                      S.new_cnt.p, S.old_ids.p, S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, S.jmid.p,
                      S.jbig.p, S.totals.p + 3, S.jflag.p + 1, step, skip, s);
