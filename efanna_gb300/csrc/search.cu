@@ -315,6 +315,15 @@ int launch_nnexp(efg_index* idx, SearchCfg cfg, uint32_t maxdeg, const float* d_
   if (cfg.T > 256) return fail(EFG_ERR_ARG, "at most 256 search trees");
   if (cfg.lsize >= 65536) return fail(EFG_ERR_ARG, "pool too large for the tree descent");
   cfg.emit_pool = d_keys ? 1 : 0;
+  if (!cfg.screened && !cfg.fp8) {  // FP32: over byte rows where the base has them
+    EFG_TRY(make_bytes(idx));
+    if (idx->bytes_state == 1) {
+      cfg.bytes = 1;
+      cfg.cprb = idx->ldb / 16;
+      cfg.gshiftb = 0;
+      while ((1u << cfg.gshiftb) < cfg.cprb) ++cfg.gshiftb;
+    }
+  }
   cfg.fixed_k = idx->graph.fixed_k >= 2 ? idx->graph.fixed_k : 0;
   if (cfg.fixed_k) {
     // item r * K + c -> (r, c) by a multiply-high: exact while items * K < 2^32
@@ -400,14 +409,14 @@ int launch_nnexp(efg_index* idx, SearchCfg cfg, uint32_t maxdeg, const float* d_
       idx->d_base, idx->n, idx->dim, idx->ld, F.nodes.p, F.nleaf.p, F.cnl.p, F.d_roots.p, F.leaves.p, idx->graph.ptr.p,
       idx->graph.ids.p, d_q, nq, qld, c1, d_out, idx->eval_counter.p, idx->ht_scratch.p, nullptr,
       two_pass ? idx->ovf_list.p : nullptr, idx->base16.p, d_keys, d_params, d_nq, d_seeds, idx->base8.p,
-      idx->scale8.p);
+      idx->scale8.p, idx->bytes.p);
   cudaError_t le = cudaGetLastError();
   *launches = 1;
   if (le == cudaSuccess && two_pass) {
     kernel<<<(unsigned)grid2, threads, smem2, s>>>(
         idx->d_base, idx->n, idx->dim, idx->ld, F.nodes.p, F.nleaf.p, F.cnl.p, F.d_roots.p, F.leaves.p, idx->graph.ptr.p,
         idx->graph.ids.p, d_q, nq, qld, c2, d_out, idx->eval_counter.p, idx->ht_scratch.p, idx->ovf_list.p, nullptr,
-        idx->base16.p, d_keys, d_params, d_nq, d_seeds, idx->base8.p, idx->scale8.p);
+        idx->base16.p, d_keys, d_params, d_nq, d_seeds, idx->base8.p, idx->scale8.p, idx->bytes.p);
     le = cudaGetLastError();
     *launches = 2;
   }

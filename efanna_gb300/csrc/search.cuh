@@ -27,6 +27,9 @@ struct SearchCfg {
   // FP8 (e4m3, one FP32 scale per row) screening instead of BF16: rows ld8 bytes apart, cpr8
   // 16-byte chunks per row, 2^gshift8 lanes per row
   uint32_t fp8, ld8, cpr8, gshift8;
+  // byte rows (exact integer distances for queries that are bytes too): rows cprb 16-byte chunks long,
+  // 2^gshiftb lanes per row in the gather; the query's bytes at o_qb
+  uint32_t bytes, cprb, gshiftb, o_qb;
   uint32_t emit_pool;   // stop after the pool and write its keys (kgraph's first stage)
   uint32_t fixed_k;     // graph degree when every row has it (0: row pointers), and
   uint32_t kmagic;      // ceil(2^32 / fixed_k) for the division of item indices
