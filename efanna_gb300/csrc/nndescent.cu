@@ -908,10 +908,11 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_kernel(
     __syncwarp();
 
     uint32_t tlo = 0;  // every record below these distance bits is done
-    bool stop = false;
+    bool stop = false, ties = false, first = true;  // ties: more than WIN records at distance bits tlo
+    K96 last{0, 0};
     while (!stop) {
       uint32_t thi = 0xffffffffu, total = B;
-      if (B > WIN || tlo) {
+      if (!ties && (B > WIN || tlo)) {
         uint32_t mn = 0xffffffffu, mx = 0;
         total = 0;
         for (uint32_t b = lane; b < B; b += 32) {
@@ -946,52 +947,56 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_kernel(
               chi = c;
             }
           }
-          if (clo == 0) {  // more than WIN records at distance bits lo
-            K96 last{0, 0};
-            for (bool first = true; !stop; first = false) {
-              const K96 batch = next_batch(rec, B, lo, last, first);
-              const uint32_t m = __popc(__ballot_sync(0xffffffffu, !is_max(batch)));
-              if (m == 0) break;
-              stop = pool.apply_batch(batch, m);
-              last = shfl_idx(batch, m - 1);
-            }
-            tlo = lo + 1;
-            continue;
-          }
           thi = lo;
           total = clo;
+          ties = clo == 0;
+          if (ties) tlo = lo;
         }
       }
-      // the records of [tlo, thi), sorted
-      if (tlo == 0 && thi == 0xffffffffu) {
-        for (uint32_t b = lane; b < B; b += 32) {
-          const K96 y = rec_k96(rec[b]);
-          wk[b] = y.k;
-          wa[b] = y.a;
+      if (ties) {  // the next 32 of them
+        const K96 batch = next_batch(rec, B, tlo, last, first);
+        total = __popc(__ballot_sync(0xffffffffu, !is_max(batch)));
+        first = total == 0;
+        if (first) {
+          ties = false;
+          ++tlo;
+          continue;
         }
-      } else {
-        uint32_t at = 0;
-        for (uint32_t b = 0; b < B; b += 32) {
-          const uint4 q = b + lane < B ? rec[b + lane] : make_uint4(0, 0xffffffffu, 0, 0);
-          const bool take = b + lane < B && q.y >= tlo && q.y < thi;
-          const uint32_t bal = __ballot_sync(0xffffffffu, take);
-          if (take) {
-            const uint32_t o = at + __popc(bal & below);
-            wk[o] = rec_key(q);
-            wa[o] = q.z;
+        last = shfl_idx(batch, total - 1);
+        wk[lane] = batch.k;
+        wa[lane] = batch.a;
+        __syncwarp();
+      } else {  // the records of [tlo, thi), sorted
+        if (tlo == 0 && thi == 0xffffffffu) {
+          for (uint32_t b = lane; b < B; b += 32) {
+            const K96 y = rec_k96(rec[b]);
+            wk[b] = y.k;
+            wa[b] = y.a;
           }
-          at += __popc(bal);
+        } else {
+          uint32_t at = 0;
+          for (uint32_t b = 0; b < B; b += 32) {
+            const uint4 q = b + lane < B ? rec[b + lane] : make_uint4(0, 0xffffffffu, 0, 0);
+            const bool take = b + lane < B && q.y >= tlo && q.y < thi;
+            const uint32_t bal = __ballot_sync(0xffffffffu, take);
+            if (take) {
+              const uint32_t o = at + __popc(bal & below);
+              wk[o] = rec_key(q);
+              wa[o] = q.z;
+            }
+            at += __popc(bal);
+          }
         }
+        __syncwarp();
+        if (WIN == 64 && total <= 32) sort_window<1>(wk, wa, total);
+        else if (total <= 64) sort_window<2>(wk, wa, total);
+        else if (WIN > 64) sort_window<(WIN > 64 ? 8 : 1)>(wk, wa, total);
       }
-      __syncwarp();
-      if (total <= 32) sort_window<1>(wk, wa, total);
-      else if (total <= 64) sort_window<2>(wk, wa, total);
-      else if (WIN > 64 && total <= 128) sort_window<(WIN > 64 ? 4 : 1)>(wk, wa, total);
-      else if (WIN > 64) sort_window<(WIN > 64 ? 8 : 1)>(wk, wa, total);
       for (uint32_t b = 0; b < total && !stop; b += 32) {
         const K96 batch = b + lane < total ? K96{wk[b + lane], wa[b + lane]} : k96_max();
         stop = pool.apply_batch(batch, min(32u, total - b));
       }
+      if (ties) continue;
       if (thi == 0xffffffffu) break;
       tlo = thi;
     }
