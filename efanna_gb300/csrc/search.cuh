@@ -15,6 +15,7 @@ struct SearchCfg {
   uint32_t ids_cap;     // candidate id buffer (u32 entries); on entry to layout(): a bound, 0 = none
   uint32_t res_cap;     // power of two >= result_size
   uint32_t nseq;        // T * lsize leaf slots
+  uint32_t tconc;       // trees a warp descends at a time
   // shared-memory byte offsets
   uint32_t o_ids, o_ht, o_u;
   uint32_t o_lstart, o_seqoff, o_tkey, o_tpos;  // fill phase (absolute)
