@@ -84,62 +84,51 @@ __device__ __forceinline__ bool ht_insert(uint32_t* ht, uint32_t size, uint32_t 
   atomicOr(ovf, 1u);
   return false;
 }
-// ht_insert continued from slot h after `done` probes of id's sequence.
-__device__ __forceinline__ bool ht_insert_from(uint32_t* ht, uint32_t size, uint32_t limit, uint32_t* count,
-                                               uint32_t* ovf, uint32_t id, uint32_t h, uint32_t done) {
-  const uint32_t st = ht_step(id, size);
-  for (uint32_t probe = done; probe < size; ++probe) {
-    uint32_t cur = *reinterpret_cast<volatile const uint32_t*>(&ht[h]);
-    if (cur == kEmpty) {
-      if (*reinterpret_cast<volatile uint32_t*>(count) >= limit) {
-        atomicOr(ovf, 1u);
-        return false;
-      }
-      uint32_t prev = atomicCAS(&ht[h], kEmpty, id);
-      if (prev == kEmpty) return true;
-      cur = prev;
-    }
-    if ((cur & ID_MASK) == id) return false;
-    h = ht_next(h, st, size);
-  }
-  atomicOr(ovf, 1u);
-  return false;
-}
-
-// XR inserts of one thread with their first probes issued together: the first slots' loads, then
-// the compare-and-swaps of the ids whose first slot was empty, then (rarely) the rest of a probe
-// sequence.  The same outcome as XR ht_insert calls in order: an id met twice in the batch takes
-// its slot once (the second CAS returns the first's id).  kEmpty entries are skipped.
+// XR inserts of one thread into a table in shared memory, their probe sequences advanced together and
+// without branches (loads and compare-and-swaps are predicated), until the warp's last one is settled:
+// as branches, each lane's probe sequences ran one after another (1024 inserts by 256 threads at half
+// to two-thirds load: 4300 cycles, 2700 this way).  The same outcome as XR ht_insert calls: an id met
+// twice takes its slot once.  kEmpty entries are skipped.  Called by whole warps.
 template <int XR>
 __device__ __forceinline__ void ht_insert_batch(uint32_t* ht, uint32_t size, uint32_t limit, uint32_t* count,
                                                 uint32_t* ovf, const uint32_t (&id)[XR], bool (&fresh)[XR]) {
-  uint32_t h[XR], cur[XR], prev[XR];
-#pragma unroll
-  for (int u = 0; u < XR; ++u) h[u] = id[u] != kEmpty ? ht_slot(id[u], size) : 0u;
-#pragma unroll
-  for (int u = 0; u < XR; ++u) cur[u] = id[u] != kEmpty ? *reinterpret_cast<volatile const uint32_t*>(&ht[h[u]]) : 0u;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(ht);
+  uint32_t at[XR], step[XR], act[XR];
   const bool full = *reinterpret_cast<volatile uint32_t*>(count) >= limit;
 #pragma unroll
-  for (int u = 0; u < XR; ++u)
-    prev[u] = (id[u] != kEmpty && cur[u] == kEmpty && !full) ? atomicCAS(&ht[h[u]], kEmpty, id[u]) : cur[u];
-#pragma unroll
   for (int u = 0; u < XR; ++u) {
+    at[u] = ht_slot(id[u], size);
+    step[u] = ht_step(id[u], size);
+    act[u] = id[u] != kEmpty ? 1u : 0u;
     fresh[u] = false;
-    if (id[u] == kEmpty) continue;
-    uint32_t c = cur[u];
-    if (c == kEmpty) {
-      if (full) {
-        atomicOr(ovf, 1u);
-        continue;
-      }
-      if (prev[u] == kEmpty) {
-        fresh[u] = true;
-        continue;
-      }
-      c = prev[u];
+  }
+  bool any = true;
+  for (uint32_t probe = 0; any && probe < size; ++probe) {
+    uint32_t c[XR];
+#pragma unroll
+    for (int u = 0; u < XR; ++u)
+      asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(c[u]) : "r"(base + at[u] * 4) : "memory");
+    bool mine = false, none = false;
+#pragma unroll
+    for (int u = 0; u < XR; ++u) {
+      const uint32_t want = act[u] && c[u] == kEmpty && !full ? 1u : 0u;
+      none |= act[u] && c[u] == kEmpty && full;
+      asm volatile("{.reg .pred p; setp.ne.u32 p, %4, 0; @p atom.shared.cas.b32 %0, [%1], %2, %3;}"
+                   : "+r"(c[u])
+                   : "r"(base + at[u] * 4), "r"(kEmpty), "r"(id[u]), "r"(want)
+                   : "memory");
     }
-    if ((c & ID_MASK) == id[u]) continue;
-    fresh[u] = ht_insert_from(ht, size, limit, count, ovf, id[u], ht_next(h[u], ht_step(id[u], size), size), 1);
+    if (none) atomicOr(ovf, 1u);
+#pragma unroll
+    for (int u = 0; u < XR; ++u) {
+      const bool won = act[u] && c[u] == kEmpty && !full;  // (c[u] is now what the slot held before)
+      fresh[u] |= won;
+      act[u] = act[u] && c[u] != kEmpty && c[u] != id[u] ? 1u : 0u;
+      const uint32_t n = ht_next(at[u], step[u], size);
+      at[u] = act[u] ? n : at[u];
+      mine |= act[u] != 0;
+    }
+    any = __any_sync(0xffffffffu, mine);
   }
 }
 
@@ -345,6 +334,32 @@ int launch_nnexp(efg_index* idx, SearchCfg cfg, uint32_t maxdeg, const float* d_
     small = std::max<uint64_t>(2048, nice(small * (uint64_t)idx->search_ht_pct / 100));
   small = std::min(small, big);
   if (big > (1ull << 28)) return fail(EFG_ERR_ARG, "search parameters visit too many candidates");
+  int dev = 0, sms = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  auto two_fit = [&](const SearchCfg& c) -> bool {  // two 256-thread CTAs on an SM
+    SearchCfg t = c;
+    const size_t need = s256::layout(t, idx->ld, maxdeg, false, (uint32_t)small);
+    int fit = 0;
+    if (need > 113 * 1024 ||
+        cudaFuncSetAttribute(s256::nnexp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need) != cudaSuccess)
+      return false;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, s256::nnexp_kernel, 256, need);
+    return fit >= 2;
+  };
+  // The visited set as a bitmap of the base -- an atomic OR per insert, nothing to probe and nothing to
+  // outgrow -- where it costs no CTA: two fit on an SM with it (a plan's 256 queries at 400k rows 177 us,
+  // with the table 199 us; 777 queries at 61k x 101 299 us, 344 us), or only one does with the table too
+  // (2000 queries at 100k x 960, degree 100: 3.8 ms, 6.5 ms), or there is no more than one query per SM
+  // (one query at 1M x 128: 106 us, 139 us).  Else two CTAs with the table are the faster (10k queries at
+  // 1M x 128: 7.75 ms against 8.09 ms), and settings that expect to visit more ids than the base has
+  // stay with it: they are the ones its hand-over to global scratch is for.
+  {
+    SearchCfg t = cfg, w = cfg;
+    t.bits = w.bits = (uint32_t)round_up((idx->n + 31) / 32, 4);
+    const bool one_fits = s512::layout(w, idx->ld, maxdeg, false, 0) <= 200 * 1024;
+    if (two_fit(t) || (one_fits && (nq <= (uint64_t)sms || (!two_fit(cfg) && expect <= idx->n)))) cfg.bits = t.bits;
+  }
   // block size: 256 threads when several CTAs fit on an SM, else 512 threads
   int per_sm = 1;
   size_t smem_probe;
@@ -366,7 +381,7 @@ int launch_nnexp(efg_index* idx, SearchCfg cfg, uint32_t maxdeg, const float* d_
   c1.ht_soft = c1.ht_limit;
   size_t smem2 = layout(c2, idx->ld, maxdeg, true, (uint32_t)big);
   c2.ht_limit = (uint32_t)big;
-  bool two_pass = big > small;
+  bool two_pass = !cfg.bits && big > small;
   if (smem1 > 200 * 1024) {  // the reduced set does not fit beside the rest: one pass, global set
     c1 = c2;
     smem1 = smem2;
@@ -376,9 +391,6 @@ int launch_nnexp(efg_index* idx, SearchCfg cfg, uint32_t maxdeg, const float* d_
     return fail(EFG_ERR_ARG, "search parameters need " + std::to_string(smem1) +
                                  " bytes of shared memory per query (pool/extend/degree too large)");
   EFG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(smem1, smem2)));
-  int dev = 0, sms = 152;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem1);
   if (idx->search_ctas_per_sm > 0) per_sm = std::min(per_sm, idx->search_ctas_per_sm);
   uint64_t grid1 = std::min<uint64_t>(nq, (uint64_t)sms * std::max(1, per_sm));
