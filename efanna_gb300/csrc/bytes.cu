@@ -240,7 +240,7 @@ int make_bytes(efg_index* idx) {
   int dev = 0, sms = 152;
   EFG_CUDA(cudaGetDevice(&dev));
   EFG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  LocalBuf<int> flag;
+  LocalBuf<int> flag(idx->stream);
   EFG_TRY(flag.reserve(1));
   EFG_CUDA(cudaMemsetAsync(flag.p, 0, 4, idx->stream));
   // a thin sample first: other data are known by it

@@ -9,27 +9,43 @@
 
 namespace efg {
 
-// A device buffer that grows on demand (never shrinks until freed).
+// A device buffer that grows on demand (never shrinks until freed).  On a stream (on()), memory up to
+// POOL_MAX comes from the device's stream-ordered pool and goes back there: for scratch that only that
+// stream uses.  A build's 50 buffers cost 0.04 ms each to allocate with cudaMalloc and as much to free;
+// blocks of gigabytes are the faster with it (0.3 ms and 0.5 ms per GB; from the pool, which gives its
+// memory back at the next synchronisation, twice that).
 template <typename T>
 struct DevBuf {
+  static constexpr size_t POOL_MAX = 32u << 20, SLACK_MAX = 64u << 20;  // bytes
   T* p = nullptr;
   size_t cap = 0;  // elements
+  cudaStream_t stream = nullptr;
+  bool pooled = false, from_pool = false;
+  void on(cudaStream_t s) {
+    release();
+    stream = s;
+    pooled = true;
+  }
   int reserve(size_t n) {
     if (n <= cap) return EFG_OK;
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
-    size_t want = n + n / 8 + 64;
-    cudaError_t e = cudaMalloc((void**)&p, want * sizeof(T));
+    release();
+    const size_t want = n + (n / 8 < SLACK_MAX / sizeof(T) ? n / 8 : SLACK_MAX / sizeof(T)) + 64;
+    from_pool = pooled && want * sizeof(T) <= POOL_MAX;
+    cudaError_t e = from_pool ? cudaMallocAsync((void**)&p, want * sizeof(T), stream)
+                              : cudaMalloc((void**)&p, want * sizeof(T));
     if (e != cudaSuccess) {
       cudaGetLastError();
-      return fail(EFG_ERR_NOMEM, "cudaMalloc of " + std::to_string(want * sizeof(T)) + " bytes failed");
+      p = nullptr;
+      return fail(EFG_ERR_NOMEM, "allocation of " + std::to_string(want * sizeof(T)) + " device bytes failed");
     }
     cap = want;
     return EFG_OK;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p) {
+      if (from_pool) cudaFreeAsync(p, stream);
+      else cudaFree(p);
+    }
     p = nullptr;
     cap = 0;
   }
@@ -62,6 +78,7 @@ struct ScopedEvents {
 template <typename T>
 struct LocalBuf : DevBuf<T> {
   LocalBuf() = default;
+  explicit LocalBuf(cudaStream_t s) { this->on(s); }
   LocalBuf(const LocalBuf&) = delete;
   LocalBuf& operator=(const LocalBuf&) = delete;
   ~LocalBuf() { this->release(); }

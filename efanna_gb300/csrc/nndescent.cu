@@ -44,7 +44,6 @@ struct NNDev {
   DevBuf<uint8_t> found;
   // scratch
   DevBuf<uint64_t> task_len, off64, scan64;
-  DevBuf<uint64_t> rec_key;  // leaf merge: records per target
   DevBuf<uint32_t> cnt, cursor, rcnt, rcur, roff, rbuf, scan32;
   DevBuf<float> bound;
   DevBuf<unsigned long long> totals;  // pairs, records, overflow records, nodes larger than a tile
@@ -60,16 +59,21 @@ struct NNDev {
   bool jexact = false;  // the tensor cores' distances are exact (integers, squared norms below 2^22)
   uint32_t W = 0;          // records per bucket
   uint64_t bucket_cap = 0, ovf_cap = 0;
-  void release_all() {
-    pd.release(); radius.release(); radiusM.release(); pid.release(); Lc.release(); Range.release();
-    new_ids.release(); new_cnt.release(); old_ids.release(); old_cnt.release(); found.release();
-    task_len.release(); off64.release(); scan64.release(); cnt.release(); cursor.release(); bound.release();
-    rcnt.release(); rcur.release(); roff.release(); rbuf.release(); scan32.release(); totals.release();
-    jctr.release(); bucket.release(); ovf.release(); ovfrec.release(); ovf_slot.release();
-    rec_key.release(); jhi.release(); jlo.release(); jnorm.release(); jflag.release();
-    jmid.release();
-    jbig.release();
-    jterms = 0;
+  // every buffer from the stream's pool: only the build's stream uses them
+  explicit NNDev(cudaStream_t s) {
+    each([s](auto& b) { b.on(s); });
+  }
+  ~NNDev() {
+    each([](auto& b) { b.release(); });
+  }
+  NNDev(const NNDev&) = delete;
+  NNDev& operator=(const NNDev&) = delete;
+  template <typename F>
+  void each(F f) {
+    auto all = [&](auto&... b) { (f(b), ...); };
+    all(pd, radius, radiusM, pid, Lc, Range, new_ids, new_cnt, old_ids, old_cnt, found, task_len, off64, scan64,
+        cnt, cursor, bound, rcnt, rcur, roff, rbuf, scan32, totals, jctr, bucket, ovf, ovfrec, ovf_slot,
+        jhi, jlo, jnorm, jflag, jmid, jbig);
   }
 };
 
@@ -1167,7 +1171,7 @@ __global__ void widen_kernel(const uint32_t* __restrict__ in, uint64_t* __restri
 static int merge_level_check(efg_index* idx, int32_t* min_level) {
   Forest& F = idx->forest;
   TreeView tv{F.nodes.p, F.n_left.p, F.n_right.p, F.n_level.p, F.n_tree.p, F.n_start.p, F.n_end.p, F.leaves.p, F.n};
-  LocalBuf<int32_t> d;
+  LocalBuf<int32_t> d(idx->stream);
   EFG_TRY(d.reserve(1));
   int32_t big = 0x7fffffff;
   EFG_CUDA(cudaMemcpyAsync(d.p, &big, 4, cudaMemcpyHostToDevice, idx->stream));
@@ -1175,8 +1179,35 @@ static int merge_level_check(efg_index* idx, int32_t* min_level) {
   EFG_CUDA(cudaGetLastError());
   EFG_CUDA(cudaMemcpyAsync(min_level, d.p, 4, cudaMemcpyDeviceToHost, idx->stream));
   EFG_CUDA(cudaStreamSynchronize(idx->stream));
-  d.release();
   return EFG_OK;
+}
+
+// Records of a first join per node, on average (every pair of the seeded lists is kept: 2 S entries),
+// and whether the first join runs in two parts (1 of FIRST_PART nodes, then the others).
+constexpr uint32_t FIRST_PART = 8;
+static uint64_t first_mean(const efg_build_params& bp) { return 2ull * bp.S * (2 * bp.S - 1); }
+static bool first_in_parts(const efg_build_params& bp, uint32_t P, bool exact) {
+  return exact && P <= TIGHTEN_MAX_P && first_mean(bp) / FIRST_PART + bp.S >= P + P / 4;
+}
+
+// Bucket width: about the records a node receives in the first join, or five pools' worth where pools
+// are large (later joins then bring more), then (see the end of an iteration) three times the last
+// iteration's mean as far as the buffer reaches -- it grows only when the mean itself nears its width:
+// a GB costs about 0.8 ms to allocate and free, more than some overflowing hubs do -- within a quarter
+// of the memory free at the start; the rest goes to the overflow list.
+static int first_width(efg_index* idx, NNDev& S) {
+  if (S.W) return EFG_OK;
+  const efg_build_params& bp = idx->bp;
+  size_t free_b = 0, total_b = 0;
+  EFG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  S.bucket_cap = std::max<uint64_t>(1, (uint64_t)free_b / 4 / sizeof(uint4) / S.n);
+  const uint64_t mean = first_mean(bp);
+  const uint64_t expect = first_in_parts(bp, S.P, true) ? mean / FIRST_PART + 8 * S.P
+                                                        : std::max<uint64_t>(mean + mean / 4, S.P > 64 ? 5 * S.P : 0);
+  S.W = (uint32_t)std::min<uint64_t>(S.bucket_cap, expect + 32);
+  S.ovf_cap = std::max<uint64_t>(S.n * (expect / 4 + 8), 1 << 16);
+  EFG_TRY(S.ovf.reserve(S.ovf_cap));
+  return S.ovf_slot.reserve(S.ovf_cap);
 }
 
 static int nnd_init_device(efg_index* idx, NNDev& S) {
@@ -1211,10 +1242,10 @@ static int nnd_init_device(efg_index* idx, NNDev& S) {
   // per-target record counts -> offsets
   EFG_TRY(S.cnt.reserve(n));
   EFG_TRY(S.cursor.reserve(n));
-  LocalBuf<uint64_t> cnt64, off64;
+  LocalBuf<uint64_t> cnt64(s), off64(s);
   EFG_TRY(cnt64.reserve(n));
   EFG_TRY(off64.reserve(n + 1));
-  LocalBuf<unsigned long long> nd;
+  LocalBuf<unsigned long long> nd(s);
   EFG_TRY(nd.reserve(1));
   EFG_CUDA(cudaMemsetAsync(S.cnt.p, 0, n * 4, s));
   EFG_CUDA(cudaMemsetAsync(S.cursor.p, 0, n * 4, s));
@@ -1224,7 +1255,7 @@ static int nnd_init_device(efg_index* idx, NNDev& S) {
   // that stays within 4 GiB; otherwise pass 1 routes again)
   uint32_t maxl = 0;
   {
-    LocalBuf<uint32_t> ml;
+    LocalBuf<uint32_t> ml(s);
     EFG_TRY(ml.reserve(1));
     EFG_CUDA(cudaMemsetAsync(ml.p, 0, 4, s));
     max_leaf_kernel<<<blocks_for(F.nnodes, 256), 256, 0, s>>>(tv, F.nnodes, ml.p);
@@ -1232,9 +1263,9 @@ static int nnd_init_device(efg_index* idx, NNDev& S) {
     EFG_CUDA(cudaStreamSynchronize(s));
   }
   const bool keep = ntasks && maxl && ntasks * (uint64_t)(maxl + 2) * 4 <= (4ull << 30);
-  LocalBuf<uint32_t> task_p;
-  LocalBuf<int32_t> task_leaf;
-  LocalBuf<float> task_d;
+  LocalBuf<uint32_t> task_p(s);
+  LocalBuf<int32_t> task_leaf(s);
+  LocalBuf<float> task_d(s);
   if (keep) {
     EFG_TRY(task_p.reserve(ntasks));
     EFG_TRY(task_leaf.reserve(ntasks));
@@ -1261,25 +1292,25 @@ static int nnd_init_device(efg_index* idx, NNDev& S) {
   EFG_CUDA(cudaMemcpyAsync(&ndist, nd.p, 8, cudaMemcpyDeviceToHost, s));
   EFG_CUDA(cudaStreamSynchronize(s));
   idx->bstats.merge_distances = ndist;
-  EFG_TRY(S.rec_key.reserve(nrec + 1));
+  // the leaf merge's records in the join's bucket buffer, allocated once for both
+  EFG_TRY(first_width(idx, S));
+  EFG_TRY(S.bucket.reserve(std::max<uint64_t>(n * S.W, nrec / 2 + 1)));
+  uint64_t* rec_key_buf = reinterpret_cast<uint64_t*>(S.bucket.p);
   if (keep) {
     merge_emit_kernel<<<(unsigned)std::min<uint64_t>(blocks_for(ntasks, 256), 152ull * 64), 256, 0, s>>>(
-        tv, ntasks, task_p.p, task_leaf.p, task_d.p, maxl, off64.p, S.cursor.p, S.rec_key.p);
+        tv, ntasks, task_p.p, task_leaf.p, task_d.p, maxl, off64.p, S.cursor.p, rec_key_buf);
     EFG_CUDA(cudaGetLastError());
   } else if (ntasks) {
     auto route = br.rows ? merge_route_kernel<1, true> : merge_route_kernel<1, false>;
     route<<<rgrid, 256, 0, s>>>(idx->d_base, ld4, br, tv, S.off64.p, F.nnodes, ntasks, nullptr, off64.p, S.cursor.p,
-                                S.rec_key.p, nullptr, nullptr, nullptr, nullptr, 0);
+                                rec_key_buf, nullptr, nullptr, nullptr, nullptr, 0);
     EFG_CUDA(cudaGetLastError());
   }
   init_select_kernel<<<blocks_for(n * 32, 256), 256, 0, s>>>(
-      idx->d_base, ld4, n, bp.S, S.P, cap, bp.seed, S.cnt.p, off64.p, S.rec_key.p, S.pd.p, S.pid.p, S.Lc.p,
+      idx->d_base, ld4, n, bp.S, S.P, cap, bp.seed, S.cnt.p, off64.p, rec_key_buf, S.pd.p, S.pid.p, S.Lc.p,
       S.Range.p, S.radius.p, S.radiusM.p, S.found.p, S.new_ids.p, S.new_cnt.p, S.old_cnt.p);
   EFG_CUDA(cudaGetLastError());
   EFG_CUDA(cudaStreamSynchronize(s));
-  cnt64.release();
-  off64.release();
-  nd.release();
   return EFG_OK;
 }
 
@@ -1296,12 +1327,11 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   EFG_TRY(S.bound.reserve(n));
   EFG_TRY(S.totals.reserve(4));
   EFG_TRY(S.jctr.reserve(8));
-  // The first join keeps every pair of the seeded lists, mean = 2 S (2S - 1) records per node (380 for
+  // The first join keeps every pair of the seeded lists, 2 S (2S - 1) records per node (380 for
   // S = 10), of which a pool of P - 1 takes a few dozen.  So in FP32 it runs on 1 of `part` nodes first,
   // where that leaves about P entries per target, the targets' bounds are tightened, and the other
   // nodes follow: 1M x 128 keeps 221 records per node instead of 380.  (On the tensor cores only
   // where their distances are exact: else an id may be found at two distances, and would count twice.)
-  const uint64_t mean = 2ull * bp.S * (2 * bp.S - 1);
   const bool tc = idx->build_precision == EFG_PRECISION_BF16;
   if (tc && !S.jterms) {
     const uint64_t W = (idx->dim + 63) / 64 * 64;
@@ -1317,21 +1347,8 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
     S.jterms = inexact[0] ? 3 : 1;
     S.jexact = !inexact[0] && !inexact[2];
   }
-  const uint32_t part = iter == 0 && (!tc || S.jexact) && S.P <= TIGHTEN_MAX_P && mean / 8 + bp.S >= S.P + S.P / 4 ? 8 : 1;
-  // Bucket width: about the records a node receives in the first join, then three times the last
-  // iteration's mean (past the buffer's size only up to 4 GiB or when the mean itself nears its width:
-  // allocating costs about 1 ms per GB, more than a few overflowing hubs do), within a quarter of the
-  // memory free at the start; the rest goes to the overflow list.
-  if (!S.W) {
-    size_t free_b = 0, total_b = 0;
-    EFG_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    S.bucket_cap = std::max<uint64_t>(1, (uint64_t)free_b / 4 / sizeof(uint4) / n);
-    const uint64_t expect = part > 1 ? mean / part + 8 * S.P : mean + mean / 4;
-    S.W = (uint32_t)std::min<uint64_t>(S.bucket_cap, expect + 32);
-    S.ovf_cap = std::max<uint64_t>(n * (expect / 4 + 8), 1 << 16);
-    EFG_TRY(S.ovf.reserve(S.ovf_cap));
-    EFG_TRY(S.ovf_slot.reserve(S.ovf_cap));
-  }
+  const uint32_t part = iter == 0 && first_in_parts(bp, S.P, !tc || S.jexact) ? FIRST_PART : 1;
+  EFG_TRY(first_width(idx, S));
   EFG_TRY(S.bucket.reserve(n * S.W));
   int sms = 152, dev = 0;
   cudaGetDevice(&dev);
@@ -1448,7 +1465,7 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   unsigned long long nrec = 0;
   EFG_CUDA(cudaMemcpyAsync(&nrec, S.totals.p + 1, 8, cudaMemcpyDeviceToHost, s));
   EFG_CUDA(cudaStreamSynchronize(s));
-  const uint64_t avg = nrec / n, have = std::max<uint64_t>(S.bucket.cap / n, (4ull << 30) / sizeof(uint4) / n);
+  const uint64_t avg = nrec / n, have = S.bucket.cap / n;
   S.W = (uint32_t)std::max<uint64_t>(
       1, std::min<uint64_t>({S.bucket_cap, 3 * avg + 64, std::max<uint64_t>(have, avg + avg / 4 + 32)}));
   if (pairs_out) *pairs_out = npairs;
@@ -1469,15 +1486,14 @@ int build_graph_device(efg_index* idx) {
     EFG_TRY(build_forest(idx, idx->bp.trees));
   }
   cudaEventRecord(ev[1], s);
-  NNDev S;
+  NNDev S(idx->stream);
   int rc;
   {
     NvtxRange r("efg: leaf-merge init");
     rc = nnd_init_device(idx, S);
   }
   if (rc != EFG_OK) {
-    S.release_all();
-    return rc;
+      return rc;
   }
   cudaEventRecord(ev[2], s);
   uint64_t pairs = 0, recs = 0;
@@ -1486,8 +1502,7 @@ int build_graph_device(efg_index* idx) {
     NvtxRange range_it("efg: nn-descent iteration");
     rc = nnd_iterate_device(idx, S, it, &p, &r);
     if (rc != EFG_OK) {
-      S.release_all();
-      return rc;
+          return rc;
     }
     pairs += p;
     recs += r;
@@ -1517,7 +1532,6 @@ int build_graph_device(efg_index* idx) {
   idx->bstats.total_ms = a + b + c;
   idx->bstats.join_pairs = pairs;
   idx->bstats.join_records = recs;
-  S.release_all();
   return EFG_OK;
 }
 
@@ -1526,6 +1540,7 @@ int build_graph_device(efg_index* idx) {
 static int state_to_device(efg_index* idx, NNDev& S, const efg_nnd_host_state* st) {
   if (st->n != idx->n || st->L != idx->bp.L) return fail(EFG_ERR_ARG, "state does not match the index");
   EFG_TRY(nn_alloc(S, st->n, st->L, st->cap));
+  EFG_CUDA(cudaStreamSynchronize(idx->stream));  // the copies below run on the default stream
   uint64_t n = st->n, np = n * S.P;
   std::vector<uint32_t> pid(np);
   for (uint64_t i = 0; i < np; ++i) pid[i] = st->pool_id[i] | (st->pool_flag[i] ? FLAG : 0u);
@@ -1540,6 +1555,7 @@ static int state_to_device(efg_index* idx, NNDev& S, const efg_nnd_host_state* s
   EFG_CUDA(cudaMemcpy(S.new_cnt.p, st->new_cnt, n * 4, cudaMemcpyHostToDevice));
   EFG_CUDA(cudaMemcpy(S.old_ids.p, st->old_ids, n * st->cap * 4, cudaMemcpyHostToDevice));
   EFG_CUDA(cudaMemcpy(S.old_cnt.p, st->old_cnt, n * 4, cudaMemcpyHostToDevice));
+  EFG_CUDA(cudaStreamSynchronize(0));
   return EFG_OK;
 }
 
@@ -1569,23 +1585,21 @@ int nnd_init_host(efg_index* idx, efg_nnd_host_state* st) {
   if (st->n != idx->n || st->L != idx->bp.L) return fail(EFG_ERR_ARG, "state does not match the index");
   uint32_t need = std::max(idx->bp.L, 2 * idx->bp.S) + idx->bp.reverse_cap;
   if (st->cap != need) return fail(EFG_ERR_ARG, "state list capacity must be " + std::to_string(need));
-  NNDev S;
+  NNDev S(idx->stream);
   int rc = nnd_init_device(idx, S);
   if (rc == EFG_OK) rc = state_to_host(S, st);
-  S.release_all();
   return rc;
 }
 
 int nnd_iterate_host(efg_index* idx, efg_nnd_host_state* st, uint32_t iter, uint64_t* pairs) {
   uint32_t need = std::max(idx->bp.L, 2 * idx->bp.S) + idx->bp.reverse_cap;
   if (st->cap < need) return fail(EFG_ERR_ARG, "state list capacity too small");
-  NNDev S;
+  NNDev S(idx->stream);
   int rc = state_to_device(idx, S, st);
   uint64_t p = 0, r = 0;
   if (rc == EFG_OK) rc = nnd_iterate_device(idx, S, iter, &p, &r);
   if (rc == EFG_OK) rc = state_to_host(S, st);
   if (pairs) *pairs = p;
-  S.release_all();
   return rc;
 }
 

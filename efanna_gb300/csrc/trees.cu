@@ -381,9 +381,9 @@ int build_forest(efg_index* idx, uint32_t ntrees) {
   const uint64_t cap_nodes = 2 * total + ntrees;  // each split adds two nodes; at most n-1 splits per tree
 
   EFG_TRY(F.leaves.reserve(total));
-  LocalBuf<uint32_t> ids_b;
-  LocalBuf<int32_t> owner;
-  LocalBuf<uint64_t> flags, pref, scan_tmp;
+  LocalBuf<uint32_t> ids_b(s);
+  LocalBuf<int32_t> owner(s);
+  LocalBuf<uint64_t> flags(s), pref(s), scan_tmp(s);
   EFG_TRY(ids_b.reserve(total));
   EFG_TRY(owner.reserve(total));
   EFG_TRY(flags.reserve(total));
@@ -395,8 +395,8 @@ int build_forest(efg_index* idx, uint32_t ntrees) {
   EFG_TRY(F.n_level.reserve(cap_nodes));
   EFG_TRY(F.n_left.reserve(cap_nodes));
   EFG_TRY(F.n_right.reserve(cap_nodes));
-  LocalBuf<int32_t> n_dim, n_split;
-  LocalBuf<float> n_val;
+  LocalBuf<int32_t> n_dim(s), n_split(s);
+  LocalBuf<float> n_val(s);
   EFG_TRY(n_dim.reserve(cap_nodes));
   EFG_TRY(n_split.reserve(cap_nodes));
   EFG_TRY(n_val.reserve(cap_nodes));
@@ -404,8 +404,8 @@ int build_forest(efg_index* idx, uint32_t ntrees) {
 
   // active lists and per-level scratch (active count <= total)
   uint64_t cap_act = std::max<uint64_t>(total, 2048);
-  LocalBuf<int32_t> act, next_cand;
-  LocalBuf<uint32_t> split_flag, child_off, mids, next_flag, next_pos, tmp32;
+  LocalBuf<int32_t> act(s), next_cand(s);
+  LocalBuf<uint32_t> split_flag(s), child_off(s), mids(s), next_flag(s), next_pos(s), tmp32(s);
   EFG_TRY(act.reserve(cap_act));
   EFG_TRY(next_cand.reserve(2 * cap_act));
   EFG_TRY(split_flag.reserve(cap_act));
@@ -502,14 +502,6 @@ int build_forest(efg_index* idx, uint32_t ntrees) {
   F.nnodes = (uint64_t)nnodes;
   F.roots = roots;
   F.has_soa = true;
-  ids_b.release();
-  owner.release();
-  flags.release();
-  pref.release();
-  scan_tmp.release();
-  n_dim.release();
-  n_split.release();
-  n_val.release();
   return EFG_OK;
 }
 
