@@ -42,6 +42,7 @@
 #include <cfloat>
 #include <cmath>
 #include <mutex>
+#include <vector>
 
 #include "internal.cuh"
 #include "tcgen05.cuh"
@@ -414,6 +415,474 @@ __global__ void bound_kernel(const uint64_t* __restrict__ lists, uint64_t nq, ui
   }
 }
 
+
+// ==============================================================================================
+// Screening against a bound: the path of every call whose candidates fit their buffers.
+//
+// With an upper bound on each query's K2-th distance, screening only has to find the values under it
+// and append them to the query's buffer; lists, and their divergent insertions, are left to the few.
+// The bound comes from cheap passes of the same kernel:
+//   * MIN pass over a sample: the rows fall into groups, every thread keeps its groups' minima, and the
+//     largest minimum of at least K2 disjoint groups bounds the K2-th distance (no list, two
+//     instructions per value);
+//   * append pass over n / 16 rows with that bound, whose K2-th key is a tight one: about 16 K2 values of
+//     the whole base lie under it.
+//
+// Data movement is what bounds a Gram tile here: 128 x 128 x 64 products take 256 cycles and read 32 KB.
+// So a work item keeps its query blocks in shared memory (where they fit) and takes two query tiles at
+// a time (256 queries, 512 TMEM columns with two buffers), which reads each base block once per 256
+// queries: 32 KB per 1024 cycles at 128 dimensions instead of 64 KB per 512.  The screening warps spend
+// one packed FMA and one three-input minimum per two values.
+constexpr uint32_t SW_ = 8;                     // screening warps
+constexpr uint32_t STH = 64 + 32 * SW_;         // threads
+constexpr uint32_t CAND_MAX = 4096;             // candidates a query's buffer can hold
+
+struct ScreenArgs {
+  const float* qnorm;     // nq FP32 squared norms
+  const float* xnorm;     // of the rows, +inf past the last up to a whole tile
+  const uint32_t* qbound; // bits of an upper bound of each query's rank-th distance, or null (+inf)
+  uint32_t* qmax;         // MIN pass: bits of the bound, combined by atomicMax (zero on entry)
+  uint32_t* cnt;          // append pass: candidates per query (may exceed cap)
+  uint64_t* buf;          // nq x cap keys
+  int* err;
+  uint64_t n, first_row;
+  uint32_t ntiles, chunk_tiles, nchunks, qgroups, nq, cap, kblocks, stages, exclude_self;
+  uint32_t group_tiles;   // MIN pass: tiles per group of a thread's 64 columns (0: groups of 16 columns)
+  uint32_t split, resident;
+  float rel;              // the bound is widened by this much (passes of the split form may round differently)
+  uint32_t stage_bytes, o_x, o_scr, o_xn;
+};
+
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+template <int NT, bool MINP>
+__global__ void __launch_bounds__(STH, 1)
+    tc_screen_kernel(const __grid_constant__ CUtensorMap mq_hi, const __grid_constant__ CUtensorMap mq_lo,
+                     const __grid_constant__ CUtensorMap mx_hi, const __grid_constant__ CUtensorMap mx_lo,
+                     const ScreenArgs a) {
+  constexpr uint32_t COLS = 2 * NT * TN;  // two buffers of NT accumulators
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t bar_full[MAX_STAGES], bar_empty[MAX_STAGES], bar_tfull[2], bar_tempty[2], bar_q,
+      bar_qfree, bar_drain;
+  __shared__ uint32_t tmem_base_sh;
+  __shared__ int abort_sh;
+  const uint32_t raw = smem_addr(smem_raw);
+  const uint32_t pad = ((raw + 1023u) & ~1023u) - raw;
+  unsigned char* smem = smem_raw + pad;
+  const uint32_t sbase = raw + pad;
+  const uint32_t parts = a.split ? 2u : 1u;  // hi, or hi and lo blocks
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (uint32_t s = 0; s < a.stages; ++s) {
+      mbar_init(smem_addr(&bar_full[s]), 1);
+      mbar_init(smem_addr(&bar_empty[s]), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_addr(&bar_tfull[b]), 1);
+      mbar_init(smem_addr(&bar_tempty[b]), 32 * SW_);
+    }
+    mbar_init(smem_addr(&bar_q), 1);
+    mbar_init(smem_addr(&bar_qfree), 1);
+    mbar_init(smem_addr(&bar_drain), 1);
+    abort_sh = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_sh)),
+                 "r"(COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_sh;
+  volatile int* abort_flag = &abort_sh;
+  const uint32_t items = a.qgroups * a.nchunks;
+  bool mma_issued = false;
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- TMA producer (one lane)
+    if (lane == 0) {
+      uint32_t s = 0, ph = 0, it = 0;
+      bool ok = true;
+      for (uint32_t w = blockIdx.x; ok && w < items; w += gridDim.x, ++it) {
+        const uint32_t chunk = w / a.qgroups, qg = w % a.qgroups;
+        const uint32_t t0 = chunk * a.chunk_tiles, t1 = min(a.ntiles, t0 + a.chunk_tiles);
+        const int yq = (int)(qg * NT * TM);
+        if (a.resident) {  // the item's query blocks, once the previous item's products have read theirs
+          if (!mbar_wait(smem_addr(&bar_qfree), (it & 1u) ^ 1u, abort_flag, a.err)) break;
+          const uint32_t qb = smem_addr(&bar_q);
+          mbar_expect_tx(qb, NT * a.kblocks * parts * PART);
+          for (uint32_t i = 0; i < NT * a.kblocks; ++i) {
+            const int x = (int)((i % a.kblocks) * TKB), y = yq + (int)((i / a.kblocks) * TM);
+            tma_load_2d(sbase + i * parts * PART, &mq_hi, qb, x, y);
+            if (a.split) tma_load_2d(sbase + (i * parts + 1) * PART, &mq_lo, qb, x, y);
+          }
+        }
+        for (uint32_t t = t0; ok && t < t1; ++t) {
+          for (uint32_t kb = 0; kb < a.kblocks; ++kb) {
+            if (!mbar_wait(smem_addr(&bar_empty[s]), ph ^ 1u, abort_flag, a.err)) {
+              ok = false;
+              break;
+            }
+            const uint32_t fb = smem_addr(&bar_full[s]);
+            mbar_expect_tx(fb, a.stage_bytes);
+            const uint32_t st = sbase + a.o_x + s * a.stage_bytes;
+            const int x = (int)(kb * TKB), yx = (int)(t * TN);
+            tma_load_2d(st, &mx_hi, fb, x, yx);
+            if (a.split) tma_load_2d(st + PART, &mx_lo, fb, x, yx);
+            if (!a.resident)
+              for (uint32_t i = 0; i < NT; ++i) {
+                const uint32_t dst = st + (1 + i) * parts * PART;
+                tma_load_2d(dst, &mq_hi, fb, x, yq + (int)(i * TM));
+                if (a.split) tma_load_2d(dst + PART, &mq_lo, fb, x, yq + (int)(i * TM));
+              }
+            if (++s == a.stages) {
+              s = 0;
+              ph ^= 1u;
+            }
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- MMA issuer (one lane)
+    if (lane == 0) {
+      uint32_t s = 0, ph = 0, tcount = 0, it = 0;
+      bool ok = true;
+      for (uint32_t w = blockIdx.x; ok && w < items; w += gridDim.x, ++it) {
+        const uint32_t chunk = w / a.qgroups;
+        const uint32_t t0 = chunk * a.chunk_tiles, t1 = min(a.ntiles, t0 + a.chunk_tiles);
+        if (a.resident && !mbar_wait(smem_addr(&bar_q), it & 1u, abort_flag, a.err)) break;
+        tc_fence_after();
+        for (uint32_t t = t0; ok && t < t1; ++t, ++tcount) {
+          const uint32_t b = tcount & 1u, tph = (tcount >> 1) & 1u;
+          if (!mbar_wait(smem_addr(&bar_tempty[b]), tph ^ 1u, abort_flag, a.err)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + b * NT * TN;
+          for (uint32_t kb = 0; kb < a.kblocks; ++kb) {
+            if (!mbar_wait(smem_addr(&bar_full[s]), ph, abort_flag, a.err)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t st = sbase + a.o_x + s * a.stage_bytes;
+            const uint64_t xh = sw128_desc(st), xl = sw128_desc(st + PART);
+#pragma unroll
+            for (uint32_t i = 0; i < NT; ++i) {
+              const uint32_t qa = a.resident ? sbase + (i * a.kblocks + kb) * parts * PART : st + (1 + i) * parts * PART;
+              const uint64_t qh = sw128_desc(qa), ql = sw128_desc(qa + PART);
+#pragma unroll
+              for (uint32_t j = 0; j < TKB / 16; ++j) {  // K = 16 per MMA: 32 bytes further along the row
+                const uint64_t o = (uint64_t)(2 * j);
+                umma_bf16(d_tmem + i * TN, qh + o, xh + o, IDESC, (kb | j) != 0 ? 1u : 0u);
+                if (a.split) {
+                  umma_bf16(d_tmem + i * TN, qh + o, xl + o, IDESC, 1u);
+                  umma_bf16(d_tmem + i * TN, ql + o, xh + o, IDESC, 1u);
+                }
+              }
+            }
+            mma_issued = true;
+            umma_commit(smem_addr(&bar_empty[s]));  // frees the stage when these MMAs have read it
+            if (++s == a.stages) {
+              s = 0;
+              ph ^= 1u;
+            }
+          }
+          if (!ok) break;
+          umma_commit(smem_addr(&bar_tfull[b]));  // buffer b holds the tile
+        }
+        if (ok && a.resident) umma_commit(smem_addr(&bar_qfree));
+      }
+    }
+  } else {
+    // ---------------------------------------------------------------- screening (warps 2 ..)
+    const uint32_t ew = warp - 2, quad = warp & 3u, half = ew >> 2;  // TMEM lanes 32 quad .., columns 64 half ..
+    float* scr = reinterpret_cast<float*>(smem + a.o_scr) + (ew * 32 + lane) * GRP;
+    const uint32_t sw = (lane >> 1) & 3u;  // (the copy of a group's 16 values: float4 slot j at j ^ sw)
+    float* xw = reinterpret_cast<float*>(smem + a.o_xn) + ew * 2 * 64;  // norms of 64 rows, two copies
+    const uint64_t m2 = pack2(__float_as_uint(-2.f), __float_as_uint(-2.f));
+    uint32_t tcount = 0;
+    bool ok = true;
+    for (uint32_t w = blockIdx.x; ok && w < items; w += gridDim.x) {
+      const uint32_t chunk = w / a.qgroups, qg = w % a.qgroups;
+      const uint32_t t0 = chunk * a.chunk_tiles, t1 = min(a.ntiles, t0 + a.chunk_tiles);
+      float qn[NT], thr[NT], lim[NT], gmin[NT], gmax[NT];
+      uint32_t qi[NT];
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        qi[i] = (qg * NT + i) * TM + quad * 32 + lane;
+        const bool valid = qi[i] < a.nq;
+        qn[i] = valid ? a.qnorm[qi[i]] : 0.f;
+        const float b = !MINP && valid && a.qbound ? __uint_as_float(a.qbound[qi[i]]) : INFINITY;
+        thr[i] = !valid ? -1.f : b < INFINITY ? b + b * a.rel : INFINITY;
+        // the group test compares xn - 2 q.x against thr - qn, widened by a few ulps so that it never
+        // rejects what the exact test (d = xn - 2 q.x + qn <= thr) accepts
+        lim[i] = valid ? thr[i] - qn[i] + (fabsf(thr[i]) + qn[i]) * 4.8e-7f : -INFINITY;
+        gmin[i] = INFINITY;
+        gmax[i] = -INFINITY;
+      }
+      reinterpret_cast<float2*>(xw + (tcount & 1u) * 64)[lane] =
+          __ldg(reinterpret_cast<const float2*>(a.xnorm + (uint64_t)t0 * TN + half * 64) + lane);
+      __syncwarp();
+      for (uint32_t t = t0; t < t1; ++t, ++tcount) {
+        const uint32_t b = tcount & 1u, tph = (tcount >> 1) & 1u;
+        const uint64_t row0 = (uint64_t)t * TN + half * 64;
+        float2 xnext = make_float2(0.f, 0.f);
+        if (t + 1 < t1) xnext = __ldg(reinterpret_cast<const float2*>(a.xnorm + row0 + TN) + lane);  // in flight meanwhile
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&bar_tfull[b]), tph, abort_flag, a.err));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + ((quad * 32u) << 16) + b * NT * TN + half * 64;
+        const float* xs = xw + (tcount & 1u) * 64;
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+          uint32_t v[64];
+          tmem_ld64(taddr + i * TN, v);
+          tmem_wait();
+#pragma unroll
+          for (uint32_t g = 0; g < 64 / GRP; ++g) {
+            const ulonglong2* x2 = reinterpret_cast<const ulonglong2*>(xs + g * GRP);
+            float m0 = INFINITY, m1 = INFINITY;
+#pragma unroll
+            for (uint32_t j = 0; j < GRP / 4; ++j) {
+              const ulonglong2 xn = x2[j];
+              const uint32_t o = g * GRP + 4 * j;
+              float p0, p1, p2, p3;
+              unpack2(fma2(m2, pack2(v[o], v[o + 1]), xn.x), p0, p1);
+              unpack2(fma2(m2, pack2(v[o + 2], v[o + 3]), xn.y), p2, p3);
+              m0 = min3(m0, p0, p1);
+              m1 = min3(m1, p2, p3);
+            }
+            const float m = fminf(m0, m1);
+            if (MINP) {
+              if (a.group_tiles) gmin[i] = fminf(gmin[i], m);
+              else gmax[i] = fmaxf(gmax[i], m);
+            } else if (__any_sync(0xffffffffu, m <= lim[i])) {
+              // the group's values under the bound, as a mask; this thread's values to its scratch
+              uint32_t hits = 0;
+              if (m <= lim[i]) {
+#pragma unroll
+                for (uint32_t j = 0; j < GRP / 4; ++j) {
+                  const float4 xn = reinterpret_cast<const float4*>(xs + g * GRP)[j];
+                  const uint32_t o = g * GRP + 4 * j;
+                  hits |= (fmaf(-2.f, __uint_as_float(v[o + 0]), xn.x) <= lim[i] ? 1u : 0u) << (4 * j);
+                  hits |= (fmaf(-2.f, __uint_as_float(v[o + 1]), xn.y) <= lim[i] ? 2u : 0u) << (4 * j);
+                  hits |= (fmaf(-2.f, __uint_as_float(v[o + 2]), xn.z) <= lim[i] ? 4u : 0u) << (4 * j);
+                  hits |= (fmaf(-2.f, __uint_as_float(v[o + 3]), xn.w) <= lim[i] ? 8u : 0u) << (4 * j);
+                  reinterpret_cast<float4*>(scr)[j ^ sw] =
+                      make_float4(__uint_as_float(v[o]), __uint_as_float(v[o + 1]), __uint_as_float(v[o + 2]),
+                                  __uint_as_float(v[o + 3]));
+                }
+              }
+              const uint64_t self = a.exclude_self ? a.first_row + qi[i] : ~0ull;
+              while (hits) {  // the exact test, then the query's buffer
+                const uint32_t j = __ffs(hits) - 1;
+                hits &= hits - 1;
+                const float val = scr[(((j >> 2) ^ sw) << 2) | (j & 3u)];
+                const float d = fmaxf(fmaf(-2.f, val, xs[g * GRP + j]) + qn[i], 0.f);
+                const uint64_t row = row0 + g * GRP + j;
+                if (d <= thr[i] && row < a.n && row != self) {
+                  const uint32_t pos = atomicAdd(&a.cnt[qi[i]], 1u);
+                  if (pos < a.cap)
+                    a.buf[(uint64_t)qi[i] * a.cap + pos] = ((uint64_t)__float_as_uint(d) << 32) | (uint32_t)row;
+                }
+              }
+              __syncwarp();
+            }
+          }
+        }
+        tc_fence_before();
+        mbar_arrive(smem_addr(&bar_tempty[b]));  // buffer b may be overwritten
+        if (t + 1 < t1) reinterpret_cast<float2*>(xw + ((tcount + 1) & 1u) * 64)[lane] = xnext;
+        if (MINP && a.group_tiles && (t + 1 - t0) % a.group_tiles == 0) {
+#pragma unroll
+          for (int i = 0; i < NT; ++i) {
+            gmax[i] = fmaxf(gmax[i], gmin[i]);
+            gmin[i] = INFINITY;
+          }
+        }
+        __syncwarp();
+      }
+      if (!ok) break;
+      if (MINP) {
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+          if (qi[i] < a.nq) atomicMax(&a.qmax[qi[i]], __float_as_uint(fmaxf(gmax[i] + qn[i], 0.f)));
+      }
+    }
+  }
+
+  // ------------------------------------------------------------------------------ teardown
+  __syncthreads();
+  if (warp == 1) {
+    if (lane == 0 && mma_issued) {  // every MMA this thread issued has finished before TMEM is freed
+      umma_commit(smem_addr(&bar_drain));
+      unsigned long long t0 = clock64();
+      while (!mbar_try_wait(smem_addr(&bar_drain), 0)) {
+        if (clock64() - t0 > WAIT_CYCLES) {
+          atomicOr(a.err, 2);
+          break;
+        }
+      }
+    }
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(COLS) : "memory");
+  }
+}
+
+// Sample rows in a scattered order: row i of the sample is base row floor(((i * step) mod S) * n / S), step
+// prime to S, so that every leading part of the sample is spread over the base too.  A warp per row,
+// 16-byte copies, W BF16 values per row; lo may be null.
+__global__ void scatter_sample_kernel(const uint4* __restrict__ hi, const uint4* __restrict__ lo,
+                                      const float* __restrict__ norms, uint64_t n, uint32_t W, uint32_t S,
+                                      uint32_t step, uint4* __restrict__ shi, uint4* __restrict__ slo,
+                                      float* __restrict__ snorms) {
+  const uint32_t lane = threadIdx.x & 31, w16 = W / 8;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < S; i += nw) {
+    const uint64_t r = (i * step % S) * n / S;
+    for (uint32_t c = lane; c < w16; c += 32) {
+      shi[i * w16 + c] = hi[r * w16 + c];
+      if (lo) slo[i * w16 + c] = lo[r * w16 + c];
+    }
+    if (lane == 0) snorms[i] = norms[r];
+  }
+}
+
+// FP32 rows -> BF16 hi (and, with lo, lo = x - hi) rows of W values (zero padded), squared norms (+inf
+// for the rows up to norm_rows), and a flag set when some lo is not zero.  A warp per row of the rows
+// r * step; a lane four values at a time.  hi null: only the flag.
+__global__ void split_bf16_kernel(const float* __restrict__ src, uint64_t rows, uint64_t step, uint32_t dim,
+                                  uint64_t ld, uint32_t W, uint2* __restrict__ hi, uint2* __restrict__ lo,
+                                  float* __restrict__ norms, uint64_t norm_rows, int* __restrict__ inexact) {
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint32_t lane = threadIdx.x & 31;
+  bool any_lo = false;
+  for (uint64_t r = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * step; r < norm_rows; r += nw * step) {
+    if (r >= rows) {
+      if (lane == 0) norms[r] = INFINITY;
+      continue;
+    }
+    float acc = 0.f;
+    for (uint32_t c = lane; c < W / 4; c += 32) {
+      float x[4] = {0.f, 0.f, 0.f, 0.f};
+      if (4 * c + 3 < dim) {
+        const float4 f = __ldg(reinterpret_cast<const float4*>(src + r * ld) + c);
+        x[0] = f.x;
+        x[1] = f.y;
+        x[2] = f.z;
+        x[3] = f.w;
+      } else {
+        for (uint32_t j = 0; 4 * c + j < dim; ++j) x[j] = src[r * ld + 4 * c + j];
+      }
+      __nv_bfloat16 h[4], l[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        h[j] = __float2bfloat16_rn(x[j]);
+        l[j] = __float2bfloat16_rn(x[j] - __bfloat162float(h[j]));
+        any_lo |= __bfloat162float(l[j]) != 0.f;
+        acc = fmaf(x[j], x[j], acc);
+      }
+      if (hi) hi[r * (W / 4) + c] = *reinterpret_cast<const uint2*>(h);
+      if (lo) lo[r * (W / 4) + c] = *reinterpret_cast<const uint2*>(l);
+    }
+    acc = warp_sum(acc);
+    if (lane == 0 && hi) norms[r] = acc;
+  }
+  if (__any_sync(0xffffffffu, any_lo) && lane == 0) atomicOr(inexact, 1);
+}
+
+// One CTA per query: the query's candidates sorted in shared memory.  With `ids` the K2 smallest are
+// re-ranked in FP64 and the first k written; else the rank-th distance becomes the query's bound (when
+// the buffer holds that many, and all of them).  *over is set when a final buffer was too short.
+__global__ void __launch_bounds__(256) select_kernel(const uint64_t* __restrict__ buf, const uint32_t* __restrict__ cnt,
+                                                     uint32_t cap, uint32_t rank, uint32_t* __restrict__ qbound,
+                                                     const float* __restrict__ base, uint32_t dim, uint32_t ld,
+                                                     const float* __restrict__ q, uint32_t qld, uint32_t k,
+                                                     int32_t* __restrict__ ids, float* __restrict__ dists,
+                                                     int* __restrict__ over) {
+  extern __shared__ __align__(16) uint64_t keys[];  // next_pow2(candidates), then K2 distances
+  const uint64_t qi = blockIdx.x;
+  const uint32_t m = cnt[qi], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (m > cap) {
+    if (threadIdx.x == 0 && ids) *over = 1;
+    return;
+  }
+  if (!ids && m < rank) return;
+  const uint32_t p2 = next_pow2(m < 2 ? 2 : m);
+  for (uint32_t i = threadIdx.x; i < p2; i += 256) keys[i] = i < m ? buf[qi * cap + i] : ~0ull;
+  __syncthreads();
+  for (uint32_t s = 2; s <= p2; s <<= 1)
+    for (uint32_t j = s >> 1; j > 0; j >>= 1) {
+      for (uint32_t i = threadIdx.x; i < p2 / 2; i += 256) {
+        const uint32_t lo = ((i & ~(j - 1)) << 1) | (i & (j - 1)), hi = lo | j;
+        const uint64_t x = keys[lo], y = keys[hi];
+        if ((x > y) == ((lo & s) == 0)) {
+          keys[lo] = y;
+          keys[hi] = x;
+        }
+      }
+      __syncthreads();
+    }
+  if (!ids) {
+    if (threadIdx.x == 0) qbound[qi] = min(qbound[qi], (uint32_t)(keys[rank - 1] >> 32));
+    return;
+  }
+  // FP64 distances of the first `rank` (= K2) keys, then their places by (distance, id)
+  const uint32_t K2 = min(rank, m);
+  double* d64 = reinterpret_cast<double*>(keys + cap);
+  const float* qr = q + qi * qld;
+  for (uint32_t i = warp; i < K2; i += 8) {
+    const float* br = base + (uint64_t)(uint32_t)keys[i] * ld;
+    double acc = 0.0;
+    for (uint32_t c = lane; c < dim; c += 32) {
+      const double t = (double)br[c] - (double)qr[c];
+      acc += t * t;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) d64[i] = acc;
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < K2; i += 256) {
+    const double d = d64[i];
+    const uint32_t id = (uint32_t)keys[i];
+    uint32_t place = 0;
+    for (uint32_t j = 0; j < K2; ++j) place += d64[j] < d || (d64[j] == d && (uint32_t)keys[j] < id);
+    if (place < k) {
+      ids[qi * k + place] = (int32_t)id;
+      if (dists) dists[qi * k + place] = (float)d;
+    }
+  }
+  for (uint32_t i = K2 + threadIdx.x; i < k; i += 256) {  // (fewer rows than k)
+    ids[qi * k + i] = -1;
+    if (dists) dists[qi * k + i] = INFINITY;
+  }
+}
+
 }  // namespace
 
 thread_local efg_knn_stats g_knn_stats = {};
@@ -422,6 +891,40 @@ thread_local efg_knn_stats g_knn_stats = {};
 // must fit in shared memory beside two pipeline stages of the split form).
 uint32_t tc_knn_max_k() { return 104; }
 
+namespace {
+
+// Converted operands of one call and what the list path needs of them.
+struct Operands {
+  const __nv_bfloat16 *xh, *xl, *qh, *ql;
+  const float *xn, *qn;
+  int* flags;
+  uint32_t terms;
+};
+
+int knn_lists(const float* base, uint64_t n, uint32_t dim, uint32_t ld, const float* q, uint64_t nq, uint32_t qld,
+              uint32_t k, int exclude_self, uint64_t first_row, int32_t* ids, float* dists, cudaStream_t s,
+              const Operands& op);
+
+// Stream-ordered memory of one call.
+struct CallBuf {
+  cudaStream_t s;
+  std::vector<void*> p;
+  explicit CallBuf(cudaStream_t st) : s(st) {}
+  ~CallBuf() {
+    for (void* x : p) cudaFreeAsync(x, s);
+  }
+  template <typename T>
+  int get(T** out, uint64_t count) {
+    void* x = nullptr;
+    EFG_CUDA(cudaMallocAsync(&x, count * sizeof(T), s));
+    p.push_back(x);
+    *out = reinterpret_cast<T*>(x);
+    return EFG_OK;
+  }
+};
+
+}  // namespace
+
 int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld, const float* q, uint64_t nq,
                        uint32_t qld, uint32_t k, int exclude_self, uint64_t first_row, int32_t* ids, float* dists,
                        cudaStream_t s, int force_split) {
@@ -429,47 +932,273 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   if (n >= (1ull << 31) || nq >= (1ull << 31)) return fail(EFG_ERR_ARG, "tensor-core k-NN: more than 2^31 rows");
   if (k > tc_knn_max_k()) return fail(EFG_ERR_ARG, "tensor-core k-NN: k above " + std::to_string(tc_knn_max_k()));
   const uint32_t K2 = (uint32_t)std::min<uint64_t>(k + 16, n);
+  const uint32_t W = (dim + TKB - 1) / TKB * TKB, kblocks = W / TKB;
+  const uint64_t qtiles = (nq + TM - 1) / TM, ntiles = (n + TN - 1) / TN;
+  int dev = 0, sms = 148, smem_max = 0;
+  EFG_CUDA(cudaGetDevice(&dev));
+  EFG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  EFG_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  cudaEvent_t ev[5] = {};
+  struct EvGuard {
+    cudaEvent_t* e;
+    ~EvGuard() {
+      for (int i = 0; i < 5; ++i)
+        if (e[i]) cudaEventDestroy(e[i]);
+    }
+  } evguard{ev};
+  for (auto& e : ev) EFG_CUDA(cudaEventCreate(&e));
+  CallBuf mem(s);
+
+  // operands: BF16 rows, norms, flags {inexact, error, a buffer too short}.  A thin sample tells whether
+  // the low parts are wanted, so that data BF16 holds are converted without them.
+  __nv_bfloat16 *xh, *xl = nullptr, *qh, *ql = nullptr;
+  float *xn, *qn;
+  int* flags;
+  EFG_TRY(mem.get(&xh, n * W));
+  EFG_TRY(mem.get(&qh, nq * W));
+  EFG_TRY(mem.get(&xn, ntiles * TN));
+  EFG_TRY(mem.get(&qn, nq));
+  EFG_TRY(mem.get(&flags, 4));
+  EFG_CUDA(cudaMemsetAsync(flags, 0, 16, s));
+  EFG_CUDA(cudaEventRecord(ev[0], s));
+  auto blocks = [&](uint64_t warps) { return (unsigned)((std::min<uint64_t>(warps, (uint64_t)sms * 64) + 7) / 8); };
+  const uint64_t thin = std::max<uint64_t>(1, n / 1024);
+  split_bf16_kernel<<<blocks(n / thin + 1), 256, 0, s>>>(base, n, thin, dim, ld, W, nullptr, nullptr, nullptr, n, flags);
+  split_bf16_kernel<<<blocks(nq), 256, 0, s>>>(q, nq, 1, dim, qld, W, nullptr, nullptr, nullptr, nq, flags);
+  EFG_CUDA(cudaGetLastError());
+  int hflags[4] = {0, 0, 0, 0};
+  EFG_CUDA(cudaMemcpyAsync(hflags, flags, 16, cudaMemcpyDeviceToHost, s));
+  EFG_CUDA(cudaStreamSynchronize(s));
+  bool split = force_split || hflags[0];
+  for (;;) {
+    if (split) {
+      EFG_TRY(mem.get(&xl, n * W));
+      EFG_TRY(mem.get(&ql, nq * W));
+    }
+    split_bf16_kernel<<<blocks(ntiles * TN), 256, 0, s>>>(base, n, 1, dim, ld, W, (uint2*)xh, (uint2*)xl, xn,
+                                                          ntiles * TN, flags);
+    split_bf16_kernel<<<blocks(nq), 256, 0, s>>>(q, nq, 1, dim, qld, W, (uint2*)qh, (uint2*)ql, qn, nq, flags);
+    EFG_CUDA(cudaGetLastError());
+    if (split) break;
+    EFG_CUDA(cudaMemcpyAsync(hflags, flags, 16, cudaMemcpyDeviceToHost, s));
+    EFG_CUDA(cudaStreamSynchronize(s));
+    if (!hflags[0]) break;
+    split = true;  // the sample missed it
+  }
+  const uint32_t terms = split ? 3u : 1u, parts = split ? 2u : 1u;
+
+  // Query tiles per item, and whether their blocks stay in shared memory: two tiles unless that would
+  // leave a tile empty for a few queries (300 queries: three tiles as three items, not two pairs);
+  // resident with at least three stages of base blocks beside them, else streamed with those.
+  const uint32_t NT = qtiles >= 8 || qtiles % 2 == 0 ? 2u : 1u;
+  const uint32_t scratch = 32 * SW_ * GRP * 4, norms_b = SW_ * 2 * 64 * 4;
+  const int64_t room = (int64_t)smem_max - 1024 - 1024 - scratch - norms_b;  // alignment pad, barriers
+  const uint32_t qbytes = NT * kblocks * parts * PART;
+  const bool resident = (int64_t)qbytes + 3 * (int64_t)(parts * PART) <= room;
+  const uint32_t stage_bytes = resident ? parts * PART : (1 + NT) * parts * PART;
+  const uint32_t stages = (uint32_t)std::min<int64_t>(MAX_STAGES, (room - (resident ? qbytes : 0)) / stage_bytes);
+  if (stages < 2) return fail(EFG_ERR_ARG, "tensor-core k-NN: shared memory");
+  const uint32_t qgroups = (uint32_t)((qtiles + NT - 1) / NT);
+
+  CUtensorMap mqh, mql, mxh, mxl;
+  EFG_TRY(make_map(&mqh, qh, nq, W));
+  EFG_TRY(make_map(&mql, split ? ql : qh, nq, W));
+  EFG_TRY(make_map(&mxh, xh, n, W));
+  EFG_TRY(make_map(&mxl, split ? xl : xh, n, W));
+
+  unsigned grid = 0;
+  uint32_t nchunks = 1;
+  uint64_t chunk_tiles = 1;
+  // One pass over `rows` rows (maps, norms): the chunk count that keeps the SMs busiest, time ~ waves x
+  // (tiles per item, and about two for an item's start); chunks of whole groups for the MIN pass.
+  auto pass = [&](bool minp, const CUtensorMap& mh, const CUtensorMap& ml, const float* xnorm, uint64_t rows,
+                  uint32_t group_tiles, const uint32_t* qbound, uint32_t* qmax, uint32_t* cnt, uint64_t* buf,
+                  uint32_t cap, int excl) -> int {
+    ScreenArgs a;
+    const uint64_t tiles = (rows + TN - 1) / TN, unit = std::max<uint32_t>(1, group_tiles);
+    const uint64_t units = (tiles + unit - 1) / unit;
+    double best = 1e300;
+    for (uint64_t nc = 1; nc <= std::min<uint64_t>(units, 512); ++nc) {
+      const uint64_t ct = (units + nc - 1) / nc * unit, real = (tiles + ct - 1) / ct;
+      const uint64_t waves = (qgroups * real + sms - 1) / sms;
+      const double cost = (double)waves * (double)(ct + 2) + 0.001 * (double)real;
+      if (cost < best) {
+        best = cost;
+        chunk_tiles = ct;
+        nchunks = (uint32_t)real;
+      }
+    }
+    a.qnorm = qn;
+    a.xnorm = xnorm;
+    a.qbound = qbound;
+    a.qmax = qmax;
+    a.cnt = cnt;
+    a.buf = buf;
+    a.err = flags + 1;
+    a.n = rows;
+    a.first_row = first_row;
+    a.ntiles = (uint32_t)tiles;
+    a.chunk_tiles = (uint32_t)chunk_tiles;
+    a.nchunks = nchunks;
+    a.qgroups = qgroups;
+    a.nq = (uint32_t)nq;
+    a.cap = cap;
+    a.kblocks = kblocks;
+    a.stages = stages;
+    a.exclude_self = excl ? 1u : 0u;
+    a.group_tiles = group_tiles;
+    a.split = split ? 1u : 0u;
+    a.resident = resident ? 1u : 0u;
+    a.rel = split ? 1e-5f : 0.f;
+    a.stage_bytes = stage_bytes;
+    a.o_x = resident ? qbytes : 0;
+    a.o_scr = a.o_x + stages * stage_bytes;
+    a.o_xn = a.o_scr + scratch;
+    const size_t smem = 1024 + (size_t)a.o_xn + norms_b;
+    auto kern = NT == 2 ? (minp ? tc_screen_kernel<2, true> : tc_screen_kernel<2, false>)
+                        : (minp ? tc_screen_kernel<1, true> : tc_screen_kernel<1, false>);
+    EFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    grid = (unsigned)std::min<uint64_t>((uint64_t)qgroups * nchunks, (uint64_t)sms);
+    kern<<<grid, STH, smem, s>>>(mqh, mql, mh, ml, a);
+    EFG_CUDA(cudaGetLastError());
+    return EFG_OK;
+  };
+
+  // 1. bounds.  rank = K2, + 1 with exclude_self (a sample may hold the query itself).
+  EFG_CUDA(cudaEventRecord(ev[1], s));
+  const uint32_t rank = K2 + (exclude_self ? 1u : 0u);
+  uint32_t cap = 1024;  // three times the 16 x rank expected under a bound from n / 16 rows
+  while (cap < 48 * rank && cap < CAND_MAX) cap *= 2;
+  uint32_t *qbound, *cnt;
+  uint64_t* buf;
+  EFG_TRY(mem.get(&qbound, nq));
+  EFG_TRY(mem.get(&cnt, nq));
+  EFG_TRY(mem.get(&buf, nq * cap));
+  EFG_CUDA(cudaMemsetAsync(qbound, 0, nq * 4, s));
+  const size_t sel_smem = (size_t)cap * 8 + (size_t)rank * 8;
+  EFG_CUDA(cudaFuncSetAttribute(select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem));
+  const uint64_t S1 = std::min<uint64_t>(n / 16, 1u << 20) / TN * TN;  // rows of the append pass's sample
+  const uint64_t gtiles = (rank + 1) / 2;                              // tiles that hold `rank` groups of 64 columns
+  uint32_t S = 0;
+  bool bounded = true;
+  if (S1 >= gtiles * TN) {
+    __nv_bfloat16 *bh, *bl = nullptr;
+    float* bn;
+    EFG_TRY(mem.get(&bh, S1 * W));
+    if (split) EFG_TRY(mem.get(&bl, S1 * W));
+    EFG_TRY(mem.get(&bn, S1));
+    uint32_t step = (uint32_t)((double)S1 * 0.6180339887) | 1u;
+    auto gcd = [](uint64_t x, uint64_t y) {
+      while (y) {
+        const uint64_t r = x % y;
+        x = y;
+        y = r;
+      }
+      return x;
+    };
+    while (gcd(step, S1) != 1) step += 2;
+    scatter_sample_kernel<<<blocks(S1), 256, 0, s>>>((const uint4*)xh, (const uint4*)xl, xn, n, W, (uint32_t)S1, step,
+                                                     (uint4*)bh, (uint4*)bl, bn);
+    EFG_CUDA(cudaGetLastError());
+    uint32_t gt = 1;  // tiles per group: up to a third of the sample for the MIN pass
+    while (gt < 16 && gtiles * (2 * gt) * TN * 3 <= S1) gt *= 2;
+    const uint64_t S0 = gtiles * gt * TN;
+    CUtensorMap m0h, m0l, m1h, m1l;
+    EFG_TRY(make_map(&m0h, bh, S0, W));
+    EFG_TRY(make_map(&m0l, split ? bl : bh, S0, W));
+    EFG_TRY(make_map(&m1h, bh, S1, W));
+    EFG_TRY(make_map(&m1l, split ? bl : bh, S1, W));
+    EFG_TRY(pass(true, m0h, m0l, bn, S0, gt, nullptr, qbound, nullptr, nullptr, 0, 0));
+    EFG_CUDA(cudaMemsetAsync(cnt, 0, nq * 4, s));
+    EFG_TRY(pass(false, m1h, m1l, bn, S1, 0, qbound, nullptr, cnt, buf, cap, 0));
+    select_kernel<<<(unsigned)nq, 256, sel_smem, s>>>(buf, cnt, cap, rank, qbound, nullptr, 0, 0, nullptr, 0, 0, nullptr,
+                                                      nullptr, nullptr);
+    EFG_CUDA(cudaGetLastError());
+    S = (uint32_t)S1;
+  } else if (n >= 16ull * (rank + 8)) {  // a small base: groups of it all (the last tile may be partly empty)
+    const uint64_t full = n / TN;
+    uint32_t gt = 0;  // groups of 16 columns, or of 64 columns x gt tiles
+    while (full / (gt ? 2 * gt : 1) * 2 >= rank) gt = gt ? 2 * gt : 1;
+    if (gt || full * 8 >= rank) {
+      const uint64_t rows = gt ? full / gt * gt * TN : full * TN;
+      CUtensorMap m0h, m0l;
+      EFG_TRY(make_map(&m0h, xh, rows, W));
+      EFG_TRY(make_map(&m0l, split ? xl : xh, rows, W));
+      EFG_TRY(pass(true, m0h, m0l, xn, rows, gt, nullptr, qbound, nullptr, nullptr, 0, 0));
+      S = (uint32_t)rows;
+    } else {
+      bounded = false;
+    }
+  } else {
+    bounded = false;
+  }
+
+  // 2. the whole base, 3. the candidates' order
+  EFG_CUDA(cudaEventRecord(ev[2], s));
+  EFG_CUDA(cudaMemsetAsync(cnt, 0, nq * 4, s));
+  EFG_TRY(pass(false, mxh, mxl, xn, n, 0, bounded ? qbound : nullptr, nullptr, cnt, buf, cap, exclude_self));
+  EFG_CUDA(cudaEventRecord(ev[3], s));
+  select_kernel<<<(unsigned)nq, 256, sel_smem, s>>>(buf, cnt, cap, K2, nullptr, base, dim, ld, q, qld, k, ids, dists,
+                                                    flags + 2);
+  EFG_CUDA(cudaGetLastError());
+  EFG_CUDA(cudaEventRecord(ev[4], s));
+  EFG_CUDA(cudaMemcpyAsync(hflags, flags, 16, cudaMemcpyDeviceToHost, s));
+  EFG_CUDA(cudaStreamSynchronize(s));
+  if (hflags[1]) return fail(EFG_ERR_DEVICE_LIMIT, "tensor-core k-NN: a pipeline wait ran out (error word " +
+                                                       std::to_string(hflags[1]) + ")");
+  if (hflags[2]) {  // more values under a bound than its buffer holds (many equal distances): sorted lists
+    if (!split) xl = xh;
+    if (!split) ql = qh;
+    return knn_lists(base, n, dim, ld, q, nq, qld, k, exclude_self, first_row, ids, dists, s,
+                     Operands{xh, xl, qh, ql, xn, qn, flags, terms});
+  }
+  float ms[4] = {0, 0, 0, 0};
+  for (int i = 0; i < 4; ++i) cudaEventElapsedTime(&ms[i], ev[i], ev[i + 1]);
+  g_knn_stats.convert_ms = ms[0];
+  g_knn_stats.bound_ms = ms[1];
+  g_knn_stats.screen_ms = ms[2];
+  g_knn_stats.merge_ms = ms[3];
+  g_knn_stats.sample_rows = S;
+  g_knn_stats.screen_flops = 2.0 * (double)nq * (double)n * (double)dim;
+  g_knn_stats.tile_flops = 2.0 * (double)(qgroups * NT * TM) * (double)(ntiles * TN) * (double)W * (double)terms;
+  g_knn_stats.terms = terms;
+  g_knn_stats.stages = stages;
+  g_knn_stats.nchunks = nchunks;
+  g_knn_stats.ctas = grid;
+  return EFG_OK;
+}
+
+namespace {
+
+// The same result with sorted lists of K2 keys per (query, chunk), whatever the number of values under a
+// bound: for calls whose candidate buffers were too short.
+int knn_lists(const float* base, uint64_t n, uint32_t dim, uint32_t ld, const float* q, uint64_t nq, uint32_t qld,
+              uint32_t k, int exclude_self, uint64_t first_row, int32_t* ids, float* dists, cudaStream_t s,
+              const Operands& op) {
+  const uint32_t K2 = (uint32_t)std::min<uint64_t>(k + 16, n);
   const uint32_t W = (dim + TKB - 1) / TKB * TKB;
   const uint32_t kblocks = W / TKB;
   const uint64_t qtiles = (nq + TM - 1) / TM;
-  const uint64_t nrows_pad = (n + TN - 1) / TN * TN;
-
   int dev = 0, sms = 148;
   EFG_CUDA(cudaGetDevice(&dev));
   EFG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   int smem_max = 0;
   EFG_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-
-  // operands: BF16 hi/lo rows, norms, the inexact flag and the error word
-  __nv_bfloat16 *xh = nullptr, *xl = nullptr, *qh = nullptr, *ql = nullptr;
-  float *xn = nullptr, *qn = nullptr;
-  int* flags = nullptr;
+  const __nv_bfloat16 *xh = op.xh, *xl = op.xl, *qh = op.qh, *ql = op.ql;
+  const float *xn = op.xn, *qn = op.qn;
+  int* flags = op.flags;
+  const uint32_t terms = op.terms;
   uint64_t* part = nullptr;
   float *sn = nullptr, *qbound = nullptr;
   auto release = [&] {
     cudaFreeAsync(sn, s);
     cudaFreeAsync(qbound, s);
-    cudaFreeAsync(xh, s);
-    cudaFreeAsync(xl, s);
-    cudaFreeAsync(qh, s);
-    cudaFreeAsync(ql, s);
-    cudaFreeAsync(xn, s);
-    cudaFreeAsync(qn, s);
-    cudaFreeAsync(flags, s);
     cudaFreeAsync(part, s);
   };
   struct Guard {
     decltype(release)& f;
     ~Guard() { f(); }
   } guard{release};
-  EFG_CUDA(cudaMallocAsync((void**)&xh, n * W * 2, s));
-  EFG_CUDA(cudaMallocAsync((void**)&xl, n * W * 2, s));
-  EFG_CUDA(cudaMallocAsync((void**)&qh, nq * W * 2, s));
-  EFG_CUDA(cudaMallocAsync((void**)&ql, nq * W * 2, s));
-  EFG_CUDA(cudaMallocAsync((void**)&xn, nrows_pad * 4, s));
-  EFG_CUDA(cudaMallocAsync((void**)&qn, nq * 4, s));
-  EFG_CUDA(cudaMallocAsync((void**)&flags, 8, s));
-  EFG_CUDA(cudaMemsetAsync(flags, 0, 8, s));
   cudaEvent_t ev[5] = {};
   struct EvGuard {
     cudaEvent_t* e;
@@ -480,19 +1209,7 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   } evguard{ev};
   for (auto& e : ev) EFG_CUDA(cudaEventCreate(&e));
   EFG_CUDA(cudaEventRecord(ev[0], s));
-  {
-    const uint64_t warps = std::min<uint64_t>(nrows_pad, (uint64_t)sms * 64);
-    to_bf16_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(base, n, dim, ld, W, xh, xl, xn, nrows_pad,
-                                                                        flags);
-    EFG_CUDA(cudaGetLastError());
-    const uint64_t qwarps = std::min<uint64_t>(nq, (uint64_t)sms * 64);
-    to_bf16_kernel<<<(unsigned)((qwarps * 32 + 255) / 256), 256, 0, s>>>(q, nq, dim, qld, W, qh, ql, qn, nq, flags);
-    EFG_CUDA(cudaGetLastError());
-  }
   int hflags[2] = {0, 0};
-  EFG_CUDA(cudaMemcpyAsync(hflags, flags, 8, cudaMemcpyDeviceToHost, s));
-  EFG_CUDA(cudaStreamSynchronize(s));
-  const uint32_t terms = (hflags[0] || force_split) ? 3u : 1u;
 
   // shared memory: pipeline stages, then the per-thread lists, scratch and norm copies
   const uint32_t stage_bytes = 2 * PART;
@@ -676,5 +1393,7 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
                                                         std::to_string(hflags[1]) + ")");
   return EFG_OK;
 }
+
+}  // namespace
 
 }  // namespace efg

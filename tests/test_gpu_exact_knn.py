@@ -129,3 +129,34 @@ def test_few_queries_over_many_chunks(efg, n, nq, k):
     tc = _knn(efg, x, q, k, "auto")
     f32 = _knn(efg, x, q, k, "fp32")
     assert np.array_equal(tc[0], f32[0]) and np.array_equal(tc[1], f32[1])
+
+
+@pytest.mark.parametrize("n,nq,k,excl", [(17, 5, 1, False), (130, 260, 20, True), (543, 129, 10, False),
+                                         (544, 64, 10, False), (2063, 257, 104, True), (2100, 1100, 104, False),
+                                         (30_000, 900, 10, True), (130_000, 300, 104, False)])
+@pytest.mark.parametrize("d", [5, 129, 300])
+def test_bound_passes_at_their_edges(efg, n, nq, k, excl, d):
+    """No bound, a bound from groups of 16 columns, of 64 and of whole tiles of the base, and from a sample;
+    one and two query tiles per item, resident and streamed (d = 300 in the split form)."""
+    rng = np.random.default_rng(n + d)
+    x = rng.integers(0, 256, (n, d)).astype(np.float32)
+    nq = min(nq, n) if excl else nq
+    q = x[:nq].copy() if excl else rng.integers(0, 256, (nq, d)).astype(np.float32)
+    k = min(k, n - 1)
+    for screening in ("auto", "split"):
+        tc = _knn(efg, x, q, k, screening, exclude=excl)
+        f32 = _knn(efg, x, q, k, "fp32", exclude=excl)
+        assert np.array_equal(tc[0], f32[0]) and np.array_equal(tc[1], f32[1])
+
+
+@pytest.mark.parametrize("n", [3000, 60_000])
+def test_many_equal_distances(efg, n):
+    """More rows at one distance than a candidate buffer holds: the lists take the call."""
+    x = np.zeros((n, 8), np.float32)
+    x[::7, 3] = 1.0
+    q = np.zeros((200, 8), np.float32)
+    q[::2, 0] = 2.0
+    tc = _knn(efg, x, q, 12, "auto")
+    ref_ids, ref_d = _numpy_exact(x, q[:2], 12)
+    for i in range(200):
+        assert np.array_equal(tc[0][i], ref_ids[i % 2]) and np.array_equal(tc[1][i], ref_d[i % 2])
