@@ -450,7 +450,7 @@ struct ScreenArgs {
   uint32_t group_tiles;   // MIN pass: tiles per group of a thread's 64 columns (0: groups of 16 columns)
   uint32_t split, resident;
   float rel;              // the bound is widened by this much (passes of the split form may round differently)
-  uint32_t stage_bytes, o_x, o_scr, o_xn;
+  uint32_t stage_bytes, o_x, o_scr, o_xn, o_queue;
 };
 
 __device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
@@ -623,6 +623,28 @@ __global__ void __launch_bounds__(STH, 1)
     const uint32_t sw = (lane >> 1) & 3u;  // (the copy of a group's 16 values: float4 slot j at j ^ sw)
     float* xw = reinterpret_cast<float*>(smem + a.o_xn) + ew * 2 * 64;  // norms of 64 rows, two copies
     const uint64_t m2 = pack2(__float_as_uint(-2.f), __float_as_uint(-2.f));
+    // candidates on their way to the queries' buffers: 32 slots are taken at once, an atomic per lane
+    // (one at a time their latency held the warp at every hit: 4.6 of 7.0 ms at 10k x 1M x 128)
+    uint64_t* queue_key = reinterpret_cast<uint64_t*>(smem + a.o_queue) + ew * 64;
+    uint32_t* queue_q = reinterpret_cast<uint32_t*>(smem + a.o_queue + SW_ * 64 * 8) + ew * 64;
+    uint32_t queued = 0;
+    auto flush = [&](uint32_t m) {
+      __syncwarp();
+      if (lane < m) {
+        const uint32_t qq = queue_q[lane];
+        const uint32_t pos = atomicAdd(&a.cnt[qq], 1u);
+        if (pos < a.cap) a.buf[(uint64_t)qq * a.cap + pos] = queue_key[lane];
+      }
+      const uint64_t rk = lane + 32 < queued ? queue_key[lane + 32] : 0;
+      const uint32_t rq = lane + 32 < queued ? queue_q[lane + 32] : 0;
+      __syncwarp();
+      if (lane + 32 < queued) {
+        queue_key[lane] = rk;
+        queue_q[lane] = rq;
+      }
+      queued -= m;
+      __syncwarp();
+    };
     uint32_t tcount = 0;
     bool ok = true;
     for (uint32_t w = blockIdx.x; ok && w < items; w += gridDim.x) {
@@ -696,18 +718,28 @@ __global__ void __launch_bounds__(STH, 1)
                                   __uint_as_float(v[o + 3]));
                 }
               }
+              // one marked value per lane per round: the exact test, then the warp's queue
               const uint64_t self = a.exclude_self ? a.first_row + qi[i] : ~0ull;
-              while (hits) {  // the exact test, then the query's buffer
-                const uint32_t j = __ffs(hits) - 1;
-                hits &= hits - 1;
-                const float val = scr[(((j >> 2) ^ sw) << 2) | (j & 3u)];
-                const float d = fmaxf(fmaf(-2.f, val, xs[g * GRP + j]) + qn[i], 0.f);
-                const uint64_t row = row0 + g * GRP + j;
-                if (d <= thr[i] && row < a.n && row != self) {
-                  const uint32_t pos = atomicAdd(&a.cnt[qi[i]], 1u);
-                  if (pos < a.cap)
-                    a.buf[(uint64_t)qi[i] * a.cap + pos] = ((uint64_t)__float_as_uint(d) << 32) | (uint32_t)row;
+              while (__any_sync(0xffffffffu, hits != 0)) {
+                uint64_t key = 0;
+                bool take = false;
+                if (hits) {
+                  const uint32_t j = __ffs(hits) - 1;
+                  hits &= hits - 1;
+                  const float val = scr[(((j >> 2) ^ sw) << 2) | (j & 3u)];
+                  const float d = fmaxf(fmaf(-2.f, val, xs[g * GRP + j]) + qn[i], 0.f);
+                  const uint64_t row = row0 + g * GRP + j;
+                  key = ((uint64_t)__float_as_uint(d) << 32) | (uint32_t)row;
+                  take = d <= thr[i] && row < a.n && row != self;
                 }
+                const uint32_t bal = __ballot_sync(0xffffffffu, take);
+                if (take) {
+                  const uint32_t e = queued + __popc(bal & ((1u << lane) - 1));
+                  queue_key[e] = key;
+                  queue_q[e] = qi[i];
+                }
+                queued += __popc(bal);
+                if (queued >= 32) flush(32);
               }
               __syncwarp();
             }
@@ -732,6 +764,7 @@ __global__ void __launch_bounds__(STH, 1)
           if (qi[i] < a.nq) atomicMax(&a.qmax[qi[i]], __float_as_uint(fmaxf(gmax[i] + qn[i], 0.f)));
       }
     }
+    if (!MINP && queued) flush(queued);
   }
 
   // ------------------------------------------------------------------------------ teardown
@@ -992,7 +1025,8 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   // resident with at least three stages of base blocks beside them, else streamed with those.
   const uint32_t NT = qtiles >= 8 || qtiles % 2 == 0 ? 2u : 1u;
   const uint32_t scratch = 32 * SW_ * GRP * 4, norms_b = SW_ * 2 * 64 * 4;
-  const int64_t room = (int64_t)smem_max - 1024 - 1024 - scratch - norms_b;  // alignment pad, barriers
+  const uint32_t queue_b = SW_ * 64 * 12;
+  const int64_t room = (int64_t)smem_max - 1024 - 1024 - scratch - norms_b - queue_b;  // alignment pad, barriers
   const uint32_t qbytes = NT * kblocks * parts * PART;
   const bool resident = (int64_t)qbytes + 3 * (int64_t)(parts * PART) <= room;
   const uint32_t stage_bytes = resident ? parts * PART : (1 + NT) * parts * PART;
@@ -1054,7 +1088,8 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     a.o_x = resident ? qbytes : 0;
     a.o_scr = a.o_x + stages * stage_bytes;
     a.o_xn = a.o_scr + scratch;
-    const size_t smem = 1024 + (size_t)a.o_xn + norms_b;
+    a.o_queue = a.o_xn + norms_b;
+    const size_t smem = 1024 + (size_t)a.o_queue + queue_b;
     auto kern = NT == 2 ? (minp ? tc_screen_kernel<2, true> : tc_screen_kernel<2, false>)
                         : (minp ? tc_screen_kernel<1, true> : tc_screen_kernel<1, false>);
     EFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

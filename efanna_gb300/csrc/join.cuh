@@ -45,27 +45,4 @@ __device__ __forceinline__ void place_record(const RecordSink& s, uint32_t t, ui
   else place_overflow(s, t, slot, d, cand, aux);
 }
 
-__device__ __forceinline__ void emit_record(const RecordSink& s, uint32_t t, float d, uint32_t cand, uint32_t aux) {
-  place_record(s, t, atomicAdd(&s.cnt[t], 1u), d, cand, aux);
-}
-
-// The record side of one join pair (a lane's pair): x is the list entry being joined, y the
-// candidate, my_new whether y comes from the new list, d their distance.  Returns whether side 0
-// dropped a candidate that a rank below check_k could have needed.
-__device__ __forceinline__ bool join_pair_records(const RecordSink& s, uint64_t i, uint32_t x, uint32_t y, bool my_new,
-                                                  float d, uint32_t P, uint32_t check_k,
-                                                  const float* __restrict__ bound) {
-  if (my_new && y == x) return false;  // equal ids: no pair
-  uint32_t a = x, b = y;
-  if (my_new && b < a) {
-    a = y;
-    b = x;
-  }
-  // side 0: candidate b into node a (its rank feeds found); side 1: a into b
-  const float ba = bound[a], bb = bound[b];
-  if (d <= ba) emit_record(s, a, d, b, (uint32_t)(i << 1));
-  if (d <= bb) emit_record(s, b, d, a, (uint32_t)(i << 1) | 1u);
-  return !(d <= ba) && P < check_k;
-}
-
 }  // namespace efg

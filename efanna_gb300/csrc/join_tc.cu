@@ -8,7 +8,7 @@
 // blocks of a BF16 copy of the base.
 //
 //   * Three launches per join.  Tiles of TR = 128 rows (128 TMEM columns, three CTAs per SM) take
-//     the nodes in order, 32 consecutive nodes at a time from a counter, packed in order; a node
+//     the nodes in order, up to 32 consecutive nodes at a time from a counter, packed in order; a node
 //     with more rows goes to a list that tiles of TR = 256 rows (two CTAs per SM) pack next; a node
 //     with more than 128 new entries or 256 rows goes to a second list, scored tile by tile: a
 //     block of new entries (the tile's first rows) with a chunk of the candidates after the block,
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
   __shared__ uint32_t cum[JM + 1];                 // pairs of the tile's new entries before each one
   __shared__ uint8_t rnode[JM];                    // tile node of each new entry
   __shared__ uint32_t rows_sh[TR];                 // the tile's rows: all new entries, then all old ones
-  __shared__ float norm_sh[TR];
+  __shared__ float norm_sh[TR], bound_sh[TR];
   __shared__ uint32_t tmem_base_sh, chn_sh, chpos_sh, tn_sh, nsum_sh, tsum_sh;
   __shared__ uint32_t next_k0_sh, next_cn_sh;  // the chunk being fetched (published after a barrier)
   __shared__ int abort_sh, rec_fail_sh, bad_sh;
@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
         }
         rows_sh[b] = r;
         norm_sh[b] = a.xnorm[r];
+        bound_sh[b] = a.bound[r];
         if (b < A) rnode[b] = 0;
       }
     } else {
@@ -209,11 +210,14 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
       // step): a warp that read it late would take another branch and miss the barriers
       const bool fetch = chpos_sh >= chn_sh;
       __syncthreads();
-      if (fetch) {  // the chunk is packed: the next JCH nodes
+      if (fetch) {  // the chunk is packed: the next nodes
         if (threadIdx.x == 0) {
           const uint32_t total = a.mode == MODE_LIST ? a.mid[0] : a.count;
-          const uint32_t k0 = *abort_flag ? total : atomicAdd(a.next_node, JCH);
-          next_cn_sh = k0 < total ? min(JCH, total - k0) : 0;
+          // up to JCH, fewer where the launch has few per CTA (a chunk of large nodes at the end would
+          // leave the others waiting)
+          const uint32_t step = min(JCH, max(total / (gridDim.x * 8), a.mode == MODE_LIST ? 2u : 8u));
+          const uint32_t k0 = *abort_flag ? total : atomicAdd(a.next_node, step);
+          next_cn_sh = k0 < total ? min(step, total - k0) : 0;
           next_k0_sh = k0;
         }
         __syncthreads();
@@ -289,6 +293,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
           const uint32_t b = e < nn ? tnb[j] + e : tob[j] + e - nn;
           rows_sh[b] = r;
           norm_sh[b] = a.xnorm[r];
+          bound_sh[b] = a.bound[r];
           if (e < nn) rnode[b] = (uint8_t)j;
         }
       }
@@ -418,33 +423,57 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
           // pairs of new entries q0 .. q1 - 1, one per thread
           const uint32_t q1 = min(Ns, q0 + 32), u1 = cum[q1];
           uint32_t r = q0;
-          for (uint32_t u = cum[q0] + t; u < u1; u += JRT) {
-            while (u >= cum[r + 1]) ++r;
-            const uint32_t off = u - cum[r];
-            uint32_t bc;    // the candidate's row in the tile
-            bool cand_new;  // the candidate is a new entry
-            uint64_t node;
-            if (big) {
-              const uint32_t tl = bm_tri ? Ns - r - 1 : 0;  // the row's pairs within the new block
-              if (off < tl) {
-                bc = r + 1 + off;
-                cand_new = true;
+          constexpr int RU = 2;  // pairs per thread at a time: their slots' atomics are in flight together
+          for (uint32_t u0 = cum[q0] + t; u0 < u1; u0 += RU * JRT) {
+            uint32_t tgt[2 * RU], slot[2 * RU], aux[RU];
+            float d[RU];
+            uint32_t put = 0;
+#pragma unroll
+            for (int p = 0; p < RU; ++p) {
+              const uint32_t u = u0 + p * JRT;
+              if (u >= u1) continue;
+              while (u >= cum[r + 1]) ++r;
+              const uint32_t off = u - cum[r];
+              uint32_t bc;    // the candidate's row in the tile
+              bool cand_new;  // the candidate is a new entry
+              uint64_t node;
+              if (big) {
+                const uint32_t tl = bm_tri ? Ns - r - 1 : 0;  // the row's pairs within the new block
+                if (off < tl) {
+                  bc = r + 1 + off;
+                  cand_new = true;
+                } else {
+                  bc = Ns + (off - tl);
+                  cand_new = bm_tc0 + (off - tl) < bm_nn;
+                }
+                node = bm_node;
               } else {
-                bc = Ns + (off - tl);
-                cand_new = bm_tc0 + (off - tl) < bm_nn;
+                const uint32_t j = rnode[r], sl = tslot[j], nn = nn_ch[sl];
+                const uint32_t cl = r - tnb[j] + 1 + off;  // candidate within the node's lists
+                bc = cl < nn ? tnb[j] + cl : tob[j] + (cl - nn);
+                cand_new = cl < nn;
+                node = id_ch[sl];
               }
-              node = bm_node;
-            } else {
-              const uint32_t j = rnode[r], sl = tslot[j], nn = nn_ch[sl];
-              const uint32_t cl = r - tnb[j] + 1 + off;  // candidate within the node's lists
-              bc = cl < nn ? tnb[j] + cl : tob[j] + (cl - nn);
-              cand_new = cl < nn;
-              node = id_ch[sl];
+              const float dot = gram[(r - q0) * DLD + bc];
+              d[p] = fmaxf(fmaf(-2.f, dot, norm_sh[r] + norm_sh[bc]), 0.f);
+              const uint32_t x = rows_sh[r], y = rows_sh[bc];
+              if (cand_new && y == x) continue;  // equal ids: no pair
+              // side 0: the larger id of two new entries into the smaller one's node, else y into x
+              const bool swap = cand_new && y < x;
+              const float b0 = bound_sh[swap ? bc : r], b1 = bound_sh[swap ? r : bc];
+              tgt[2 * p] = swap ? y : x;
+              tgt[2 * p + 1] = swap ? x : y;
+              aux[p] = (uint32_t)(node << 1);
+              if (d[p] <= b0) put |= 1u << (2 * p);
+              else if (a.P < a.check_k) a.found[node] = 1;
+              if (d[p] <= b1) put |= 2u << (2 * p);
             }
-            const float dot = gram[(r - q0) * DLD + bc];
-            const float d = fmaxf(fmaf(-2.f, dot, norm_sh[r] + norm_sh[bc]), 0.f);
-            if (join_pair_records(a.sink, node, rows_sh[r], rows_sh[bc], cand_new, d, a.P, a.check_k, a.bound))
-              a.found[node] = 1;
+#pragma unroll
+            for (int e = 0; e < 2 * RU; ++e)
+              if (put >> e & 1u) slot[e] = atomicAdd(&a.sink.cnt[tgt[e]], 1u);
+#pragma unroll
+            for (int e = 0; e < 2 * RU; ++e)
+              if (put >> e & 1u) place_record(a.sink, tgt[e], slot[e], d[e >> 1], tgt[e ^ 1], aux[e >> 1] | (e & 1));
           }
           rec_sync();  // the Gram rows are overwritten by the next 32 entries
         }
