@@ -433,7 +433,7 @@ __global__ void bound_kernel(const uint64_t* __restrict__ lists, uint64_t nq, ui
 // a time (256 queries, 512 TMEM columns with two buffers), which reads each base block once per 256
 // queries: 32 KB per 1024 cycles at 128 dimensions instead of 64 KB per 512.  The screening warps spend
 // one packed FMA and one three-input minimum per two values.
-constexpr uint32_t SW_ = 8;                     // screening warps
+constexpr uint32_t SW_ = 16;                    // screening warps: eight per accumulator buffer
 constexpr uint32_t STH = 64 + 32 * SW_;         // threads
 constexpr uint32_t CAND_MAX = 4096;             // candidates a query's buffer can hold
 
@@ -447,7 +447,8 @@ struct ScreenArgs {
   int* err;
   uint64_t n, first_row;
   uint32_t ntiles, chunk_tiles, nchunks, qgroups, nq, cap, kblocks, stages, exclude_self;
-  uint32_t group_tiles;   // MIN pass: tiles per group of a thread's 64 columns (0: groups of 16 columns)
+  uint32_t group_tiles;   // MIN pass: a thread's tiles (every other one) per group of its 64 columns (0: groups of
+                          // 16 columns); a chunk holds a multiple of 2 group_tiles
   uint32_t split, resident;
   float rel;              // the bound is widened by this much (passes of the split form may round differently)
   uint32_t stage_bytes, o_x, o_scr, o_xn, o_queue;
@@ -488,7 +489,8 @@ __global__ void __launch_bounds__(STH, 1)
   unsigned char* smem = smem_raw + pad;
   const uint32_t sbase = raw + pad;
   const uint32_t parts = a.split ? 2u : 1u;  // hi, or hi and lo blocks
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (the shuffle tells the compiler that the warp index is the same in all lanes)
+  const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < a.stages; ++s) {
       mbar_init(smem_addr(&bar_full[s]), 1);
@@ -496,7 +498,7 @@ __global__ void __launch_bounds__(STH, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_addr(&bar_tfull[b]), 1);
-      mbar_init(smem_addr(&bar_tempty[b]), 32 * SW_);
+      mbar_init(smem_addr(&bar_tempty[b]), 16 * SW_);
     }
     mbar_init(smem_addr(&bar_q), 1);
     mbar_init(smem_addr(&bar_qfree), 1);
@@ -564,64 +566,78 @@ __global__ void __launch_bounds__(STH, 1)
       }
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer (one lane)
-    if (lane == 0) {
+    // ---------------------------------------------------------------- MMA issuer
+    // The whole warp walks the loops, so that descriptors and addresses stay in uniform registers, and one
+    // elected lane issues.  With the loops inside one lane's branch every tcgen05.mma cost about 144
+    // cycles of issue, more than twice its 64 cycles in the tensor cores.
+    {
       uint32_t s = 0, ph = 0, tcount = 0, it = 0;
       bool ok = true;
+      const bool one = elect_one();
       for (uint32_t w = blockIdx.x; ok && w < items; w += gridDim.x, ++it) {
         const uint32_t chunk = w / a.qgroups;
         const uint32_t t0 = chunk * a.chunk_tiles, t1 = min(a.ntiles, t0 + a.chunk_tiles);
-        if (a.resident && !mbar_wait(smem_addr(&bar_q), it & 1u, abort_flag, a.err)) break;
+        if (a.resident && !warp_wait(smem_addr(&bar_q), it & 1u, abort_flag, a.err)) break;
         tc_fence_after();
         for (uint32_t t = t0; ok && t < t1; ++t, ++tcount) {
           const uint32_t b = tcount & 1u, tph = (tcount >> 1) & 1u;
-          if (!mbar_wait(smem_addr(&bar_tempty[b]), tph ^ 1u, abort_flag, a.err)) {
+          if (!warp_wait(smem_addr(&bar_tempty[b]), tph ^ 1u, abort_flag, a.err)) {
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + b * NT * TN;
           for (uint32_t kb = 0; kb < a.kblocks; ++kb) {
-            if (!mbar_wait(smem_addr(&bar_full[s]), ph, abort_flag, a.err)) {
+            if (!warp_wait(smem_addr(&bar_full[s]), ph, abort_flag, a.err)) {
               ok = false;
               break;
             }
             tc_fence_after();
             const uint32_t st = sbase + a.o_x + s * a.stage_bytes;
             const uint64_t xh = sw128_desc(st), xl = sw128_desc(st + PART);
+            const uint32_t qa = a.resident ? sbase + kb * parts * PART : st + parts * PART;
+            const uint32_t qstep = a.resident ? a.kblocks * parts * PART : parts * PART;
+            const uint32_t free_bar = smem_addr(&bar_empty[s]), done_bar = smem_addr(&bar_tfull[b]);
+            const bool last = kb + 1 == a.kblocks;
+            if (one) {
 #pragma unroll
-            for (uint32_t i = 0; i < NT; ++i) {
-              const uint32_t qa = a.resident ? sbase + (i * a.kblocks + kb) * parts * PART : st + (1 + i) * parts * PART;
-              const uint64_t qh = sw128_desc(qa), ql = sw128_desc(qa + PART);
+              for (uint32_t i = 0; i < NT; ++i) {
+                const uint64_t qh = sw128_desc(qa + i * qstep), ql = sw128_desc(qa + i * qstep + PART);
 #pragma unroll
-              for (uint32_t j = 0; j < TKB / 16; ++j) {  // K = 16 per MMA: 32 bytes further along the row
-                const uint64_t o = (uint64_t)(2 * j);
-                umma_bf16(d_tmem + i * TN, qh + o, xh + o, IDESC, (kb | j) != 0 ? 1u : 0u);
-                if (a.split) {
-                  umma_bf16(d_tmem + i * TN, qh + o, xl + o, IDESC, 1u);
-                  umma_bf16(d_tmem + i * TN, ql + o, xh + o, IDESC, 1u);
+                for (uint32_t j = 0; j < TKB / 16; ++j) {  // K = 16 per MMA: 32 bytes further along the row
+                  const uint64_t o = (uint64_t)(2 * j);
+                  umma_bf16(d_tmem + i * TN, qh + o, xh + o, IDESC, (kb | j) != 0 ? 1u : 0u);
+                  if (a.split) {
+                    umma_bf16(d_tmem + i * TN, qh + o, xl + o, IDESC, 1u);
+                    umma_bf16(d_tmem + i * TN, ql + o, xh + o, IDESC, 1u);
+                  }
                 }
               }
+              umma_commit(free_bar);               // frees the stage when these MMAs have read it
+              if (last) umma_commit(done_bar);     // buffer b holds the tile
             }
             mma_issued = true;
-            umma_commit(smem_addr(&bar_empty[s]));  // frees the stage when these MMAs have read it
+            __syncwarp();
             if (++s == a.stages) {
               s = 0;
               ph ^= 1u;
             }
           }
-          if (!ok) break;
-          umma_commit(smem_addr(&bar_tfull[b]));  // buffer b holds the tile
         }
-        if (ok && a.resident) umma_commit(smem_addr(&bar_qfree));
+        if (ok && a.resident && one) umma_commit(smem_addr(&bar_qfree));
+        __syncwarp();
       }
+      if (one && mma_issued) umma_commit(smem_addr(&bar_drain));  // by the lane that issued them
     }
   } else {
     // ---------------------------------------------------------------- screening (warps 2 ..)
-    const uint32_t ew = warp - 2, quad = warp & 3u, half = ew >> 2;  // TMEM lanes 32 quad .., columns 64 half ..
+    // eight warps screen the tiles of one accumulator buffer, eight the other's: a tile's chain of waiting,
+    // TMEM reads and tests takes longer than its products, and two run side by side this way
+    const uint32_t ew = warp - 2, quad = warp & 3u, half = (ew >> 2) & 1u, b = ew >> 3;  // TMEM lanes 32 quad ..,
+    const uint32_t taddr0 = tmem_base + ((quad * 32u) << 16) + b * NT * TN + half * 64;  // columns 64 half ..
     float* scr = reinterpret_cast<float*>(smem + a.o_scr) + (ew * 32 + lane) * GRP;
     const uint32_t sw = (lane >> 1) & 3u;  // (the copy of a group's 16 values: float4 slot j at j ^ sw)
-    float* xw = reinterpret_cast<float*>(smem + a.o_xn) + ew * 2 * 64;  // norms of 64 rows, two copies
+    float* xw = reinterpret_cast<float*>(smem + a.o_xn) + ew * 2 * 64;  // norms of 64 rows, this tile's and the next
     const uint64_t m2 = pack2(__float_as_uint(-2.f), __float_as_uint(-2.f));
     // candidates on their way to the queries' buffers: 32 slots are taken at once, an atomic per lane
     // (one at a time their latency held the warp at every hit: 4.6 of 7.0 ms at 10k x 1M x 128)
@@ -665,32 +681,38 @@ __global__ void __launch_bounds__(STH, 1)
         gmin[i] = INFINITY;
         gmax[i] = -INFINITY;
       }
-      reinterpret_cast<float2*>(xw + (tcount & 1u) * 64)[lane] =
-          __ldg(reinterpret_cast<const float2*>(a.xnorm + (uint64_t)t0 * TN + half * 64) + lane);
+      const uint32_t first = t0 + ((tcount & 1u) ^ b);  // this buffer's tiles: first, first + 2, ...
+      const uint32_t item_end = tcount + (t1 - t0);
+      uint32_t flip = 0, in_group = 0;
+      if (first < t1)
+        reinterpret_cast<float2*>(xw)[lane] =
+            __ldg(reinterpret_cast<const float2*>(a.xnorm + (uint64_t)first * TN + half * 64) + lane);
       __syncwarp();
-      for (uint32_t t = t0; t < t1; ++t, ++tcount) {
-        const uint32_t b = tcount & 1u, tph = (tcount >> 1) & 1u;
+      for (uint32_t t = first; t < t1; t += 2, flip ^= 1u) {
+        const uint32_t tph = ((tcount + (t - t0)) >> 1) & 1u;
         const uint64_t row0 = (uint64_t)t * TN + half * 64;
         float2 xnext = make_float2(0.f, 0.f);
-        if (t + 1 < t1) xnext = __ldg(reinterpret_cast<const float2*>(a.xnorm + row0 + TN) + lane);  // in flight meanwhile
+        if (t + 2 < t1) xnext = __ldg(reinterpret_cast<const float2*>(a.xnorm + row0 + 2 * TN) + lane);  // in flight meanwhile
         ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&bar_tfull[b]), tph, abort_flag, a.err));
         if (!ok) break;
         tc_fence_after();
-        const uint32_t taddr = tmem_base + ((quad * 32u) << 16) + b * NT * TN + half * 64;
-        const float* xs = xw + (tcount & 1u) * 64;
+        const float* xs = xw + flip * 64;
 #pragma unroll
         for (int i = 0; i < NT; ++i) {
-          uint32_t v[64];
-          tmem_ld64(taddr + i * TN, v);
-          tmem_wait();
+          uint32_t v[32];
 #pragma unroll
           for (uint32_t g = 0; g < 64 / GRP; ++g) {
+            if (g % 2 == 0) {  // 32 columns at a time (64 would not leave 16 warps their registers)
+              tmem_ld16(taddr0 + i * TN + g * GRP, v);
+              tmem_ld16(taddr0 + i * TN + g * GRP + 16, v + 16);
+              tmem_wait();
+            }
             const ulonglong2* x2 = reinterpret_cast<const ulonglong2*>(xs + g * GRP);
             float m0 = INFINITY, m1 = INFINITY;
 #pragma unroll
             for (uint32_t j = 0; j < GRP / 4; ++j) {
               const ulonglong2 xn = x2[j];
-              const uint32_t o = g * GRP + 4 * j;
+              const uint32_t o = (g % 2) * GRP + 4 * j;
               float p0, p1, p2, p3;
               unpack2(fma2(m2, pack2(v[o], v[o + 1]), xn.x), p0, p1);
               unpack2(fma2(m2, pack2(v[o + 2], v[o + 3]), xn.y), p2, p3);
@@ -708,7 +730,7 @@ __global__ void __launch_bounds__(STH, 1)
 #pragma unroll
                 for (uint32_t j = 0; j < GRP / 4; ++j) {
                   const float4 xn = reinterpret_cast<const float4*>(xs + g * GRP)[j];
-                  const uint32_t o = g * GRP + 4 * j;
+                  const uint32_t o = (g % 2) * GRP + 4 * j;
                   hits |= (fmaf(-2.f, __uint_as_float(v[o + 0]), xn.x) <= lim[i] ? 1u : 0u) << (4 * j);
                   hits |= (fmaf(-2.f, __uint_as_float(v[o + 1]), xn.y) <= lim[i] ? 2u : 0u) << (4 * j);
                   hits |= (fmaf(-2.f, __uint_as_float(v[o + 2]), xn.z) <= lim[i] ? 4u : 0u) << (4 * j);
@@ -747,8 +769,9 @@ __global__ void __launch_bounds__(STH, 1)
         }
         tc_fence_before();
         mbar_arrive(smem_addr(&bar_tempty[b]));  // buffer b may be overwritten
-        if (t + 1 < t1) reinterpret_cast<float2*>(xw + ((tcount + 1) & 1u) * 64)[lane] = xnext;
-        if (MINP && a.group_tiles && (t + 1 - t0) % a.group_tiles == 0) {
+        if (t + 2 < t1) reinterpret_cast<float2*>(xw + (flip ^ 1u) * 64)[lane] = xnext;
+        if (MINP && a.group_tiles && ++in_group == a.group_tiles) {
+          in_group = 0;
 #pragma unroll
           for (int i = 0; i < NT; ++i) {
             gmax[i] = fmaxf(gmax[i], gmin[i]);
@@ -758,6 +781,7 @@ __global__ void __launch_bounds__(STH, 1)
         __syncwarp();
       }
       if (!ok) break;
+      tcount = item_end;
       if (MINP) {
 #pragma unroll
         for (int i = 0; i < NT; ++i)
@@ -770,8 +794,7 @@ __global__ void __launch_bounds__(STH, 1)
   // ------------------------------------------------------------------------------ teardown
   __syncthreads();
   if (warp == 1) {
-    if (lane == 0 && mma_issued) {  // every MMA this thread issued has finished before TMEM is freed
-      umma_commit(smem_addr(&bar_drain));
+    if (lane == 0 && mma_issued) {  // every MMA has finished before TMEM is freed
       unsigned long long t0 = clock64();
       while (!mbar_try_wait(smem_addr(&bar_drain), 0)) {
         if (clock64() - t0 > WAIT_CYCLES) {
@@ -1021,17 +1044,20 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   const uint32_t terms = split ? 3u : 1u, parts = split ? 2u : 1u;
 
   // Query tiles per item, and whether their blocks stay in shared memory: two tiles unless that would
-  // leave a tile empty for a few queries (300 queries: three tiles as three items, not two pairs);
-  // resident with at least three stages of base blocks beside them, else streamed with those.
-  const uint32_t NT = qtiles >= 8 || qtiles % 2 == 0 ? 2u : 1u;
-  const uint32_t scratch = 32 * SW_ * GRP * 4, norms_b = SW_ * 2 * 64 * 4;
-  const uint32_t queue_b = SW_ * 64 * 12;
+  // leave a tile empty for a few queries (300 queries: three tiles as three items, not two pairs) or the
+  // stages would not fit; resident with at least three stages of base blocks beside them, else streamed
+  // with those.
+  const uint32_t scratch = 32 * SW_ * GRP * 4, norms_b = SW_ * 2 * 64 * 4, queue_b = SW_ * 64 * 12;
   const int64_t room = (int64_t)smem_max - 1024 - 1024 - scratch - norms_b - queue_b;  // alignment pad, barriers
-  const uint32_t qbytes = NT * kblocks * parts * PART;
-  const bool resident = (int64_t)qbytes + 3 * (int64_t)(parts * PART) <= room;
-  const uint32_t stage_bytes = resident ? parts * PART : (1 + NT) * parts * PART;
-  const uint32_t stages = (uint32_t)std::min<int64_t>(MAX_STAGES, (room - (resident ? qbytes : 0)) / stage_bytes);
-  if (stages < 2) return fail(EFG_ERR_ARG, "tensor-core k-NN: shared memory");
+  uint32_t NT = qtiles >= 8 || qtiles % 2 == 0 ? 2u : 1u, qbytes, stage_bytes, stages;
+  bool resident;
+  for (;; NT = 1) {
+    qbytes = NT * kblocks * parts * PART;
+    resident = (int64_t)qbytes + 3 * (int64_t)(parts * PART) <= room;
+    stage_bytes = resident ? parts * PART : (1 + NT) * parts * PART;
+    stages = (uint32_t)std::min<int64_t>(MAX_STAGES, (room - (resident ? qbytes : 0)) / stage_bytes);
+    if (stages >= 2 || NT == 1) break;
+  }
   const uint32_t qgroups = (uint32_t)((qtiles + NT - 1) / NT);
 
   CUtensorMap mqh, mql, mxh, mxl;
@@ -1049,7 +1075,7 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
                   uint32_t group_tiles, const uint32_t* qbound, uint32_t* qmax, uint32_t* cnt, uint64_t* buf,
                   uint32_t cap, int excl) -> int {
     ScreenArgs a;
-    const uint64_t tiles = (rows + TN - 1) / TN, unit = std::max<uint32_t>(1, group_tiles);
+    const uint64_t tiles = (rows + TN - 1) / TN, unit = std::max<uint32_t>(1, 2 * group_tiles);
     const uint64_t units = (tiles + unit - 1) / unit;
     double best = 1e300;
     for (uint64_t nc = 1; nc <= std::min<uint64_t>(units, 512); ++nc) {
@@ -1113,7 +1139,7 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   const size_t sel_smem = (size_t)cap * 8 + (size_t)rank * 8;
   EFG_CUDA(cudaFuncSetAttribute(select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem));
   const uint64_t S1 = std::min<uint64_t>(n / 16, 1u << 20) / TN * TN;  // rows of the append pass's sample
-  const uint64_t gtiles = (rank + 1) / 2;                              // tiles that hold `rank` groups of 64 columns
+  const uint64_t gtiles = (rank + 3) / 4 * 2;                          // tiles that hold `rank` groups of 64 columns, an even number
   uint32_t S = 0;
   bool bounded = true;
   if (S1 >= gtiles * TN) {
@@ -1153,9 +1179,9 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   } else if (n >= 16ull * (rank + 8)) {  // a small base: groups of it all (the last tile may be partly empty)
     const uint64_t full = n / TN;
     uint32_t gt = 0;  // groups of 16 columns, or of 64 columns x gt tiles
-    while (full / (gt ? 2 * gt : 1) * 2 >= rank) gt = gt ? 2 * gt : 1;
+    while (full / (gt ? 4 * gt : 2) * 4 >= rank) gt = gt ? 2 * gt : 1;
     if (gt || full * 8 >= rank) {
-      const uint64_t rows = gt ? full / gt * gt * TN : full * TN;
+      const uint64_t rows = gt ? full / (2 * gt) * (2 * gt) * TN : full * TN;
       CUtensorMap m0h, m0l;
       EFG_TRY(make_map(&m0h, xh, rows, W));
       EFG_TRY(make_map(&m0l, split ? xl : xh, rows, W));
