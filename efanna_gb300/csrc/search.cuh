@@ -21,6 +21,7 @@ struct SearchCfg {
   uint32_t o_ids, o_ht, o_u;
   uint32_t o_lstart, o_seqoff, o_tkey, o_tpos;  // fill phase (absolute)
   uint32_t o_res, o_tmp, o_newk, o_surv;                // select phase (absolute)
+  uint32_t sel_cap;     // pool keys the select phase holds at once (0: not the whole pool)
   uint32_t q4;          // staged query length in float4 (covers both row layouts)
   // reduced-precision screening (BF16 or FP8): BF16 rows ld16 values apart, cpr16 16-byte chunks
   // per row, 2^gshift16 lanes per row in the gather; the first `rerank` results are re-scored in
