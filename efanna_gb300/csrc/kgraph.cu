@@ -15,6 +15,12 @@
 //
 // Equal distances are ordered by id (the reference orders them by arrival).  The visited set is
 // the reference's N-bit `flags`: one bitset per warp in global memory, cleared per query.
+//
+// A query is a serial chain of expansions (graph row, visited bits and rows, list), so latency and the
+// number of warps in flight bound it.  Over byte rows the row loads don't wait for the visited bits, the
+// new keys are ranked instead of sorted, eight lanes share a row (128 dimensions) so that an expansion's
+// rows are one pass, and 64 registers hold 32 warps per SM: 4000 queries (1M x 128, 6 rounds, pool 4000,
+// extend 500) in 18.3 ms, 28.2 ms in FP32 rows with 24 warps per SM.
 #include <algorithm>
 
 #include "search.cuh"
@@ -35,6 +41,8 @@ struct KgCfg {
   uint32_t ld4, words;       // float4 per base row; bitset words per warp (multiple of 4)
   uint32_t warp_bytes;       // shared memory per warp
   uint32_t o_list, o_res, o_res2;
+  uint32_t cprb, gshiftb;    // byte rows: 16-byte chunks per row, 2^gshiftb >= cprb lanes per row
+  uint32_t o_qb;             // the query's bytes in the warp's shared memory
   uint32_t full_rows;        // 1: an expansion visits the whole graph row, else its first E ids
 };
 
@@ -140,22 +148,66 @@ __device__ __forceinline__ void row_dists_pass(const float4* qv, uint32_t ld4, c
 
 // Squared distances from the query (shared memory, ld4 float4, zero padded) to the rows named by
 // lanes 0..cnt-1 (`id`); lane u returns row u's distance.  Eight rows are in flight per pass, four
-// in a last pass of at most four rows (most expansions bring fewer than five new neighbours).
+// in a last pass of at most four rows (most expansions bring fewer than five new neighbours), or always
+// (EIGHT false: fewer registers).
+template <bool EIGHT>
 __device__ __forceinline__ float warp_row_dists(const float4* qv, uint32_t ld4, const float* __restrict__ base, uint32_t ld,
                                 uint32_t id, uint32_t cnt, uint32_t lane) {
   float mine = 0.f;
-  for (uint32_t u0 = 0; u0 < cnt; u0 += 8) {
-    if (cnt - u0 <= 4) row_dists_pass<4>(qv, ld4, base, ld, id, cnt, u0, lane, mine);
+  for (uint32_t u0 = 0; u0 < cnt; u0 += EIGHT ? 8 : 4) {
+    if (!EIGHT || cnt - u0 <= 4) row_dists_pass<4>(qv, ld4, base, ld, id, cnt, u0, lane, mine);
     else row_dists_pass<8>(qv, ld4, base, ld, id, cnt, u0, lane, mine);
   }
   return mine;
 }
 
-__global__ void __launch_bounds__(KG_WARPS * 32, 6) kgraph_kernel(
+// The same from byte rows for a query of bytes (qb its 16-byte chunks, qn its squared norm), for all cnt
+// <= 32 lanes' ids at once: eight lanes (at 128 dimensions) share a row, d = qn + sum x (x - 2 q).
+__device__ __forceinline__ float warp_row_dists_bytes(const uint4* qb, uint32_t qn, const uint8_t* __restrict__ rows,
+                                                      uint32_t cpr, uint32_t gshift, uint32_t id, uint32_t cnt,
+                                                      uint32_t lane) {
+  const uint32_t G = 1u << gshift, rpi = 32u >> gshift, sub = lane >> gshift, cl = lane & (G - 1);
+  const uint4* rows4 = reinterpret_cast<const uint4*>(rows);
+  const bool on = cl < cpr;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  const uint4 q = on ? qb[cl] : zero;
+  int mine = 0;
+  for (uint32_t r0 = 0; r0 < cnt; r0 += 4 * rpi) {
+    uint4 x[4];
+    int acc[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t r = r0 + u * rpi + sub, rid = __shfl_sync(FULL, id, r & 31);
+      x[u] = on && r < cnt ? __ldg(rows4 + (uint64_t)rid * cpr + cl) : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t xx = __dp4a(x[u].x, x[u].x, __dp4a(x[u].y, x[u].y, __dp4a(x[u].z, x[u].z, __dp4a(x[u].w, x[u].w, 0u))));
+      const uint32_t xq = __dp4a(x[u].x, q.x, __dp4a(x[u].y, q.y, __dp4a(x[u].z, q.z, __dp4a(x[u].w, q.w, 0u))));
+      acc[u] = (int)xx - 2 * (int)xq;
+    }
+    for (uint32_t o = G >> 1; o > 0; o >>= 1) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[u] += __shfl_xor_sync(FULL, acc[u], o);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {  // row r0 + u rpi + i sits with group i
+      const uint32_t rel = lane - r0 - u * rpi;
+      const int t = __shfl_sync(FULL, acc[u], (rel & (rpi - 1)) << gshift);
+      if (rel < rpi) mine = t;
+    }
+  }
+  return (float)((int)qn + mine);
+}
+
+// BYTES: over byte rows (a query that is no byte row goes to the FP32 rows).  Registers bound the warps per
+// SM, and a call ends with its last wave of queries: 4000 queries on 24 warps per SM are two waves.
+template <bool BYTES>
+__global__ void __launch_bounds__(KG_WARPS * 32, BYTES ? 8 : 6) kgraph_kernel(
     const float* __restrict__ base, uint32_t dim, uint32_t ld, const uint64_t* __restrict__ gptr,
     const uint32_t* __restrict__ gids, const float* __restrict__ queries, uint64_t nq, uint64_t qld,
     const uint64_t* __restrict__ keys, KgCfg c, int32_t* __restrict__ out, uint32_t* __restrict__ bits,
-    unsigned long long* __restrict__ stats, uint32_t* __restrict__ next_query) {
+    unsigned long long* __restrict__ stats, uint32_t* __restrict__ next_query, const uint8_t* __restrict__ rowsb) {
   extern __shared__ __align__(16) unsigned char smem[];
   const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   unsigned char* ws = smem + (size_t)wib * c.warp_bytes;
@@ -182,6 +234,22 @@ __global__ void __launch_bounds__(KG_WARPS * 32, 6) kgraph_kernel(
       v.z = e + 2 < dim ? qrow[e + 2] : 0.f;
       v.w = e + 3 < dim ? qrow[e + 3] : 0.f;
       qv[i] = v;
+    }
+    bool qbytes = false;
+    uint32_t qn = 0;
+    if (BYTES) {  // the query's bytes, where it has them, and its squared norm
+      bool other = false;
+      __syncwarp();
+      for (uint32_t i = lane; i < c.cprb * 4; i += 32) {
+        const float4 v = i < c.ld4 ? qv[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const bool o = !is_byte(v.x) || !is_byte(v.y) || !is_byte(v.z) || !is_byte(v.w);
+        const uint32_t w = o ? 0u : (uint32_t)v.x | (uint32_t)v.y << 8 | (uint32_t)v.z << 16 | (uint32_t)v.w << 24;
+        reinterpret_cast<uint32_t*>(ws + c.o_qb)[i] = w;
+        qn = __dp4a(w, w, qn);
+        other |= o;
+      }
+      qn = __reduce_add_sync(FULL, qn);
+      qbytes = !__any_sync(FULL, other);
     }
     uint4* v4 = reinterpret_cast<uint4*>(vis);
     for (uint32_t i = lane; i < c.words / 4; i += 32) v4[i] = make_uint4(0, 0, 0, 0);
@@ -249,32 +317,65 @@ __global__ void __launch_bounds__(KG_WARPS * 32, 6) kgraph_kernel(
             uint32_t bit = 1u << (nb & 31);
             fresh = !(atomicOr(&vis[nb >> 5], bit) & bit);
           }
-          uint32_t fm = __ballot_sync(FULL, fresh);
-          uint32_t cnt = __popc(fm);
-          if (cnt == 0) continue;
-          uint32_t src = lane < cnt ? __fns(fm, 0, lane + 1) : 0;
-          uint32_t my = __shfl_sync(FULL, nb, src);
-          float d = warp_row_dists(qv, c.ld4, base, ld, my, cnt, lane);
+          uint32_t fm, cnt;
+          uint64_t dk = ~0ULL;  // lane l < cnt: the l-th smallest new key
+          if (BYTES && qbytes) {
+            // all neighbours' distances, without waiting for the visited bits (a byte row is one line); the
+            // fresh ones are ranked by counting
+            const float d = warp_row_dists_bytes(reinterpret_cast<const uint4*>(ws + c.o_qb), qn, rowsb, c.cprb,
+                                                 c.gshiftb, nb, min(32u, maxM - m0), lane);
+            fm = __ballot_sync(FULL, fresh);
+            cnt = __popc(fm);
+            if (cnt == 0) continue;
+            const uint64_t key = pack_key(d, nb);
+            uint32_t rank = 0;
+            for (uint32_t left = fm; left; left &= left - 1) {
+              const uint64_t o = __shfl_sync(FULL, key, __ffs(left) - 1);
+              rank += o < key;
+            }
+            uint64_t* slot = list + c.list_slots;  // 32 keys of scratch behind the list
+            if (fresh) slot[rank] = key;
+            __syncwarp();
+            if (lane < cnt) dk = slot[lane];
+          } else {
+            fm = __ballot_sync(FULL, fresh);
+            cnt = __popc(fm);
+            if (cnt == 0) continue;
+            uint32_t src = lane < cnt ? __fns(fm, 0, lane + 1) : 0;
+            uint32_t my = __shfl_sync(FULL, nb, src);
+            float d = warp_row_dists<!BYTES>(qv, c.ld4, base, ld, my, cnt, lane);
+            dk = warp_sort32(lane < cnt ? pack_key(d, my) : ~0ULL, lane);
+          }
           evals += cnt;
-          uint64_t dk = warp_sort32(lane < cnt ? pack_key(d, my) : ~0ULL, lane);
           // merge the cnt sorted keys into the list (capacity C)
           uint32_t lb = lane < cnt ? lower_bound_keys(list, L, dk) : L;
           uint32_t newL = min(c.C, L + cnt);
           uint32_t first = __shfl_sync(FULL, lb, 0);
-          // old entries move right: those in [lb_j, lb_{j+1}) (lb_cnt = L) by j + 1, the highest
-          // segment first, each copied from its top down (reads before writes within a round)
-          for (int32_t j = (int32_t)cnt - 1; j >= 0; --j) {
-            const uint32_t s_lo = __shfl_sync(FULL, lb, j);
-            const uint32_t s_hi = __shfl_sync(FULL, lb, j + 1 < (int32_t)cnt ? j + 1 : j);
-            const uint32_t top = j + 1 < (int32_t)cnt ? s_hi : L;
-            for (int32_t hi = (int32_t)top; hi > (int32_t)s_lo; hi -= 32) {
-              int32_t i = hi - 32 + (int32_t)lane;
-              bool act = i >= (int32_t)s_lo;
-              uint64_t v = act ? list[i] : 0;
-              __syncwarp();
-              if (act && (uint32_t)i + j + 1 < newL) list[i + j + 1] = v;
-              __syncwarp();
+          // old entry i moves right by the new keys at or before it; from the top down, 128 entries at a
+          // time, each read before any of them is written (they move by 32 at most, into places already read)
+          for (int32_t hi = (int32_t)L; hi > (int32_t)first; hi -= 128) {
+            uint64_t v[4];
+            uint32_t to[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int32_t i = hi - 128 + u * 32 + (int32_t)lane;
+              const bool act = i >= (int32_t)first;
+              v[u] = act ? list[i] : 0;
+              to[u] = act ? (uint32_t)i : 0xffffffffu;
             }
+            for (uint32_t j = 0; j < cnt; ++j) {
+              const uint32_t lbj = __shfl_sync(FULL, lb, j);
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                const int32_t i = hi - 128 + u * 32 + (int32_t)lane;
+                to[u] += i >= (int32_t)first && (int32_t)lbj <= i ? 1u : 0u;
+              }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (to[u] < newL) list[to[u]] = v[u];
+            __syncwarp();
           }
           if (lane < cnt && lb + lane < newL) list[lb + lane] = dk;
           __syncwarp();
@@ -353,12 +454,20 @@ int kgraph_search_device(efg_index* idx, const float* d_q, uint64_t nq, uint64_t
   kc.ld4 = idx->ld / 4;
   kc.words = (uint32_t)round_up((idx->n + 31) / 32, 4);
   kc.o_list = (uint32_t)round_up((uint64_t)kc.ld4 * 16, 16);
-  kc.o_res = (uint32_t)round_up(kc.o_list + (uint64_t)kc.list_slots * 8, 16);
+  kc.o_res = (uint32_t)round_up(kc.o_list + ((uint64_t)kc.list_slots + 32) * 8, 16);  // (32 keys of scratch)
   kc.o_res2 = (uint32_t)round_up(kc.o_res + (uint64_t)k * 8, 16);
-  kc.warp_bytes = (uint32_t)round_up(kc.o_res2 + (uint64_t)k * 8, 16);
+  kc.o_qb = (uint32_t)round_up(kc.o_res2 + (uint64_t)k * 8, 16);
+  EFG_TRY(make_bytes(idx));
+  const bool bytes = idx->bytes_state == 1;
+  if (bytes) {
+    kc.cprb = idx->ldb / 16;
+    while ((1u << kc.gshiftb) < kc.cprb) ++kc.gshiftb;
+  }
+  kc.warp_bytes = kc.o_qb + kc.cprb * 16;
   kc.full_rows = hs ? 1 : 0;
-  size_t smem = (size_t)KG_WARPS * kc.warp_bytes;
-  if (smem > 200 * 1024) return fail(EFG_ERR_ARG, "kgraph search: k + extend_to too large for shared memory");
+  const size_t smem = (size_t)KG_WARPS * kc.warp_bytes;
+  // 200 KB for the query and the lists; the 32 keys and the query's bytes (at most 2.1 KB) come on top
+  if (smem - KG_WARPS * (32 * 8 + kc.cprb * 16) > 200 * 1024) return fail(EFG_ERR_ARG, "kgraph search: k + extend_to too large for shared memory");
 
   SearchCfg cfg{};  // stage 1: the nnexp kernel up to the pool
   cfg.T = T;
@@ -384,11 +493,12 @@ int kgraph_search_device(efg_index* idx, const float* d_q, uint64_t nq, uint64_t
     EFG_TRY(hs->cnt->reserve(chunk));
     cfg.seed_cnt = hs->cnt->p;
   }
-  EFG_CUDA(cudaFuncSetAttribute(kgraph_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto kern = bytes ? kgraph_kernel<true> : kgraph_kernel<false>;
+  EFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int dev = 0, sms = 152, per_sm = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kgraph_kernel, KG_WARPS * 32, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, KG_WARPS * 32, smem);
   uint64_t max_warps = std::max<uint64_t>(KG_WARPS, (512ull << 20) / ((uint64_t)kc.words * 4));
   uint64_t warps = std::min<uint64_t>({round_up(chunk, KG_WARPS), (uint64_t)sms * std::max(1, per_sm) * KG_WARPS,
                                        round_up(max_warps, KG_WARPS)});
@@ -422,10 +532,10 @@ int kgraph_search_device(efg_index* idx, const float* d_q, uint64_t nq, uint64_t
       launches += (int)((m + 65534) / 65535);
     }
     if (rc != EFG_OK) break;
-    kgraph_kernel<<<(unsigned)grid, KG_WARPS * 32, smem, s>>>(idx->d_base, idx->dim, idx->ld, idx->graph.ptr.p,
+    kern<<<(unsigned)grid, KG_WARPS * 32, smem, s>>>(idx->d_base, idx->dim, idx->ld, idx->graph.ptr.p,
                                                               idx->graph.ids.p, d_q + q0 * qld, m, qld,
                                                               idx->kg_keys.p, kc, d_out + q0 * k, idx->kg_bits.p,
-                                                              idx->eval_counter.p, qctr.p + q0 / chunk);
+                                                              idx->eval_counter.p, qctr.p + q0 / chunk, idx->bytes.p);
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) rc = fail(EFG_ERR_CUDA, std::string("kgraph launch: ") + cudaGetErrorString(le));
     ++launches;
