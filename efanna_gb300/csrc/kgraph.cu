@@ -17,10 +17,10 @@
 // the reference's N-bit `flags`: one bitset per warp in global memory, cleared per query.
 //
 // A query is a serial chain of expansions (graph row, visited bits and rows, list), so latency and the
-// number of warps in flight bound it.  Over byte rows the row loads don't wait for the visited bits, the
-// new keys are ranked instead of sorted, eight lanes share a row (128 dimensions) so that an expansion's
-// rows are one pass, and 64 registers hold 32 warps per SM: 4000 queries (1M x 128, 6 rounds, pool 4000,
-// extend 500) in 18.3 ms, 28.2 ms in FP32 rows with 24 warps per SM.
+// number of warps in flight bound it.  Over byte rows the row loads don't wait for the visited bits,
+// eight lanes share a row (128 dimensions) so that an expansion's rows are one pass, and 64 registers hold 32
+// warps per SM: 4000 queries (1M x 128, 6 rounds, pool 4000, extend 500) in 18.4 ms, 28.0 ms from FP32 rows
+// on 24 warps per SM with the new keys sorted instead of ranked.
 #include <algorithm>
 
 #include "search.cuh"
@@ -74,19 +74,6 @@ __device__ void warp_sort_keys(uint64_t* a, uint32_t n, uint32_t lane) {
       }
       __syncwarp();
     }
-}
-
-// Bitonic sort of one key per lane, ascending with the lane index.
-__device__ __forceinline__ uint64_t warp_sort32(uint64_t v, uint32_t lane) {
-#pragma unroll
-  for (uint32_t k = 2; k <= 32; k <<= 1)
-#pragma unroll
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      uint64_t o = __shfl_xor_sync(FULL, v, j);
-      bool keep_min = ((lane & j) == 0) == ((lane & k) == 0);
-      v = keep_min ? (o < v ? o : v) : (o > v ? o : v);
-    }
-  return v;
 }
 
 // Sums v[0..4) over the warp's 32 lanes; lane l returns the total of v[(l >> 3) & 3].
@@ -147,16 +134,15 @@ __device__ __forceinline__ void row_dists_pass(const float4* qv, uint32_t ld4, c
 }
 
 // Squared distances from the query (shared memory, ld4 float4, zero padded) to the rows named by
-// lanes 0..cnt-1 (`id`); lane u returns row u's distance.  Eight rows are in flight per pass, four
-// in a last pass of at most four rows (most expansions bring fewer than five new neighbours), or always
-// (EIGHT false: fewer registers).
-template <bool EIGHT>
-__device__ __forceinline__ float warp_row_dists(const float4* qv, uint32_t ld4, const float* __restrict__ base, uint32_t ld,
-                                uint32_t id, uint32_t cnt, uint32_t lane) {
+// lanes 0..cnt-1 (`id`); lane u returns row u's distance.  U rows are in flight per pass; of eight, four
+// in a last pass of at most four rows (most expansions bring fewer than five new neighbours).
+template <int U>
+__device__ __forceinline__ float warp_row_dists(const float4* qv, uint32_t ld4, const float* __restrict__ base,
+                                                uint32_t ld, uint32_t id, uint32_t cnt, uint32_t lane) {
   float mine = 0.f;
-  for (uint32_t u0 = 0; u0 < cnt; u0 += EIGHT ? 8 : 4) {
-    if (!EIGHT || cnt - u0 <= 4) row_dists_pass<4>(qv, ld4, base, ld, id, cnt, u0, lane, mine);
-    else row_dists_pass<8>(qv, ld4, base, ld, id, cnt, u0, lane, mine);
+  for (uint32_t u0 = 0; u0 < cnt; u0 += U) {
+    if (U == 8 && cnt - u0 > 4) row_dists_pass<8>(qv, ld4, base, ld, id, cnt, u0, lane, mine);
+    else row_dists_pass<4>(qv, ld4, base, ld, id, cnt, u0, lane, mine);
   }
   return mine;
 }
@@ -200,10 +186,10 @@ __device__ __forceinline__ float warp_row_dists_bytes(const uint4* qb, uint32_t 
   return (float)((int)qn + mine);
 }
 
-// BYTES: over byte rows (a query that is no byte row goes to the FP32 rows).  Registers bound the warps per
-// SM, and a call ends with its last wave of queries: 4000 queries on 24 warps per SM are two waves.
-template <bool BYTES>
-__global__ void __launch_bounds__(KG_WARPS * 32, BYTES ? 8 : 6) kgraph_kernel(
+// U: FP32 rows per pass, 8 (80 registers, 24 warps per SM) or 4 (64 registers, 32 warps); with BYTES over
+// byte rows (a query that is no byte row goes to the FP32 rows).
+template <bool BYTES, int U>
+__global__ void __launch_bounds__(KG_WARPS * 32, U == 8 ? 6 : 8) kgraph_kernel(
     const float* __restrict__ base, uint32_t dim, uint32_t ld, const uint64_t* __restrict__ gptr,
     const uint32_t* __restrict__ gids, const float* __restrict__ queries, uint64_t nq, uint64_t qld,
     const uint64_t* __restrict__ keys, KgCfg c, int32_t* __restrict__ out, uint32_t* __restrict__ bits,
@@ -317,35 +303,32 @@ __global__ void __launch_bounds__(KG_WARPS * 32, BYTES ? 8 : 6) kgraph_kernel(
             uint32_t bit = 1u << (nb & 31);
             fresh = !(atomicOr(&vis[nb >> 5], bit) & bit);
           }
-          uint32_t fm, cnt;
-          uint64_t dk = ~0ULL;  // lane l < cnt: the l-th smallest new key
+          uint32_t fm, cnt, my = nb;
+          float d;
           if (BYTES && qbytes) {
-            // all neighbours' distances, without waiting for the visited bits (a byte row is one line); the
-            // fresh ones are ranked by counting
-            const float d = warp_row_dists_bytes(reinterpret_cast<const uint4*>(ws + c.o_qb), qn, rowsb, c.cprb,
-                                                 c.gshiftb, nb, min(32u, maxM - m0), lane);
+            // all neighbours' distances, without waiting for the visited bits (a byte row is one line)
+            d = warp_row_dists_bytes(reinterpret_cast<const uint4*>(ws + c.o_qb), qn, rowsb, c.cprb, c.gshiftb, nb,
+                                     min(32u, maxM - m0), lane);
             fm = __ballot_sync(FULL, fresh);
             cnt = __popc(fm);
             if (cnt == 0) continue;
-            const uint64_t key = pack_key(d, nb);
-            uint32_t rank = 0;
-            for (uint32_t left = fm; left; left &= left - 1) {
-              const uint64_t o = __shfl_sync(FULL, key, __ffs(left) - 1);
-              rank += o < key;
-            }
-            uint64_t* slot = list + c.list_slots;  // 32 keys of scratch behind the list
-            if (fresh) slot[rank] = key;
-            __syncwarp();
-            if (lane < cnt) dk = slot[lane];
-          } else {
+          } else {  // the fresh ones' distances, gathered in the first cnt lanes
             fm = __ballot_sync(FULL, fresh);
             cnt = __popc(fm);
             if (cnt == 0) continue;
-            uint32_t src = lane < cnt ? __fns(fm, 0, lane + 1) : 0;
-            uint32_t my = __shfl_sync(FULL, nb, src);
-            float d = warp_row_dists<!BYTES>(qv, c.ld4, base, ld, my, cnt, lane);
-            dk = warp_sort32(lane < cnt ? pack_key(d, my) : ~0ULL, lane);
+            my = __shfl_sync(FULL, nb, lane < cnt ? __fns(fm, 0, lane + 1) : 0);
+            d = warp_row_dists<U>(qv, c.ld4, base, ld, my, cnt, lane);
+            fresh = lane < cnt;
+            fm = __ballot_sync(FULL, fresh);
           }
+          // each new key's rank counted (usually a few keys); lane l < cnt gets the l-th smallest
+          const uint64_t key = pack_key(d, my);
+          uint32_t rank = 0;
+          for (uint32_t left = fm; left; left &= left - 1) rank += __shfl_sync(FULL, key, __ffs(left) - 1) < key;
+          uint64_t* slot = list + c.list_slots;  // 32 keys of scratch behind the list
+          if (fresh) slot[rank] = key;
+          __syncwarp();
+          const uint64_t dk = lane < cnt ? slot[lane] : ~0ULL;
           evals += cnt;
           // merge the cnt sorted keys into the list (capacity C)
           uint32_t lb = lane < cnt ? lower_bound_keys(list, L, dk) : L;
@@ -493,13 +476,17 @@ int kgraph_search_device(efg_index* idx, const float* d_q, uint64_t nq, uint64_t
     EFG_TRY(hs->cnt->reserve(chunk));
     cfg.seed_cnt = hs->cnt->p;
   }
-  auto kern = bytes ? kgraph_kernel<true> : kgraph_kernel<false>;
-  EFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int dev = 0, sms = 152, per_sm = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const uint64_t max_warps = std::max<uint64_t>(KG_WARPS, (512ull << 20) / ((uint64_t)kc.words * 4));
+  // Eight FP32 rows a pass while the queries fit the 24 warps per SM that leaves (300 queries at 100k x 960:
+  // 27.4 ms, 34.7 with four), four for more of them (4000 at 300k x 100: 19.6 ms, 26.4 with eight; at
+  // 100k x 480: 30.8 and 36.6).
+  auto kern = bytes ? kgraph_kernel<true, 4>
+                    : std::min(chunk, max_warps) > (uint64_t)sms * 6 * KG_WARPS ? kgraph_kernel<false, 4> : kgraph_kernel<false, 8>;
+  EFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, KG_WARPS * 32, smem);
-  uint64_t max_warps = std::max<uint64_t>(KG_WARPS, (512ull << 20) / ((uint64_t)kc.words * 4));
   uint64_t warps = std::min<uint64_t>({round_up(chunk, KG_WARPS), (uint64_t)sms * std::max(1, per_sm) * KG_WARPS,
                                        round_up(max_warps, KG_WARPS)});
   uint64_t grid = std::max<uint64_t>(1, warps / KG_WARPS);

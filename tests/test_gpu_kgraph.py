@@ -103,3 +103,15 @@ def test_kgraph_device_api_and_edges(efg, oracle_lib):
     idx.set_search_params(2, 100, 10, 8, -1, 7)
     with pytest.raises(efg.EfannaError):
         idx.knn_search(5, q[:3])
+
+
+def test_kgraph_more_queries_than_warps(efg, oracle_lib):
+    """Float rows and a batch beyond the warps of the eight-row kernel (24 per SM): the same queries,
+    each many times over, answered as in a small batch."""
+    x = np.random.default_rng(5).standard_normal((3000, 40)).astype(np.float32)
+    q = np.random.default_rng(6).standard_normal((50, 40)).astype(np.float32)
+    idx = efg.Index(x, efg.IndexParams(trees=8, merge_level=4, epochs=4, L=30, K=20))
+    idx.build_index()
+    idx.set_search_params(3, 300, 40, 8, -1, 1)
+    few = idx.knn_search(10, q)
+    assert np.array_equal(idx.knn_search(10, np.tile(q, (80, 1))), np.tile(few, (80, 1)))
