@@ -834,9 +834,25 @@ __device__ __forceinline__ void sort_window(uint64_t* wk, uint32_t* wa, uint32_t
   __syncwarp();
 }
 
-// Next 32 records of distance bits g in ascending (key, aux) order after `last`.
-__device__ __forceinline__ K96 next_batch(const uint4* __restrict__ rec, uint32_t B, uint32_t g, K96 last, bool first) {
+// Next 32 records of distance bits g in ascending (key, aux) order after `last`.  With `single` a lone id's
+// copies count as its first record: a pass without sorting finds whether there is one id.
+__device__ __forceinline__ K96 next_batch(const uint4* __restrict__ rec, uint32_t B, uint32_t g, K96 last, bool first,
+                                          bool single) {
   const uint32_t lane = threadIdx.x & 31;
+  if (single) {
+    K96 mn = k96_max();
+    uint32_t mx = 0;
+    for (uint32_t b = lane; b < B; b += 32) {
+      if (rec[b].y != g) continue;
+      const K96 y = rec_k96(rec[b]);
+      if (!first && !lt(last, y)) continue;
+      if (lt(y, mn)) mn = y;
+      mx = max(mx, key_id(y.k));
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    mn = shfl_idx(warp_sort32(mn), 0);
+    if (is_max(mn) || key_id(mn.k) == mx) return lane == 0 ? mn : k96_max();
+  }
   K96 run = k96_max();
   for (uint32_t b = 0; b < B; b += 32) {
     K96 x = k96_max();
@@ -857,14 +873,17 @@ __device__ __forceinline__ K96 next_batch(const uint4* __restrict__ rec, uint32_
 // interpolation and bisection on the distance bits) so that at most WIN and, as a rule, at least half
 // as many fall below it, sorted in registers and applied 32 at once (Pool::apply_batch); a pool of 30
 // is done after one window of the 78 records per node and iteration that 1M x 128 has.  More than WIN
-// records at one distance are pulled 32 at a time.  A record equal to an earlier one in all four fields
+// records at one distance are pulled 32 at a time; from a pool of check_k entries on without the copies of
+// a pair (found again from every common neighbour), which change nothing there: they are duplicates, or
+// land in the overflow slot again, at a rank of check_k or more.  A record equal to an earlier one in all four fields
 // changes nothing, so the windows need not keep its copies apart.
 // The reference rejects a candidate whose id sits among the entries of equal distance; a pair's
 // distance is the same wherever the reference computes it, so that finds every repeat.  With
 // any_dist a repeat is found at any distance: the tensor-core join's distances can differ in the
 // last bits from the FP32 ones a pool entry was inserted with, and an equal-distance test would
 // let the id in twice.
-// Bound: instruction issue and the latency of the record reads.  Sorting every record in shared memory
+// Bound: instruction issue and the latency of the record reads.  (Hubs are the tail: one of 4800 records at
+// 30 distances took 21M cycles with all copies pulled in order, 8 of its iteration's 10.8 ms.)  Sorting every record in shared memory
 // and inserting them one by one took 40 ms of the 1M x 128 build's 8 iterations and 65 ms of 6
 // iterations at 100k x 960 (P = 201).
 template <int NS>
@@ -958,7 +977,8 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_kernel(
         }
       }
       if (ties) {  // the next 32 of them
-        const K96 batch = next_batch(rec, B, tlo, last, first);
+        const bool quiet = pool.L >= check_k;
+        const K96 batch = next_batch(rec, B, tlo, last, first, quiet);
         total = __popc(__ballot_sync(0xffffffffu, !is_max(batch)));
         first = total == 0;
         if (first) {
@@ -967,6 +987,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_kernel(
           continue;
         }
         last = shfl_idx(batch, total - 1);
+        if (quiet) last.a = 0xffffffffu;  // past all its copies
         wk[lane] = batch.k;
         wa[lane] = batch.a;
         __syncwarp();
