@@ -48,6 +48,7 @@ __global__ void to_bytes_kernel(const float* __restrict__ base, uint64_t n, uint
 
 constexpr uint32_t BW = 4;       // warps per CTA
 constexpr uint32_t BROWS = 64;   // rows per tile
+constexpr uint32_t QUEUE = 256;  // records made at a time (a round of 32 blocks has 1024 at most)
 constexpr uint32_t BBLOCK = 32;  // new entries per tile of a node with more rows
 
 struct JoinBytesArgs {
@@ -77,16 +78,22 @@ __device__ __forceinline__ uint32_t row_slot(uint32_t r) { return (r & 3u) * (BR
 // The join (InitIndex::join, base_index.hpp:328-371), a warp per node: the node's rows (new entries
 // first, then old ones; a node of more than 64 rows tile by tile) go to shared memory once, then a lane
 // computes the distances of a 4 x 4 block of pairs, on or above the diagonal of (new groups x all
-// groups).  Bound: the latency of a node's chain (lists, rows, records' slots), which 20 warps per SM
-// overlap, and the records' atomics; products are 64 __dp4a per 16-byte chunk and block.
-__global__ void __launch_bounds__(BW * 32, 5) join_bytes_kernel(const JoinBytesArgs a) {
+// groups).  The pairs that make records (a fifth of them) are queued and their records made by whole warps.
+// Bound: instruction issue (half of all slots) and the latency of a node's chain (lists, rows, records'
+// slots), which 16 warps per SM overlap; products are 64 __dp4a per 16-byte chunk and block.  The 1M x 128
+// build's joins: 34.0 ms, 46.7 with each lane making the records of its own pairs, four at a time (half as
+// many instructions again), and 37.1 with 48 rows a tile and 20 warps per SM.
+__global__ void __launch_bounds__(BW * 32, 4) join_bytes_kernel(const JoinBytesArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ uint32_t id_all[BW][BROWS], norm_all[BW][BROWS];
-  __shared__ float bound_all[BW][BROWS];
+  __shared__ __align__(16) uint32_t id_all[BW][BROWS], norm_all[BW][BROWS], bound_all[BW][BROWS];
+  __shared__ uint32_t blk_all[BW][32];
+  __shared__ uint16_t queue_all[BW][QUEUE];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t* id_sh = id_all[warp];
   uint32_t* norm_sh = norm_all[warp];
-  float* bound_sh = bound_all[warp];
+  uint32_t* bound_sh = bound_all[warp];
+  uint32_t* blk_sh = blk_all[warp];
+  uint16_t* queue = queue_all[warp];
   const uint32_t rows0 = (uint32_t)__cvta_generic_to_shared(smem) + warp * BROWS * a.stride;
   uint32_t* dot_sh = reinterpret_cast<uint32_t*>(smem + BW * BROWS * a.stride) + warp * 512;
   uint32_t nk = 0;
@@ -109,7 +116,7 @@ __global__ void __launch_bounds__(BW * 32, 5) join_bytes_kernel(const JoinBytesA
         const uint32_t id = e < nn ? a.new_ids[node * a.cap + e] : a.old_ids[node * a.cap + e - nn];
         id_sh[r] = id;
         norm_sh[r] = a.norm[id];
-        bound_sh[r] = a.bound[id];
+        bound_sh[r] = __float2uint_rd(a.bound[id]);  // (distances are integers)
       }
       __syncwarp();
       for (uint32_t e = lane; e < R * a.chunks; e += 32) {
@@ -123,9 +130,11 @@ __global__ void __launch_bounds__(BW * 32, 5) join_bytes_kernel(const JoinBytesA
       // blocks (gx, gy): new group gx with group gy >= gx, or with the candidates' groups
       const uint32_t GX = (A + 3) / 4, GY = (R + 3) / 4, g0 = tri ? 0 : A / 4;
       const uint32_t nb = tri ? GX * GY - GX * (GX - 1) / 2 : GX * (GY - g0);
-      for (uint32_t b = lane; b < nb; b += 32) {
+      for (uint32_t b0 = 0; b0 < nb; b0 += 32) {
+        const uint32_t b = b0 + lane;
         uint32_t gx = 0, gy = 0;
-        if (tri) {
+        if (b >= nb) {  // (computed for nothing)
+        } else if (tri) {
           uint32_t r = b;
           while (r >= GY - gx) {
             r -= GY - gx;
@@ -159,58 +168,69 @@ __global__ void __launch_bounds__(BW * 32, 5) join_bytes_kernel(const JoinBytesA
               acc[i * 4 + j] = s;
             }
         }
-        // the lane's 16 products through shared memory, so that the record code below exists once per
-        // column and not 16 times: unrolled over the rows too it outgrew the instruction cache
+        // which of the 16 pairs make a record: bit q = 4 i + j for x's node, 16 + q for y's
+        uint32_t put = 0;
+        {
+          const uint4 xn = *reinterpret_cast<const uint4*>(norm_sh + gx * 4), yn = *reinterpret_cast<const uint4*>(norm_sh + gy * 4);
+          const uint4 xb = *reinterpret_cast<const uint4*>(bound_sh + gx * 4), yb = *reinterpret_cast<const uint4*>(bound_sh + gy * 4);
+          const uint32_t nx[4] = {xn.x, xn.y, xn.z, xn.w}, ny[4] = {yn.x, yn.y, yn.z, yn.w};
+          const uint32_t bx[4] = {xb.x, xb.y, xb.z, xb.w}, by[4] = {yb.x, yb.y, yb.z, yb.w};
+#pragma unroll
+          for (int q = 0; q < 16; ++q) {
+            acc[q] = nx[q / 4] + ny[q % 4] - 2 * acc[q];
+            put |= (acc[q] <= bx[q / 4] ? 1u << q : 0u) | (acc[q] <= by[q % 4] ? 0x10000u << q : 0u);
+          }
+        }
+        // pairs of the tile: rows x < A, columns y < R, above the diagonal or past the new entries
+        uint32_t ok = 0;
+        if (b < nb) {
+          const uint32_t na = min(A - gx * 4, 4u), ny = min(R - gy * 4, 4u), y0 = tri ? 0 : max(A, gy * 4) - gy * 4;
+          ok = (0xffffu >> (16 - 4 * na)) & (0x1111u * ((1u << ny) - (1u << y0)));
+          if (tri && gx == gy) ok &= 0x08ceu;  // j > i
+        }
+        put &= ok | ok << 16;
+        // the distances to shared memory: the records are made by whole warps, a lane each, from a queue of
+        // (block, pair, side) -- made by the lanes that found them, a lane's 32 chances had each to be tried
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           *reinterpret_cast<uint4*>(dot_sh + (i * 32 + lane) * 4) =
               make_uint4(acc[i * 4], acc[i * 4 + 1], acc[i * 4 + 2], acc[i * 4 + 3]);
-#pragma unroll 1
-        for (uint32_t i = 0; i < 4; ++i) {
-          const uint32_t rx = gx * 4 + i;
-          if (rx >= A) break;
-          const uint32_t x = id_sh[rx], nx = norm_sh[rx];
-          const float bx = bound_sh[rx];
-          const uint4 dv = *reinterpret_cast<const uint4*>(dot_sh + (i * 32 + lane) * 4);
-          const uint32_t dot[4] = {dv.x, dv.y, dv.z, dv.w};
-          // four pairs' slots first, then their records: the atomics' latencies overlap
-          uint32_t slot[8], ta[8];
-          float dd[4];
-          uint32_t put = 0;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t ry = gy * 4 + j;
-            const bool pair = ry < R && (tri ? ry > rx : ry >= A);
-            const uint32_t y = id_sh[ry];
-            const float by = bound_sh[ry];
+        blk_sh[lane] = gx * 4 | gy * 4 << 16;
+        if (a.P < a.check_k) {  // a pair whose first side is rejected
+          for (uint32_t q = 0; q < 16; ++q) {
+            const uint32_t rx = gx * 4 + q / 4, ry = gy * 4 + q % 4;
+            if (!(ok >> q & 1u)) continue;
             const bool my_new = (ry < A ? a0 + ry : c0 + (ry - A)) < nn;
-            dd[j] = (float)(nx + norm_sh[ry] - 2 * dot[j]);
-            const bool ok = pair && !(my_new && y == x);
-            const bool swap = my_new && y < x;  // side 0: the larger id into the smaller id's node
-            const bool in0 = dd[j] <= (swap ? by : bx), in1 = dd[j] <= (swap ? bx : by);
-            put |= (ok && in0 ? 1u : 0u) << (2 * j) | (ok && in1 ? 2u : 0u) << (2 * j);
-            drop |= ok && !in0;
-            ta[2 * j] = swap ? y : x;
-            ta[2 * j + 1] = swap ? x : y;
+            const uint32_t x = id_sh[rx], y = id_sh[ry];
+            drop |= !(my_new && y == x) && !(put >> (my_new && y < x ? 16 + q : q) & 1u);
           }
+        }
+        while (__any_sync(0xffffffffu, put != 0)) {
+          uint32_t end = __popc(put);
+          uint32_t at = end;
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-            if (put >> q & 1u) slot[q] = atomicAdd(&a.sink.cnt[ta[q]], 1u);
-          uint32_t over = 0;
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            if (put >> q & 1u) {
-              if (slot[q] < a.sink.W)
-                a.sink.bucket[(uint64_t)ta[q] * a.sink.W + slot[q]] =
-                    make_uint4(ta[q ^ 1], __float_as_uint(dd[q >> 1]), (uint32_t)(node << 1) | (q & 1), ta[q]);
-              else over |= 1u << q;
-            }
-          if (over) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-              if (over >> q & 1u)
-                place_overflow(a.sink, ta[q], slot[q], dd[q >> 1], ta[q ^ 1], (uint32_t)(node << 1) | (q & 1));
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= (uint32_t)o) end += y;
           }
+          at = end - at;
+          for (; put && at < QUEUE; put &= put - 1) queue[at++] = (uint16_t)(lane << 5 | (__ffs(put) - 1));
+          const uint32_t total = min(__shfl_sync(0xffffffffu, end, 31), QUEUE);
+          __syncwarp();
+          for (uint32_t r = lane; r < total; r += 32) {
+            const uint32_t code = queue[r], src = code >> 5, q = code & 15u, blk = blk_sh[src];
+            const uint32_t rx = (blk & 0xffffu) + q / 4, ry = (blk >> 16) + q % 4;
+            const float d = (float)dot_sh[(q / 4 * 32 + src) * 4 + q % 4];
+            const bool to_y = code & 16u;
+            const uint32_t x = id_sh[rx], y = id_sh[ry];
+            const bool my_new = (ry < A ? a0 + ry : c0 + (ry - A)) < nn;
+            if (my_new && y == x) continue;
+            // side 0: the larger id into the smaller id's node (an old y into x's)
+            const uint32_t t = to_y ? y : x, cand = to_y ? x : y, side = to_y != (my_new && y < x) ? 1u : 0u;
+            const uint32_t aux = (uint32_t)(node << 1) | side;
+            place_record(a.sink, t, atomicAdd(&a.sink.cnt[t], 1u), d, cand, aux);
+          }
+          __syncwarp();
         }
       }
       __syncwarp();  // the tile's rows are no longer read
