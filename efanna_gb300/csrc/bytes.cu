@@ -59,7 +59,8 @@ struct JoinBytesArgs {
   RecordSink sink;
   uint8_t* found;
   uint32_t* next_node;
-  uint32_t count, step, skip;
+  NodeSet set;
+  uint32_t count;           // of its nodes
   uint32_t chunks, cmagic;  // 16-byte chunks per row, and ceil(2^16 / chunks) for the division by it
   uint32_t stride;          // of a row in shared memory: an odd number of chunks, in bytes
   uint32_t cap, P, check_k;
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(BW * 32, 4) join_bytes_kernel(const JoinBytesA
     const uint32_t k = __shfl_sync(0xffffffffu, nk, 0);
     if (k >= a.count) return;
     if (lane == 0) nk = atomicAdd(a.next_node, 1u);  // the next node's, in flight meanwhile
-    const uint64_t node = a.skip ? (uint64_t)k + k / (a.step - 1) + 1 : (uint64_t)k * a.step;
+    const uint64_t node = a.set.node(k);
     const uint32_t nn = a.new_cnt[node], T = nn + a.old_cnt[node];
     bool drop = false;
     // tiles: A new entries from a0 with C entries from c0 on; the first of a block (tri) also covers the
@@ -289,7 +290,7 @@ int make_bytes(efg_index* idx) {
 int join_bytes(const uint8_t* rows, const uint32_t* norm, uint64_t n, uint32_t ldb, uint32_t cap, uint32_t P,
                uint32_t check_k, const uint32_t* new_ids, const uint32_t* new_cnt, const uint32_t* old_ids,
                const uint32_t* old_cnt, const float* bound, const RecordSink& sink, uint8_t* found, uint32_t* counter,
-               uint32_t step, uint32_t skip, cudaStream_t s) {
+               const NodeSet& set, cudaStream_t s) {
   JoinBytesArgs a;
   a.rows = rows;
   a.norm = norm;
@@ -301,10 +302,8 @@ int join_bytes(const uint8_t* rows, const uint32_t* norm, uint64_t n, uint32_t l
   a.sink = sink;
   a.found = found;
   a.next_node = counter;
-  a.step = step;
-  a.skip = skip;
-  const uint64_t first = (n + step - 1) / step;  // nodes k * step
-  a.count = (uint32_t)(skip ? n - first : first);
+  a.set = set;
+  a.count = (uint32_t)set.count(n);
   a.chunks = ldb / 16;  // <= 17
   a.cmagic = (65536 + a.chunks - 1) / a.chunks;  // exact for e < 64 * 17 (error e / 65536 * (chunks - 1) < 1 / chunks)
   a.stride = (a.chunks | 1) * 16;

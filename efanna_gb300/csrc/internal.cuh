@@ -201,26 +201,37 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
 // 256 rows over the nodes listed in mid, the nodes listed in big tile by tile; counters: three node
 // counters); err is set when a wait ran out or a list holds an id >= n.
 struct RecordSink;
+// The nodes i with first <= i % step < first + width: the k-th of them, and how many of n they are.
+struct NodeSet {
+  uint32_t step, first, width;
+  __host__ __device__ __forceinline__ uint64_t node(uint32_t k) const {
+    return (uint64_t)(k / width) * step + first + k % width;
+  }
+  uint64_t count(uint64_t n) const {
+    const uint64_t rest = n % step;
+    return n / step * width + (rest > first ? std::min<uint64_t>(rest - first, width) : 0);
+  }
+};
 int tc_join_prepare(const float* base, uint64_t n, uint32_t dim, uint32_t ld, __nv_bfloat16* hi, __nv_bfloat16* lo,
                     float* norms, int* flags, cudaStream_t s);
 int tc_join(const __nv_bfloat16* hi, const __nv_bfloat16* lo, const float* norms, uint64_t n, uint32_t dim,
             uint32_t terms, uint32_t cap, uint32_t P, uint32_t check_k, const uint32_t* new_ids,
             const uint32_t* new_cnt, const uint32_t* old_ids, const uint32_t* old_cnt, const float* bound,
             const RecordSink& sink, uint8_t* found, uint32_t* counters, uint32_t* mid, uint32_t* big,
-            unsigned long long* nlarge, int* err, uint32_t step, uint32_t skip, cudaStream_t s);
-// join_fp32.cu: the NN-descent join in FP32 over the nodes k * step (skip 0) or the others (skip 1);
+            unsigned long long* nlarge, int* err, const NodeSet& set, cudaStream_t s);
+// join_fp32.cu: the NN-descent join in FP32 over a subset of the nodes;
 // counters: two node counters, zero on entry; big: n + 1 words, word 0 zero on entry.
 int join_fp32(const float* base, uint64_t n, uint32_t ld, uint32_t cap, uint32_t P, uint32_t check_k,
               const uint32_t* new_ids, const uint32_t* new_cnt, const uint32_t* old_ids, const uint32_t* old_cnt,
               const float* bound, const RecordSink& sink, uint8_t* found, uint32_t* counters, uint32_t* big,
-              uint32_t step, uint32_t skip, cudaStream_t s);
+              const NodeSet& set, cudaStream_t s);
 // bytes.cu: the byte rows of an index's base, where it has them (idx->bytes_state == 1 afterwards), and
 // the join over byte rows, with the FP32 join's records.
 int make_bytes(efg_index* idx);
 int join_bytes(const uint8_t* rows, const uint32_t* norm, uint64_t n, uint32_t ldb, uint32_t cap, uint32_t P,
                uint32_t check_k, const uint32_t* new_ids, const uint32_t* new_cnt, const uint32_t* old_ids,
                const uint32_t* old_cnt, const float* bound, const RecordSink& sink, uint8_t* found, uint32_t* counter,
-               uint32_t step, uint32_t skip, cudaStream_t s);
+               const NodeSet& set, cudaStream_t s);
 __host__ __device__ __forceinline__ bool is_byte(float x) { return x >= 0.f && x <= 255.f && (float)(uint32_t)x == x; }
 // mlp_tc.cu: the learned form's dense layers on the tensor cores, C = act(A W^T + bias) (A: M x K,
 // W: N x K, BF16 row-major; C FP32 and / or Cb BF16, M x N); EFG_ERR_ARG when the shape does not fit.

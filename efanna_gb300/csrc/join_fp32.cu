@@ -32,7 +32,8 @@ struct JoinFp32Args {
   uint8_t* found;
   uint32_t* next_node;
   uint32_t* big;               // big[0]: nodes listed, then their ids
-  uint32_t count, step, skip;  // nodes: k * step (skip 0), or the others of every step (skip 1)
+  NodeSet set;
+  uint32_t count;  // of its nodes
   uint32_t ld4, cap, P, check_k;
 };
 
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(JW * 32, 2) join_fp32_kernel(const JoinFp32Arg
     if (lane == 0) kk = atomicAdd(a.next_node, 1u);
     const uint32_t k = __shfl_sync(0xffffffffu, kk, 0);
     if (k >= a.count) break;
-    const uint64_t i = a.skip ? (uint64_t)k + k / (a.step - 1) + 1 : (uint64_t)k * a.step;
+    const uint64_t i = a.set.node(k);
     const uint32_t nn = a.new_cnt[i], no = a.old_cnt[i];
     if (nn == 0) continue;
     if ((uint64_t)nn * (nn / 2 + no) > JBIG) {
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(JW * 32, 2) join_fp32_big_kernel(const JoinFp3
 int join_fp32(const float* base, uint64_t n, uint32_t ld, uint32_t cap, uint32_t P, uint32_t check_k,
               const uint32_t* new_ids, const uint32_t* new_cnt, const uint32_t* old_ids, const uint32_t* old_cnt,
               const float* bound, const RecordSink& sink, uint8_t* found, uint32_t* counters, uint32_t* big,
-              uint32_t step, uint32_t skip, cudaStream_t s) {
+              const NodeSet& set, cudaStream_t s) {
   JoinFp32Args a;
   a.base = base;
   a.new_ids = new_ids;
@@ -301,10 +302,8 @@ int join_fp32(const float* base, uint64_t n, uint32_t ld, uint32_t cap, uint32_t
   a.found = found;
   a.next_node = counters;
   a.big = big;
-  a.step = step;
-  a.skip = skip;
-  const uint64_t first = (n + step - 1) / step;  // nodes k * step
-  a.count = (uint32_t)(skip ? n - first : first);
+  a.set = set;
+  a.count = (uint32_t)set.count(n);
   a.ld4 = ld / 4;
   a.cap = cap;
   a.P = P;

@@ -71,7 +71,8 @@ struct JoinArgs {
   uint64_t n;
   unsigned long long* nlarge;  // counts the nodes larger than a tile
   uint32_t W, cap, P, check_k, kblocks, terms, nstages, mode;
-  uint32_t count, step, skip;  // MODE_ORDER: the nodes k * step (skip 0), or the others (skip 1)
+  NodeSet set;     // MODE_ORDER: the nodes
+  uint32_t count;  // of them
 };
 
 __device__ __forceinline__ void rec_sync() { asm volatile("bar.sync 1, %0;" ::"r"(JRT) : "memory"); }
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
         if (cn == 0) break;
         if (threadIdx.x < cn) {
           const uint32_t k = next_k0_sh + threadIdx.x;
-          const uint32_t i = a.mode == MODE_LIST ? a.mid[1 + k] : a.skip ? k + k / (a.step - 1) + 1 : k * a.step;
+          const uint32_t i = a.mode == MODE_LIST ? a.mid[1 + k] : (uint32_t)a.set.node(k);
           uint32_t nn = a.new_cnt[i];
           const uint32_t no = a.old_cnt[i];
           if (nn > a.cap || no > a.cap) {  // not a list: reported, the node left out
@@ -565,12 +566,13 @@ int tc_join_prepare(const float* base, uint64_t n, uint32_t dim, uint32_t ld, __
 // The join on the tensor cores: three launches (tiles of 128 rows over every node, tiles of 256
 // rows over the nodes listed in mid, and the nodes listed in big tile by tile).  counters: three
 // node counters, zero on entry; mid and big: n + 1 words each, their counts (word 0) zero on entry;
-// *err zero on entry; *nlarge counts the nodes larger than a tile.  step, skip: the nodes k * step (skip 0) or the others (skip 1).  terms: 1 (BF16 holds the base) or 3 (hi + lo products).
+// *err zero on entry; *nlarge counts the nodes larger than a tile.  set: the nodes.
+// terms: 1 (BF16 holds the base) or 3 (hi + lo products).
 int tc_join(const __nv_bfloat16* hi, const __nv_bfloat16* lo, const float* norms, uint64_t n, uint32_t dim,
             uint32_t terms, uint32_t cap, uint32_t P, uint32_t check_k, const uint32_t* new_ids,
             const uint32_t* new_cnt, const uint32_t* old_ids, const uint32_t* old_cnt, const float* bound,
             const RecordSink& sink, uint8_t* found, uint32_t* counters, uint32_t* mid, uint32_t* big,
-            unsigned long long* nlarge, int* err, uint32_t step, uint32_t skip, cudaStream_t s) {
+            unsigned long long* nlarge, int* err, const NodeSet& set, cudaStream_t s) {
   if (terms != 1 && terms != 3) return fail(EFG_ERR_ARG, "tensor-core join: terms must be 1 or 3");
   if (n >= 0xffffffffull) return fail(EFG_ERR_ARG, "tensor-core join: more than 2^32 - 2 rows");
   const uint32_t W = (dim + 63) / 64 * 64;
@@ -601,10 +603,8 @@ int tc_join(const __nv_bfloat16* hi, const __nv_bfloat16* lo, const float* norms
   a.terms = terms;
   a.nstages = terms == 1 ? 2 : 1;
   a.nlarge = nlarge;
-  a.step = step;
-  a.skip = skip;
-  const uint64_t first = (n + step - 1) / step;
-  a.count = (uint32_t)(skip ? n - first : first);
+  a.set = set;
+  a.count = (uint32_t)set.count(n);
   a.mode = MODE_ORDER;
   a.next_node = counters;
   EFG_TRY(launch_join<128>(a, sms, smem_max, s));

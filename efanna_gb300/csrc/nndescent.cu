@@ -47,7 +47,7 @@ struct NNDev {
   DevBuf<uint32_t> cnt, cursor, rcnt, rcur, roff, rbuf, scan32;
   DevBuf<float> bound;
   DevBuf<unsigned long long> totals;  // pairs, records, overflow records, nodes larger than a tile
-  DevBuf<uint32_t> jctr;              // node counters: the merge's, the join's (up to three launches in each of two parts)
+  DevBuf<uint32_t> jctr;              // node counters: the merge's, the join's (up to three launches)
   DevBuf<uint4> bucket, ovf, ovfrec;  // join records: per-target buckets, overflow list, hub targets' records
   DevBuf<uint32_t> ovf_slot;
   // tensor-core join: BF16 rows (hi, lo), FP32 norms, flags {inexact, error}, nodes left to FP32
@@ -1204,11 +1204,13 @@ static int merge_level_check(efg_index* idx, int32_t* min_level) {
 }
 
 // Records of a first join per node, on average (every pair of the seeded lists is kept: 2 S entries),
-// and whether the first join runs in two parts (1 of FIRST_PART nodes, then the others).
-constexpr uint32_t FIRST_PART = 8;
+// and whether the first join runs in parts: of every FIRST_STEP nodes those from one entry of FIRST_PARTS to
+// the next, the targets' bounds tightened in between (1M x 128: 8.7 ms; in two parts, 1 and 7, 10.9 ms
+// with half as many records again).
+constexpr uint32_t FIRST_STEP = 8, FIRST_PARTS[] = {0, 1, 3, 8};
 static uint64_t first_mean(const efg_build_params& bp) { return 2ull * bp.S * (2 * bp.S - 1); }
 static bool first_in_parts(const efg_build_params& bp, uint32_t P, bool exact) {
-  return exact && P <= TIGHTEN_MAX_P && first_mean(bp) / FIRST_PART + bp.S >= P + P / 4;
+  return exact && P <= TIGHTEN_MAX_P && first_mean(bp) / FIRST_STEP + bp.S >= P + P / 4;
 }
 
 // Bucket width: about the records a node receives in the first join, or five pools' worth where pools
@@ -1223,7 +1225,7 @@ static int first_width(efg_index* idx, NNDev& S) {
   EFG_CUDA(cudaMemGetInfo(&free_b, &total_b));
   S.bucket_cap = std::max<uint64_t>(1, (uint64_t)free_b / 4 / sizeof(uint4) / S.n);
   const uint64_t mean = first_mean(bp);
-  const uint64_t expect = first_in_parts(bp, S.P, true) ? mean / FIRST_PART + 8 * S.P
+  const uint64_t expect = first_in_parts(bp, S.P, true) ? mean / FIRST_STEP + 6 * S.P
                                                         : std::max<uint64_t>(mean + mean / 4, S.P > 64 ? 5 * S.P : 0);
   S.W = (uint32_t)std::min<uint64_t>(S.bucket_cap, expect + 32);
   S.ovf_cap = std::max<uint64_t>(S.n * (expect / 4 + 8), 1 << 16);
@@ -1368,7 +1370,7 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
     S.jterms = inexact[0] ? 3 : 1;
     S.jexact = !inexact[0] && !inexact[2];
   }
-  const uint32_t part = iter == 0 && first_in_parts(bp, S.P, !tc || S.jexact) ? FIRST_PART : 1;
+  const bool parts = iter == 0 && first_in_parts(bp, S.P, !tc || S.jexact);
   EFG_TRY(first_width(idx, S));
   EFG_TRY(S.bucket.reserve(n * S.W));
   int sms = 152, dev = 0;
@@ -1386,28 +1388,32 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
     EFG_CUDA(cudaGetLastError());
     const RecordSink sink{S.cnt.p, S.bucket.p, S.ovf.p, S.ovf_slot.p, S.totals.p + 2, S.ovf_cap, S.W};
     if (tc) EFG_CUDA(cudaMemsetAsync(S.jflag.p + 1, 0, 4, s));
-    auto join = [&](uint32_t counter, uint32_t step, uint32_t skip) -> int {
+    auto join = [&](const NodeSet& set) -> int {
+      EFG_CUDA(cudaMemsetAsync(S.jctr.p + 1, 0, 12, s));
       if (!tc && idx->bytes_state == 1)
         return join_bytes(idx->bytes.p, idx->bnorm.p, n, idx->ldb, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p,
-                          S.old_ids.p, S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, step, skip, s);
+                          S.old_ids.p, S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + 1, set, s);
       EFG_TRY(S.jbig.reserve(n + 1));
       EFG_CUDA(cudaMemsetAsync(S.jbig.p, 0, 4, s));
       if (!tc)
         return join_fp32(idx->d_base, n, idx->ld, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p, S.old_ids.p,
-                         S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, S.jbig.p, step, skip, s);
+                         S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + 1, S.jbig.p, set, s);
       EFG_CUDA(cudaMemsetAsync(S.jmid.p, 0, 4, s));
       return tc_join(S.jhi.p, S.jlo.p, S.jnorm.p, n, idx->dim, S.jterms, S.cap, S.P, bp.check_k, S.new_ids.p,
-                     S.new_cnt.p, S.old_ids.p, S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + counter, S.jmid.p,
-                     S.jbig.p, S.totals.p + 3, S.jflag.p + 1, step, skip, s);
+                     S.new_cnt.p, S.old_ids.p, S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + 1, S.jmid.p,
+                     S.jbig.p, S.totals.p + 3, S.jflag.p + 1, set, s);
     };
-    if (part > 1) {
-      EFG_TRY(join(1, part, 0));
-      tighten_kernel<<<blocks_for(n * 32, 256), 256, 0, s>>>(n, S.P, S.W, S.cnt.p, S.bucket.p, S.pd.p, S.pid.p,
-                                                             S.Lc.p, S.bound.p);
-      EFG_CUDA(cudaGetLastError());
-      EFG_TRY(join(4, part, 1));
+    if (parts) {
+      for (uint32_t p = 0; p + 1 < sizeof(FIRST_PARTS) / 4; ++p) {
+        if (p) {
+          tighten_kernel<<<blocks_for(n * 32, 256), 256, 0, s>>>(n, S.P, S.W, S.cnt.p, S.bucket.p, S.pd.p, S.pid.p,
+                                                                 S.Lc.p, S.bound.p);
+          EFG_CUDA(cudaGetLastError());
+        }
+        EFG_TRY(join(NodeSet{FIRST_STEP, FIRST_PARTS[p], FIRST_PARTS[p + 1] - FIRST_PARTS[p]}));
+      }
     } else {
-      EFG_TRY(join(1, 1, 0));
+      EFG_TRY(join(NodeSet{1, 0, 1}));
     }
     unsigned long long tot[4] = {0, 0, 0, 0};
     EFG_CUDA(cudaMemcpyAsync(tot, S.totals.p, 32, cudaMemcpyDeviceToHost, s));
