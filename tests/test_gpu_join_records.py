@@ -64,3 +64,17 @@ def test_overflowing_buckets_match_oracle(efg, oracle_lib, nodes, nn, no, hub, b
     g = st.copy()
     assert idx.nnd_iterate(g, 0) == pairs
     assert _state_diff(nxt, g) is None, _state_diff(nxt, g)
+
+
+@pytest.mark.parametrize("reverse_cap", [5, 31, 32, 33, 64])
+def test_reverse_lists_match_oracle(efg, oracle_lib, reverse_cap):
+    """Reverse lists below, at and beyond a warp's lanes, sampled and whole."""
+    O = oracle_lib
+    x, params, p, cur = _start(O, 2000, 6, 40, 30, 25, seed=9, reverse_cap=reverse_cap)
+    idx = efg.Index(x, efg.IndexParams(**params))
+    for it in range(2):
+        nxt, pairs = O.nnd_iterate(x, cur, p, it, O.CANON)
+        g = cur.copy()
+        assert idx.nnd_iterate(g, it) == pairs
+        assert _state_diff(nxt, g) is None, (it, _state_diff(nxt, g))
+        cur = nxt
