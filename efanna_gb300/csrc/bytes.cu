@@ -277,8 +277,12 @@ int make_bytes(efg_index* idx) {
     }
   }
   idx->ldb = (uint32_t)round_up(idx->dim, 16);
-  EFG_TRY(idx->bytes.reserve(idx->n * idx->ldb));
-  EFG_TRY(idx->bnorm.reserve(idx->n));
+  if (idx->bytes.reserve(idx->n * idx->ldb) != EFG_OK || idx->bnorm.reserve(idx->n) != EFG_OK) {
+    idx->bytes.release();  // no room: the FP32 rows serve as well
+    idx->bnorm.release();
+    idx->bytes_state = 2;
+    return EFG_OK;
+  }
   to_bytes_kernel<<<sms * 8, 256, 0, idx->stream>>>(idx->d_base, idx->n, idx->ld / 4, idx->ldb, idx->bytes.p,
                                                     idx->bnorm.p);
   EFG_CUDA(cudaGetLastError());
