@@ -947,7 +947,7 @@ def knn_line(kst, form):
     peak = float(json.load(open(pk))["bf16_tflops"]) if os.path.exists(pk) else 1900.0
     tf = kst.screen_flops / (kst.screen_ms * 1e-3) / 1e12 if kst.screen_ms else 0.0
     ti = kst.tile_flops / (kst.screen_ms * 1e-3) / 1e12 if kst.screen_ms else 0.0
-    return {"kernel": "tc_knn_kernel", "form": form, "convert_ms": round(kst.convert_ms, 3),
+    return {"kernel": "tc_screen_kernel", "form": form, "convert_ms": round(kst.convert_ms, 3),
             "bound_ms": round(kst.bound_ms, 3), "screen_ms": round(kst.screen_ms, 3),
             "merge_ms": round(kst.merge_ms, 3),
             "roofline": {"bound": "tensor", "achieved": round(tf, 1), "issued": round(ti, 1), "peak": peak,

@@ -12,28 +12,21 @@
 //     below 2^24, so the screened distances equal the exact ones.  Other data are split as
 //     x = hi + lo (two BF16 values) and each tile accumulates hi.hi + hi.lo + lo.hi, which leaves
 //     an error near 2^-16 of |q.x| instead of 2^-8.
-//   * a CTA owns one work item at a time: 128 queries (the MMA's M, one TMEM lane each) against
-//     one chunk of base rows, walked in tiles of 128 rows (N).  Warp 0 streams the operand
-//     k-blocks into a ring of shared-memory stages with cp.async.bulk.tensor (TMA, 128-byte
-//     swizzle), one (query block, base block) pair per stage -- in the split form three pairs per
-//     k-block: (hi, hi), (hi, lo), (lo, hi); one thread of warp 1 issues the MMAs (K = 16 each) into one of two TMEM
-//     accumulators and commits them to mbarriers; warps 2-5 read the other accumulator with
-//     tcgen05.ld, one query per thread, turn each Gram value into a distance and keep the
-//     query's best K2 = k + 16 (distance, id) keys of the chunk.  The two accumulators let the
-//     MMAs of tile t + 1 run while tile t is being screened.
-//   * every query starts with a bound on its K2-th distance: the K2-th distance over a strided
-//     sample of the base, from a first pass of the same kernel over the sample alone (any subset's
-//     K2-th distance bounds the whole base's from above).  Per group of 64 values a branch-free
-//     test (one FMA, one compare per value) builds each thread's mask of values under its bound;
-//     only values in some mask reach the exact test, one per lane per round, and go straight into
-//     the thread's sorted list in shared memory, which tightens the bound once it holds K2 keys.
-//     The base-row norms of the next tile are loaded while the current one is screened, and the
-//     second half of the accumulator is read from TMEM during the first.
+//   * tc_screen_kernel: a CTA owns one work item at a time, 128 or 256 queries (the MMA's M, one TMEM
+//     lane each; one or two accumulators) against one chunk of base rows, walked in tiles of 128 rows
+//     (N).  The queries' blocks stay in shared memory where they fit; warp 0 streams the base's
+//     k-blocks into a ring of stages with cp.async.bulk.tensor (TMA, 128-byte swizzle), warp 1 issues
+//     the MMAs (K = 16 each) into double-buffered accumulators, and sixteen warps in two sets read
+//     the finished ones with tcgen05.ld and screen them.
+//   * every query has an upper bound on its K2-th distance (K2 = k + 16) from cheap passes of the
+//     same kernel over samples; the pass over the whole base appends the few values under it to the
+//     query's candidate buffer, and select_kernel sorts them and re-ranks the K2 smallest in FP64.
+//   * tc_knn_kernel, the path of a call whose candidates overran their buffers (many rows at nearly one
+//     distance): per-(query, chunk) sorted lists of K2 keys in shared memory, as the FP32 kernel writes
+//     them (distance.cu), ranked by the same merge kernel.
 //
-// The chunks' lists are the same per-(query, chunk) lists the FP32 kernel writes (distance.cu);
-// the same merge kernel then re-ranks the K2 survivors of each query in FP64.  Every wait on an
-// mbarrier is bounded: a wait that runs out sets an error word and the CTA leaves its loops,
-// drains its tensor-core work and frees its TMEM; the host turns the word into
+// Every wait on an mbarrier is bounded: a wait that runs out sets an error word and the CTA leaves its
+// loops, drains its tensor-core work and frees its TMEM; the host turns the word into
 // EFG_ERR_DEVICE_LIMIT.
 #include <cuda.h>
 #include <cuda_bf16.h>

@@ -1,5 +1,5 @@
-// The record side of the NN-descent join (base_index.hpp:328-371), shared by the FP32 join
-// kernel (nndescent.cu) and the tensor-core join (join_tc.cu): which of a pair's two sides becomes
+// The record side of the NN-descent join (base_index.hpp:328-371), shared by the join over FP32 rows
+// (join_fp32.cu), over byte rows (bytes.cu) and on the tensor cores (join_tc.cu): which of a pair's two sides becomes
 // a pool-insert record, and where the record goes.
 #pragma once
 #include "internal.cuh"

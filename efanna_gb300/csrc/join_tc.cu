@@ -23,8 +23,8 @@
 //     per thread: distance ||x||^2 + ||y||^2 - 2 x.y, then the join's record step -- the same records
 //     and `found` flags as the FP32 join kernel.
 //   * When BF16 holds every value of the base, one product per value; with integer values and
-//     squared norms below 2^23 (byte data up to 128 dimensions) every sum is exact, so the distances
-//     equal the FP32 join's and the graph is identical.  Other data take the hi + lo split
+//     squared norms below 2^22 (byte data of 64 dimensions whatever the values) every sum is exact, so
+//     the distances equal the FP32 join's and the graph is identical.  Other data take the hi + lo split
 //     (hi.hi + hi.lo + lo.hi, a relative error near 2^-17 of sum |x_k y_k|): distances, and so pools,
 //     can then differ from the FP32 join's in the last bits.
 //   * Shared memory is sized so that the CTAs an SM can hold never need more than its 512 TMEM

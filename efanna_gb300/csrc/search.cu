@@ -18,15 +18,20 @@
 //      graph row, add the unvisited neighbours, keep the resultSize best (:444-484).
 //   5. emit the first k ids (:486-492).
 // Candidate lists are packed (dist_bits << 32 | id) keys, which order exactly like the reference's
-// pair<float, size_t>.  The resultSize best are kept as one sorted list; candidates are folded
-// into it 1024 at a time: keys at or above the current worst are dropped, the rest sorted and
-// merged by rank.  Ids are unique, so the result does not depend on the order threads find them.
+// pair<float, size_t>.  The resultSize best are kept as one sorted list: the pool's by one selection and
+// sort where the pool's keys fit shared memory, later candidates folded into it 1024 at a time (keys at
+// or above the current worst dropped, the rest sorted and merged by rank).  Ids are unique, so the result
+// does not depend on the order threads find them.
 //
-// The visited set (the reference's N-bit tbflag) is a double-hashing table in shared memory sized
-// for the expected number of visits; the reference's newflag ("expanded") is a bit of the result
-// keys.  A query whose set reaches 80% of the table at a phase boundary moves it to a worst-case
-// table in global scratch; one that fills 90% within a phase is abandoned and listed, and a second
-// launch answers the listed queries with worst-case tables in global memory.
+// The visited set (the reference's N-bit tbflag) is, where one bit per row fits shared memory without
+// costing a CTA that would otherwise run, a bitmap; else a double-hashing table sized for the expected
+// number of visits.  The reference's newflag ("expanded") is a bit of the result keys.  A query whose
+// table reaches 80% at a phase boundary moves it to a worst-case table in global scratch; one that fills
+// 90% within a phase is abandoned and listed, and a second launch answers the listed queries with
+// worst-case tables in global memory.
+//
+// A base of bytes (integers in [0, 255], at most 258 dimensions) is searched over its byte rows for
+// queries of bytes: the distances are the same integers at a quarter of the FP32 rows' traffic.
 #include <algorithm>
 
 #include <cuda_bf16.h>
