@@ -93,27 +93,32 @@ __device__ __forceinline__ bool ht_insert(uint32_t* ht, uint32_t size, uint32_t 
 // without branches (loads and compare-and-swaps are predicated), until the warp's last one is settled:
 // as branches, each lane's probe sequences ran one after another (1024 inserts by 256 threads at half
 // to two-thirds load: 4300 cycles, 2700 this way).  The same outcome as XR ht_insert calls: an id met
-// twice takes its slot once.  kEmpty entries are skipped.  Called by whole warps.
+// twice takes its slot once.  kEmpty entries are skipped.  Called by whole warps.  The warps' counts come
+// after their inserts, so together they can pass the limit and fill the table: an id that finds no place
+// in PROBES steps (at the limit's 90% load a chance of 2e-12) gives the query to the overflow pass.
+static constexpr uint32_t PROBES = 256;
 template <int XR>
 __device__ __forceinline__ void ht_insert_batch(uint32_t* ht, uint32_t size, uint32_t limit, uint32_t* count,
                                                 uint32_t* ovf, const uint32_t (&id)[XR], bool (&fresh)[XR]) {
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(ht);
   uint32_t at[XR], step[XR], act[XR];
   const bool full = *reinterpret_cast<volatile uint32_t*>(count) >= limit;
+  const bool dead = *reinterpret_cast<volatile uint32_t*>(ovf) != 0;  // the query is the overflow pass's already
 #pragma unroll
   for (int u = 0; u < XR; ++u) {
     at[u] = ht_slot(id[u], size);
     step[u] = ht_step(id[u], size);
-    act[u] = id[u] != kEmpty ? 1u : 0u;
+    act[u] = id[u] != kEmpty && !dead ? 1u : 0u;
     fresh[u] = false;
   }
-  bool any = true;
-  for (uint32_t probe = 0; any && probe < size; ++probe) {
+  bool any = true, mine = false;
+  for (uint32_t probe = 0; any && probe < PROBES; ++probe) {
     uint32_t c[XR];
 #pragma unroll
     for (int u = 0; u < XR; ++u)
       asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(c[u]) : "r"(base + at[u] * 4) : "memory");
-    bool mine = false, none = false;
+    bool none = false;
+    mine = false;
 #pragma unroll
     for (int u = 0; u < XR; ++u) {
       const uint32_t want = act[u] && c[u] == kEmpty && !full ? 1u : 0u;
@@ -135,6 +140,7 @@ __device__ __forceinline__ void ht_insert_batch(uint32_t* ht, uint32_t size, uin
     }
     any = __any_sync(0xffffffffu, mine);
   }
+  if (mine) atomicOr(ovf, 1u);
 }
 
 __device__ __forceinline__ bool ht_contains(const uint32_t* ht, uint32_t size, uint32_t id) {
