@@ -1131,11 +1131,26 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   EFG_CUDA(cudaMemsetAsync(qbound, 0, nq * 4, s));
   const size_t sel_smem = (size_t)cap * 8 + (size_t)rank * 8;
   EFG_CUDA(cudaFuncSetAttribute(select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem));
-  const uint64_t S1 = std::min<uint64_t>(n / 16, 1u << 20) / TN * TN;  // rows of the append pass's sample
+  uint64_t S1 = std::min<uint64_t>(n / 16, 1u << 20) / TN * TN;  // rows of the append pass's sample
   const uint64_t gtiles = (rank + 3) / 4 * 2;                          // tiles that hold `rank` groups of 64 columns, an even number
   uint32_t S = 0;
   bool bounded = true;
   if (S1 >= gtiles * TN) {
+    uint32_t gt = 1;  // tiles per group: up to a third of the sample for the MIN pass
+    while (gt < 16 && gtiles * (2 * gt) * TN * 3 <= S1) gt *= 2;
+    // Values of the sample under the MIN pass's bound: a share p of them, where all of the `rank` groups of
+    // 64 gt columns have one below it; (1 - p)^(64 gt) rank nq = 1 / 32 says what their buffers must hold.  A
+    // call that overran them goes through the lists after all (k = 100, 10k queries at 1M x 960: 167 ms, 114
+    // through the lists at once), so the sample is cut while the base's expected candidates (six deviations
+    // up) still fit, else the groups doubled.
+    const double tail = std::log(32.0 * (double)rank * (double)nq);
+    while ((double)S1 * tail > (double)cap * 64 * gt) {
+      const uint64_t cut = (uint64_t)((double)cap * 64 * gt / tail) / TN * TN;
+      const double expect = (double)n / (double)std::max<uint64_t>(cut, 1) * (double)rank;
+      if (cut >= gtiles * gt * TN && expect * (1 + 6 / std::sqrt((double)rank)) <= (double)cap) S1 = cut;
+      else if (gtiles * (2 * gt) * TN <= S1) gt *= 2;
+      else break;
+    }
     __nv_bfloat16 *bh, *bl = nullptr;
     float* bn;
     EFG_TRY(mem.get(&bh, S1 * W));
@@ -1154,8 +1169,6 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     scatter_sample_kernel<<<blocks(S1), 256, 0, s>>>((const uint4*)xh, (const uint4*)xl, xn, n, W, (uint32_t)S1, step,
                                                      (uint4*)bh, (uint4*)bl, bn);
     EFG_CUDA(cudaGetLastError());
-    uint32_t gt = 1;  // tiles per group: up to a third of the sample for the MIN pass
-    while (gt < 16 && gtiles * (2 * gt) * TN * 3 <= S1) gt *= 2;
     const uint64_t S0 = gtiles * gt * TN;
     CUtensorMap m0h, m0l, m1h, m1l;
     EFG_TRY(make_map(&m0h, bh, S0, W));

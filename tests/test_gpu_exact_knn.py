@@ -160,3 +160,23 @@ def test_many_equal_distances(efg, n):
     ref_ids, ref_d = _numpy_exact(x, q[:2], 12)
     for i in range(200):
         assert np.array_equal(tc[0][i], ref_ids[i % 2]) and np.array_equal(tc[1][i], ref_d[i % 2])
+
+
+@pytest.mark.parametrize("n,nq", [(330_000, 4000), (520_000, 2000), (1_000_000, 3000)])
+def test_long_lists_over_large_bases(efg, n, nq):
+    """k = 100 over bases whose sample is cut or whose groups are doubled; ids and distances equal the FP32
+    screening's, and the call does not end in the lists."""
+    import torch
+    x = torch.randint(0, 256, (n, 16), device="cuda", dtype=torch.int32).float()
+    q = torch.randint(0, 256, (nq, 16), device="cuda", dtype=torch.int32).float()
+    out = {}
+    for screening in ("fp32", "auto"):
+        ids = torch.zeros((nq, 100), dtype=torch.int32, device="cuda")
+        dist = torch.zeros((nq, 100), dtype=torch.float32, device="cuda")
+        efg.brute_force_knn_device(x.data_ptr(), n, 16, 16, q.data_ptr(), nq, 16, 100, ids.data_ptr(),
+                                   dist.data_ptr(), screening=screening)
+        torch.cuda.synchronize()
+        out[screening] = (ids.cpu().numpy(), dist.cpu().numpy())
+    assert efg.knn_stats().convert_ms > 0.05  # (the lists' rerun has nothing left to convert)
+    assert np.array_equal(out["auto"][0], out["fp32"][0])
+    assert np.array_equal(out["auto"][1], out["fp32"][1])
