@@ -58,7 +58,7 @@ struct NNDev {
   uint32_t jterms = 0;  // 0: not prepared; 1 or 3 products per value
   bool jexact = false;  // the tensor cores' distances are exact (integers, squared norms below 2^22)
   uint32_t W = 0;          // records per bucket
-  uint64_t bucket_cap = 0, ovf_cap = 0;
+  uint64_t bucket_cap = 0, ovf_cap = 0, last_ovf = 0;  // last_ovf: the last iteration's overflow records
   // every buffer from the stream's pool: only the build's stream uses them
   explicit NNDev(cudaStream_t s) {
     each([s](auto& b) { b.on(s); });
@@ -1390,6 +1390,12 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   if (!tc) EFG_TRY(make_bytes(idx));
   EFG_CUDA(cudaMemsetAsync(S.found.p, 0, n, s));
   uint64_t npairs = 0, novf = 0;
+  if (S.last_ovf + S.last_ovf / 4 > S.ovf_cap) {  // lists that fill up grow before a join has to run again
+    const uint64_t want = S.last_ovf + S.last_ovf / 2;
+    if (S.ovf.reserve(want) == EFG_OK && S.ovf_slot.reserve(want) == EFG_OK) S.ovf_cap = want;
+    EFG_TRY(S.ovf.reserve(S.ovf_cap));  // (where there is no room for more)
+    EFG_TRY(S.ovf_slot.reserve(S.ovf_cap));
+  }
   for (;;) {  // again only when the overflow list was too short for its records
     EFG_CUDA(cudaMemsetAsync(S.totals.p, 0, 32, s));
     EFG_CUDA(cudaMemsetAsync(S.cnt.p, 0, n * 4, s));
@@ -1443,6 +1449,7 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
     EFG_TRY(S.ovf.reserve(S.ovf_cap));
     EFG_TRY(S.ovf_slot.reserve(S.ovf_cap));
   }
+  S.last_ovf = novf;
   if (novf) {  // the hub targets' records gathered in one array
     hub_len_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, S.W, S.cnt.p, S.task_len.p);
     EFG_CUDA(cudaGetLastError());
