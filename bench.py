@@ -275,7 +275,7 @@ def run_gpu(args):
         st = idx.search_stats()
         evals_q = st.distance_evals / nq
         exp_q = st.expanded_nodes / nq
-        row_bytes = {"fp32": 128 * 4, "bf16": 128 * 2, "fp8": 128 + 4}[precision]  # fp8: bytes + row scale
+        row_bytes = {"fp32": 128, "bf16": 128 * 2, "fp8": 128 + 4}[precision]  # fp32: byte rows, this base being bytes; fp8: bytes + row scale
         # algorithmic bytes per query: screened rows + graph rows of expanded nodes + leaf ids + query
         # (+ the FP32 rows re-ranked after BF16/FP8 screening)
         bytes_q = evals_q * row_bytes + exp_q * GRAPH["K"] * 4 + point[1] * 4 + 128 * 4 + st.reranked * 128 * 4
