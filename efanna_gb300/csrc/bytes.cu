@@ -82,7 +82,8 @@ __device__ __forceinline__ uint32_t row_slot(uint32_t r) { return (r & 3u) * (BR
 // groups).  The pairs that make records (a fifth of them) are queued and their records made by whole warps.
 // Bound: instruction issue (half of all slots) and the latency of a node's chain (lists, rows, records'
 // slots), which 16 warps per SM overlap; products are 64 __dp4a per 16-byte chunk and block.  The 1M x 128
-// build's joins: 34.0 ms, 46.7 with each lane making the records of its own pairs, four at a time (half as
+// build's joins: 34.0 ms (28.2 since the first one runs in three parts and overflowing lanes share an atomic),
+// 46.7 with each lane making the records of its own pairs, four at a time (half as
 // many instructions again), and 37.1 with 48 rows a tile and 20 warps per SM.
 __global__ void __launch_bounds__(BW * 32, 4) join_bytes_kernel(const JoinBytesArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
