@@ -1214,14 +1214,37 @@ static int merge_level_check(efg_index* idx, int32_t* min_level) {
   return EFG_OK;
 }
 
-// Records of a first join per node, on average (every pair of the seeded lists is kept: 2 S entries),
-// and whether the first join runs in parts: of every FIRST_STEP nodes those from one entry of FIRST_PARTS to
-// the next, the targets' bounds tightened in between (1M x 128: 8.7 ms; in two parts, 1 and 7, 10.9 ms
-// with half as many records again).
+// The first join keeps every pair of the seeded lists, 2 S (2S - 1) records per node on average (380 for
+// S = 10), of which a pool of P - 1 takes a few dozen.  Where an eighth of the nodes leaves more than P
+// entries per target it runs in parts: of every FIRST_STEP nodes those from one entry of FIRST_PARTS to the
+// next, the targets' bounds tightened in between (1M x 128: 8.7 ms; in two parts, 1 and 7, 10.9 ms with
+// half as many records again).  On the tensor cores only where their distances are exact: else an id may be
+// found at two distances, and would count twice.
 constexpr uint32_t FIRST_STEP = 8, FIRST_PARTS[] = {0, 1, 3, 8};
 static uint64_t first_mean(const efg_build_params& bp) { return 2ull * bp.S * (2 * bp.S - 1); }
-static bool first_in_parts(const efg_build_params& bp, uint32_t P, bool exact) {
-  return exact && P <= TIGHTEN_MAX_P && first_mean(bp) / FIRST_STEP + bp.S >= P + P / 4;
+static bool first_in_parts(const efg_index* idx, const NNDev& S) {
+  const efg_build_params& bp = idx->bp;
+  const bool exact = idx->build_precision != EFG_PRECISION_BF16 || S.jexact;
+  return exact && S.P <= TIGHTEN_MAX_P && first_mean(bp) / FIRST_STEP + bp.S >= S.P + S.P / 4;
+}
+
+// The tensor-core join's rows, and whether its distances are exact (once per build; nothing in FP32).
+static int prepare_tc(efg_index* idx, NNDev& S) {
+  if (idx->build_precision != EFG_PRECISION_BF16 || S.jterms) return EFG_OK;
+  cudaStream_t s = idx->stream;
+  const uint64_t n = S.n, W = (idx->dim + 63) / 64 * 64;
+  EFG_TRY(S.jhi.reserve(n * W));
+  EFG_TRY(S.jlo.reserve(n * W));
+  EFG_TRY(S.jnorm.reserve(n));
+  EFG_TRY(S.jflag.reserve(3));
+  EFG_TRY(S.jmid.reserve(n + 1));
+  EFG_TRY(tc_join_prepare(idx->d_base, n, idx->dim, idx->ld, S.jhi.p, S.jlo.p, S.jnorm.p, S.jflag.p, s));
+  int flags[3] = {0, 0, 0};
+  EFG_CUDA(cudaMemcpyAsync(flags, S.jflag.p, 12, cudaMemcpyDeviceToHost, s));
+  EFG_CUDA(cudaStreamSynchronize(s));
+  S.jterms = flags[0] ? 3 : 1;
+  S.jexact = !flags[0] && !flags[2];
+  return EFG_OK;
 }
 
 // Bucket width: about the records a node receives in the first join, or five pools' worth where pools
@@ -1231,12 +1254,13 @@ static bool first_in_parts(const efg_build_params& bp, uint32_t P, bool exact) {
 // of the memory free at the start; the rest goes to the overflow list.
 static int first_width(efg_index* idx, NNDev& S) {
   if (S.W) return EFG_OK;
+  EFG_TRY(prepare_tc(idx, S));  // (the first join in parts or not: up to twice the records)
   const efg_build_params& bp = idx->bp;
   size_t free_b = 0, total_b = 0;
   EFG_CUDA(cudaMemGetInfo(&free_b, &total_b));
   S.bucket_cap = std::max<uint64_t>(1, (uint64_t)free_b / 4 / sizeof(uint4) / S.n);
   const uint64_t mean = first_mean(bp);
-  const uint64_t expect = first_in_parts(bp, S.P, true) ? mean / FIRST_STEP + 6 * S.P
+  const uint64_t expect = first_in_parts(idx, S) ? mean / FIRST_STEP + 6 * S.P
                                                         : std::max<uint64_t>(mean + mean / 4, S.P > 64 ? 5 * S.P : 0);
   S.W = (uint32_t)std::min<uint64_t>(S.bucket_cap, expect + 32);
   S.ovf_cap = std::max<uint64_t>(S.n * (expect / 4 + 8), 1 << 16);
@@ -1361,27 +1385,9 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   EFG_TRY(S.bound.reserve(n));
   EFG_TRY(S.totals.reserve(4));
   EFG_TRY(S.jctr.reserve(8));
-  // The first join keeps every pair of the seeded lists, 2 S (2S - 1) records per node (380 for
-  // S = 10), of which a pool of P - 1 takes a few dozen.  So in FP32 it runs on 1 of `part` nodes first,
-  // where that leaves about P entries per target, the targets' bounds are tightened, and the other
-  // nodes follow: 1M x 128 keeps 221 records per node instead of 380.  (On the tensor cores only
-  // where their distances are exact: else an id may be found at two distances, and would count twice.)
   const bool tc = idx->build_precision == EFG_PRECISION_BF16;
-  if (tc && !S.jterms) {
-    const uint64_t W = (idx->dim + 63) / 64 * 64;
-    EFG_TRY(S.jhi.reserve(n * W));
-    EFG_TRY(S.jlo.reserve(n * W));
-    EFG_TRY(S.jnorm.reserve(n));
-    EFG_TRY(S.jflag.reserve(3));
-    EFG_TRY(S.jmid.reserve(n + 1));
-    EFG_TRY(tc_join_prepare(idx->d_base, n, idx->dim, idx->ld, S.jhi.p, S.jlo.p, S.jnorm.p, S.jflag.p, s));
-    int inexact[3] = {0, 0, 0};
-    EFG_CUDA(cudaMemcpyAsync(inexact, S.jflag.p, 12, cudaMemcpyDeviceToHost, s));
-    EFG_CUDA(cudaStreamSynchronize(s));
-    S.jterms = inexact[0] ? 3 : 1;
-    S.jexact = !inexact[0] && !inexact[2];
-  }
-  const bool parts = iter == 0 && first_in_parts(bp, S.P, !tc || S.jexact);
+  EFG_TRY(prepare_tc(idx, S));
+  const bool parts = iter == 0 && first_in_parts(idx, S);
   EFG_TRY(first_width(idx, S));
   EFG_TRY(S.bucket.reserve(n * S.W));
   int sms = 152, dev = 0;
@@ -1445,6 +1451,7 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
       idx->bstats.join_large_nodes += tot[3];
       break;
     }
+    ++idx->bstats.join_reruns;
     S.ovf_cap = novf + novf / 4;
     EFG_TRY(S.ovf.reserve(S.ovf_cap));
     EFG_TRY(S.ovf_slot.reserve(S.ovf_cap));

@@ -63,6 +63,7 @@ typedef struct efg_build_stats {
   uint64_t join_records;    /* neighbour-list insert candidates kept after the radius filter    */
   uint64_t merge_distances; /* leaf-merge distances of the initial graph                        */
   int32_t max_merge_depth;  /* on EFG_ERR_MERGE_LEVEL: deepest usable merge level               */
+  uint32_t join_reruns;     /* joins run again because their records outgrew the overflow list   */
   uint64_t join_large_nodes; /* BF16 build precision: node joins larger than one tensor-core tile */
 } efg_build_stats;
 
