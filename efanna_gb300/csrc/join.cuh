@@ -25,6 +25,9 @@ struct RecordSink {
   unsigned long long* ovf_n;   // overflow records found (may exceed ovf_cap: the join runs again)
   uint64_t ovf_cap;
   uint32_t W;
+  // With little memory (W = 0, ovf_cap = 0) a join counts its records first; its second run has their
+  // places, off[t] .. off[t + 1] of ovf for target t: 16 bytes a record and no more.
+  const uint64_t* off;
 };
 
 // A record whose slot lies past its target's bucket.  (Not inlined: rare, and its code would be
@@ -36,6 +39,11 @@ static __device__ __noinline__ void place_overflow(const RecordSink& s, uint32_t
   unsigned long long o = 0;
   if (lane == leader) o = atomicAdd(s.ovf_n, (unsigned long long)__popc(mask));
   o = __shfl_sync(mask, o, leader) + __popc(mask & ((1u << lane) - 1));
+  if (s.off) {
+    const uint64_t at = s.off[t] + slot;
+    if (at < s.off[t + 1]) s.ovf[at] = make_uint4(cand, __float_as_uint(d), aux, t);
+    return;
+  }
   if (o < s.ovf_cap) {
     s.ovf[o] = make_uint4(cand, __float_as_uint(d), aux, t);
     s.ovf_slot[o] = slot;

@@ -59,6 +59,7 @@ struct NNDev {
   bool jexact = false;  // the tensor cores' distances are exact (integers, squared norms below 2^22)
   uint32_t W = 0;          // records per bucket
   uint64_t bucket_cap = 0, ovf_cap = 0, last_ovf = 0;  // last_ovf: the last iteration's overflow records
+  bool scarce = false;  // memory for buckets and lists fell short: every join counts, then places, its records
   // every buffer from the stream's pool: only the build's stream uses them
   explicit NNDev(cudaStream_t s) {
     each([s](auto& b) { b.on(s); });
@@ -68,6 +69,24 @@ struct NNDev {
   }
   NNDev(const NNDev&) = delete;
   NNDev& operator=(const NNDev&) = delete;
+  // Gives the record buffers back (their contents are lost); the build goes on in 16 bytes a record, with
+  // every join run twice.
+  void run_scarce() {
+    bucket.release();
+    ovf.release();
+    ovf_slot.release();
+    ovfrec.release();
+    W = 0;
+    ovf_cap = last_ovf = 0;
+    scarce = true;
+  }
+  // Room in b, at the record buffers' cost when there is no other (while they hold nothing).
+  template <typename B>
+  int room(B& b, uint64_t count) {
+    if (b.reserve(count) == EFG_OK) return EFG_OK;
+    run_scarce();
+    return b.reserve(count);
+  }
   template <typename F>
   void each(F f) {
     auto all = [&](auto&... b) { (f(b), ...); };
@@ -1253,7 +1272,7 @@ static int prepare_tc(efg_index* idx, NNDev& S) {
 // a GB costs about 0.8 ms to allocate and free, more than some overflowing hubs do -- within a quarter
 // of the memory free at the start; the rest goes to the overflow list.
 static int first_width(efg_index* idx, NNDev& S) {
-  if (S.W) return EFG_OK;
+  if (S.W || S.scarce) return EFG_OK;
   EFG_TRY(prepare_tc(idx, S));  // (the first join in parts or not: up to twice the records)
   const efg_build_params& bp = idx->bp;
   size_t free_b = 0, total_b = 0;
@@ -1263,9 +1282,10 @@ static int first_width(efg_index* idx, NNDev& S) {
   const uint64_t expect = first_in_parts(idx, S) ? mean / FIRST_STEP + 6 * S.P
                                                         : std::max<uint64_t>(mean + mean / 4, S.P > 64 ? 5 * S.P : 0);
   S.W = (uint32_t)std::min<uint64_t>(S.bucket_cap, expect + 32);
-  S.ovf_cap = std::max<uint64_t>(S.n * (expect / 4 + 8), 1 << 16);
-  EFG_TRY(S.ovf.reserve(S.ovf_cap));
-  return S.ovf_slot.reserve(S.ovf_cap);
+  // (a list of more than an eighth of the free memory grows to it only when a join finds that many)
+  S.ovf_cap = std::max<uint64_t>(std::min<uint64_t>(S.n * (expect / 4 + 8), (uint64_t)free_b / 8 / 20), 1 << 16);
+  if (S.ovf.reserve(S.ovf_cap) != EFG_OK || S.ovf_slot.reserve(S.ovf_cap) != EFG_OK) S.run_scarce();
+  return EFG_OK;
 }
 
 static int nnd_init_device(efg_index* idx, NNDev& S) {
@@ -1352,7 +1372,7 @@ static int nnd_init_device(efg_index* idx, NNDev& S) {
   idx->bstats.merge_distances = ndist;
   // the leaf merge's records in the join's bucket buffer, allocated once for both
   EFG_TRY(first_width(idx, S));
-  EFG_TRY(S.bucket.reserve(std::max<uint64_t>(n * S.W, nrec / 2 + 1)));
+  if (S.bucket.reserve(std::max<uint64_t>(n * S.W, nrec / 2 + 1)) != EFG_OK) EFG_TRY(S.room(S.bucket, nrec / 2 + 1));
   uint64_t* rec_key_buf = reinterpret_cast<uint64_t*>(S.bucket.p);
   if (keep) {
     merge_emit_kernel<<<(unsigned)std::min<uint64_t>(blocks_for(ntasks, 256), 152ull * 64), 256, 0, s>>>(
@@ -1376,47 +1396,47 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   cudaStream_t s = idx->stream;
   const efg_build_params& bp = idx->bp;
   uint64_t n = S.n;
-  uint32_t ld4 = idx->ld / 4;
   // ---- join
-  EFG_TRY(S.off64.reserve(n + 1));
-  EFG_TRY(S.scan64.reserve(scan_tmp_elems<uint64_t>(2 * n) + 1));
-  EFG_TRY(S.task_len.reserve(n + 1));
-  EFG_TRY(S.cnt.reserve(2 * n));
-  EFG_TRY(S.bound.reserve(n));
-  EFG_TRY(S.totals.reserve(4));
-  EFG_TRY(S.jctr.reserve(8));
   const bool tc = idx->build_precision == EFG_PRECISION_BF16;
   EFG_TRY(prepare_tc(idx, S));
-  const bool parts = iter == 0 && first_in_parts(idx, S);
   EFG_TRY(first_width(idx, S));
-  EFG_TRY(S.bucket.reserve(n * S.W));
+  if (S.scarce) S.bucket.release();  // (the leaf merge's records)
+  EFG_TRY(S.room(S.off64, n + 1));
+  EFG_TRY(S.room(S.scan64, scan_tmp_elems<uint64_t>(2 * n) + 1));
+  EFG_TRY(S.room(S.task_len, n + 1));
+  EFG_TRY(S.room(S.cnt, 2 * n));
+  EFG_TRY(S.room(S.bound, n));
+  EFG_TRY(S.room(S.totals, 4));
+  EFG_TRY(S.room(S.jctr, 8));
+  if (!tc) EFG_TRY(make_bytes(idx));
+  if (tc || idx->bytes_state != 1) EFG_TRY(S.room(S.jbig, n + 1));
+  if (!S.scarce && S.bucket.reserve(n * S.W) != EFG_OK) S.run_scarce();
   int sms = 152, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (!tc) EFG_TRY(make_bytes(idx));
   EFG_CUDA(cudaMemsetAsync(S.found.p, 0, n, s));
-  uint64_t npairs = 0, novf = 0;
-  if (S.last_ovf + S.last_ovf / 4 > S.ovf_cap) {  // lists that fill up grow before a join has to run again
+  uint64_t npairs = 0, novf = 0, large = 0;
+  if (!S.scarce && S.last_ovf + S.last_ovf / 4 > S.ovf_cap) {  // lists that fill up grow before a join has to run again
     const uint64_t want = S.last_ovf + S.last_ovf / 2;
     if (S.ovf.reserve(want) == EFG_OK && S.ovf_slot.reserve(want) == EFG_OK) S.ovf_cap = want;
-    EFG_TRY(S.ovf.reserve(S.ovf_cap));  // (where there is no room for more)
-    EFG_TRY(S.ovf_slot.reserve(S.ovf_cap));
+    else if (S.ovf.reserve(S.ovf_cap) != EFG_OK || S.ovf_slot.reserve(S.ovf_cap) != EFG_OK) S.run_scarce();
   }
-  for (;;) {  // again only when the overflow list was too short for its records
+  bool counted = false;  // (scarce memory) the records of the second run have their places
+  for (;;) {  // again when the overflow list was too short for its records, and with scarce memory
     EFG_CUDA(cudaMemsetAsync(S.totals.p, 0, 32, s));
     EFG_CUDA(cudaMemsetAsync(S.cnt.p, 0, n * 4, s));
     EFG_CUDA(cudaMemsetAsync(S.jctr.p, 0, 32, s));
     bound_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, S.P, S.pd.p, S.Lc.p, S.radius.p, S.new_cnt.p, S.old_cnt.p,
                                                     S.bound.p, S.totals.p);
     EFG_CUDA(cudaGetLastError());
-    const RecordSink sink{S.cnt.p, S.bucket.p, S.ovf.p, S.ovf_slot.p, S.totals.p + 2, S.ovf_cap, S.W};
+    const RecordSink sink{S.cnt.p, S.bucket.p, counted ? S.ovfrec.p : S.ovf.p, S.ovf_slot.p, S.totals.p + 2, S.ovf_cap,
+                          S.W, counted ? S.off64.p : nullptr};
     if (tc) EFG_CUDA(cudaMemsetAsync(S.jflag.p + 1, 0, 4, s));
     auto join = [&](const NodeSet& set) -> int {
       EFG_CUDA(cudaMemsetAsync(S.jctr.p + 1, 0, 12, s));
       if (!tc && idx->bytes_state == 1)
         return join_bytes(idx->bytes.p, idx->bnorm.p, n, idx->ldb, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p,
                           S.old_ids.p, S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + 1, set, s);
-      EFG_TRY(S.jbig.reserve(n + 1));
       EFG_CUDA(cudaMemsetAsync(S.jbig.p, 0, 4, s));
       if (!tc)
         return join_fp32(idx->d_base, n, idx->ld, S.cap, S.P, bp.check_k, S.new_ids.p, S.new_cnt.p, S.old_ids.p,
@@ -1426,7 +1446,7 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
                      S.new_cnt.p, S.old_ids.p, S.old_cnt.p, S.bound.p, sink, S.found.p, S.jctr.p + 1, S.jmid.p,
                      S.jbig.p, S.totals.p + 3, S.jflag.p + 1, set, s);
     };
-    if (parts) {
+    if (iter == 0 && !S.scarce && first_in_parts(idx, S)) {
       for (uint32_t p = 0; p + 1 < sizeof(FIRST_PARTS) / 4; ++p) {
         if (p) {
           tighten_kernel<<<blocks_for(n * 32, 256), 256, 0, s>>>(n, S.P, S.W, S.cnt.p, S.bucket.p, S.pd.p, S.pid.p,
@@ -1446,30 +1466,43 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
     if (jerr & 4) return fail(EFG_ERR_ARG, "tensor-core join: a join list holds an id >= n");
     if (jerr) return fail(EFG_ERR_DEVICE_LIMIT, "tensor-core join: a wait ran out on the device");
     npairs = tot[0];
-    novf = tot[2];
-    if (novf <= S.ovf_cap) {
-      idx->bstats.join_large_nodes += tot[3];
+    large = tot[3];
+    if (counted) {
+      if (tot[2] != novf) return fail(EFG_ERR_STATE, "NN-descent: a join's two runs found different records");
       break;
     }
-    ++idx->bstats.join_reruns;
-    S.ovf_cap = novf + novf / 4;
-    EFG_TRY(S.ovf.reserve(S.ovf_cap));
-    EFG_TRY(S.ovf_slot.reserve(S.ovf_cap));
-  }
-  S.last_ovf = novf;
-  if (novf) {  // the hub targets' records gathered in one array
+    novf = tot[2];
+    if (!S.scarce && novf > S.ovf_cap) {
+      ++idx->bstats.join_reruns;
+      S.ovf_cap = novf + novf / 4;
+      if (S.ovf.reserve(S.ovf_cap) != EFG_OK || S.ovf_slot.reserve(S.ovf_cap) != EFG_OK) S.run_scarce();
+      continue;
+    }
+    if (novf == 0) break;
+    // one array for the hub targets' records (scarce: for all of them, which the second run writes)
     hub_len_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, S.W, S.cnt.p, S.task_len.p);
     EFG_CUDA(cudaGetLastError());
     EFG_TRY(device_scan<uint64_t>(S.task_len.p, n, S.off64.p, S.scan64.p, s));
     uint64_t hub_total = 0;
     EFG_CUDA(cudaMemcpyAsync(&hub_total, S.off64.p + n, 8, cudaMemcpyDeviceToHost, s));
     EFG_CUDA(cudaStreamSynchronize(s));
-    EFG_TRY(S.ovfrec.reserve(hub_total));
+    if (S.scarce) {
+      EFG_TRY(S.ovfrec.reserve(hub_total));
+      counted = true;
+      continue;
+    }
+    if (S.ovfrec.reserve(hub_total) != EFG_OK) {
+      S.run_scarce();
+      continue;
+    }
     hub_copy_kernel<<<blocks_for(n * 32, 256), 256, 0, s>>>(n, S.W, S.cnt.p, S.off64.p, S.bucket.p, S.ovfrec.p);
     EFG_CUDA(cudaGetLastError());
     hub_scatter_kernel<<<blocks_for(novf, 256), 256, 0, s>>>(novf, S.ovf.p, S.ovf_slot.p, S.off64.p, S.ovfrec.p);
     EFG_CUDA(cudaGetLastError());
+    break;
   }
+  S.last_ovf = novf;
+  idx->bstats.join_large_nodes += large;
   auto launch_merge = [&](auto kern, uint32_t warp_bytes) -> int {
     const size_t msmem = (size_t)MERGE_WARPS * warp_bytes;
     EFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem));
@@ -1491,10 +1524,10 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   update_range_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, S.P, bp.S, S.pd.p, S.pid.p, S.Lc.p, S.Range.p,
                                                          S.radius.p, S.radiusM.p, S.found.p);
   EFG_CUDA(cudaGetLastError());
-  EFG_TRY(S.rcnt.reserve(2 * n));
-  EFG_TRY(S.rcur.reserve(2 * n));
-  EFG_TRY(S.roff.reserve(2 * n + 1));
-  EFG_TRY(S.scan32.reserve(scan_tmp_elems<uint32_t>(2 * n) + 1));
+  EFG_TRY(S.room(S.rcnt, 2 * n));  // (the records have been merged)
+  EFG_TRY(S.room(S.rcur, 2 * n));
+  EFG_TRY(S.room(S.roff, 2 * n + 1));
+  EFG_TRY(S.room(S.scan32, scan_tmp_elems<uint32_t>(2 * n) + 1));
   EFG_CUDA(cudaMemsetAsync(S.rcnt.p, 0, 2 * n * 4, s));
   EFG_CUDA(cudaMemsetAsync(S.rcur.p, 0, 2 * n * 4, s));
   update_lists_kernel<0><<<blocks_for(n * 32, 256), 256, 0, s>>>(n, S.P, S.cap, S.pd.p, S.pid.p, S.Range.p, S.radiusM.p,
@@ -1505,7 +1538,7 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   uint32_t nrev = 0;
   EFG_CUDA(cudaMemcpyAsync(&nrev, S.roff.p + 2 * n, 4, cudaMemcpyDeviceToHost, s));
   EFG_CUDA(cudaStreamSynchronize(s));
-  EFG_TRY(S.rbuf.reserve((uint64_t)nrev + 1));
+  EFG_TRY(S.room(S.rbuf, (uint64_t)nrev + 1));
   update_lists_kernel<1><<<blocks_for(n * 32, 256), 256, 0, s>>>(n, S.P, S.cap, S.pd.p, S.pid.p, S.Range.p, S.radiusM.p,
                                                             S.new_ids.p, S.new_cnt.p, S.old_ids.p, S.old_cnt.p,
                                                             S.rcnt.p, S.roff.p, S.rcur.p, S.rbuf.p);
@@ -1518,8 +1551,9 @@ static int nnd_iterate_device(efg_index* idx, NNDev& S, uint32_t iter, uint64_t*
   EFG_CUDA(cudaMemcpyAsync(&nrec, S.totals.p + 1, 8, cudaMemcpyDeviceToHost, s));
   EFG_CUDA(cudaStreamSynchronize(s));
   const uint64_t avg = nrec / n, have = S.bucket.cap / n;
-  S.W = (uint32_t)std::max<uint64_t>(
-      1, std::min<uint64_t>({S.bucket_cap, 3 * avg + 64, std::max<uint64_t>(have, avg + avg / 4 + 32)}));
+  if (!S.scarce)
+    S.W = (uint32_t)std::max<uint64_t>(
+        1, std::min<uint64_t>({S.bucket_cap, 3 * avg + 64, std::max<uint64_t>(have, avg + avg / 4 + 32)}));
   if (pairs_out) *pairs_out = npairs;
   if (recs_out) *recs_out = nrec;
   return EFG_OK;
