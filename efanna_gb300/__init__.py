@@ -657,7 +657,7 @@ class KnnStats(C.Structure):
     _fields_ = [("convert_ms", C.c_double), ("bound_ms", C.c_double), ("screen_ms", C.c_double),
                 ("merge_ms", C.c_double), ("screen_flops", C.c_double), ("tile_flops", C.c_double),
                 ("terms", C.c_uint32), ("stages", C.c_uint32), ("nchunks", C.c_uint32), ("ctas", C.c_uint32),
-                ("sample_rows", C.c_uint32)]
+                ("sample_rows", C.c_uint32), ("list_queries", C.c_uint32)]
 
 
 def knn_stats() -> KnnStats:

@@ -68,6 +68,7 @@ struct TcArgs {
   const float* xnorm;  // squared norms of the base rows, +inf past n (rounded up to a tile)
   const float* qbound; // per query an upper bound of its K2-th distance, or null (+inf)
   uint64_t* part;      // nq x nchunks x K2 keys
+  const uint32_t* qid; // the queries' numbers in the call (exclude_self), or null: 0, 1, ...
   int* err;
   uint64_t n, chunk, first_row;
   uint32_t nq, qtiles, nchunks, K2, kblocks, terms, stages, exclude_self;
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(kThreads<EW>, 1)
       const uint32_t q = qt * TM + et;
       const bool qvalid = q < a.nq;
       const float qn = qvalid ? a.qnorm[q] : 0.f;
-      const uint64_t self = a.exclude_self ? a.first_row + q : ~0ull;
+      const uint64_t self = a.exclude_self && qvalid ? a.first_row + (a.qid ? a.qid[q] : q) : ~0ull;
       uint32_t lcnt = 0;
       // distance bound: the K2-th key's once the list is full; a thread past the queries accepts nothing
       float thr = qvalid ? (a.qbound ? a.qbound[q] : INFINITY) : -1.f;
@@ -866,18 +867,19 @@ __global__ void split_bf16_kernel(const float* __restrict__ src, uint64_t rows, 
 
 // One CTA per query: the query's candidates sorted in shared memory.  With `ids` the K2 smallest are
 // re-ranked in FP64 and the first k written; else the rank-th distance becomes the query's bound (when
-// the buffer holds that many, and all of them).  *over is set when a final buffer was too short.
+// the buffer holds that many, and all of them).  A query whose final buffer was too short is left to the
+// lists: its number goes to over_list, which *over counts.
 __global__ void __launch_bounds__(256) select_kernel(const uint64_t* __restrict__ buf, const uint32_t* __restrict__ cnt,
                                                      uint32_t cap, uint32_t rank, uint32_t* __restrict__ qbound,
                                                      const float* __restrict__ base, uint32_t dim, uint32_t ld,
                                                      const float* __restrict__ q, uint32_t qld, uint32_t k,
                                                      int32_t* __restrict__ ids, float* __restrict__ dists,
-                                                     int* __restrict__ over) {
+                                                     int* __restrict__ over, uint32_t* __restrict__ over_list) {
   extern __shared__ __align__(16) uint64_t keys[];  // next_pow2(candidates), then K2 distances
   const uint64_t qi = blockIdx.x;
   const uint32_t m = cnt[qi], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (m > cap) {
-    if (threadIdx.x == 0 && ids) *over = 1;
+    if (threadIdx.x == 0 && ids) over_list[atomicAdd(over, 1)] = (uint32_t)qi;
     return;
   }
   if (!ids && m < rank) return;
@@ -932,6 +934,40 @@ __global__ void __launch_bounds__(256) select_kernel(const uint64_t* __restrict_
   }
 }
 
+// The listed queries' operands and FP32 rows, one after another (a warp per query), and their results back
+// to their places.
+__global__ void gather_queries_kernel(const uint32_t* __restrict__ list, uint64_t m, const uint4* __restrict__ hi,
+                                      const uint4* __restrict__ lo, const float* __restrict__ norms,
+                                      const float* __restrict__ q, uint32_t W, uint32_t dim, uint64_t qld, uint32_t gld,
+                                      uint4* __restrict__ ghi, uint4* __restrict__ glo, float* __restrict__ gnorms,
+                                      float* __restrict__ gq) {
+  const uint32_t lane = threadIdx.x & 31, w16 = W / 8;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += nw) {
+    const uint64_t r = list[i];
+    for (uint32_t c = lane; c < w16; c += 32) {
+      ghi[i * w16 + c] = hi[r * w16 + c];
+      if (lo) glo[i * w16 + c] = lo[r * w16 + c];
+    }
+    for (uint32_t c = lane; c < gld; c += 32) gq[i * gld + c] = c < dim ? q[r * qld + c] : 0.f;
+    if (lane == 0) gnorms[i] = norms[r];
+  }
+}
+
+__global__ void scatter_results_kernel(const uint32_t* __restrict__ list, uint64_t m, uint32_t k,
+                                       const int32_t* __restrict__ gi, const float* __restrict__ gd,
+                                       int32_t* __restrict__ ids, float* __restrict__ dists) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += nw) {
+    const uint64_t r = list[i];
+    for (uint32_t c = lane; c < k; c += 32) {
+      ids[r * k + c] = gi[i * k + c];
+      if (dists) dists[r * k + c] = gd[i * k + c];
+    }
+  }
+}
+
 }  // namespace
 
 thread_local efg_knn_stats g_knn_stats = {};
@@ -952,7 +988,7 @@ struct Operands {
 
 int knn_lists(const float* base, uint64_t n, uint32_t dim, uint32_t ld, const float* q, uint64_t nq, uint32_t qld,
               uint32_t k, int exclude_self, uint64_t first_row, int32_t* ids, float* dists, cudaStream_t s,
-              const Operands& op);
+              const Operands& op, const uint32_t* qid);
 
 // Stream-ordered memory of one call.
 struct CallBuf {
@@ -1126,7 +1162,8 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   uint32_t *qbound, *cnt;
   uint64_t* buf;
   EFG_TRY(mem.get(&qbound, nq));
-  EFG_TRY(mem.get(&cnt, nq));
+  EFG_TRY(mem.get(&cnt, 2 * nq));
+  uint32_t* over_list = cnt + nq;  // queries whose buffer was too short
   EFG_TRY(mem.get(&buf, nq * cap));
   EFG_CUDA(cudaMemsetAsync(qbound, 0, nq * 4, s));
   const size_t sel_smem = (size_t)cap * 8 + (size_t)rank * 8;
@@ -1179,7 +1216,7 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     EFG_CUDA(cudaMemsetAsync(cnt, 0, nq * 4, s));
     EFG_TRY(pass(false, m1h, m1l, bn, S1, 0, qbound, nullptr, cnt, buf, cap, 0));
     select_kernel<<<(unsigned)nq, 256, sel_smem, s>>>(buf, cnt, cap, rank, qbound, nullptr, 0, 0, nullptr, 0, 0, nullptr,
-                                                      nullptr, nullptr);
+                                                      nullptr, nullptr, nullptr);
     EFG_CUDA(cudaGetLastError());
     S = (uint32_t)S1;
   } else if (n >= 16ull * (rank + 8)) {  // a small base: groups of it all (the last tile may be partly empty)
@@ -1206,42 +1243,69 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   EFG_TRY(pass(false, mxh, mxl, xn, n, 0, bounded ? qbound : nullptr, nullptr, cnt, buf, cap, exclude_self));
   EFG_CUDA(cudaEventRecord(ev[3], s));
   select_kernel<<<(unsigned)nq, 256, sel_smem, s>>>(buf, cnt, cap, K2, nullptr, base, dim, ld, q, qld, k, ids, dists,
-                                                    flags + 2);
+                                                    flags + 2, over_list);
   EFG_CUDA(cudaGetLastError());
   EFG_CUDA(cudaEventRecord(ev[4], s));
   EFG_CUDA(cudaMemcpyAsync(hflags, flags, 16, cudaMemcpyDeviceToHost, s));
   EFG_CUDA(cudaStreamSynchronize(s));
   if (hflags[1]) return fail(EFG_ERR_DEVICE_LIMIT, "tensor-core k-NN: a pipeline wait ran out (error word " +
                                                        std::to_string(hflags[1]) + ")");
-  if (hflags[2]) {  // more values under a bound than its buffer holds (many equal distances): sorted lists
-    if (!split) xl = xh;
-    if (!split) ql = qh;
-    return knn_lists(base, n, dim, ld, q, nq, qld, k, exclude_self, first_row, ids, dists, s,
-                     Operands{xh, xl, qh, ql, xn, qn, flags, terms});
+  const uint64_t over = (uint64_t)hflags[2];
+  efg_knn_stats lists = {};
+  if (over) {
+    // more values under a bound than a buffer holds (many rows at nearly one distance): sorted lists for
+    // these queries, gathered unless they are all of the call's
+    Operands op{xh, split ? xl : xh, qh, split ? ql : qh, xn, qn, flags, terms};
+    if (over == nq) {
+      EFG_TRY(knn_lists(base, n, dim, ld, q, nq, qld, k, exclude_self, first_row, ids, dists, s, op, nullptr));
+    } else {
+      __nv_bfloat16 *gh, *gl = nullptr;
+      float *gn, *gq, *gd = nullptr;
+      int32_t* gi;
+      const uint32_t gld = (uint32_t)round_up(dim, 4);
+      EFG_TRY(mem.get(&gh, over * W));
+      if (split) EFG_TRY(mem.get(&gl, over * W));
+      EFG_TRY(mem.get(&gn, over));
+      EFG_TRY(mem.get(&gq, over * gld));
+      EFG_TRY(mem.get(&gi, over * k));
+      if (dists) EFG_TRY(mem.get(&gd, over * k));
+      gather_queries_kernel<<<blocks(over), 256, 0, s>>>(over_list, over, (const uint4*)qh, (const uint4*)ql, qn, q, W,
+                                                         dim, qld, gld, (uint4*)gh, (uint4*)gl, gn, gq);
+      EFG_CUDA(cudaGetLastError());
+      op.qh = gh;
+      op.ql = split ? gl : gh;
+      op.qn = gn;
+      EFG_TRY(knn_lists(base, n, dim, ld, gq, over, gld, k, exclude_self, first_row, gi, gd, s, op, over_list));
+      scatter_results_kernel<<<blocks(over), 256, 0, s>>>(over_list, over, k, gi, gd, ids, dists);
+      EFG_CUDA(cudaGetLastError());
+      EFG_CUDA(cudaStreamSynchronize(s));  // (a call has its results when it returns)
+    }
+    lists = g_knn_stats;
   }
   float ms[4] = {0, 0, 0, 0};
   for (int i = 0; i < 4; ++i) cudaEventElapsedTime(&ms[i], ev[i], ev[i + 1]);
   g_knn_stats.convert_ms = ms[0];
-  g_knn_stats.bound_ms = ms[1];
-  g_knn_stats.screen_ms = ms[2];
-  g_knn_stats.merge_ms = ms[3];
+  g_knn_stats.bound_ms = ms[1] + lists.bound_ms;
+  g_knn_stats.screen_ms = ms[2] + lists.screen_ms;
+  g_knn_stats.merge_ms = ms[3] + lists.merge_ms;
   g_knn_stats.sample_rows = S;
   g_knn_stats.screen_flops = 2.0 * (double)nq * (double)n * (double)dim;
-  g_knn_stats.tile_flops = 2.0 * (double)(qgroups * NT * TM) * (double)(ntiles * TN) * (double)W * (double)terms;
+  g_knn_stats.tile_flops = 2.0 * (double)(qgroups * NT * TM) * (double)(ntiles * TN) * (double)W * (double)terms + lists.tile_flops;
   g_knn_stats.terms = terms;
   g_knn_stats.stages = stages;
   g_knn_stats.nchunks = nchunks;
   g_knn_stats.ctas = grid;
+  g_knn_stats.list_queries = (uint32_t)over;
   return EFG_OK;
 }
 
 namespace {
 
 // The same result with sorted lists of K2 keys per (query, chunk), whatever the number of values under a
-// bound: for calls whose candidate buffers were too short.
+// bound: for queries whose candidate buffers were too short (qid: their numbers in the call, or null for all).
 int knn_lists(const float* base, uint64_t n, uint32_t dim, uint32_t ld, const float* q, uint64_t nq, uint32_t qld,
               uint32_t k, int exclude_self, uint64_t first_row, int32_t* ids, float* dists, cudaStream_t s,
-              const Operands& op) {
+              const Operands& op, const uint32_t* qid) {
   const uint32_t K2 = (uint32_t)std::min<uint64_t>(k + 16, n);
   const uint32_t W = (dim + TKB - 1) / TKB * TKB;
   const uint32_t kblocks = W / TKB;
@@ -1306,6 +1370,7 @@ int knn_lists(const float* base, uint64_t n, uint32_t dim, uint32_t ld, const fl
     a.xnorm = xnorm;
     a.qbound = qb;
     a.part = out;
+    a.qid = qid;
     a.err = flags + 1;
     a.n = rows;
     a.chunk = chunk_rows;

@@ -383,6 +383,7 @@ typedef struct efg_knn_stats {
   uint32_t terms;       /* BF16 products per value: 1 (exact data) or 3 (hi.hi + hi.lo + lo.hi)      */
   uint32_t stages, nchunks, ctas;
   uint32_t sample_rows; /* base rows of the bound pass (0: none, small bases)                        */
+  uint32_t list_queries; /* queries with more candidates than their buffer holds, done by sorted lists */
 } efg_knn_stats;
 int efg_get_knn_stats(efg_knn_stats* out);
 /* The same with the screening in FP32 on CUDA cores (squared differences, any k <= 256). */
