@@ -31,3 +31,39 @@ def test_only_queries_among_copies_take_the_lists(efg, k, d, near, exclude, scre
     tc = _knn(efg, x, q, k, screening, exclude=exclude, first_row=first if exclude else 0)
     assert efg.knn_stats().list_queries == near
     assert np.array_equal(tc[0], f32[0]) and np.array_equal(tc[1], f32[1])
+
+
+def _classes(rng, n, nq, d, classes, order):
+    """Rows and queries of `classes` distant classes; the rows class by class or in turn."""
+    centres = rng.integers(0, 200, (classes, d))
+    of = np.arange(n) * classes // n if order == "sorted" else np.arange(n) % classes
+    x = centres[of] + rng.integers(0, 50, (n, d))
+    q = centres[rng.integers(0, classes, nq)] + rng.integers(0, 50, (nq, d))
+    return x.astype(np.float32), q.astype(np.float32)
+
+
+@pytest.mark.parametrize("n,nq,k,order,classes", [
+    (20_000, 300, 10, "sorted", 4), (60_011, 300, 100, "sorted", 10), (7_000, 200, 104, "sorted", 5),
+    (60_011, 300, 100, "in turn", 2), (1 << 16, 300, 10, "sorted", 8), (300_000, 300, 10, "sorted", 30)])
+def test_bounds_hold_whatever_the_order_of_the_rows(efg, n, nq, k, order, classes):
+    """Rows in class order and classes in turn: the bounds' groups and samples reach every class, so that no
+    query finds a whole class under its bound."""
+    x, q = _classes(np.random.default_rng(n + k), n, nq, 64, classes, order)
+    for screening in ("auto", "split"):
+        tc = _knn(efg, x, q, k, screening)
+        assert efg.knn_stats().list_queries == 0
+        f32 = _knn(efg, x, q, k, "fp32")
+        assert np.array_equal(tc[0], f32[0]) and np.array_equal(tc[1], f32[1])
+
+
+@pytest.mark.parametrize("n", [544, 545, 607, 1_791, 2_063, 4_300, 28_799])
+@pytest.mark.parametrize("k,d", [(1, 5), (10, 64), (10, 129)])
+def test_strided_groups_at_their_edges(efg, n, k, d):
+    """Boxes of 16 and 64 rows a prime number apart, with empty columns at their ends."""
+    rng = np.random.default_rng(n + d)
+    x = rng.integers(0, 256, (n, d)).astype(np.float32)
+    q = rng.integers(0, 256, (150, d)).astype(np.float32)
+    for screening in ("auto", "split"):
+        tc = _knn(efg, x, q, k, screening)
+        f32 = _knn(efg, x, q, k, "fp32")
+        assert np.array_equal(tc[0], f32[0]) and np.array_equal(tc[1], f32[1])
