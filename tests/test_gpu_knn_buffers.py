@@ -44,7 +44,8 @@ def _classes(rng, n, nq, d, classes, order):
 
 @pytest.mark.parametrize("n,nq,k,order,classes", [
     (20_000, 300, 10, "sorted", 4), (60_011, 300, 100, "sorted", 10), (7_000, 200, 104, "sorted", 5),
-    (60_011, 300, 100, "in turn", 2), (1 << 16, 300, 10, "sorted", 8), (300_000, 300, 10, "sorted", 30)])
+    (60_011, 300, 100, "in turn", 2), (1 << 16, 300, 10, "sorted", 8), (1 << 18, 500, 10, "in turn", 16),
+    (1 << 18, 500, 100, "in turn", 8), (300_000, 300, 10, "sorted", 30)])
 def test_bounds_hold_whatever_the_order_of_the_rows(efg, n, nq, k, order, classes):
     """Rows in class order and classes in turn: the bounds' groups and samples reach every class, so that no
     query finds a whole class under its bound."""
