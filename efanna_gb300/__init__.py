@@ -175,6 +175,7 @@ def lib():
         "efg_brute_force_knn_noalloc": (i32, [vp, u64, u32, u64, vp, u64, u64, u32, i32, u64, vp, vp, vp]),
         "efg_brute_force_knn_fp32": (i32, [vp, u64, u32, u64, vp, u64, u64, u32, i32, u64, vp, vp, vp]),
         "efg_get_knn_stats": (i32, [vp]),
+        "efg_brute_force_knn_within": (i32, [vp, u64, u32, u64, vp, u64, u64, u32, i32, u64, vp, vp, u64, vp]),
         "efg_brute_force_knn_split": (i32, [vp, u64, u32, u64, vp, u64, u64, u32, i32, u64, vp, vp, vp]),
         "efg_knn_search_batch": (i32, [vp, f32p, u64, u32, u64, vp, u32, C.POINTER(C.c_int32)]),
         "efg_knn_search_batch_device": (i32, [vp, vp, u64, u64, vp, C.POINTER(QueryParams), vp, vp, vp]),

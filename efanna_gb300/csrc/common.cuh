@@ -17,9 +17,11 @@ int fail(int code, const std::string& msg);
 #define EFG_CUDA(call)                                                                  \
   do {                                                                                  \
     cudaError_t e_ = (call);                                                            \
-    if (e_ != cudaSuccess)                                                              \
+    if (e_ != cudaSuccess) {                                                            \
+      cudaGetLastError(); /* a later launch's check must not find this error */         \
       return ::efg::fail(e_ == cudaErrorMemoryAllocation ? EFG_ERR_NOMEM : EFG_ERR_CUDA, \
                          std::string(#call) + ": " + cudaGetErrorString(e_));          \
+    }                                                                                   \
   } while (0)
 
 #define EFG_TRY(expr)        \

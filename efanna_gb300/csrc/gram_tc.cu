@@ -430,6 +430,9 @@ __global__ void bound_kernel(const uint64_t* __restrict__ lists, uint64_t nq, ui
 constexpr uint32_t SW_ = 16;                    // screening warps: eight per accumulator buffer
 constexpr uint32_t STH = 64 + 32 * SW_;         // threads
 constexpr uint32_t CAND_MAX = 4096;             // candidates a query's buffer can hold
+// Bytes of candidate buffers: more queries than they serve (262,144 at k = 1, 131,072 at k = 10, 65,536 from
+// k = 27 on, far more than keep the chip busy) are taken in blocks.
+constexpr uint64_t CAND_BYTES = 2ull << 30;
 
 struct ScreenArgs {
   const float* qnorm;     // nq FP32 squared norms
@@ -892,18 +895,19 @@ __global__ void split_bf16_kernel(const float* __restrict__ src, uint64_t rows, 
 // One CTA per query: the query's candidates sorted in shared memory.  With `ids` the K2 smallest are
 // re-ranked in FP64 and the first k written; else the rank-th distance becomes the query's bound (when
 // the buffer holds that many, and all of them).  A query whose final buffer was too short is left to the
-// lists: its number goes to over_list, which *over counts.
+// lists: its number (q0 the first's) goes to over_list, which *over counts.
 __global__ void __launch_bounds__(256) select_kernel(const uint64_t* __restrict__ buf, const uint32_t* __restrict__ cnt,
                                                      uint32_t cap, uint32_t rank, uint32_t* __restrict__ qbound,
                                                      const float* __restrict__ base, uint32_t dim, uint32_t ld,
                                                      const float* __restrict__ q, uint32_t qld, uint32_t k,
                                                      int32_t* __restrict__ ids, float* __restrict__ dists,
-                                                     int* __restrict__ over, uint32_t* __restrict__ over_list) {
+                                                     int* __restrict__ over, uint32_t* __restrict__ over_list,
+                                                     uint32_t q0) {
   extern __shared__ __align__(16) uint64_t keys[];  // next_pow2(candidates), then K2 distances
   const uint64_t qi = blockIdx.x;
   const uint32_t m = cnt[qi], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (m > cap) {
-    if (threadIdx.x == 0 && ids) over_list[atomicAdd(over, 1)] = (uint32_t)qi;
+    if (threadIdx.x == 0 && ids) over_list[atomicAdd(over, 1)] = q0 + (uint32_t)qi;
     return;
   }
   if (!ids && m < rank) return;
@@ -1028,7 +1032,8 @@ struct CallBuf {
   std::vector<void*> p;
   explicit CallBuf(cudaStream_t st) : s(st) {}
   ~CallBuf() {
-    for (void* x : p) cudaFreeAsync(x, s);
+    for (void* x : p)
+      if (x) cudaFreeAsync(x, s);
   }
   template <typename T>
   int get(T** out, uint64_t count) {
@@ -1038,32 +1043,50 @@ struct CallBuf {
     *out = reinterpret_cast<T*>(x);
     return EFG_OK;
   }
+  void drop(void* x) {
+    for (void*& y : p)
+      if (y == x) {
+        cudaFreeAsync(x, s);
+        y = nullptr;
+      }
+  }
 };
 
 }  // namespace
 
 int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld, const float* q, uint64_t nq,
                        uint32_t qld, uint32_t k, int exclude_self, uint64_t first_row, int32_t* ids, float* dists,
-                       cudaStream_t s, int force_split) {
+                       cudaStream_t s, int force_split, uint64_t cand_bytes) {
   if (nq == 0) return EFG_OK;
   if (n >= (1ull << 31) || nq >= (1ull << 31)) return fail(EFG_ERR_ARG, "tensor-core k-NN: more than 2^31 rows");
   if (k > tc_knn_max_k()) return fail(EFG_ERR_ARG, "tensor-core k-NN: k above " + std::to_string(tc_knn_max_k()));
   const uint32_t K2 = (uint32_t)std::min<uint64_t>(k + 16, n);
   const uint32_t W = (dim + TKB - 1) / TKB * TKB, kblocks = W / TKB;
-  const uint64_t qtiles = (nq + TM - 1) / TM, ntiles = (n + TN - 1) / TN;
+  const uint64_t ntiles = (n + TN - 1) / TN;
   int dev = 0, sms = 148, smem_max = 0;
   EFG_CUDA(cudaGetDevice(&dev));
   EFG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   EFG_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  cudaEvent_t ev[5] = {};
-  struct EvGuard {
-    cudaEvent_t* e;
-    ~EvGuard() {
-      for (int i = 0; i < 5; ++i)
-        if (e[i]) cudaEventDestroy(e[i]);
+  // start, then bounds, screening and selection of each block of queries, end
+  struct Events {
+    std::vector<cudaEvent_t> e;
+    size_t n = 0;  // recorded
+    ~Events() {
+      for (cudaEvent_t x : e) cudaEventDestroy(x);
     }
-  } evguard{ev};
-  for (auto& e : ev) EFG_CUDA(cudaEventCreate(&e));
+    int make() {
+      cudaEvent_t x;
+      EFG_CUDA(cudaEventCreate(&x));
+      e.push_back(x);
+      return EFG_OK;
+    }
+    int record(cudaStream_t st) {
+      if (n == e.size()) EFG_TRY(make());
+      EFG_CUDA(cudaEventRecord(e[n++], st));
+      return EFG_OK;
+    }
+  } ev;
+  for (int i = 0; i < 5; ++i) EFG_TRY(ev.make());  // (one block's)
   CallBuf mem(s);
 
   // operands: BF16 rows, norms, flags {inexact, error, a buffer too short}.  A thin sample tells whether
@@ -1077,7 +1100,7 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   EFG_TRY(mem.get(&qn, nq));
   EFG_TRY(mem.get(&flags, 4));
   EFG_CUDA(cudaMemsetAsync(flags, 0, 16, s));
-  EFG_CUDA(cudaEventRecord(ev[0], s));
+  EFG_TRY(ev.record(s));
   auto blocks = [&](uint64_t warps) { return (unsigned)((std::min<uint64_t>(warps, (uint64_t)sms * 64) + 7) / 8); };
   const uint64_t thin = std::max<uint64_t>(1, n / 1024);
   split_bf16_kernel<<<blocks(n / thin + 1), 256, 0, s>>>(base, n, thin, dim, ld, W, nullptr, nullptr, nullptr, n, flags);
@@ -1104,6 +1127,33 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   }
   const uint32_t terms = split ? 3u : 1u, parts = split ? 2u : 1u;
 
+  EFG_TRY(ev.record(s));
+
+  // Candidate buffers, and the block of queries they serve at a time (in whole query groups; fewer where
+  // memory is short).  rank = K2, + 1 with exclude_self (a sample may hold the query itself).
+  const uint32_t rank = K2 + (exclude_self ? 1u : 0u);
+  uint32_t cap = 1024;  // three times the 16 x rank expected under a bound from n / 16 rows
+  while (cap < 48 * rank && cap < CAND_MAX) cap *= 2;
+  constexpr uint64_t QGROUP = 2 * TM;
+  const uint64_t most = std::max<uint64_t>(1, (cand_bytes ? cand_bytes : CAND_BYTES) / (8 * cap) / QGROUP) * QGROUP;
+  uint64_t QB = nq;
+  if (nq > most) {  // blocks of about one size
+    const uint64_t nb = (nq + most - 1) / most;
+    QB = round_up((nq + nb - 1) / nb, QGROUP);
+  }
+  uint32_t *qbound, *cnt;
+  uint64_t* buf;
+  EFG_TRY(mem.get(&qbound, nq));
+  EFG_TRY(mem.get(&cnt, 2 * nq));
+  uint32_t* over_list = cnt + nq;  // queries whose buffer was too short
+  for (;;) {
+    const int rc = mem.get(&buf, QB * cap);
+    if (rc == EFG_OK) break;
+    if (rc != EFG_ERR_NOMEM || QB <= QGROUP) return rc;
+    QB = round_up(QB / 2, QGROUP);
+  }
+  const uint64_t qtiles = (QB + TM - 1) / TM;
+
   // Query tiles per item, and whether their blocks stay in shared memory: two tiles unless that would
   // leave a tile empty for a few queries (300 queries: three tiles as three items, not two pairs) or the
   // stages would not fit; resident with at least three stages of base blocks beside them, else streamed
@@ -1119,18 +1169,14 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     stages = (uint32_t)std::min<int64_t>(MAX_STAGES, (room - (resident ? qbytes : 0)) / stage_bytes);
     if (stages >= 2 || NT == 1) break;
   }
-  const uint32_t qgroups = (uint32_t)((qtiles + NT - 1) / NT);
-
   CUtensorMap mqh, mql, mxh, mxl;
-  EFG_TRY(make_map(&mqh, qh, nq, W));
-  EFG_TRY(make_map(&mql, split ? ql : qh, nq, W));
   EFG_TRY(make_map(&mxh, xh, n, W));
   EFG_TRY(make_map(&mxl, split ? xl : xh, n, W));
 
   unsigned grid = 0;
-  uint32_t nchunks = 1;
-  uint64_t chunk_tiles = 1;
-  // One pass over `rows` rows (maps, norms): the chunk count that keeps the SMs busiest, time ~ waves x
+  uint32_t nchunks = 1, qgroups = 0;
+  uint64_t chunk_tiles = 1, q0 = 0, nqb = 0;  // the block: its first query, its queries (and their groups, maps)
+  // One pass of the block's queries over `rows` rows (maps, norms): the chunk count that keeps the SMs busiest, time ~ waves x
   // (tiles per item, and about two for an item's start); chunks of whole groups for the MIN pass.
   auto pass = [&](bool minp, const CUtensorMap& mh, const CUtensorMap& ml, const float* xnorm, uint64_t rows,
                   uint32_t group_tiles, const uint32_t* qbound, uint32_t* qmax, uint32_t* cnt, uint64_t* buf,
@@ -1153,7 +1199,7 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
         nchunks = (uint32_t)real;
       }
     }
-    a.qnorm = qn;
+    a.qnorm = qn + q0;
     a.xnorm = xnorm;
     a.qbound = qbound;
     a.qmax = qmax;
@@ -1161,12 +1207,12 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     a.buf = buf;
     a.err = flags + 1;
     a.n = rows;
-    a.first_row = first_row;
+    a.first_row = first_row + q0;
     a.ntiles = (uint32_t)tiles;
     a.chunk_tiles = (uint32_t)chunk_tiles;
     a.nchunks = nchunks;
     a.qgroups = qgroups;
-    a.nq = (uint32_t)nq;
+    a.nq = (uint32_t)nqb;
     a.cap = cap;
     a.kblocks = kblocks;
     a.stages = stages;
@@ -1190,26 +1236,19 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     return EFG_OK;
   };
 
-  // 1. bounds.  rank = K2, + 1 with exclude_self (a sample may hold the query itself).
-  EFG_CUDA(cudaEventRecord(ev[1], s));
-  const uint32_t rank = K2 + (exclude_self ? 1u : 0u);
-  uint32_t cap = 1024;  // three times the 16 x rank expected under a bound from n / 16 rows
-  while (cap < 48 * rank && cap < CAND_MAX) cap *= 2;
-  uint32_t *qbound, *cnt;
-  uint64_t* buf;
-  EFG_TRY(mem.get(&qbound, nq));
-  EFG_TRY(mem.get(&cnt, 2 * nq));
-  uint32_t* over_list = cnt + nq;  // queries whose buffer was too short
-  EFG_TRY(mem.get(&buf, nq * cap));
-  EFG_CUDA(cudaMemsetAsync(qbound, 0, nq * 4, s));
+  // 1. bounds: how, and the sample
   const size_t sel_smem = (size_t)cap * 8 + (size_t)rank * 8;
   EFG_CUDA(cudaFuncSetAttribute(select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem));
   uint64_t S1 = std::min<uint64_t>(n / 16, 1u << 20) / TN * TN;  // rows of the append pass's sample
   const uint64_t gtiles = (rank + 3) / 4 * 2;                          // tiles that hold `rank` groups of 64 columns, an even number
-  uint32_t S = 0;
-  bool bounded = true;
-  if (S1 >= gtiles * TN) {
-    uint32_t gt = 1;  // tiles per group: up to a third of the sample for the MIN pass
+  uint32_t S = 0, gt = 0;  // rows of the last bound pass (0: no bounds); tiles per group
+  CUtensorMap m0h, m0l, m1h, m1l;  // of the MIN pass and the append pass
+  uint64_t min_rows = 0;
+  const float* min_norms = xn;
+  uint32_t min_stride = 0, min_box = TN;
+  const bool sampled = S1 >= gtiles * TN;
+  if (sampled) {
+    gt = 1;  // up to a third of the sample for the MIN pass
     while (gt < 16 && gtiles * (2 * gt) * TN * 3 <= S1) gt *= 2;
     // Values of the sample under the MIN pass's bound: a share p of them, where all of the `rank` groups of
     // 64 gt columns have one below it; (1 - p)^(64 gt) rank nq = 1 / 32 says what their buffers must hold.  A
@@ -1242,52 +1281,61 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     scatter_sample_kernel<<<blocks(S1), 256, 0, s>>>((const uint4*)xh, (const uint4*)xl, xn, n, W, (uint32_t)S1, step,
                                                      (uint4*)bh, (uint4*)bl, bn);
     EFG_CUDA(cudaGetLastError());
-    const uint64_t S0 = gtiles * gt * TN;
-    CUtensorMap m0h, m0l, m1h, m1l;
-    EFG_TRY(make_map(&m0h, bh, S0, W));
-    EFG_TRY(make_map(&m0l, split ? bl : bh, S0, W));
+    min_rows = gtiles * gt * TN;
+    min_norms = bn;
+    EFG_TRY(make_map(&m0h, bh, min_rows, W));
+    EFG_TRY(make_map(&m0l, split ? bl : bh, min_rows, W));
     EFG_TRY(make_map(&m1h, bh, S1, W));
     EFG_TRY(make_map(&m1l, split ? bl : bh, S1, W));
-    EFG_TRY(pass(true, m0h, m0l, bn, S0, gt, nullptr, qbound, nullptr, nullptr, 0, 0));
-    EFG_CUDA(cudaMemsetAsync(cnt, 0, nq * 4, s));
-    EFG_TRY(pass(false, m1h, m1l, bn, S1, 0, qbound, nullptr, cnt, buf, cap, 0));
-    select_kernel<<<(unsigned)nq, 256, sel_smem, s>>>(buf, cnt, cap, rank, qbound, nullptr, 0, 0, nullptr, 0, 0, nullptr,
-                                                      nullptr, nullptr, nullptr);
-    EFG_CUDA(cudaGetLastError());
     S = (uint32_t)S1;
   } else if (n >= 16ull * (rank + 8)) {  // a small base: groups of it all (the last tile may be partly empty)
     const uint64_t full = n / TN;
-    uint32_t gt = 0;  // groups of 16 columns, or of 64 columns x gt tiles
+    // groups of 16 columns, or of 64 columns x gt tiles
     while (full / (gt ? 4 * gt : 2) * 4 >= rank) gt = gt ? 2 * gt : 1;
     if (gt || full * 8 >= rank) {
       // Boxes of 64 or 16 rows (one of a group's) whose rows are a prime number apart, the least that spreads
       // them over the whole base: groups of neighbouring rows would give bounds that let a whole class
       // through where rows come class by class, a multiple of its period where classes alternate (20k x
       // 128 in four classes, 10k queries: 4.2 ms with all of them in the lists, 1.3 ms this way).
-      const uint64_t rows = gt ? full / (2 * gt) * (2 * gt) * TN : full * TN;
-      const uint32_t box = gt ? 64 : 16;
-      const uint32_t stride = next_prime((uint32_t)((n + box - 1) / box));
-      CUtensorMap m0h, m0l;
-      EFG_TRY(make_map(&m0h, xh, std::min<uint64_t>(box, n / stride), stride * W, box));
-      EFG_TRY(make_map(&m0l, split ? xl : xh, std::min<uint64_t>(box, n / stride), stride * W, box));
-      EFG_TRY(pass(true, m0h, m0l, xn, rows, gt, nullptr, qbound, nullptr, nullptr, 0, 0, stride, box));
-      S = (uint32_t)rows;
-    } else {
-      bounded = false;
+      min_rows = gt ? full / (2 * gt) * (2 * gt) * TN : full * TN;
+      min_box = gt ? 64 : 16;
+      min_stride = next_prime((uint32_t)((n + min_box - 1) / min_box));
+      EFG_TRY(make_map(&m0h, xh, std::min<uint64_t>(min_box, n / min_stride), min_stride * W, min_box));
+      EFG_TRY(make_map(&m0l, split ? xl : xh, std::min<uint64_t>(min_box, n / min_stride), min_stride * W, min_box));
+      S = (uint32_t)min_rows;
     }
-  } else {
-    bounded = false;
   }
 
-  // 2. the whole base, 3. the candidates' order
-  EFG_CUDA(cudaEventRecord(ev[2], s));
-  EFG_CUDA(cudaMemsetAsync(cnt, 0, nq * 4, s));
-  EFG_TRY(pass(false, mxh, mxl, xn, n, 0, bounded ? qbound : nullptr, nullptr, cnt, buf, cap, exclude_self));
-  EFG_CUDA(cudaEventRecord(ev[3], s));
-  select_kernel<<<(unsigned)nq, 256, sel_smem, s>>>(buf, cnt, cap, K2, nullptr, base, dim, ld, q, qld, k, ids, dists,
-                                                    flags + 2, over_list);
-  EFG_CUDA(cudaGetLastError());
-  EFG_CUDA(cudaEventRecord(ev[4], s));
+  double tile_rows = 0;  // queries' rows in the tiles
+  for (q0 = 0; q0 < nq; q0 += QB) {
+    nqb = std::min(QB, nq - q0);
+    qgroups = (uint32_t)(((nqb + TM - 1) / TM + NT - 1) / NT);
+    tile_rows += (double)(qgroups * NT * TM);
+    EFG_TRY(make_map(&mqh, qh + q0 * W, nqb, W));
+    EFG_TRY(make_map(&mql, (split ? ql : qh) + q0 * W, nqb, W));
+    if (q0) EFG_TRY(ev.record(s));
+    if (S) {
+      EFG_CUDA(cudaMemsetAsync(qbound, 0, nqb * 4, s));
+      EFG_TRY(pass(true, m0h, m0l, min_norms, min_rows, gt, nullptr, qbound, nullptr, nullptr, 0, 0, min_stride, min_box));
+    }
+    if (sampled) {
+      EFG_CUDA(cudaMemsetAsync(cnt, 0, nqb * 4, s));
+      EFG_TRY(pass(false, m1h, m1l, min_norms, S1, 0, qbound, nullptr, cnt, buf, cap, 0));
+      select_kernel<<<(unsigned)nqb, 256, sel_smem, s>>>(buf, cnt, cap, rank, qbound, nullptr, 0, 0, nullptr, 0, 0,
+                                                         nullptr, nullptr, nullptr, nullptr, 0);
+      EFG_CUDA(cudaGetLastError());
+    }
+    // 2. the whole base, 3. the candidates' order
+    EFG_TRY(ev.record(s));
+    EFG_CUDA(cudaMemsetAsync(cnt, 0, nqb * 4, s));
+    EFG_TRY(pass(false, mxh, mxl, xn, n, 0, S ? qbound : nullptr, nullptr, cnt, buf, cap, exclude_self));
+    EFG_TRY(ev.record(s));
+    select_kernel<<<(unsigned)nqb, 256, sel_smem, s>>>(buf, cnt, cap, K2, nullptr, base, dim, ld, q + q0 * qld, qld, k,
+                                                       ids + q0 * k, dists ? dists + q0 * k : nullptr, flags + 2,
+                                                       over_list, (uint32_t)q0);
+    EFG_CUDA(cudaGetLastError());
+  }
+  EFG_TRY(ev.record(s));
   EFG_CUDA(cudaMemcpyAsync(hflags, flags, 16, cudaMemcpyDeviceToHost, s));
   EFG_CUDA(cudaStreamSynchronize(s));
   if (hflags[1]) return fail(EFG_ERR_DEVICE_LIMIT, "tensor-core k-NN: a pipeline wait ran out (error word " +
@@ -1295,6 +1343,7 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   const uint64_t over = (uint64_t)hflags[2];
   efg_knn_stats lists = {};
   if (over) {
+    mem.drop(buf);
     // more values under a bound than a buffer holds (many rows at nearly one distance): sorted lists for
     // these queries, gathered unless they are all of the call's
     Operands op{xh, split ? xl : xh, qh, split ? ql : qh, xn, qn, flags, terms};
@@ -1324,15 +1373,19 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     }
     lists = g_knn_stats;
   }
-  float ms[4] = {0, 0, 0, 0};
-  for (int i = 0; i < 4; ++i) cudaEventElapsedTime(&ms[i], ev[i], ev[i + 1]);
+  double ms[4] = {0, 0, 0, 0};
+  for (size_t i = 0; i + 1 < ev.n; ++i) {
+    float t = 0;
+    cudaEventElapsedTime(&t, ev.e[i], ev.e[i + 1]);
+    ms[i ? 1 + (i - 1) % 3 : 0] += t;
+  }
   g_knn_stats.convert_ms = ms[0];
   g_knn_stats.bound_ms = ms[1] + lists.bound_ms;
   g_knn_stats.screen_ms = ms[2] + lists.screen_ms;
   g_knn_stats.merge_ms = ms[3] + lists.merge_ms;
   g_knn_stats.sample_rows = S;
   g_knn_stats.screen_flops = 2.0 * (double)nq * (double)n * (double)dim;
-  g_knn_stats.tile_flops = 2.0 * (double)(qgroups * NT * TM) * (double)(ntiles * TN) * (double)W * (double)terms + lists.tile_flops;
+  g_knn_stats.tile_flops = 2.0 * tile_rows * (double)(ntiles * TN) * (double)W * (double)terms + lists.tile_flops;
   g_knn_stats.terms = terms;
   g_knn_stats.stages = stages;
   g_knn_stats.nchunks = nchunks;

@@ -707,6 +707,15 @@ int efg_brute_force_knn(const float* d_base, uint64_t n, uint32_t dim, uint64_t 
                    d_ids, d_dists, (cudaStream_t)stream);
 }
 
+int efg_brute_force_knn_within(const float* d_base, uint64_t n, uint32_t dim, uint64_t row_stride, const float* d_q,
+                               uint64_t nq, uint64_t q_stride, uint32_t k, int exclude_self, uint64_t first_row,
+                               int32_t* d_ids, float* d_dists, uint64_t candidate_bytes, void* stream) {
+  EFG_TRY(efg::bf_check_args(d_base, n, dim, row_stride, d_q, nq, q_stride, k, exclude_self, first_row, d_ids));
+  if (k > tc_knn_max_k()) return fail(EFG_ERR_ARG, "k above the tensor-core path's limit");
+  return brute_force_knn_tc(d_base, n, dim, (uint32_t)row_stride, d_q, nq, (uint32_t)q_stride, k, exclude_self,
+                            first_row, d_ids, d_dists, (cudaStream_t)stream, 0, candidate_bytes);
+}
+
 int efg_get_knn_stats(efg_knn_stats* out) {
   if (!out) return fail(EFG_ERR_ARG, "null argument");
   *out = g_knn_stats;

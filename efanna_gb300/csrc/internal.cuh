@@ -194,7 +194,7 @@ uint32_t tc_knn_max_k();
 extern thread_local efg_knn_stats g_knn_stats;  // the calling thread's last tensor-core k-NN call
 int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld, const float* q, uint64_t nq,
                        uint32_t qld, uint32_t k, int exclude_self, uint64_t first_row, int32_t* ids, float* dists,
-                       cudaStream_t s, int force_split = 0);
+                       cudaStream_t s, int force_split = 0, uint64_t cand_bytes = 0);
 // join_tc.cu: the NN-descent join on the tensor cores.  tc_join_prepare converts the base
 // to BF16 hi / lo rows of round_up(dim, 64) values with FP32 norms and sets flags[0] when some lo is
 // not zero, flags[2] when the distances may not be exact; tc_join scores the nodes in three launches (tiles of 128 rows over all nodes, tiles of

@@ -396,6 +396,13 @@ int efg_brute_force_knn_split(const float* d_base, uint64_t n, uint32_t dim, uin
                               uint64_t nq, uint64_t q_stride, uint32_t k, int exclude_self, uint64_t first_row,
                               int32_t* d_ids, float* d_dists, void* stream);
 
+/* The tensor-core path with a bound on its candidate buffers (8 to 32 KB a query, so that more queries than
+ * the bound serves, but at least 256, are taken in blocks).  0: the other calls' bound of 2 GB.  The
+ * results don't depend on it (k <= 104). */
+int efg_brute_force_knn_within(const float* d_base, uint64_t n, uint32_t dim, uint64_t row_stride, const float* d_q,
+                               uint64_t nq, uint64_t q_stride, uint32_t k, int exclude_self, uint64_t first_row,
+                               int32_t* d_ids, float* d_dists, uint64_t candidate_bytes, void* stream);
+
 /* efg_brute_force_knn without any device allocation, for callers that must not have a library
  * allocate GPU memory during the call (their device memory is owned by another allocator, or the
  * call sits in a loop that cannot afford an allocation).  No counterpart in the reference.

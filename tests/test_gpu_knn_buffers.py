@@ -68,3 +68,58 @@ def test_strided_groups_at_their_edges(efg, n, k, d):
         tc = _knn(efg, x, q, k, screening)
         f32 = _knn(efg, x, q, k, "fp32")
         assert np.array_equal(tc[0], f32[0]) and np.array_equal(tc[1], f32[1])
+
+
+@pytest.mark.parametrize("n,k,copies", [(400, 10, 0), (5_000, 10, 0), (40_000, 10, 0), (140_011, 100, 5_000),
+                                        (60_011, 100, 0), (20_000, 10, 3_000)])
+@pytest.mark.parametrize("nq,groups", [(1_300, 1), (1_300, 2), (1_281, 1), (513, 2)])
+@pytest.mark.parametrize("exclude", [False, True])
+def test_queries_in_blocks(efg, n, k, copies, nq, groups, exclude):
+    """Candidate buffers for 256 or 512 queries at a time: even and ragged last blocks, with queries in
+    several blocks that overrun their buffers."""
+    rng = np.random.default_rng(n + nq)
+    d, first = 24, 50
+    x = rng.integers(0, 100, (n, d)).astype(np.float32)
+    if exclude:
+        nq = min(nq, n - first)
+        if copies:
+            x[first:first + nq:199] = 220
+        q = x[first:first + nq].copy()
+    else:
+        q = rng.integers(0, 100, (nq, d)).astype(np.float32)
+        if copies:
+            q[::199] = 220
+    if copies:
+        x[n - copies:] = 220
+    X, Q = torch.from_numpy(x).cuda(), torch.from_numpy(q).cuda()
+    ids = torch.full((nq, k), -7, dtype=torch.int32, device="cuda")
+    dist = torch.full((nq, k), -1.0, dtype=torch.float32, device="cuda")
+    per = 8 * (4096 if k == 100 else 2048)  # bytes of a query's buffer
+    f32 = _knn(efg, x, q, k, "fp32", exclude=exclude, first_row=first)
+    efg._check(efg.lib().efg_brute_force_knn_within(X.data_ptr(), n, d, d, Q.data_ptr(), nq, d, k, int(exclude), first,
+                                                    ids.data_ptr(), dist.data_ptr(), groups * 256 * per + 100, None))
+    torch.cuda.synchronize()
+    assert efg.knn_stats().list_queries == (-(-nq // 199) if copies else 0)
+    assert np.array_equal(ids.cpu().numpy(), f32[0]) and np.array_equal(dist.cpu().numpy(), f32[1])
+
+
+def test_many_queries_with_little_memory(efg):
+    """80,000 queries with 2.6 GB of candidate buffers between them where 1 GB is left: taken in blocks."""
+    n, nq, d, k = 20_000, 80_000, 16, 100
+    g = torch.Generator(device="cuda").manual_seed(1)
+    X = torch.randint(0, 256, (n, d), generator=g, device="cuda").float()
+    Q = torch.randint(0, 256, (nq, d), generator=g, device="cuda").float()
+    ids = torch.empty((nq, k), dtype=torch.int32, device="cuda")
+    dist = torch.empty((nq, k), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    ballast = torch.empty(torch.cuda.mem_get_info()[0] - (1 << 30), dtype=torch.uint8, device="cuda")
+    try:
+        efg.brute_force_knn_device(X.data_ptr(), n, d, d, Q.data_ptr(), nq, d, k, ids.data_ptr(), dist.data_ptr())
+        torch.cuda.synchronize()
+    finally:
+        del ballast
+        torch.cuda.empty_cache()
+    some = torch.arange(0, nq, 131, device="cuda")
+    f32 = _knn(efg, X.cpu().numpy(), Q[some].cpu().numpy(), k, "fp32")
+    assert np.array_equal(ids[some].cpu().numpy(), f32[0]) and np.array_equal(dist[some].cpu().numpy(), f32[1])
