@@ -1239,7 +1239,11 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   // 1. bounds: how, and the sample
   const size_t sel_smem = (size_t)cap * 8 + (size_t)rank * 8;
   EFG_CUDA(cudaFuncSetAttribute(select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem));
-  uint64_t S1 = std::min<uint64_t>(n / 16, 1u << 20) / TN * TN;  // rows of the append pass's sample
+  // Rows of the append pass's sample: n / 16 up to 2^20 of them, more for bases so large that the values
+  // under the bound of 2^20 rows, n / 2^20 x rank and six deviations, would not fit a buffer (from 23
+  // million rows at k = 100; 2000 queries over 45M x 8: 144 ms with all of them in the lists, 40.7 this way).
+  const double spread = (double)rank * (1 + 6 / std::sqrt((double)rank));
+  uint64_t S1 = std::min<uint64_t>(n / 16, std::max<uint64_t>(1u << 20, (uint64_t)((double)n * spread / cap) + TN)) / TN * TN;
   const uint64_t gtiles = (rank + 3) / 4 * 2;                          // tiles that hold `rank` groups of 64 columns, an even number
   uint32_t S = 0, gt = 0;  // rows of the last bound pass (0: no bounds); tiles per group
   CUtensorMap m0h, m0l, m1h, m1l;  // of the MIN pass and the append pass
@@ -1258,8 +1262,8 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     const double tail = std::log(32.0 * (double)rank * (double)nq);
     while ((double)S1 * tail > (double)cap * 64 * gt) {
       const uint64_t cut = (uint64_t)((double)cap * 64 * gt / tail) / TN * TN;
-      const double expect = (double)n / (double)std::max<uint64_t>(cut, 1) * (double)rank;
-      if (cut >= gtiles * gt * TN && expect * (1 + 6 / std::sqrt((double)rank)) <= (double)cap) S1 = cut;
+      const double expect = (double)n / (double)std::max<uint64_t>(cut, 1) * spread;
+      if (cut >= gtiles * gt * TN && expect <= (double)cap) S1 = cut;
       else if (gtiles * (2 * gt) * TN <= S1) gt *= 2;
       else break;
     }

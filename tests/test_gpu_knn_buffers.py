@@ -123,3 +123,22 @@ def test_many_queries_with_little_memory(efg):
     some = torch.arange(0, nq, 131, device="cuda")
     f32 = _knn(efg, X.cpu().numpy(), Q[some].cpu().numpy(), k, "fp32")
     assert np.array_equal(ids[some].cpu().numpy(), f32[0]) and np.array_equal(dist[some].cpu().numpy(), f32[1])
+
+
+def test_sample_grows_with_the_base(efg):
+    """45 million rows: a bound from 2^20 of them leaves more values under it (45 / 1.05 x 116 = 4980) than
+    a buffer's 4096, so the sample has to be larger."""
+    n, nq, d, k = 45_000_000, 64, 8, 100
+    g = torch.Generator(device="cuda").manual_seed(1)
+    X = torch.randint(0, 256, (n, d), generator=g, device="cuda", dtype=torch.uint8).float()
+    Q = torch.randint(0, 256, (nq, d), generator=g, device="cuda", dtype=torch.uint8).float()
+    out = {}
+    for screening in ("fp32", "auto"):
+        ids = torch.empty((nq, k), dtype=torch.int32, device="cuda")
+        dist = torch.empty((nq, k), dtype=torch.float32, device="cuda")
+        efg.brute_force_knn_device(X.data_ptr(), n, d, d, Q.data_ptr(), nq, d, k, ids.data_ptr(), dist.data_ptr(),
+                                   screening=screening)
+        torch.cuda.synchronize()
+        out[screening] = ids.cpu().numpy(), dist.cpu().numpy()
+    assert efg.knn_stats().list_queries == 0
+    assert np.array_equal(out["auto"][0], out["fp32"][0]) and np.array_equal(out["auto"][1], out["fp32"][1])
