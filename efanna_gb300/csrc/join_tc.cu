@@ -75,6 +75,15 @@ struct JoinArgs {
   uint32_t count;  // of them
 };
 
+// max(x, 0), NaN for NaN: a row with a NaN or an infinity (or a norm past FP32's range) is at no distance
+// from any other, and its pairs make no records, as in the FP32 join.  With fmaxf they were at distance
+// zero: such a row came nearest to all, with millions of records.
+__device__ __forceinline__ float max0_nan(float x) {
+  float r;
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 __device__ __forceinline__ void rec_sync() { asm volatile("bar.sync 1, %0;" ::"r"(JRT) : "memory"); }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
@@ -456,7 +465,7 @@ __global__ void __launch_bounds__(JTHREADS, Tile<TR>::CTAS) tc_join_kernel(const
                 node = id_ch[sl];
               }
               const float dot = gram[(r - q0) * DLD + bc];
-              d[p] = fmaxf(fmaf(-2.f, dot, norm_sh[r] + norm_sh[bc]), 0.f);
+              d[p] = max0_nan(fmaf(-2.f, dot, norm_sh[r] + norm_sh[bc]));
               const uint32_t x = rows_sh[r], y = rows_sh[bc];
               if (cand_new && y == x) continue;  // equal ids: no pair
               // side 0: the larger id of two new entries into the smaller one's node, else y into x
