@@ -855,8 +855,9 @@ __device__ __forceinline__ void sort_window(uint64_t* wk, uint32_t* wa, uint32_t
 
 // Next 32 records of distance bits g in ascending (key, aux) order after `last`.  With `single` a lone id's
 // copies count as its first record: a pass without sorting finds whether there is one id.
-__device__ __forceinline__ K96 next_batch(const uint4* __restrict__ rec, uint32_t B, uint32_t g, K96 last, bool first,
-                                          bool single) {
+// (Not inlined: rare, and the code around its place runs for every node.)
+static __device__ __noinline__ K96 next_batch(const uint4* __restrict__ rec, uint32_t B, uint32_t g, K96 last, bool first,
+                                              bool single) {
   const uint32_t lane = threadIdx.x & 31;
   if (single) {
     K96 mn = k96_max();
@@ -872,7 +873,7 @@ __device__ __forceinline__ K96 next_batch(const uint4* __restrict__ rec, uint32_
     mn = shfl_idx(warp_sort32(mn), 0);
     if (is_max(mn) || key_id(mn.k) == mx) return lane == 0 ? mn : k96_max();
   }
-  K96 run = k96_max();
+  K96 run = k96_max(), worst = run;  // the 32 smallest so far, and the largest of them
   for (uint32_t b = 0; b < B; b += 32) {
     K96 x = k96_max();
     if (b + lane < B) {
@@ -880,11 +881,47 @@ __device__ __forceinline__ K96 next_batch(const uint4* __restrict__ rec, uint32_
       const K96 y = rec_k96(q);
       if (q.y == g && (first || lt(last, y))) x = y;
     }
-    if (__all_sync(0xffffffffu, is_max(x))) continue;
+    if (__all_sync(0xffffffffu, !lt(x, worst))) continue;
     x = warp_sort32(x);
     run = warp_merge_min32(run, x);
+    worst = shfl_idx(run, 31);
   }
   return run;
+}
+
+// The records of distance bits g after `last`, for a pool full up to that distance (entries [0, P - 1), the
+// radius and the last of them at it): each of them lands in the overflow slot or is a duplicate, so the
+// last one that is none stays there, at a rank of P - 1 (a duplicate's is P; check_k is not P).
+static __device__ __noinline__ void overflow_ties(const uint4* __restrict__ rec, uint32_t B, uint32_t g, K96 last,
+                                                  bool first, float* pd, uint32_t* pid, uint32_t P, bool any_dist,
+                                                  bool mark, uint8_t* __restrict__ found) {
+  const uint32_t lane = threadIdx.x & 31;
+  const float d = __uint_as_float(g);
+  for (uint64_t limit = 1ull << 32; limit;) {  // the largest id below `limit`
+    uint64_t mx = 0;                           // (+ 1; 0: none)
+    for (uint32_t b = lane; b < B; b += 32) {
+      const uint4 q = rec[b];
+      if (q.y != g) continue;
+      const K96 y = rec_k96(q);
+      if (!first && !lt(last, y)) continue;
+      if (q.x < limit) mx = max(mx, (uint64_t)q.x + 1);
+      if (mark && limit == 1ull << 32 && !(q.z & 1u)) found[q.z >> 1] = 1;
+    }
+    const uint32_t top = __reduce_max_sync(0xffffffffu, (uint32_t)mx);  // (ids are < 2^30)
+    if (!top) break;
+    const uint32_t cand = top - 1;
+    bool dup = false;
+    for (uint32_t e = lane; e + 1 < P; e += 32) dup |= (any_dist || pd[e] == d) && (pid[e] & IDM) == cand;
+    if (!__any_sync(0xffffffffu, dup)) {
+      if (lane == 0) {
+        pd[P - 1] = d;
+        pid[P - 1] = cand | FLAG;
+      }
+      break;
+    }
+    limit = cand;
+  }
+  __syncwarp();
 }
 
 // One warp per target node: applies its records in ascending (dist, id, source, side) order until one
@@ -997,6 +1034,14 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_kernel(
       }
       if (ties) {  // the next 32 of them
         const bool quiet = pool.L >= check_k;
+        const float dt = __uint_as_float(tlo);
+        if (pool.L == P - 1 && pool.rad == dt && pool.pd[P - 2] == dt && check_k != P) {  // nothing left but its last
+          overflow_ties(rec, B, tlo, last, first, pool.pd, pool.pid, P, any_dist, check_k > P, found);
+          ties = false;
+          first = true;
+          ++tlo;
+          continue;
+        }
         const K96 batch = next_batch(rec, B, tlo, last, first, quiet);
         total = __popc(__ballot_sync(0xffffffffu, !is_max(batch)));
         first = total == 0;
