@@ -13,6 +13,9 @@ device->host copy of the ids inside the timed region).  The graph build is timed
 reported under "build".  The base set (512 MB) is larger than the 129 MB L2, so no L2 flush is
 needed between steps.
 
+Standard output gets one short JSON line; the whole report, with every ladder and workload, goes to
+standard error as a line that starts with "report:".
+
 --impl reference times the CPU baseline: the oracle's OpenMP restatement of the reference
 (ORC_OMP: the reference's parallel build and nnexp search), on all host cores, same workload and
 operating point, each step a bounded sample of the queries.
@@ -84,6 +87,30 @@ def recall_ties(res: np.ndarray, gt: np.ndarray, base: np.ndarray, queries: np.n
         dr = ((np.asarray(base[np.where(ok, r, 0)], np.float64) - qq) ** 2).sum(-1)
         hits += int(((dr <= kth[:, None]) & ok).sum())
     return hits / (k * len(res))
+
+
+HEADLINE = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "build", "e2e", "roofline", "gpu_launches", "clocks")
+
+
+def headline(report: dict) -> dict:
+    """The line on standard output, short enough for a reader that keeps the last few KB: the measurement
+    itself, and of the report's other workloads (whole on standard error) the value, end-to-end value and
+    recall of each."""
+    line = {k: report[k] for k in HEADLINE if k in report}
+    line["config"] = {k: v for k, v in report["config"].items() if k != "ladder"}
+    if "cpu_baseline" in report:
+        line["cpu_baseline"] = {k: report["cpu_baseline"][k] for k in ("value", "unit", "cores", "kind", "recall@10")
+                                if k in report["cpu_baseline"]}
+    also = {}
+    for name, part in [(k, report.get(k)) for k in ("bf16", "fp8", "bf16_learned", "kgraph", "hashing", "batching")] + \
+            [("trees48", report.get("trees48", {}).get("fp32"))]:
+        if part:
+            r = part.get("recall@10", part.get("operating_point", {}).get("recall@10"))
+            also[name] = {k: v for k, v in (("value", part.get("value")), ("e2e", part.get("e2e")), ("recall@10", r))
+                          if isinstance(v, (int, float))}
+    line["also"] = also
+    return line
 
 
 class ClockSampler:
@@ -423,7 +450,8 @@ def run_gpu(args):
             plain_ladder=[(4, 400, 40), (4, 1000, 100), (4, 1500, 150), (4, 2000, 200), (4, 3000, 300),
                           (6, 4000, 400), (8, 6000, 600), (8, 8000, 800)], reference=(12, 12000, 800))
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        log("report:", json.dumps(line))
+        print(json.dumps(headline(line)), flush=True)
     if idx is not None:
         idx.close()
     replicas.finish()

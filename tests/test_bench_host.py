@@ -99,3 +99,32 @@ def test_recall_with_ties_counts_equally_near_points():
     assert bench.recall_ties(exact, exact, x, qq) == 1.0
     shuffled = np.argsort(d + rng.random(d.shape) * 1e-3, axis=1)[:, :10]  # other members of the ties
     assert bench.recall_ties(shuffled, exact, x, qq) == 1.0
+
+
+def test_headline_is_short_and_complete():
+    """The line on standard output holds the measurement's keys in less than 3 KB, however long the report."""
+    import bench
+    ladder = [{"epochs": 4, "pool": 400 * i, "extend": 75 * i, "recall@10": 0.95} for i in range(60)]
+    form = {"value": 1174307.5, "unit": "queries/s", "ms_per_step": 8.5157, "e2e": 1116830.3, "ladder": ladder,
+            "operating_point": {"epochs": 4, "pool": 4000, "extend": 750, "recall@10": 0.9537}}
+    report = {k: 1234567.8 for k in bench.HEADLINE}
+    report.update(
+        metric=bench.METRIC, data="synthetic (seeded integer-valued Gaussian mixture)",
+        config={"workload": bench.workload(1_000_000, 10_000), "n": 1_000_000, "ladder": ladder, "operating_point": ladder[0],
+                "config_point": ladder[1], "l2": "inputs larger than L2 (512 MB base), no flush", "parallelism": "single GPU"},
+        build={"x%d" % i: 123456.789 for i in range(18)}, e2e={"value": 1369669.9, "unit": "queries/s",
+                                                               "h2d_bytes_per_step": 5120000, "d2h_bytes_per_step": 400000},
+        roofline={"y%d" % i: "profiles/nnexp_traffic_1Mx128.md" for i in range(10)},
+        clocks={"sm_mhz": 2070.0, "sm_max_mhz": 2070.0, "reasons": ["sw_power_cap"], "samples": 40},
+        cpu_baseline={"value": 4940.9, "unit": "queries/s", "cores": 16, "kind": "port", "sample": "s" * 400},
+        bf16=form, fp8=form, kgraph=form, hashing=form, batching=dict(form, sweep=ladder), trees48={"fp32": form, "bf16": form},
+        bf16_learned={"value": 930656.3, "recall@10": 0.953, "sweep": ladder}, learned_aniso={"learned": ladder})
+    line = bench.headline(report)
+    text = json.dumps(line)
+    assert len(text) < 3000
+    for key in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+                "vs_baseline", "dtype", "data", "config", "e2e", "gpu_launches", "clocks"):
+        assert line[key] == report[key] or key == "config"
+    assert line["config"]["operating_point"] == ladder[0] and "ladder" not in line["config"]
+    assert line["also"]["bf16"] == {"value": 1174307.5, "e2e": 1116830.3, "recall@10": 0.9537}
+    assert line["also"]["bf16_learned"] == {"value": 930656.3, "recall@10": 0.953}
