@@ -21,7 +21,7 @@
 //   * every query has an upper bound on its K2-th distance (K2 = k + 16) from cheap passes of the
 //     same kernel over samples; the pass over the whole base appends the few values under it to the
 //     query's candidate buffer, and select_kernel sorts them and re-ranks the K2 smallest in FP64.
-//   * tc_knn_kernel, the path of a call whose candidates overran their buffers (many rows at nearly one
+//   * tc_knn_kernel, for the queries whose candidates overran their buffers (many rows at nearly one
 //     distance): per-(query, chunk) sorted lists of K2 keys in shared memory, as the FP32 kernel writes
 //     them (distance.cu), ranked by the same merge kernel.
 //
@@ -411,7 +411,7 @@ __global__ void bound_kernel(const uint64_t* __restrict__ lists, uint64_t nq, ui
 
 
 // ==============================================================================================
-// Screening against a bound: the path of every call whose candidates fit their buffers.
+// Screening against a bound: every query whose candidates fit its buffer.
 //
 // With an upper bound on each query's K2-th distance, screening only has to find the values under it
 // and append them to the query's buffer; lists, and their divergent insertions, are left to the few.
@@ -446,10 +446,10 @@ struct ScreenArgs {
   uint32_t ntiles, chunk_tiles, nchunks, qgroups, nq, cap, kblocks, stages, exclude_self;
   uint32_t group_tiles;   // MIN pass: a thread's tiles (every other one) per group of its 64 columns (0: groups of
                           // 16 columns); a chunk holds a multiple of 2 group_tiles
-  // MIN pass over a base in its own order: rows `stride` apart fill a box of `box` columns (row i stride + u
-  // is column i of box u, for i < rows_box; the others are empty), so that every group reaches over the
-  // whole base; W values per row.  stride 0: rows in order.
-  uint32_t stride, box, rows_box, W;
+  // MIN_STRIDED: rows `stride` apart fill a box of 2^box_shift columns (row i stride + u is column i of box
+  // u, for i < rows_box; the others are empty), so that every group reaches over the whole base; W values
+  // per row.
+  uint32_t stride, box_shift, rows_box, W;
   uint32_t split, resident;
   float rel;              // the bound is widened by this much (passes of the split form may round differently)
   uint32_t stage_bytes, o_x, o_scr, o_xn, o_queue;
@@ -474,12 +474,15 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
   return r;
 }
 
-template <int NT, bool MINP>
+// PASS: values under the bound appended, groups' minima of rows in order, or of strided rows.
+enum { APPEND = 0, MIN_ROWS = 1, MIN_STRIDED = 2 };
+template <int NT, int PASS>
 __global__ void __launch_bounds__(STH, 1)
     tc_screen_kernel(const __grid_constant__ CUtensorMap mq_hi, const __grid_constant__ CUtensorMap mq_lo,
                      const __grid_constant__ CUtensorMap mx_hi, const __grid_constant__ CUtensorMap mx_lo,
                      const ScreenArgs a) {
   constexpr uint32_t COLS = 2 * NT * TN;  // two buffers of NT accumulators
+  constexpr bool MINP = PASS != APPEND;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[MAX_STAGES], bar_empty[MAX_STAGES], bar_tfull[2], bar_tempty[2], bar_q,
       bar_qfree, bar_drain;
@@ -550,9 +553,9 @@ __global__ void __launch_bounds__(STH, 1)
             mbar_expect_tx(fb, a.stage_bytes);
             const uint32_t st = sbase + a.o_x + s * a.stage_bytes;
             const int x = (int)(kb * TKB), yx = (int)(t * TN);
-            if (MINP && a.stride) {
-              for (uint32_t c = 0; c < TN; c += a.box) {
-                const int xb = x + (int)((t * TN + c) / a.box * a.W);
+            if (PASS == MIN_STRIDED) {
+              for (uint32_t c = 0; c < TN; c += 1u << a.box_shift) {
+                const int xb = x + (int)(((t * TN + c) >> a.box_shift) * a.W);
                 tma_load_2d(st + c * TKB * 2, &mx_hi, fb, xb, 0);
                 if (a.split) tma_load_2d(st + PART + c * TKB * 2, &mx_lo, fb, xb, 0);
               }
@@ -672,7 +675,7 @@ __global__ void __launch_bounds__(STH, 1)
     };
     // norms of this lane's two of the 64 columns from col on, where the rows are not in order
     auto strided_norms = [&](uint32_t col) -> float2 {
-      const uint32_t c = col + 2 * lane, u = c / a.box, i = c % a.box;  // (both in one box)
+      const uint32_t c = col + 2 * lane, u = c >> a.box_shift, i = c & ((1u << a.box_shift) - 1);  // (both in one box)
       return make_float2(i < a.rows_box ? __ldg(a.xnorm + (uint64_t)i * a.stride + u) : INFINITY,
                          i + 1 < a.rows_box ? __ldg(a.xnorm + (uint64_t)(i + 1) * a.stride + u) : INFINITY);
     };
@@ -701,7 +704,7 @@ __global__ void __launch_bounds__(STH, 1)
       uint32_t flip = 0, in_group = 0;
       if (first < t1)
         reinterpret_cast<float2*>(xw)[lane] =
-            MINP && a.stride ? strided_norms(first * TN + half * 64)
+            PASS == MIN_STRIDED ? strided_norms(first * TN + half * 64)
                              : __ldg(reinterpret_cast<const float2*>(a.xnorm + (uint64_t)first * TN + half * 64) + lane);
       __syncwarp();
       for (uint32_t t = first; t < t1; t += 2, flip ^= 1u) {
@@ -709,7 +712,7 @@ __global__ void __launch_bounds__(STH, 1)
         const uint64_t row0 = (uint64_t)t * TN + half * 64;
         float2 xnext = make_float2(0.f, 0.f);
         if (t + 2 < t1)  // in flight meanwhile
-          xnext = MINP && a.stride ? strided_norms((uint32_t)row0 + 2 * TN)
+          xnext = PASS == MIN_STRIDED ? strided_norms((uint32_t)row0 + 2 * TN)
                                    : __ldg(reinterpret_cast<const float2*>(a.xnorm + row0 + 2 * TN) + lane);
         ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&bar_tfull[b]), tph, abort_flag, a.err));
         if (!ok) break;
@@ -827,7 +830,7 @@ __global__ void __launch_bounds__(STH, 1)
   }
 }
 
-// Sample rows in a scattered order: the base falls into S strata of n / S rows, and row i of the sample is a
+// Sample rows in a scattered order: the base falls into S strata of n / S (per) rows, and row i of the sample is a
 // row of stratum (i * step) mod S, step prime to S, so that every leading part of the sample is spread
 // over the base too.  Which row of the stratum is hashed: the first one of each would be of one class where
 // classes alternate with a period that divides n / S (2^20 rows of 16 classes in turn, 10k queries: 54.9
@@ -835,12 +838,12 @@ __global__ void __launch_bounds__(STH, 1)
 // values per row; lo may be null.
 __global__ void scatter_sample_kernel(const uint4* __restrict__ hi, const uint4* __restrict__ lo,
                                       const float* __restrict__ norms, uint64_t n, uint32_t W, uint32_t S,
-                                      uint32_t step, uint4* __restrict__ shi, uint4* __restrict__ slo,
+                                      uint32_t step, uint32_t per, uint4* __restrict__ shi, uint4* __restrict__ slo,
                                       float* __restrict__ snorms) {
   const uint32_t lane = threadIdx.x & 31, w16 = W / 8;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < S; i += nw) {
-    const uint64_t p = i * step % S, r = p * n / S + mix64(p) % (n / S);
+    const uint64_t p = i * step % S, r = p * n / S + __umulhi((uint32_t)mix64(p), per);
     for (uint32_t c = lane; c < w16; c += 32) {
       shi[i * w16 + c] = hi[r * w16 + c];
       if (lo) slo[i * w16 + c] = lo[r * w16 + c];
@@ -1180,11 +1183,11 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   // (tiles per item, and about two for an item's start); chunks of whole groups for the MIN pass.
   auto pass = [&](bool minp, const CUtensorMap& mh, const CUtensorMap& ml, const float* xnorm, uint64_t rows,
                   uint32_t group_tiles, const uint32_t* qbound, uint32_t* qmax, uint32_t* cnt, uint64_t* buf,
-                  uint32_t cap, int excl, uint32_t stride = 0, uint32_t box = TN) -> int {
+                  uint32_t cap, int excl, uint32_t stride = 0, uint32_t box_shift = 0) -> int {
     ScreenArgs a;
     a.stride = stride;
-    a.box = box;
-    a.rows_box = stride ? (uint32_t)std::min<uint64_t>(box, n / stride) : box;
+    a.box_shift = box_shift;
+    a.rows_box = stride ? (uint32_t)std::min<uint64_t>(1u << box_shift, n / stride) : 0;
     a.W = W;
     const uint64_t tiles = (rows + TN - 1) / TN, unit = std::max<uint32_t>(1, 2 * group_tiles);
     const uint64_t units = (tiles + unit - 1) / unit;
@@ -1227,8 +1230,12 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     a.o_xn = a.o_scr + scratch;
     a.o_queue = a.o_xn + norms_b;
     const size_t smem = 1024 + (size_t)a.o_queue + queue_b;
-    auto kern = NT == 2 ? (minp ? tc_screen_kernel<2, true> : tc_screen_kernel<2, false>)
-                        : (minp ? tc_screen_kernel<1, true> : tc_screen_kernel<1, false>);
+    auto kern = NT == 2 ? (!minp    ? tc_screen_kernel<2, APPEND>
+                           : stride ? tc_screen_kernel<2, MIN_STRIDED>
+                                    : tc_screen_kernel<2, MIN_ROWS>)
+                        : (!minp    ? tc_screen_kernel<1, APPEND>
+                           : stride ? tc_screen_kernel<1, MIN_STRIDED>
+                                    : tc_screen_kernel<1, MIN_ROWS>);
     EFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     grid = (unsigned)std::min<uint64_t>((uint64_t)qgroups * nchunks, (uint64_t)sms);
     kern<<<grid, STH, smem, s>>>(mqh, mql, mh, ml, a);
@@ -1249,15 +1256,15 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
   CUtensorMap m0h, m0l, m1h, m1l;  // of the MIN pass and the append pass
   uint64_t min_rows = 0;
   const float* min_norms = xn;
-  uint32_t min_stride = 0, min_box = TN;
+  uint32_t min_stride = 0, box_shift = 0;
   const bool sampled = S1 >= gtiles * TN;
   if (sampled) {
     gt = 1;  // up to a third of the sample for the MIN pass
     while (gt < 16 && gtiles * (2 * gt) * TN * 3 <= S1) gt *= 2;
     // Values of the sample under the MIN pass's bound: a share p of them, where all of the `rank` groups of
-    // 64 gt columns have one below it; (1 - p)^(64 gt) rank nq = 1 / 32 says what their buffers must hold.  A
-    // call that overran them goes through the lists after all (k = 100, 10k queries at 1M x 960: 167 ms, 114
-    // through the lists at once), so the sample is cut while the base's expected candidates (six deviations
+    // 64 gt columns have one below it; (1 - p)^(64 gt) rank nq = 1 / 32 says what their buffers must hold.
+    // Queries that overrun them go through the lists after all (k = 100, 10k queries at 1M x 960: 167 ms when
+    // all did, 65 ms), so the sample is cut while the base's expected candidates (six deviations
     // up) still fit, else the groups doubled.
     const double tail = std::log(32.0 * (double)rank * (double)nq);
     while ((double)S1 * tail > (double)cap * 64 * gt) {
@@ -1283,7 +1290,7 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     };
     while (gcd(step, S1) != 1) step += 2;
     scatter_sample_kernel<<<blocks(S1), 256, 0, s>>>((const uint4*)xh, (const uint4*)xl, xn, n, W, (uint32_t)S1, step,
-                                                     (uint4*)bh, (uint4*)bl, bn);
+                                                     (uint32_t)(n / S1), (uint4*)bh, (uint4*)bl, bn);
     EFG_CUDA(cudaGetLastError());
     min_rows = gtiles * gt * TN;
     min_norms = bn;
@@ -1302,10 +1309,11 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
       // through where rows come class by class, a multiple of its period where classes alternate (20k x
       // 128 in four classes, 10k queries: 4.2 ms with all of them in the lists, 1.3 ms this way).
       min_rows = gt ? full / (2 * gt) * (2 * gt) * TN : full * TN;
-      min_box = gt ? 64 : 16;
-      min_stride = next_prime((uint32_t)((n + min_box - 1) / min_box));
-      EFG_TRY(make_map(&m0h, xh, std::min<uint64_t>(min_box, n / min_stride), min_stride * W, min_box));
-      EFG_TRY(make_map(&m0l, split ? xl : xh, std::min<uint64_t>(min_box, n / min_stride), min_stride * W, min_box));
+      box_shift = gt ? 6 : 4;
+      const uint32_t box = 1u << box_shift;
+      min_stride = next_prime((uint32_t)((n + box - 1) / box));
+      EFG_TRY(make_map(&m0h, xh, std::min<uint64_t>(box, n / min_stride), min_stride * W, box));
+      EFG_TRY(make_map(&m0l, split ? xl : xh, std::min<uint64_t>(box, n / min_stride), min_stride * W, box));
       S = (uint32_t)min_rows;
     }
   }
@@ -1320,7 +1328,7 @@ int brute_force_knn_tc(const float* base, uint64_t n, uint32_t dim, uint32_t ld,
     if (q0) EFG_TRY(ev.record(s));
     if (S) {
       EFG_CUDA(cudaMemsetAsync(qbound, 0, nqb * 4, s));
-      EFG_TRY(pass(true, m0h, m0l, min_norms, min_rows, gt, nullptr, qbound, nullptr, nullptr, 0, 0, min_stride, min_box));
+      EFG_TRY(pass(true, m0h, m0l, min_norms, min_rows, gt, nullptr, qbound, nullptr, nullptr, 0, 0, min_stride, box_shift));
     }
     if (sampled) {
       EFG_CUDA(cudaMemsetAsync(cnt, 0, nqb * 4, s));

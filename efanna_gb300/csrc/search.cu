@@ -359,11 +359,11 @@ int launch_nnexp(efg_index* idx, SearchCfg cfg, uint32_t maxdeg, const float* d_
     return fit >= 2;
   };
   // The visited set as a bitmap of the base -- an atomic OR per insert, nothing to probe and nothing to
-  // outgrow -- where it costs no CTA: two fit on an SM with it (a plan's 256 queries at 400k rows 177 us,
-  // with the table 199 us; 777 queries at 61k x 101 299 us, 344 us), or only one does with the table too
-  // (2000 queries at 100k x 960, degree 100: 3.8 ms, 6.5 ms), or there is no more than one query per SM
-  // (one query at 1M x 128: 106 us, 139 us).  Else two CTAs with the table are the faster (10k queries at
-  // 1M x 128: 7.75 ms against 8.09 ms), and settings that expect to visit more ids than the base has
+  // outgrow -- where it costs no CTA: two fit on an SM with it (a plan's 256 queries at 400k rows 157 us,
+  // with the table 181 us; 777 queries at 61k x 101 287 us, 333 us), or only one does with the table too
+  // (2000 queries at 100k x 960, degree 100: 3.68 ms, 6.41 ms), or there is no more than one query per SM
+  // (one query at 1M x 128: 113 us, 148 us).  Else two CTAs with the table are the faster (10k queries at
+  // 1M x 128: 6.75 ms against 6.80 ms), and settings that expect to visit more ids than the base has
   // stay with it: they are the ones its hand-over to global scratch is for.
   {
     SearchCfg t = cfg, w = cfg;

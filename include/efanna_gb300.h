@@ -122,9 +122,10 @@ int efg_set_search_precision(efg_index* idx, int precision);
  * EFG_PRECISION_BF16: per node, one Gram tile of its new x (new + old) rows on the tensor cores from
  * a BF16 copy of the base made at the start of each build, distance = |x|^2 + |y|^2 - 2 x.y; when
  * BF16 holds every value one product per value, else three (hi + lo split, a relative error near
- * 2^-17 of sum |x_k y_k|).  For integer data with squared norms below 2^23 (bytes up to 128
- * dimensions) every distance, and so the graph, equals the FP32 build's; for other data pools can
- * differ where distances tie within that error.  Several nodes share a tile of up to 128 new
+ * 2^-17 of sum |x_k y_k|).  For integers with squared norms below 2^22 (below 2^23 where none is
+ * negative: bytes up to 128 dimensions) every distance, and so the graph, equals the FP32 build's; for
+ * other data pools can differ where distances tie within that error.  Rows with a NaN, an infinity or a
+ * norm beyond FP32 are at no distance from others: they enter no pool by the join, in either form.  Several nodes share a tile of up to 128 new
  * entries x 128 (or, for larger nodes, 256) rows; a node with more than 128 new entries or 256
  * rows is scored as blocks of its new entries x chunks of its candidates
  * (efg_build_stats.join_large_nodes counts them).  A pair already in a pool is rejected as a
@@ -367,17 +368,18 @@ int efg_l2_pairs(const float* d_base, uint64_t n, uint32_t dim, uint64_t row_str
  * (tcgen05 BF16 Gram tiles, FP32 accumulation): exact on data BF16 holds exactly (integers up to
  * 256 in magnitude, as the byte-valued data sets), otherwise split into hi + lo BF16 parts with an
  * error near 2^-16 of |q.x|.  Larger k screen with the FP32 kernel below.  Ids are exact whenever
- * the true k nearest are among the k + 16 screened survivors of their chunk -- always on exactly
- * representable data. */
+ * the true k nearest are among the k + 16 nearest as screened -- always on exactly representable
+ * data.  Scratch: BF16 copies of base and queries, and at most 2 GB of candidate buffers (see
+ * efg_brute_force_knn_within). */
 int efg_brute_force_knn(const float* d_base, uint64_t n, uint32_t dim, uint64_t row_stride, const float* d_q,
                         uint64_t nq, uint64_t q_stride, uint32_t k, int exclude_self, uint64_t first_row,
                         int32_t* d_ids, float* d_dists, void* stream);
 /* Timing of this thread's last tensor-core k-NN call (CUDA events on the call's stream). */
 typedef struct efg_knn_stats {
   double convert_ms;    /* BF16 hi/lo rows and FP32 norms of base and queries                       */
-  double bound_ms;      /* the per-query distance bounds from a strided sample of the base          */
-  double screen_ms;     /* the tcgen05 screening kernel                                             */
-  double merge_ms;      /* per-query merge of the chunk lists and FP64 re-rank                      */
+  double bound_ms;      /* the per-query distance bounds, from a sample of the base or groups of it */
+  double screen_ms;     /* the tcgen05 screening kernel over the whole base                         */
+  double merge_ms;      /* per-query selection among the candidates and FP64 re-rank                */
   double screen_flops;  /* algorithmic: 2 x queries x base rows x dim (one Gram contraction)          */
   double tile_flops;    /* issued by the MMAs: whole tiles, 64-value k-blocks, x products per value  */
   uint32_t terms;       /* BF16 products per value: 1 (exact data) or 3 (hi.hi + hi.lo + lo.hi)      */
