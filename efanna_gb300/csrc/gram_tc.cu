@@ -834,7 +834,7 @@ __global__ void __launch_bounds__(STH, 1)
 // row of stratum (i * step) mod S, step prime to S, so that every leading part of the sample is spread
 // over the base too.  Which row of the stratum is hashed: the first one of each would be of one class where
 // classes alternate with a period that divides n / S (2^20 rows of 16 classes in turn, 10k queries: 54.9
-// ms with nearly all queries in the lists, 6.5 ms this way).  A warp per row, 16-byte copies, W BF16
+// ms with nearly all queries in the lists, 5.8 ms this way).  A warp per row, 16-byte copies, W BF16
 // values per row; lo may be null.
 __global__ void scatter_sample_kernel(const uint4* __restrict__ hi, const uint4* __restrict__ lo,
                                       const float* __restrict__ norms, uint64_t n, uint32_t W, uint32_t S,

