@@ -316,7 +316,9 @@ int launch_nnexp(efg_index* idx, SearchCfg cfg, uint32_t maxdeg, const float* d_
   if (cfg.lsize >= 65536) return fail(EFG_ERR_ARG, "pool too large for the tree descent");
   cfg.emit_pool = d_keys ? 1 : 0;
   if (!cfg.screened && !cfg.fp8) {  // FP32: over byte rows where the base has them
-    EFG_TRY(make_bytes(idx));
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!idx->bytes_state) EFG_CUDA(cudaStreamIsCapturing(s, &capture));
+    if (capture == cudaStreamCaptureStatusNone) EFG_TRY(make_bytes(idx));  // (allocates; the FP32 rows serve a capture)
     if (idx->bytes_state == 1) {
       cfg.bytes = 1;
       cfg.cprb = idx->ldb / 16;
