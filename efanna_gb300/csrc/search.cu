@@ -395,12 +395,13 @@ int launch_nnexp(efg_index* idx, SearchCfg cfg, uint32_t maxdeg, const float* d_
   size_t smem2 = layout(c2, idx->ld, maxdeg, true, (uint32_t)big);
   c2.ht_limit = (uint32_t)big;
   bool two_pass = !cfg.bits && big > small;
-  if (smem1 > 200 * 1024) {  // the reduced set does not fit beside the rest: one pass, global set
+  const size_t qb = (size_t)cfg.cprb * 16;  // the query's bytes (272 at most) come on top of the limits below
+  if (smem1 - qb > 200 * 1024) {  // the reduced set does not fit beside the rest: one pass, global set
     c1 = c2;
     smem1 = smem2;
     two_pass = false;
   }
-  if (smem1 > 220 * 1024)
+  if (smem1 - qb > 220 * 1024)
     return fail(EFG_ERR_ARG, "search parameters need " + std::to_string(smem1) +
                                  " bytes of shared memory per query (pool/extend/degree too large)");
   EFG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(smem1, smem2)));
